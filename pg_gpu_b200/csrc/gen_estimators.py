@@ -645,9 +645,8 @@ def emit_geno(P):
     feats = geno_features_needed(P)
     calls, stats = plan(P, geno=True)
     L = [f"// genotype path, P = {P}: {len(stats)} statistics from {len(calls)} distinct raw calls",
-         "// (PREP false: the reciprocals are already set, e.g. by geno_prepare_from)",
-         "template <typename T, bool PREP = true>", f"LDK_DEV void geno_features_P{P}(GenoFeat<T>& x) {{",
-         "    if constexpr (PREP) geno_prepare(x);"]
+         "template <typename T>", f"LDK_DEV void geno_features_P{P}(GenoFeat<T>& x) {{",
+         "    geno_prepare(x);"]
     for n, e in geno_features():
         if n in feats:
             L.append(f"    x.{n} = {_cexpr(e)};")
@@ -750,246 +749,217 @@ def emit_hap(P):
 # fused-path forms (tensor-core parse)
 # ---------------------------------------------------------------------------
 #
-# Statistic-level expressions over per-population *scaled* features (numerator factors
-# times their reciprocal denominators), written as one accumulate per product term so
-# that every term is a single FMA into its sum.  Every raw call's numerator is an
-# integer polynomial of the counts, exact in FP64 below 2^53, so regrouping it changes
-# only the final roundings.  Two identities shorten the pi2 cases:
-#   L_k = c_{5-k} ns - sigma_k E  (sigma = +1, -1, -1, +1), hence
-#   F_k = L_k - c_{5-k} = c_{5-k} (ns - 1) - sigma_k E, and the pi2(i,j,i,j) correction
-#   sum_k (Q_k^i c_{5-k}^j - c_k^i L_k^j) = X (1 - ns_i - ns_j) - (E_i s_j + E_j s_i),
-#   X = sum_k c_{5-k}^i c_k^j, symmetric in (i, j): pi2_ijij(i, j) = pi2_ijij(j, i).
-# ``check()`` verifies both symbolically.
+# Spin moments.  Let sigma = 1 - 2a, a being the individual's frequency of allele 1 at the
+# left SNP (haplotypes: 0 or 1; genotypes: half the dosage, so sigma = 1 - g), tau the same
+# at the right SNP, both 0 where the call is missing.  The tensor-core kernel counts the
+# sums over a population's jointly called individuals
+#   n,  S = sum sigma,  T = sum tau,  R = sum sigma tau,
+#   (genotypes) SS = sum sigma^2, TT, SST = sum sigma^2 tau, STT, SSTT,
+# and every statistic is an unbiased mean over distinct individuals of products of sigma and
+# tau (a U-statistic), i.e. a polynomial of these integers over n(n-1)..., for both paths:
+#   E  = n R - S T            = sum over k != l of sigma_k (tau_k - tau_l)   (4 x / -D)
+#   W  = S T - R              = sum over k != l of sigma_k tau_l
+#   u  = S^2 - SS, v = T^2 - TT;   hA = n(n-1) - u, hB = n(n-1) - v   (heterozygosities)
+#   Q2 = R^2 - SSTT           = sum over k != m of sigma_k tau_k sigma_m tau_m
+#   Q3 = R W - S STT - T SST + 2 SSTT   = sum over distinct k, m, o of sigma_k tau_k sigma_m tau_o
+#   Q4 = u v - 4 Q3 - 2 Q2    = sum over distinct k, m, l, o of sigma_k sigma_m tau_l tau_o
+# (the pairs {k, m} and {l, o} of u v overlap in one index in four ways, in both in two).
+# A haplotype has sigma^2 = 1, so SS = TT = SSTT = n, SST = T, STT = S and Q3 = R W - u - v.
+# All numerators are integers, exact in FP64 below 2^53 (populations of up to ~8,000), so a
+# statistic that is exactly zero stays zero; each is scaled by the tabulated reciprocals and
+# added with one FMA.  The constant factors (powers of two) are applied once per staged sum
+# (SPIN weights), not per pair.  ``check()`` proves the forms equal to the raw calls.
+#
+# Expressions are C and Python syntax over the names below, suffixed with the population.
 
-# (name, expression): x = f[p] (HapFeat), g = this population's scaled features
-FUSED_SCALED = [
-    ("Er2", "x.E * x.r2"),
-    ("Er2h", "0.5 * g.Er2"),
-    ("Er3h", "x.E * (0.5 * x.r3)"),
-    ("aEr3h", "x.a * g.Er3h"),
-    ("bEr3h", "x.b * g.Er3h"),
-    ("ar1", "x.a * x.r1"),
-    ("br1", "x.b * x.r1"),
-    ("Sr2", "(x.s + x.a * x.b) * x.r2"),
-    ("r3h", "0.5 * x.r3"),
-    ("T1r3h", "x.T1 * g.r3h"),
-    ("T2r3h", "x.T2 * g.r3h"),
-    ("pAr1", "x.pA * x.r1"),
-    ("qAr1", "x.qA * x.r1"),
-    ("pBr1", "x.pB * x.r1"),
-    ("qBr1", "x.qB * x.r1"),
-    ("r2h", "0.5 * x.r2"),
-    ("fAr2h", "x.fA * g.r2h"),
-    ("fBr2", "x.fB * x.r2"),
-    ("r2q", "0.25 * x.r2"),
-    ("fAr2q", "x.fA * g.r2q"),
-    ("fBr2q", "x.fB * g.r2q"),
-    ("r2e", "0.125 * x.r2"),
-    ("m1", "x.ns - 1"),
-    ("F1h", "(x.c4 * g.m1 - x.E) * g.r2e"),
-    ("F2h", "(x.c3 * g.m1 + x.E) * g.r2e"),
-    ("F3h", "(x.c2 * g.m1 + x.E) * g.r2e"),
-    ("F4h", "(x.c1 * g.m1 - x.E) * g.r2e"),
-]
-
-# features of HapFeat the fused forms read directly
-FUSED_BASE = ["c1", "c2", "c3", "c4", "ns", "pA", "qA", "pB", "qB", "E", "a", "b", "s", "fA", "fB",
-              "T1", "T2", "DDs", "DZs", "PIs"]
+SPIN_INPUTS = ["n", "S", "T", "R", "r1", "r2", "r3", "r4"]
+SPIN_INPUTS_GENO = SPIN_INPUTS + ["SS", "TT", "SST", "STT", "SSTT"]
 
 
-def fused_plan(P):
-    """Per statistic, the list of (weight, case, args) with pi2_ijij merged over its
-    two argument orders."""
+def _spin_pop(p, geno):
+    """Definitions (name, expression) of population p's features."""
+    d = [
+        ("m", "n# - 1.0"), ("nu", "n# * m#"), ("nux", "nu# + nu#"), ("ST", "S# * T#"), ("E", "fma(n#, R#, -ST#)"),
+        ("W", "ST# - R#"), ("u", "fma(S#, S#, -SS#)" if geno else "fma(S#, S#, -n#)"),
+        ("v", "fma(T#, T#, -TT#)" if geno else "fma(T#, T#, -n#)"), ("hA", "nu# - u#"), ("hB", "nu# - v#"),
+        ("uv", "u# + v#"), ("n2", "n# - 2.0"), ("n3", "n# - 3.0"),
+        ("Q2", "fma(R#, R#, -SSTT#)" if geno else "fma(R#, R#, -n#)"),
+        ("Q3", "fma(-T#, SST#, fma(-S#, STT#, fma(R#, W#, SSTT# + SSTT#)))" if geno else "fma(R#, W#, -uv#)"),
+        ("Qx", "Q3# + Q3#"), ("Q4", "fma(-2.0, Qx# + Q2#, u# * v#)"),
+        ("DD", "fma(n3#, fma(n2#, Q2#, -Qx#), Q4#)"), ("DZ", "fma(n3#, Q3#, -Q4#)"),
+        ("PI", "fma(n2# * n3#, nu# - uv#, Q4#)"),
+        ("De", "E# * r2#"), ("Er", "E# * r3#"),
+        ("U", "fma(n#, fma(R#, S#, -SST#), -(u# * T#)) * r3#" if geno else "S# * Er#"),
+        ("V", "fma(n#, fma(R#, T#, -STT#), -(v# * S#)) * r3#" if geno else "T# * Er#"),
+        ("al", "S# * r1#"), ("be", "T# * r1#"), ("w", "W# * r2#"), ("hAr", "hA# * r2#"), ("hBr", "hB# * r2#"),
+        ("Sm", "m# * S#"), ("Tm", "m# * T#"),
+        # pi2 with one population three times: (X n_s - Y T_s [- Yb S_s]) r3 r1_s
+        ("P", "fma(R#, S#, -SST#)" if geno else "fma(R#, S#, -T#)"), ("Y", "fma(fma(-2.0, m#, hA#), T#, P# + P#)"),
+        ("X", "n2# * (hA# + hB#)" if geno else "n2# * hA#"),
+        ("Pb", "fma(R#, T#, -STT#)" if geno else "fma(R#, T#, -S#)"), ("Yb", "fma(fma(-2.0, m#, hB#), S#, Pb# + Pb#)"),
+        # variances behind r^2 (of population 0)
+        ("vx", "fma(n#, SS#, -(S# * S#))" if geno else "hA#"), ("vy", "fma(n#, TT#, -(T# * T#))" if geno else "hB#"),
+    ]
+    return [(n + str(p), e.replace("#", str(p))) for n, e in d]
+
+
+def _spin_pair(i, j):
+    """Definitions of the pair (i < j): symmetric products, suffix ij."""
+    d = [("rr", "r2I * r2J"), ("rho", "r1I * r1J"), ("nn", "nI * nJ"), ("HA", "fma(-SI, SJ, nn@)"),
+         ("HB", "fma(-TI, TJ, nn@)"), ("K", "fma(SI, TJ, SJ * TI)"), ("Kr", "K@ * rho@"),
+         ("La", "fma(SI, nJ, SJ * nI)"), ("Lb", "fma(TI, nJ, TJ * nI)")]
+    k = f"{i}{j}"
+    return [(n + k, e.replace("r1I", f"r1{i}").replace("r1J", f"r1{j}").replace("r2I", f"r2{i}")
+             .replace("r2J", f"r2{j}").replace("SI", f"S{i}").replace("SJ", f"S{j}").replace("TI", f"T{i}")
+             .replace("TJ", f"T{j}").replace("nI", f"n{i}").replace("nJ", f"n{j}").replace("@", k)) for n, e in d]
+
+
+def spin_defs(P, geno):
+    d = {}
+    for p in range(P):
+        d.update(_spin_pop(p, geno))
+    for i in range(P):
+        for j in range(i + 1, P):
+            d.update(_spin_pair(i, j))
+    return d
+
+
+def spin_stats(P, geno):
+    """[(name, weight, [(A, B), ...], rank)]: the statistic is weight * sum of A * B; rank
+    orders the emission (single populations, pairs, triples, quadruples)."""
+    c = 2.0 if geno else 1.0  # the genotype D is the composite one, twice as large
+    pr = lambda a, b: f"{min(a, b)}{max(a, b)}"  # noqa: E731
     out = []
-    for name, cl in stat_specs(P):
-        terms = {}
-        for w, kind, p in cl:
-            case, args = canonical(kind, p)
-            if case == "pi2_ijij":
-                args = tuple(sorted(args))
-            terms[(case, args)] = terms.get((case, args), 0.0) + w
-        out.append((name, [(w, c, a) for (c, a), w in terms.items()]))
+    for kind, q in ld_names(P):
+        pops = sorted(set(q))
+        rank = (len(pops), pops)
+        if kind == "dd":
+            i, j = q
+            t = (c * c / 16, [(f"DD{i}", f"r4{i}")] if i == j else [(f"De{i}", f"De{j}")])
+        elif kind == "dz":
+            i, j, k = q
+            if i == j == k:
+                t = (c / 4, [(f"DZ{i}", f"r4{i}")])
+            elif j == k:
+                t = (c / 4, [(f"De{i}", f"w{j}")])
+            elif i in (j, k):
+                o = k if i == j else j
+                t = (c / 8, [(f"U{i}", f"be{o}"), (f"V{i}", f"al{o}")])
+            else:
+                t = (c / 8, [(f"De{i}", f"Kr{pr(j, k)}")])
+        else:
+            i, j, k, l = q
+            case = _pi2_case(q)
+            if case == "same":
+                t = (1 / 16, [(f"PI{i}", f"r4{i}")])
+            elif case == "iikk":
+                t = (1 / 32, [(f"hAr{i}", f"hBr{k}"), (f"hBr{i}", f"hAr{k}")])
+            elif case == "triple":
+                cnt = _counts_of(q)
+                a = [x for x, m in cnt.items() if m == 3][0]
+                s = [x for x, m in cnt.items() if m == 1][0]
+                num = f"fma(-Y{a}, T{s}, X{a} * n{s})"
+                if geno:
+                    num = f"fma(-Yb{a}, S{s}, {num})"
+                t = (1 / 32 if geno else 1 / 16, [(num, f"(r3{a} * r1{s})")])
+            elif case in ("iikl", "ijkk"):
+                a, x, y = (i, k, l) if i == j else (k, i, j)
+                t = (1 / 32, [(f"fma(hAr{a}, HB{pr(x, y)}, hBr{a} * HA{pr(x, y)})", f"rho{pr(x, y)}")])
+            elif case == "ijij":
+                t = (1 / 16, [(f"fma(-Sm{i}, Sm{j}, fma(-Tm{i}, Tm{j}, fma(W{i}, W{j}, nu{i} * nu{j})))", f"rr{pr(i, j)}")])
+                # Sm = (n - 1) S on both sides would carry (n_i - 1)(n_j - 1): exactly the form's factor
+            elif case == "shared":
+                s = [x for x in (i, j) if x in (k, l)][0]
+                x, y = (j if i == s else i), (l if k == s else k)
+                g = pr(x, y)
+                t = (1 / 32, [(f"fma(W{s}, K{g}, fma(-Tm{s}, Lb{g}, fma(-Sm{s}, La{g}, nux{s} * nn{g})))",
+                               f"(r2{s} * rho{g})")])
+            else:
+                a, b = pr(i, j), pr(k, l)
+                t = (1 / 32, [(f"fma(HA{a}, HB{b}, HA{b} * HB{a})", f"(rho{a} * rho{b})")])
+        out.append((stat_name(kind, q), t[0], t[1], rank))
     return out
 
 
-def fused_terms(case, args, w):
-    """Product terms (A, B) whose sum is w * call(case, args); A and B use f[p].name for
-    HapFeat fields and g{p}_name for scaled features."""
-    g = lambda p, n: f"g{p}_{n}"  # noqa: E731
-    f = lambda p, n: f"f[{p}].{n}"  # noqa: E731
-    need = {"dd1": 1.0, "dd2": 1.0, "dz_iii": 1.0, "dz_iij": 0.5, "dz_iji": 0.5, "dz_ijj": 1.0,
-            "dz_ijk": 0.5, "pi2_same": 1.0, "pi2_triple": 1.0, "pi2_iikk": 0.5, "pi2_iikl": 0.5,
-            "pi2_ijkk": 0.5, "pi2_alldiff": 0.5, "pi2_ijij": 1.0, "pi2_shared": 0.5}[case]
-    if w != need:
-        raise ValueError(f"weight {w} of {case}{args}: fused form assumes {need}")
-    if case == "dd1":
-        (i,) = args
-        return [(f(i, "DDs"), f(i, "r4"))]
-    if case == "dd2":
-        i, j = args
-        return [(g(i, "Er2"), g(j, "Er2"))]
-    if case == "dz_iii":
-        (i,) = args
-        return [(f(i, "DZs"), f(i, "r4"))]
-    if case == "dz_iij":
-        i, j = args
-        return [(g(i, "aEr3h"), g(j, "br1"))]
-    if case == "dz_iji":
-        i, j = args
-        return [(g(i, "bEr3h"), g(j, "ar1"))]
-    if case == "dz_ijj":
-        i, j = args
-        return [(g(i, "Er2"), g(j, "Sr2"))]
-    if case == "dz_ijk":
-        i, j, k = args
-        return [(g(i, "Er2h"), f"({g(j, 'ar1')} * {g(k, 'br1')})")]
-    if case == "pi2_same":
-        (i,) = args
-        return [(f(i, "PIs"), f(i, "r4"))]
-    if case == "pi2_triple":
-        t, s_ = args
-        return [(g(t, "T1r3h"), g(s_, "pBr1")), (g(t, "T2r3h"), g(s_, "qBr1"))]
-    if case == "pi2_iikk":
-        i, k = args
-        return [(g(i, "fAr2h"), g(k, "fBr2"))]
-    if case == "pi2_iikl":
-        i, k, l = args
-        return [(g(i, "fAr2q"), f"({g(k, 'pBr1')} * {g(l, 'qBr1')} + {g(k, 'qBr1')} * {g(l, 'pBr1')})")]
-    if case == "pi2_ijkk":
-        i, j, k = args
-        return [(g(k, "fBr2q"), f"({g(i, 'pAr1')} * {g(j, 'qAr1')} + {g(i, 'qAr1')} * {g(j, 'pAr1')})")]
-    if case == "pi2_alldiff":
-        i, j, k, l = args
-        return [(f"(0.125 * ({g(i, 'pAr1')} * {g(j, 'qAr1')} + {g(i, 'qAr1')} * {g(j, 'pAr1')}))",
-                 f"({g(k, 'pBr1')} * {g(l, 'qBr1')} + {g(k, 'qBr1')} * {g(l, 'pBr1')})")]
-    if case == "pi2_shared":
-        s_, a, b = args
-        return [(g(a, "pAr1"), f"({g(b, 'pBr1')} * {g(s_, 'F1h')} + {g(b, 'qBr1')} * {g(s_, 'F2h')})"),
-                (g(a, "qAr1"), f"({g(b, 'pBr1')} * {g(s_, 'F3h')} + {g(b, 'qBr1')} * {g(s_, 'F4h')})")]
-    if case == "pi2_ijij":
-        i, j = args
-        HA = f"({f(i, 'pA')} * {f(j, 'qA')} + {f(i, 'qA')} * {f(j, 'pA')})"
-        HB = f"({f(i, 'pB')} * {f(j, 'qB')} + {f(i, 'qB')} * {f(j, 'pB')})"
-        X = (f"({f(i, 'c4')} * {f(j, 'c1')} + {f(i, 'c3')} * {f(j, 'c2')} + {f(i, 'c2')} * {f(j, 'c3')}"
-             f" + {f(i, 'c1')} * {f(j, 'c4')})")
-        body = (f"({HA} * {HB} + {X} * (1 - {f(i, 'ns')} - {f(j, 'ns')})"
-                f" - ({f(i, 'E')} * {f(j, 's')} + {f(j, 'E')} * {f(i, 's')}))")
-        return [(f"({g(i, 'r2h')} * {g(j, 'r2h')})", body)]
-    raise ValueError(case)
+# Split point of the statistics where two epilogue warps share them: Dz | pi2 (the two halves
+# need nearly disjoint features).
+def spin_split(P):
+    return sum(1 for k, _ in ld_names(P) if k != "pi2")
 
 
-def _term_cost(A, B):
-    return 1 + sum(t.count("*") + t.count(" + ") + t.count(" - ") for t in (A, B))
-
-
-# Four populations: the split the tensor-core kernel uses to divide the 105 statistics
-# between the two epilogue warps of a TMEM lane quarter, set by register pressure rather than
-# cost.  Measured (4 populations of 100-160 haplotypes, 16 bins): the cost-balanced point
-# (72) leaves one warp 72 accumulators and spills ~1.1 KB per thread, 4.1e9 pairs/s; 56
-# spills ~0.5 KB, 7.9e9 pairs/s; 60: 7.4e9.
-FUSED_SPLIT_AT = {4: 56}
-
-
-def fused_split(P):
-    """Split point K of the statistics into two contiguous halves: of about equal cost, or
-    FUSED_SPLIT_AT[P]."""
-    if P in FUSED_SPLIT_AT:
-        return FUSED_SPLIT_AT[P]
-    costs = [sum(_term_cost(A, B) for w, c, a in terms for A, B in fused_terms(c, a, w))
-             for _, terms in fused_plan(P)]
-    tot, run, best = sum(costs), 0, (None, 0)
-    for k in range(1, len(costs)):
-        run += costs[k - 1]
-        d = abs(2 * run - tot)
-        if best[0] is None or d < best[0]:
-            best = (d, k)
-    return best[1]
-
-
-def _scaled_closure(used):
-    """(p, name) scaled features needed by the used set, in definition order."""
-    defs = dict(FUSED_SCALED)
+def _names_in(e):
     import re
-    need = set(used)
-    changed = True
-    while changed:
-        changed = False
-        for p, n in list(need):
-            for dep in re.findall(r"g\.(\w+)", defs[n]):
-                if (p, dep) not in need:
-                    need.add((p, dep))
-                    changed = True
-    order = [n for n, _ in FUSED_SCALED]
-    return sorted(need, key=lambda t: (t[0], order.index(t[1])))
+    return re.findall(r"[A-Za-z]\w*", e)
 
 
-def emit_hap_fused(P):
-    """hap_fused_P{P}_{part}: part 0 = all statistics, 1 = [0, K), 2 = [K, NS)."""
-    import re
-    plan_ = fused_plan(P)
-    K = fused_split(P)
-    ranges = {0: (0, len(plan_)), 1: (0, K), 2: (K, len(plan_))}
-    L = [f"// P = {P}, fused path: statistics split at {K} of {len(plan_)}"]
-    for part, (lo, hi) in ranges.items():
-        lines, used = [], set()
-        for si in range(lo, hi):
-            name, terms = plan_[si]
-            for w, case, args in terms:
-                for A, B in fused_terms(case, args, w):
-                    for m in re.finditer(r"g(\d)_(\w+)", A + " " + B):
-                        used.add((int(m.group(1)), m.group(2)))
-                    lines.append(f"    acc[{si - lo}] += {_cexpr(A)} * {_cexpr(B)};  // {name}: {case}{args}")
-        defs = dict(FUSED_SCALED)
-        L.append("template <typename T>")
-        L.append(f"LDK_DEV void hap_fused_P{P}_{part}(const HapFeat<T>* f, T* acc) {{")
-        for p, n in _scaled_closure(used):
-            e = defs[n].replace("x.", f"f[{p}].")
-            e = re.sub(r"g\.(\w+)", lambda m: f"g{p}_{m.group(1)}", e)
-            L.append(f"    const T g{p}_{n} = {_cexpr(e)};")
-        L.extend(lines)
+def emit_spin(P, geno):
+    """spin_{hap,geno}_P{P}_{part}: part 0 = all statistics and r^2, 1 = [0, K), 2 = [K, NS)
+    and r^2 (the last accumulator)."""
+    path = "geno" if geno else "hap"
+    defs, stats, K = spin_defs(P, geno), spin_stats(P, geno), spin_split(P)
+    inputs = SPIN_INPUTS_GENO if geno else SPIN_INPUTS
+    L = [f"// {path}, P = {P}: {len(stats)} statistics, split at {K}"]
+    parts = {0: (0, len(stats)), 1: (0, K), 2: (K, len(stats))}
+    if geno or P < 4:
+        parts = {0: parts[0]}
+    else:
+        parts.pop(0)
+    for part, (lo, hi) in parts.items():
+        lines, done = [], set()
+
+        def use(expr):
+            for nm in _names_in(expr):
+                if nm in done or nm == "fma":
+                    continue
+                done.add(nm)
+                if nm in defs:
+                    use(defs[nm])
+                    lines.append(f"    const double {nm} = {defs[nm]};")
+                else:
+                    base = nm.rstrip("0123456789") if not nm.startswith("r") else nm[:2]
+                    assert base in inputs, nm
+                    lines.append(f"    const double {nm} = f[{nm[-1]}].{base};")
+
+        for si in sorted(range(lo, hi), key=lambda k: stats[k][3]):
+            name, _, terms, _ = stats[si]
+            for A, B in terms:
+                use(A)
+                use(B)
+                lines.append(f"    acc[{si - lo}] = fma({A}, {B}, acc[{si - lo}]);  // {name}")
+        if part != 1:
+            use("E0 vx0 vy0")
+            lines += ["    const double den = vx0 * vy0;", "    if (den > 0.0) {",
+                      f"        acc[{hi - lo}] = fma(E0 * E0, recip_cubic(den), acc[{hi - lo}]);", "        ++nr2;", "    }"]
+        L.append(f"LDK_DEV void spin_{path}_P{P}_{part}(const SpinPop* f, double* acc, unsigned& nr2) {{")
+        L += lines
         L.append("}")
+    w = [x[1] for x in stats]
+    L.append(f"static __constant__ double spin_weight_{path}_P{P}[{len(w) + 1}] = {{{', '.join(repr(x) for x in w)}, 1.0}};")
     return "\n".join(L)
 
 
-def fused_features_ok():
-    """Every HapFeat field the fused forms read is computed by hap_features_P*."""
-    import re
-    for P in (1, 2, 3, 4):
-        have = set(hap_features_needed(P)[0]) | {"c1", "c2", "c3", "c4", "ns", "n", "r1", "r2", "r3", "r4"}
-        text = " ".join(A + " " + B for _, terms in fused_plan(P) for w, c, a in terms for A, B in fused_terms(c, a, w))
-        text += " " + " ".join(e for _, e in FUSED_SCALED)
-        used = set(re.findall(r"f\[\d\]\.(\w+)", text))
-        scaled_used = {n for p_, n in _scaled_closure(
-            {(int(m.group(1)), m.group(2)) for m in re.finditer(r"g(\d)_(\w+)", text)})}
-        used |= {d for n, e in FUSED_SCALED if n in scaled_used for d in re.findall(r"x\.(\w+)", e)}
-        if not used <= have:
-            raise AssertionError(f"P={P}: fused forms read {sorted(used - have)} not computed")
-    return True
+def emit_spin_numerators(geno):
+    """The DD and pi2 numerators of one population (16 times each, over n(n-1)(n-2)(n-3))."""
+    defs, lines, done = spin_defs(1, geno), [], set()
 
+    def use(expr):
+        for nm in _names_in(expr):
+            if nm in done or nm == "fma":
+                continue
+            done.add(nm)
+            if nm in defs:
+                use(defs[nm])
+                lines.append(f"    const double {nm} = {defs[nm]};")
 
-def numpy_hap_fused(counts_list, n_list=None, part=0):
-    """Evaluate the fused forms with NumPy float64 (test helper); columns of the part."""
-    import re
-    import numpy as np
-    P = len(counts_list)
-    xs = _numpy_hap_feats(counts_list, n_list, all_features=True)
-    env = {}
-    for p, x in enumerate(xs):
-        for n, e in FUSED_SCALED:
-            g = _NS()
-            for k, v in env.items():
-                if k.startswith(f"g{p}_"):
-                    setattr(g, k[len(f"g{p}_"):], v)
-            env[f"g{p}_{n}"] = eval(e, {}, {"x": x, "g": g})
-    plan_ = fused_plan(P)
-    K = fused_split(P)
-    lo, hi = {0: (0, len(plan_)), 1: (0, K), 2: (K, len(plan_))}[part]
-    out = np.zeros((len(xs[0].c1), hi - lo))
-    for si in range(lo, hi):
-        for w, case, args in plan_[si][1]:
-            for A, B in fused_terms(case, args, w):
-                out[:, si - lo] += eval(A, {}, {"f": xs, **env}) * eval(B, {}, {"f": xs, **env})
-    return out
+    use("DD0 PI0")
+    if geno:
+        head = ["LDK_DEV void spin_geno_numerators(const uint32_t (&G)[3][4], double& dd, double& pi2) {"]
+        cells = {"R": (0, 0), "STT": (0, 1), "S": (0, 2), "SST": (1, 0), "SSTT": (1, 1), "SS": (1, 2), "T": (2, 0),
+                 "TT": (2, 1), "n": (2, 2)}
+        head += [f"    const double {k}0 = i2d_exact((int)G[{x}][{y}]);" for k, (x, y) in cells.items() if f"{k}0" in done]
+    else:
+        head = ["LDK_DEV void spin_hap_numerators(double n0, double S0, double T0, double R0, double& dd, double& pi2) {"]
+    return "\n".join(head + lines + ["    dd = DD0;", "    pi2 = PI0;", "}"])
 
 
 def _cexpr(e):
@@ -1004,7 +974,7 @@ HEADER = """// GENERATED by gen_estimators.py -- do not edit by hand.
 // Statistic order and averaging weights follow moments.LD (pg_gpu ld_pipeline.py:357-457);
 // raw-call algebra restates pg_gpu haplotype_kernels.py:69-304 in factored form.
 // hap_stats_P* evaluate every distinct raw call (plain kernel, raw-call entry points);
-// hap_fused_P* are the statistic-level forms of the tensor-core parse.
+// spin_hap_P* / spin_geno_P* are the statistic-level forms of the tensor-core parse.
 #pragma once
 """
 
@@ -1015,22 +985,26 @@ def generate(path=None):
     for P in (1, 2, 3, 4):
         parts.append(emit_hap(P))
         parts.append("")
-    for P in (1, 2, 3, 4):
-        parts.append(emit_hap_fused(P))
-        parts.append("")
-    parts.append('#include "ldk_geno_feat.cuh"')
+    parts.append('#include "ldk_geno_feat.cuh"\n#include "ldk_spin.cuh"')
     for P in (1, 2, 3, 4):
         parts.append(emit_geno(P))
+        parts.append("")
+    for geno in (False, True):
+        for P in (1, 2, 3, 4):
+            parts.append(emit_spin(P, geno))
+            parts.append("")
+    for geno in (False, True):
+        parts.append(emit_spin_numerators(geno))
         parts.append("")
     parts.append(emit_raw_dispatch())
     parts.append("")
     parts.append("template <int P> struct HapNStats;")
     for P in (1, 2, 3, 4):
         parts.append(f"template <> struct HapNStats<{P}> {{ static constexpr int value = {len(stat_specs(P))}; }};")
-    parts.append("// first statistic of the second half of the fused path's two-way split")
-    parts.append("template <int P> struct HapFusedSplit;")
+    parts.append("// first statistic of the second half of the two-way split")
+    parts.append("template <int P> struct SpinSplit;")
     for P in (1, 2, 3, 4):
-        parts.append(f"template <> struct HapFusedSplit<{P}> {{ static constexpr int value = {fused_split(P)}; }};")
+        parts.append(f"template <> struct SpinSplit<{P}> {{ static constexpr int value = {spin_split(P)}; }};")
     parts.append("""
 template <typename T, int P>
 LDK_DEV void hap_features(HapFeat<T>& x) {
@@ -1039,12 +1013,12 @@ LDK_DEV void hap_features(HapFeat<T>& x) {
     else if constexpr (P == 3) hap_features_P3<T>(x);
     else hap_features_P4<T>(x);
 }
-template <typename T, int P, bool PREP = true>
+template <typename T, int P>
 LDK_DEV void geno_features(GenoFeat<T>& x) {
-    if constexpr (P == 1) geno_features_P1<T, PREP>(x);
-    else if constexpr (P == 2) geno_features_P2<T, PREP>(x);
-    else if constexpr (P == 3) geno_features_P3<T, PREP>(x);
-    else geno_features_P4<T, PREP>(x);
+    if constexpr (P == 1) geno_features_P1<T>(x);
+    else if constexpr (P == 2) geno_features_P2<T>(x);
+    else if constexpr (P == 3) geno_features_P3<T>(x);
+    else geno_features_P4<T>(x);
 }
 template <typename T, int P, int S = 1>
 LDK_DEV void geno_stats(const GenoFeat<T>* f, T* acc) {
@@ -1053,21 +1027,30 @@ LDK_DEV void geno_stats(const GenoFeat<T>* f, T* acc) {
     else if constexpr (P == 3) geno_stats_P3<T, S>(f, acc);
     else geno_stats_P4<T, S>(f, acc);
 }
-// Fused-path statistics of part PART (0: all, 1: [0, split), 2: [split, NS)) added into
-// acc[0 ..) of that part.
-template <typename T, int P, int PART>
-LDK_DEV void hap_fused(const HapFeat<T>* f, T* acc) {
-#define LDK_FUSED_CASE(PP) \\
-    if constexpr (P == PP) { \\
-        if constexpr (PART == 0) hap_fused_P##PP##_0<T>(f, acc); \\
-        else if constexpr (PART == 1) hap_fused_P##PP##_1<T>(f, acc); \\
-        else hap_fused_P##PP##_2<T>(f, acc); \\
+// Spin-form statistics of part PART (0: all and r^2, 1: [0, split), 2: [split, NS) and r^2)
+// added into acc[0 ..) of that part, before their weights (spin_weight).
+template <int P, bool GENO, int PART>
+LDK_DEV void spin_stats(const SpinPop* f, double* acc, unsigned& nr2) {
+    if constexpr (GENO) {
+        if constexpr (P == 1) spin_geno_P1_0(f, acc, nr2);
+        else if constexpr (P == 2) spin_geno_P2_0(f, acc, nr2);
+        else if constexpr (P == 3) spin_geno_P3_0(f, acc, nr2);
+        else spin_geno_P4_0(f, acc, nr2);
+    } else {
+        if constexpr (P == 1) spin_hap_P1_0(f, acc, nr2);
+        else if constexpr (P == 2) spin_hap_P2_0(f, acc, nr2);
+        else if constexpr (P == 3) spin_hap_P3_0(f, acc, nr2);
+        else if constexpr (PART == 1) spin_hap_P4_1(f, acc, nr2);
+        else spin_hap_P4_2(f, acc, nr2);
     }
-    LDK_FUSED_CASE(1)
-    LDK_FUSED_CASE(2)
-    LDK_FUSED_CASE(3)
-    LDK_FUSED_CASE(4)
-#undef LDK_FUSED_CASE
+}
+// Weight of statistic s of P populations (s = number of statistics: r^2, weight 1).
+template <int P, bool GENO>
+LDK_DEV double spin_weight(int s) {
+    if constexpr (GENO)
+        return P == 1 ? spin_weight_geno_P1[s] : P == 2 ? spin_weight_geno_P2[s] : P == 3 ? spin_weight_geno_P3[s] : spin_weight_geno_P4[s];
+    else
+        return P == 1 ? spin_weight_hap_P1[s] : P == 2 ? spin_weight_hap_P2[s] : P == 3 ? spin_weight_hap_P3[s] : spin_weight_hap_P4[s];
 }
 template <typename T, int P, int S = 1>
 LDK_DEV void hap_stats(const HapFeat<T>* f, T* acc) {
@@ -1131,8 +1114,67 @@ def numpy_hap_stats(counts_list, n_list=None):
     return out
 
 
+def check_spin(seed=0, trials=12, small_haplotypes=False):
+    """Exact check (rational arithmetic, random integer counts: a polynomial identity test) of
+    every spin form against the weighted raw calls it stands for, both paths, P = 1..4.
+    ``small_haplotypes``: haplotype samples of 0 to 5 instead (reciprocals of zero products
+    are 0); the genotype path divides by n(n-1)(n-2) and has no value there."""
+    import random
+    import re
+    from fractions import Fraction as Fr
+    rng = random.Random(seed)
+    lit = lambda e: re.sub(r"(?<![\w.])(\d+\.\d+|\d+)(?![\w.\]])", r"Fr('\1')", e)  # noqa: E731
+    inv = lambda d: Fr(1) / d if d > 0 else Fr(0)  # noqa: E731
+    code = lambda e: compile(lit(e), "<form>", "eval")  # noqa: E731
+    feats = {False: [(n, code(e)) for n, e in HAP_FEATURES], True: [(n, code(e)) for n, e in GENO_FEATURES]}
+    for geno in ((False,) if small_haplotypes else (False, True)):
+        for P in (1, 2, 3, 4):
+            calls, raw = plan(P, geno)
+            expr = [code((geno_call_expr if geno else hap_call_expr)(c, a)) for c, a in calls]
+            defs = {k: code(e) for k, e in spin_defs(P, geno).items()}
+            stats = [(w, [(code(A), code(B)) for A, B in t]) for _, w, t, _ in spin_stats(P, geno)]
+            for _ in range(trials):
+                f, env = [], {"Fr": Fr, "fma": lambda a, b, c: a * b + c}
+                for p in range(P):
+                    x = _NS()
+                    if small_haplotypes:
+                        c = [0, 0, 0, 0]
+                        for _ in range(rng.randint(0, 5)):
+                            c[rng.randrange(4)] += 1
+                    else:
+                        c = [rng.randint(0, 9) for _ in range(9 if geno else 4)]
+                        c[-1] += 4  # at least four individuals: every denominator positive
+                    n = Fr(sum(c))
+                    x.n = x.ns = n
+                    d = [n, n * (n - 1), n * (n - 1) * (n - 2), n * (n - 1) * (n - 2) * (n - 3)]
+                    x.r1, x.r2, x.r3, x.r4 = x.u1, x.u2, x.u3, x.w4 = [inv(q) for q in d]
+                    x.invn, x.inn1 = x.r1, inv(4 * n * (n - 1))
+                    # (sigma, tau) of every cell: genotype cells g1..g9 = n22 .. n00
+                    st = [(1 - a, 1 - b) for a in (2, 1, 0) for b in (2, 1, 0)] if geno else [(-1, -1), (-1, 1), (1, -1), (1, 1)]
+                    for m, k in enumerate(c):
+                        setattr(x, f"g{m + 1}" if geno else f"c{m + 1}", Fr(k))
+                    for name, e in feats[geno]:
+                        setattr(x, name, eval(e, {"x": x, "Fr": Fr}))
+                    f.append(x)
+                    for name, (a, b) in {"S": (1, 0), "T": (0, 1), "R": (1, 1), "SS": (2, 0), "TT": (0, 2), "SST": (2, 1),
+                                         "STT": (1, 2), "SSTT": (2, 2)}.items():
+                        env[f"{name}{p}"] = Fr(sum(k * s ** a * t ** b for k, (s, t) in zip(c, st)))
+                    env[f"n{p}"] = n
+                    for k in range(4):
+                        env[f"r{k + 1}{p}"] = inv(d[k])
+                for k, e in defs.items():
+                    env[k] = eval(e, env)
+                vals = [eval(e, {"f": f, "Fr": Fr}) for e in expr]
+                for (w, terms), (name, rt) in zip(stats, raw):
+                    want = sum(Fr(q) * vals[idx] for idx, q in rt)
+                    got = Fr(w) * sum(eval(A, env) * eval(B, env) for A, B in terms)
+                    assert got == want, (geno, P, name)
+    return True
+
+
 def check():
     """Symbolic check of the factored forms against the reference formulas (sympy)."""
+    check_spin()
     import sympy as sp
     for poly in _HORNER_POLYS.values():
         e, _, g = _horner_sympy(poly)
@@ -1170,13 +1212,6 @@ def check():
     corr = (X.Q1 * b4 + X.Q2 * b3 + X.Q3 * b2 + X.Q4 * b1
             - (a1 * Y.L1 + a2 * Y.L2 + a3 * Y.L3 + a4 * Y.L4))
     assert sp.expand(ref_ijij - (HA * HB + corr) / 4) == 0
-    # fused path: the symmetric pi2(i,j,i,j) correction and F_k = L_k - c_{5-k}
-    Xs = a4 * b1 + a3 * b2 + a2 * b3 + a1 * b4
-    corr2 = Xs * (1 - X.ns - Y.ns) - (X.E * Y.s + Y.E * X.s)
-    assert sp.expand(corr - corr2) == 0
-    m1 = X.ns - 1
-    for Lk, ck, sig in ((X.L1, a4, 1), (X.L2, a3, -1), (X.L3, a2, -1), (X.L4, a1, 1)):
-        assert sp.expand((Lk - ck) - (ck * m1 - sig * X.E)) == 0
     # single-population numerators, haplotype_kernels.py:76, 102-104, 298-301
     c1, c2, c3, c4 = a
     assert sp.expand(X.DDs - (c1 * (c1 - 1) * c4 * (c4 - 1) + c2 * (c2 - 1) * c3 * (c3 - 1)
@@ -1214,5 +1249,4 @@ def check():
 
 if __name__ == "__main__":
     check()
-    fused_features_ok()
     print(generate())

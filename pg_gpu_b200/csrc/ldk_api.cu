@@ -129,9 +129,9 @@ Layout layout_of(const ldk_parse_t* d, const ParseShape& sh) {
             L.rtab_off = off;
             off = align_up(off + (size_t)(sh.max_n + 1) * 4 * sizeof(double), 256);
         }
-        if (sh.genotypes && sh.P <= 3) {  // GenoRecip per valid count
+        if (sh.genotypes) {
             L.gtab_off = off;
-            off = align_up(off + (size_t)(sh.max_n + 1) * 9 * sizeof(double), 256);
+            off = align_up(off + (size_t)(sh.max_n + 1) * 4 * sizeof(double), 256);
         }
     }
     L.total = off;
@@ -242,7 +242,7 @@ int prepare(const ldk_parse_t* d, void* workspace, size_t workspace_bytes, Prepa
     P.w.items = reinterpret_cast<int32_t*>(ws + P.L.items_off);
     P.w.hv = ws + P.L.hv_off;
     P.w.rtab = P.sh.rtab_global ? static_cast<void*>(ws + P.L.rtab_off) : nullptr;
-    P.w.gtab = (d->method != LDK_METHOD_PLAIN_FP64 && P.sh.genotypes && P.sh.P <= 3)
+    P.w.gtab = (d->method != LDK_METHOD_PLAIN_FP64 && P.sh.genotypes)
                    ? static_cast<void*>(ws + P.L.gtab_off)
                    : nullptr;
     return LDK_OK;
@@ -318,7 +318,7 @@ int clear(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepared& P, c
     return LDK_OK;
 }
 
-// Device work of one parse (after the plan is in the workspace): pair ranges, indicator
+// Device work of one parse (after the plan is in the workspace): pair ranges, spin
 // planes and the parse kernel.  Host work: tensor-map encoding and launch configuration.
 // ---- autotuning: the fastest (tile variant, row-block order) per shape class (ldk_tune.cu)
 std::atomic<int> g_autotune{-1};  // -1: LDK_AUTOTUNE not read yet
@@ -381,7 +381,7 @@ int enqueue_device(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepa
         if (prof) cudaEventRecord(g_ev[1], s);
         if ((rc = check_cuda(launch_fx_finish(&dd, out, P.w, P.sh.n_stats, s), "bin sums"))) return rc;
     } else {
-        if ((rc = check_cuda(launch_prep_planes(&dd, P.w, P.sh, s), "indicator planes"))) return rc;
+        if ((rc = check_cuda(launch_prep_planes(&dd, P.w, P.sh, s), "spin planes"))) return rc;
         if (P.w.rtab && (rc = check_cuda(launch_fill_rtab(P.w.rtab, P.sh.max_n, s), "reciprocal table"))) return rc;
         if (P.w.gtab && (rc = check_cuda(launch_fill_gtab(P.w.gtab, P.sh.max_n, s), "reciprocal table"))) return rc;
         if (tune && n_variants(d, P.sh) * n_orders(d) > 1 && tuned_variant(d, P.sh) < 0) {

@@ -51,12 +51,6 @@ LDK_DEV int bin_advance(const double* __restrict__ e, int n_bins, int b, double 
 LDK_DEV double i2d_exact(int x) {
     return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0;
 }
-template <typename T>
-LDK_DEV T count_to(int x) {
-    if constexpr (sizeof(T) == sizeof(double)) return i2d_exact(x);
-    else return T(x);
-}
-
 LDK_DEV uint64_t global_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));

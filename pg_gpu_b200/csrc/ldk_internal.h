@@ -16,14 +16,14 @@ struct Scratch {
     int32_t* jmax;         // (n_var) exclusive end of each SNP's partner range
     int64_t* win_off;      // (n_windows + 1) window SNP offsets
     int64_t* anc_end;      // (n_windows) end of each window's anchor SNPs
-    uint8_t* hv;           // TC path: (n_var, planes, Ktot) indicator planes
+    uint8_t* hv;           // TC path: (n_var, planes, Ktot) spin planes
     int32_t* row_blocks;   // TC path: (n_row_blocks, 2) row blocks [row0, row1) in claim order
     int32_t* items;        // TC path: work items (row0, row1, t0, t1): rows [row0, row1),
                            // partner tiles [t0, t1) of that row block
     int* n_items;          // TC path: items in use
     void* rtab;            // TC haplotype path: (max_n + 1) double4 reciprocal table in the
                            // workspace, or null when it lives in shared memory
-    void* gtab;            // TC genotype path: (max_n + 1) GenoRecip reciprocal table
+    void* gtab;            // TC genotype path: (max_n + 1) double4 reciprocal table
     unsigned long long* fx;  // (n_blocks, n_bins, n_stats + 1, kFxLimbs) fixed-point bin sums
 };
 
@@ -34,7 +34,7 @@ struct ParseShape {
     int n_bins;
     int kofs[LDK_MAX_POPS + 1];  // TC path: K offset (bytes) of each population segment
     int ktot;                    // TC path: total K bytes (multiple of 128)
-    int planes;                  // TC path: indicator planes per SNP (2 haplotype, 4 genotype)
+    int planes;                  // TC path: spin planes per SNP (2 haplotype, 4 genotype)
     int max_n;                   // largest population size
     int rtab_global;             // TC haplotype path: the reciprocal table (32 B per n_valid)
                                  // does not fit beside the pipeline in shared memory

@@ -13,7 +13,7 @@
 #include <vector>
 
 #include "ldk_tc_kernel.cuh"
-#include "ldk_geno_feat.cuh"
+#include "ldk_spin.cuh"
 
 namespace ldk {
 
@@ -159,48 +159,49 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&tempty[buf]);
                     }
-                    // lane 2r: (hh, hv) of partners 2q, 2q+1; lane 2r+1: (vh, vv)
+                    // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
                     const uint32_t sx = role ? v[0][0] : v[0][2];
                     const uint32_t sy = role ? v[0][1] : v[0][3];
                     const uint32_t rx = __shfl_xor_sync(0xffffffffu, sx, 1);
                     const uint32_t ry = __shfl_xor_sync(0xffffffffu, sy, 1);
-                    int hh, hv, vh, vv;
-                    if (role == 0) { hh = (int)v[0][0]; hv = (int)v[0][1]; vh = (int)rx; vv = (int)ry; }
-                    else { vh = (int)v[0][2]; vv = (int)v[0][3]; hh = (int)rx; hv = (int)ry; }
+                    const int iR = (int)(role ? rx : v[0][0]), iS = (int)(role ? ry : v[0][1]);
+                    const int iT = (int)(role ? v[0][2] : rx), in = (int)(role ? v[0][3] : ry);
                     const int j = j0 + jj;
                     const bool valid = row_ok && j > i && j < jend;
                     double val = 0.0;
                     if (valid) {
-                        const double c1 = hh, c2 = hv - hh, c3 = vh - hh, c4 = vv - hv - vh + hh, n = vv;
+                        const double n = i2d_exact(in);
                         if constexpr (EST == 0) {
-                            // haplotype_matrix.py:1122-1128, 1171-1175
-                            const double pab = n > 0.0 ? c1 * recip_newton(n) : 0.0;
+                            // haplotype_matrix.py:1122-1128, 1171-1175; n11 = (n - S - T + R) / 4
+                            const double c1 = i2d_exact((in - iS - iT + iR) >> 2);
+                            const double pab = n > 0.0 ? c1 * recip_cubic(n) : 0.0;
                             const double D = pab - pi * pj;
                             const double den = (pi * (1.0 - pi)) * (pj * (1.0 - pj));
-                            val = den > 0.0 ? (D * D) * recip_newton(den) : 0.0;
+                            val = den > 0.0 ? (D * D) * recip_cubic(den) : 0.0;
                             zsum += val;
                             zcnt += 1.0;
-                        } else if constexpr (EST == 1) {
-                            // ld_statistics.py:326-343 (exact integers in FP64)
-                            const double dd = c1 * (c1 - 1) * c4 * (c4 - 1) + c2 * (c2 - 1) * c3 * (c3 - 1) -
-                                              2.0 * c1 * c2 * c3 * c4;
-                            const double s12 = c1 + c2, s13 = c1 + c3, s24 = c2 + c4, s34 = c3 + c4;
-                            const double pi2 = s12 * s13 * s24 * s34 - c1 * c4 * (-1.0 + c1 + 3.0 * c2 + 3.0 * c3 + c4) -
-                                               c2 * c3 * (-1.0 + 3.0 * c1 + c2 + c3 + 3.0 * c4);
-                            const bool nok = n >= 4.0;
-                            val = (nok && pi2 != 0.0) ? dd * recip_newton(pi2) : 0.0;
-                            zsum += val;
-                            zcnt += nok ? 1.0 : 0.0;
                         } else {
-                            // haplotype_kernels.py:32-42: NaN where pA qA pB qB = 0
-                            const double D = c1 * c4 - c2 * c3;
-                            const double den = (c1 + c2) * (c3 + c4) * ((c1 + c3) * (c2 + c4));
-                            if (den > 0.0) {
-                                val = (D * D) * recip_newton(den);
+                            const double S = i2d_exact(iS), T = i2d_exact(iT), R = i2d_exact(iR);
+                            if constexpr (EST == 1) {
+                                // ld_statistics.py:326-343: the DD and pi2 numerators (exact
+                                // integers in FP64), 16 times each
+                                double dd, pi2;
+                                spin_hap_numerators(n, S, T, R, dd, pi2);
+                                const bool nok = n >= 4.0;
+                                val = (nok && pi2 != 0.0) ? dd * recip_cubic(pi2) : 0.0;
                                 zsum += val;
-                                zcnt += 1.0;
+                                zcnt += nok ? 1.0 : 0.0;
                             } else {
-                                val = CUDART_NAN;
+                                // haplotype_kernels.py:32-42: NaN where pA qA pB qB = 0
+                                const double E = fma(n, R, -(S * T));
+                                const double den = fma(n, n, -(S * S)) * fma(n, n, -(T * T));
+                                if (den > 0.0) {
+                                    val = (E * E) * recip_cubic(den);
+                                    zsum += val;
+                                    zcnt += 1.0;
+                                } else {
+                                    val = CUDART_NAN;
+                                }
                             }
                         }
                     }
@@ -376,17 +377,14 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
                     const bool valid = row_ok && j > i && j < jend;
                     double val = 0.0;
                     if (valid) {
-                        // G[x][y]: plane x of SNP i . plane y of SNP j (0: g == 1, 1: g == 2, 2: valid)
-                        const int n11 = (int)G[0][0], n12 = (int)G[0][1], n21 = (int)G[1][0], n22 = (int)G[1][1];
-                        const int n10 = (int)G[0][2] - n11 - n12, n20 = (int)G[1][2] - n21 - n22;
-                        const int n01 = (int)G[2][0] - n11 - n21, n02 = (int)G[2][1] - n12 - n22;
-                        const int nv = (int)G[2][2];
+                        // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma = 1 - g,
+                        // 1: sigma^2, 2: valid)
+                        const int nv = (int)G[2][2], iS = (int)G[0][2], iT = (int)G[2][0], iR = (int)G[0][0];
                         if constexpr (EST == 3 || EST == 4) {
-                            const double sxy = (double)(n11 + 2 * (n12 + n21) + 4 * n22);
+                            const double sxy = (double)(nv - iS - iT + iR);  // sum of dosage products
                             if constexpr (EST == 3) {
                                 // centred dosages zeroed where missing (ld_statistics.py:1000-1018)
-                                const double sx = (double)((n10 + n11 + n12) + 2 * (n20 + n21 + n22));
-                                const double sy = (double)((n01 + n11 + n21) + 2 * (n02 + n12 + n22));
+                                const double sx = (double)(nv - iS), sy = (double)(nv - iT);
                                 const double cov = sxy - muj * sx - mui * sy + mui * muj * (double)nv;
                                 const double vv = vari * varj;
                                 val = vv > 0.0 ? (cov * cov) / vv : 0.0;
@@ -405,16 +403,11 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
                                 }
                             }
                         } else {
-                            // DD over pi2 numerators of one population (genotype_kernels.py:91-170)
-                            const int n00 = nv - n01 - n02 - n10 - n11 - n12 - n20 - n21 - n22;
-                            const double cd[9] = {(double)n00, (double)n01, (double)n02, (double)n10, (double)n11,
-                                                  (double)n12, (double)n20, (double)n21, (double)n22};
-                            GenoFeat<double> f;
-                            geno_set_counts(f, cd);
-                            f.n = (double)nv;
-                            geno_features<double, 1>(f);
-                            if (nv >= 4 && f.PI1 > 0.0) {
-                                val = f.DD1 / f.PI1;
+                            // DD over pi2 of one population (genotype_kernels.py:91-170)
+                            double dd, pi2;
+                            spin_geno_numerators(G, dd, pi2);
+                            if (nv >= 4 && pi2 > 0.0) {
+                                val = 4.0 * dd / pi2;
                                 zsum += val;
                                 zcnt += 1.0;
                             } else {
@@ -568,7 +561,7 @@ cudaError_t launch_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const
             X, ld_x, n_var, rows, n_sel, estimator != LDK_LDM_DIPLOID_R2, psite, svar, status);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    // the indicator planes of the selected rows, as for a one-population parse
+    // the spin planes of the selected rows, as for a one-population parse
     ldk_parse_t d{};
     d.genotypes = geno ? 1 : 0;
     d.X = X;

@@ -1,4 +1,4 @@
-// Tensor-core path of the binned parse: indicator-plane preparation, tile-variant
+// Tensor-core path of the binned parse: spin-plane preparation, tile-variant
 // dispatch and the peak probes (the kernel itself is in ldk_tc_kernel.cuh).
 #include "ldk_tc_kernel.cuh"
 
@@ -6,8 +6,8 @@ namespace ldk {
 
 namespace {
 // ---------------------------------------------------------------------------
-// indicator planes.  Haplotypes: planes[v][0][k] = [x == 1], planes[v][1][k] = [x in {0, 1}].
-// Genotypes: planes[v][0..3][k] = [x == 1], [x == 2], [x in {0, 1, 2}], 0.
+// spin planes (s8).  Haplotypes: planes[v][0][k] = sigma = 1 - 2x, planes[v][1][k] = [x in {0, 1}].
+// Genotypes: planes[v][0..3][k] = sigma = 1 - x, sigma^2, [x in {0, 1, 2}], 0.  Missing: 0.
 // ---------------------------------------------------------------------------
 
 struct PrepArgs {
@@ -32,8 +32,8 @@ constexpr int kPrepV = 128, kPrepK = 128;
 // threads, consecutive SNPs) into a SNP-major shared tile, the scatter turns each 4-byte K
 // quad of a SNP into its plane bytes with byte-wise compares and writes every plane as
 // 128-byte runs along K.  Plane bytes (GENO: 4 planes, haplotypes: 2):
-//   haplotypes  h = [x == 1], v = [x in {0, 1}]
-//   genotypes   [x == 1], [x == 2], [x in {0, 1, 2}], 0
+//   haplotypes  sigma = 1 - 2x, v = [x in {0, 1}]
+//   genotypes   sigma = 1 - x, sigma^2, v = [x in {0, 1, 2}], 0
 // Padding (127) and invalid codes give 0 in every plane; invalid codes also raise
 // LDK_DEVERR_BAD_INPUT.
 //
@@ -139,12 +139,12 @@ __global__ void __launch_bounds__(256) k_prep_planes(PrepArgs a) {
         uint8_t* dst = a.planes_out + v * PL * (int64_t)a.ktot + k0 + 4 * kq;
         if constexpr (GENO) {
             const uint32_t eq2 = __vcmpeq4(w, 2u * kOne);
-            *reinterpret_cast<uint32_t*>(dst) = eq1 & kOne;
-            *reinterpret_cast<uint32_t*>(dst + a.ktot) = eq2 & kOne;
+            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq2;  // 0xFF = -1
+            *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq2) & kOne;
             *reinterpret_cast<uint32_t*>(dst + 2 * (int64_t)a.ktot) = (eq0 | eq1 | eq2) & kOne;
             *reinterpret_cast<uint32_t*>(dst + 3 * (int64_t)a.ktot) = 0u;
         } else {
-            *reinterpret_cast<uint32_t*>(dst) = eq1 & kOne;
+            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq1;
             *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq1) & kOne;
         }
     }
@@ -184,12 +184,12 @@ __global__ void __launch_bounds__(128, 1) k_probe_i8(int iters) {
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     if (threadIdx.x == 0) {
-        constexpr uint32_t idesc = idesc_u8<kProbeN>();
+        constexpr uint32_t idesc = idesc_s8<kProbeN>();
         const uint32_t a_addr = su32(base), b_addr = a_addr + A_BYTES;
         for (int it = 0; it < iters; ++it)
 #pragma unroll
             for (int ks = 0; ks < kKChunk / 32; ++ks)
-                mma_u8(tmem, sw128_desc(a_addr + ks * 32), sw128_desc(b_addr + ks * 32), idesc, (it | ks) ? 1u : 0u);
+                mma_i8(tmem, sw128_desc(a_addr + ks * 32), sw128_desc(b_addr + ks * 32), idesc, (it | ks) ? 1u : 0u);
         mma_commit(&bar);
         mbar_wait(&bar, 0u, &abort_s, &g_probe_status);
     }
@@ -262,14 +262,14 @@ __global__ void k_fill_rtab(double4* t, int max_n) {
 }  // namespace
 
 namespace {
-__global__ void k_fill_gtab(GenoRecip* t, int max_n) {
+__global__ void k_fill_gtab(double4* t, int max_n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= max_n) t[i] = geno_recip_entry(i);
+    if (i <= max_n) t[i] = recip_entry_geno(i);
 }
 }  // namespace
 
 cudaError_t launch_fill_gtab(void* gtab, int max_n, cudaStream_t s) {
-    k_fill_gtab<<<(max_n + 256) / 256, 256, 0, s>>>(static_cast<GenoRecip*>(gtab), max_n);
+    k_fill_gtab<<<(max_n + 256) / 256, 256, 0, s>>>(static_cast<double4*>(gtab), max_n);
     return cudaGetLastError();
 }
 

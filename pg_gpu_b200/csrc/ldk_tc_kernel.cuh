@@ -1,21 +1,30 @@
 // Tensor-core path of the binned parse (sm_100a): the kernel template and its launcher,
 // instantiated per path and tile variant in ldk_tc_hap0.cu, ldk_tc_hap1.cu, ldk_tc_geno.cu.
 //
-// Counting as a Gram product.  For SNPs i, j and one population, with per-haplotype
-// indicators h = [allele == 1] and v = [allele != missing], the four products
-//   hh = sum_k h_ik h_jk,  hv = sum_k h_ik v_jk,  vh = sum_k v_ik h_jk,  vv = sum_k v_ik v_jk
-// give the two-locus counts exactly: n11 = hh, n10 = hv - hh, n01 = vh - hh,
-// n00 = vv - hv - vh + hh, n_valid = vv (pg_gpu ld_pipeline.py:155-172).
+// Counting as a Gram product.  For SNPs i, j and one population, with per-haplotype spins
+// sigma = 1 - 2 [allele == 1] (0 where missing) and v = [allele != missing], the four products
+//   R = sum_k sigma_ik sigma_jk,  S = sum_k sigma_ik v_jk,  T = sum_k v_ik sigma_jk,  n = sum_k v_ik v_jk
+// determine the two-locus counts exactly (n11 = (n - S - T + R) / 4, ...; pg_gpu
+// ld_pipeline.py:155-172) and are the moments the estimators are polynomials of
+// (ldk_spin.cuh), so no count is rebuilt per pair.  Genotypes: sigma = 1 - g, sigma^2 and v.
 //
-// Layout in HBM (built by k_prep_planes): per SNP two 0/1 byte planes (h, v) over the
+// Layout in HBM (built by k_prep_planes): per SNP two s8 planes (sigma, v) over the
 // concatenated haplotypes of all populations, each population padded to a multiple of
 // 32 bytes, the whole K axis to a multiple of 128 bytes:  planes[snp][plane][k].
 // A 3-D TMA box {128 k, 2 planes, R snps} then lands in shared memory as 2R interleaved
-// rows (h_i0, v_i0, h_i1, v_i1, ...) in the 128-byte-swizzled K-major layout that
+// rows (sigma_i0, v_i0, sigma_i1, ...) in the 128-byte-swizzled K-major layout that
 // tcgen05.mma reads directly.  One MMA per 32-byte K step and population:
-//   D[128 x 2NJ] (+)= A[128 rows = 64 SNPs x {h,v}] . B[2NJ rows = NJ SNPs x {h,v}]^T
-// with u8 inputs and s32 accumulation in tensor memory: TMEM lane 2r holds (hh, hv) and
-// lane 2r+1 holds (vh, vv) of SNP i0+r against every j of the tile.
+//   D[128 x 2NJ] (+)= A[128 rows = 64 SNPs x {sigma, v}] . B[2NJ rows = NJ SNPs x {sigma, v}]^T
+// with s8 inputs and s32 accumulation in tensor memory: TMEM lane 2r holds (R, S) and
+// lane 2r+1 holds (T, n) of SNP i0+r against every j of the tile.
+//
+// What bounds it: the FP64 estimators of the epilogue, not the counts.  The spin forms take
+// 30 / 112 / 267 FP64 operations a pair for 1 / 2 / 3 haplotype populations (the factored
+// raw-call forms they replaced: 404 measured for three) and 35 / 144 / 316 for genotypes
+// (the nine-cell polynomials: 404 for one population's numerators alone).  B200, 1965 MHz:
+// 500 diploids x 100,000 SNPs 9.63 -> 3.79 ms a pass, two genotype populations x 20,001 SNPs
+// 5.28 -> 2.77, three haplotype populations x 200 windows 48.0 -> 39.5, two x 50,000 SNPs
+// 6.93 -> 5.74, four x 8,000 SNPs 5.59 -> 4.72.
 //
 // Warp roles (one CTA per SM, persistent over work items: runs of one row block's partner
 // tiles, claimed dynamically):
@@ -57,9 +66,9 @@ constexpr int kRegCtrl = 24;
 constexpr size_t kMinSmem = 116 * 1024;
 constexpr size_t kMaxSmem = 227 * 1024;
 
-// Tile geometry.  Haplotype path: a row block of 64 SNPs x {h, v} = 128 MMA rows against
-// NJ partners x {h, v} (N = 2 NJ), one MMA per K step and population.  Genotype path: a row
-// block of 128 SNPs; four stored planes per SNP {g == 1, g == 2, valid, 0}; per K step and
+// Tile geometry.  Haplotype path: a row block of 64 SNPs x {sigma, v} = 128 MMA rows against
+// NJ partners x {sigma, v} (N = 2 NJ), one MMA per K step and population.  Genotype path: a row
+// block of 128 SNPs; four stored planes per SNP {sigma, sigma^2, valid, 0}; per K step and
 // population three MMAs, plane x (< 3) of the row block against all four planes of NJ
 // partners (N = 4 NJ) into region x, so TMEM lane r holds all nine Gram products of SNP r
 // (and a zero column per partner, which keeps every partner's columns 4-aligned).
@@ -189,16 +198,16 @@ LDK_DEV uint64_t sw128_desc(uint32_t saddr) {
     return d;
 }
 
-// kind::i8 instruction descriptor: u8 x u8 -> s32, K-major A and B, M = 128.
+// kind::i8 instruction descriptor: s8 x s8 -> s32, K-major A and B, M = 128.
 template <int N>
-__host__ __device__ constexpr uint32_t idesc_u8() {
+__host__ __device__ constexpr uint32_t idesc_s8() {
     return (2u << 4)                      // D format s32
-           | (0u << 7) | (0u << 10)       // A, B unsigned 8-bit
+           | (1u << 7) | (1u << 10)       // A, B signed 8-bit
            | ((uint32_t)(N >> 3) << 17)   // N / 8
            | ((uint32_t)(128 >> 4) << 24);  // M / 16
 }
 
-LDK_DEV void mma_u8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+LDK_DEV void mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
@@ -275,7 +284,7 @@ struct TcArgs {
     unsigned* status;
     const double4* rtab_g;  // haplotype path: reciprocal table in global memory, or null when
                             // each CTA builds it in shared memory
-    const GenoRecip* gtab;  // genotype path, P <= 3: geno_prepare's reciprocals per valid count
+    const double4* gtab;    // genotype path: reciprocal table in global memory
 };
 
 // Shared-memory state of the persistent pipeline (one CTA).
@@ -322,7 +331,7 @@ LDK_DEV void issue_loads(const Pipe& S, const CUtensorMap* tmA, const CUtensorMa
 // MMAs of K chunk c (in stage s) into accumulator buffer buf; frees the stage on completion.
 template <class C, int P>
 LDK_DEV void issue_mmas(const Pipe& S, uint32_t tmem, const TcArgs& a, int s, int c, uint32_t buf) {
-    constexpr uint32_t idesc = idesc_u8<C::N>();
+    constexpr uint32_t idesc = idesc_s8<C::N>();
     const uint32_t a_addr = su32(S.stages + s * C::STAGE_BYTES);
     const uint32_t b_addr = a_addr + C::A_BYTES;
 #pragma unroll
@@ -335,7 +344,7 @@ LDK_DEV void issue_mmas(const Pipe& S, uint32_t tmem, const TcArgs& a, int s, in
 #pragma unroll
         for (int x = 0; x < C::REGIONS; ++x) {
             const uint32_t d = tmem + buf * C::COLS + (p * C::REGIONS + x) * C::N;
-            mma_u8(d, sw128_desc(a_addr + x * C::A_BOX + ks * 32), sw128_desc(b_addr + ks * 32), idesc, first ^ 1u);
+            mma_i8(d, sw128_desc(a_addr + x * C::A_BOX + ks * 32), sw128_desc(b_addr + ks * 32), idesc, first ^ 1u);
         }
     }
     mma_commit(&S.empty_bar[s]);
@@ -501,7 +510,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
         // each holds about half of the 105 accumulators.  (The same split of the genotype
         // path measured slower: both warps then compute all four populations' features.)
         constexpr bool SSPL = !GENO && P == 4;
-        constexpr int K = HapFusedSplit<P>::value;
+        constexpr int K = SpinSplit<P>::value;
         constexpr int NA = SSPL ? ((K > NS - K + 1 ? K : NS - K + 1)) : NS + 1;  // accumulators per lane
         constexpr int MY_STEPS = SSPL ? STEPS : STEPS / PARTS;  // ... each reading a contiguous share
         const int part = e >> 2;
@@ -648,85 +657,51 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                         for (int s = 0; s < NA; ++s) acc[s] = T(0);
                         np = nr2 = 0;
                     }
-                    if constexpr (!GENO) {
-                        HapFeat<T> f[P];
-                        int nval[P];
+                    SpinPop f[P];
+                    int nval[P];
 #pragma unroll
-                        for (int p = 0; p < P; ++p) {
-                            // lane 2r: (hh, hv) of partners 2q, 2q+1; lane 2r+1: (vh, vv)
+                    for (int p = 0; p < P; ++p) {
+                        if constexpr (!GENO) {
+                            // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
                             const uint32_t* w = v[p][0];
                             const uint32_t sx = role ? w[0] : w[2];
                             const uint32_t sy = role ? w[1] : w[3];
                             const uint32_t rx = __shfl_xor_sync(0xffffffffu, sx, 1);
                             const uint32_t ry = __shfl_xor_sync(0xffffffffu, sy, 1);
-                            int hh, hv, vh, vv;
-                            if (role == 0) { hh = (int)w[0]; hv = (int)w[1]; vh = (int)rx; vv = (int)ry; }
-                            else { vh = (int)w[2]; vv = (int)w[3]; hh = (int)rx; hv = (int)ry; }
-                            hap_set_counts(f[p], count_to<T>(hh), count_to<T>(hv - hh), count_to<T>(vh - hh),
-                                           count_to<T>(vv - hv - vh + hh));
-                            nval[p] = vv;
+                            f[p].R = i2d_exact((int)(role ? rx : w[0]));
+                            f[p].S = i2d_exact((int)(role ? ry : w[1]));
+                            f[p].T = i2d_exact((int)(role ? w[2] : rx));
+                            nval[p] = (int)(role ? w[3] : ry);
+                        } else {
+                            // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma,
+                            // 1: sigma^2, 2: valid)
+                            const uint32_t (&G)[3][4] = v[p];
+                            f[p].R = i2d_exact((int)G[0][0]);
+                            f[p].STT = i2d_exact((int)G[0][1]);
+                            f[p].S = i2d_exact((int)G[0][2]);
+                            f[p].SST = i2d_exact((int)G[1][0]);
+                            f[p].SSTT = i2d_exact((int)G[1][1]);
+                            f[p].SS = i2d_exact((int)G[1][2]);
+                            f[p].T = i2d_exact((int)G[2][0]);
+                            f[p].TT = i2d_exact((int)G[2][1]);
+                            nval[p] = (int)G[2][2];
                         }
-                        if (valid && cur >= 0 && cur < nb) {
+                    }
+                    if (valid && cur >= 0 && cur < nb) {
 #pragma unroll
-                            for (int p = 0; p < P; ++p) {
-                                hap_features<T, P>(f[p]);
-                                if constexpr (GT) hap_reciprocals_from(f[p], a.rtab_g[nval[p]]);
-                                else hap_reciprocals_from(f[p], rtab[nval[p]]);
-                            }
-                            if constexpr (SSPL) {
-                                if (part == 0) {
-                                    hap_fused<T, P, 1>(f, acc);
-                                } else {
-                                    hap_fused<T, P, 2>(f, acc);
-                                    T r2;
-                                    // r^2 is this part's last staged value (global index NS)
-                                    if (hap_r2(f[0], r2)) { acc[NS - K] += r2; ++nr2; }
-                                }
-                            } else {
-                                hap_fused<T, P, 0>(f, acc);
-                                T r2;
-                                if (hap_r2(f[0], r2)) { acc[NS] += r2; ++nr2; }
-                            }
-                            ++np;
+                        for (int p = 0; p < P; ++p) {
+                            f[p].n = i2d_exact(nval[p]);
+                            if constexpr (GENO) spin_reciprocals(f[p], a.gtab[nval[p]]);
+                            else if constexpr (GT) spin_reciprocals(f[p], a.rtab_g[nval[p]]);
+                            else spin_reciprocals(f[p], rtab[nval[p]]);
                         }
-                    } else {
-                        if (valid && cur >= 0 && cur < nb) {
-                            // Gram products G[x][y] = plane x of SNP i . plane y of SNP j
-                            // (0: g == 1, 1: g == 2, 2: valid); cells in the order of pg_gpu's
-                            // counting kernel, column g_i * 3 + g_j (ld_pipeline.py:183-263)
-                            GenoFeat<T> f[P];
-                            T c0[9];
-#pragma unroll
-                            for (int p = 0; p < P; ++p) {
-                                const uint32_t (&G)[3][4] = v[p];
-                                const int n11 = (int)G[0][0], n12 = (int)G[0][1], n21 = (int)G[1][0], n22 = (int)G[1][1];
-                                const int n10 = (int)G[0][2] - n11 - n12, n20 = (int)G[1][2] - n21 - n22;
-                                const int n01 = (int)G[2][0] - n11 - n21, n02 = (int)G[2][1] - n12 - n22;
-                                const int nv = (int)G[2][2];
-                                const int n00 = nv - n01 - n02 - n10 - n11 - n12 - n20 - n21 - n22;
-                                const T cd[9] = {count_to<T>(n00), count_to<T>(n01), count_to<T>(n02),
-                                                 count_to<T>(n10), count_to<T>(n11), count_to<T>(n12),
-                                                 count_to<T>(n20), count_to<T>(n21), count_to<T>(n22)};
-                                if (p == 0) {
-#pragma unroll
-                                    for (int m = 0; m < 9; ++m) c0[m] = cd[m];
-                                }
-                                geno_set_counts(f[p], cd);
-                                f[p].n = count_to<T>(nv);
-                                if constexpr (P <= 3) {
-                                    geno_prepare_from(f[p], a.gtab + nv);  // n = ns = nv here
-                                    geno_features<T, P, false>(f[p]);
-                                } else {
-                                    // four populations divide: the table's registers deepen
-                                    // their spill (measured 0.45 vs 0.60 Gpairs/s)
-                                    geno_features<T, P>(f[p]);
-                                }
-                            }
-                            geno_stats<T, P>(f, acc);
-                            T r2;
-                            if (geno_dosage_r2(c0, r2)) { acc[NS] += r2; ++nr2; }
-                            ++np;
+                        if constexpr (SSPL) {
+                            if (part == 0) spin_stats<P, GENO, 1>(f, acc, nr2);
+                            else spin_stats<P, GENO, 2>(f, acc, nr2);
+                        } else {
+                            spin_stats<P, GENO, 0>(f, acc, nr2);
                         }
+                        ++np;
                     }
                 }
             }
@@ -747,7 +722,8 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 const int bb = rem / (NS + 1), s = rem % (NS + 1);
                 const int blk = blk0 + sl;
                 if (val != 0.0 && blk < a.n_blocks)
-                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + s) * kFxLimbs, val, a.status);
+                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + s) * kFxLimbs, val * spin_weight<P, GENO>(s),
+                           a.status);
             }
             for (int idx = et; idx < SLOTS * nb; idx += 32 * EPI) {
                 unsigned long long c0 = 0, c1 = 0;
@@ -879,7 +855,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     a.r2_counts = reinterpret_cast<unsigned long long*>(o->r2_counts);
     a.status = w.status;
     a.rtab_g = static_cast<const double4*>(w.rtab);
-    a.gtab = static_cast<const GenoRecip*>(w.gtab);
+    a.gtab = static_cast<const double4*>(w.gtab);
     // at least half of an SM's shared memory, so that one CTA (holding all 512 TMEM
     // columns) runs per SM
     size_t smem = smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), PRIV ? C::EPI : 1);
