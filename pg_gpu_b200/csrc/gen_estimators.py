@@ -881,10 +881,16 @@ def spin_stats(P, geno):
     return out
 
 
-# Split point of the statistics where two epilogue warps share them: Dz | pi2 (the two halves
-# need nearly disjoint features).
-def spin_split(P):
-    return sum(1 for k, _ in ld_names(P) if k != "pi2")
+def spin_order(P, geno):
+    """(order, K): the statistics in the order they are staged (r^2 is index NS) and, for four
+    haplotype populations, where two epilogue warps that share a pair split them: [0, K)
+    holds DD, Dz, the one-population pi2 (all from Q2, Q3, Q4) and r^2, the rest the other
+    pi2, so that the halves need nearly disjoint features.  K = 0: one warp takes all."""
+    names = ld_names(P)
+    if geno or P < 4:
+        return list(range(len(names) + 1)), 0
+    first = [k for k, (kind, q) in enumerate(names) if kind != "pi2" or len(set(q)) == 1] + [len(names)]
+    return first + [k for k in range(len(names)) if k not in first], len(first)
 
 
 def _names_in(e):
@@ -893,18 +899,14 @@ def _names_in(e):
 
 
 def emit_spin(P, geno):
-    """spin_{hap,geno}_P{P}_{part}: part 0 = all statistics and r^2, 1 = [0, K), 2 = [K, NS)
-    and r^2 (the last accumulator)."""
+    """spin_{hap,geno}_P{P}_{part}: part 0 = all statistics and r^2; with a split, part 1 =
+    staged sums [0, K) and part 2 = [K, NS]."""
     path = "geno" if geno else "hap"
-    defs, stats, K = spin_defs(P, geno), spin_stats(P, geno), spin_split(P)
+    defs, stats, (order, K) = spin_defs(P, geno), spin_stats(P, geno), spin_order(P, geno)
     inputs = SPIN_INPUTS_GENO if geno else SPIN_INPUTS
-    L = [f"// {path}, P = {P}: {len(stats)} statistics, split at {K}"]
-    parts = {0: (0, len(stats)), 1: (0, K), 2: (K, len(stats))}
-    if geno or P < 4:
-        parts = {0: parts[0]}
-    else:
-        parts.pop(0)
-    for part, (lo, hi) in parts.items():
+    NS = len(stats)
+    L = [f"// {path}, P = {P}: {NS} statistics" + (f", split at {K}" if K else "")]
+    for part, mine in ({1: order[:K], 2: order[K:]} if K else {0: order}).items():
         lines, done = [], set()
 
         def use(expr):
@@ -920,21 +922,25 @@ def emit_spin(P, geno):
                     assert base in inputs, nm
                     lines.append(f"    const double {nm} = f[{nm[-1]}].{base};")
 
-        for si in sorted(range(lo, hi), key=lambda k: stats[k][3]):
+        for si in sorted((k for k in mine if k < NS), key=lambda k: stats[k][3]):
             name, _, terms, _ = stats[si]
+            at = mine.index(si)
             for A, B in terms:
                 use(A)
                 use(B)
-                lines.append(f"    acc[{si - lo}] = fma({A}, {B}, acc[{si - lo}]);  // {name}")
-        if part != 1:
+                lines.append(f"    acc[{at}] = fma({A}, {B}, acc[{at}]);  // {name}")
+        if NS in mine:
+            at = mine.index(NS)
             use("E0 vx0 vy0")
             lines += ["    const double den = vx0 * vy0;", "    if (den > 0.0) {",
-                      f"        acc[{hi - lo}] = fma(E0 * E0, recip_cubic(den), acc[{hi - lo}]);", "        ++nr2;", "    }"]
+                      f"        acc[{at}] = fma(E0 * E0, recip_cubic(den), acc[{at}]);", "        ++nr2;", "    }"]
         L.append(f"LDK_DEV void spin_{path}_P{P}_{part}(const SpinPop* f, double* acc, unsigned& nr2) {{")
         L += lines
         L.append("}")
-    w = [x[1] for x in stats]
-    L.append(f"static __constant__ double spin_weight_{path}_P{P}[{len(w) + 1}] = {{{', '.join(repr(x) for x in w)}, 1.0}};")
+    w = [x[1] for x in stats] + [1.0]
+    L.append(f"static __constant__ double spin_weight_{path}_P{P}[{NS + 1}] = {{{', '.join(repr(w[k]) for k in order)}}};")
+    if K:
+        L.append(f"static __constant__ int spin_stat_{path}_P{P}[{NS + 1}] = {{{', '.join(map(str, order))}}};")
     return "\n".join(L)
 
 
@@ -1001,10 +1007,10 @@ def generate(path=None):
     parts.append("template <int P> struct HapNStats;")
     for P in (1, 2, 3, 4):
         parts.append(f"template <> struct HapNStats<{P}> {{ static constexpr int value = {len(stat_specs(P))}; }};")
-    parts.append("// first statistic of the second half of the two-way split")
+    parts.append("// staged sums of the first of two warps that share a pair (haplotypes), 0: no split")
     parts.append("template <int P> struct SpinSplit;")
     for P in (1, 2, 3, 4):
-        parts.append(f"template <> struct SpinSplit<{P}> {{ static constexpr int value = {spin_split(P)}; }};")
+        parts.append(f"template <> struct SpinSplit<{P}> {{ static constexpr int value = {spin_order(P, False)[1]}; }};")
     parts.append("""
 template <typename T, int P>
 LDK_DEV void hap_features(HapFeat<T>& x) {
@@ -1027,8 +1033,8 @@ LDK_DEV void geno_stats(const GenoFeat<T>* f, T* acc) {
     else if constexpr (P == 3) geno_stats_P3<T, S>(f, acc);
     else geno_stats_P4<T, S>(f, acc);
 }
-// Spin-form statistics of part PART (0: all and r^2, 1: [0, split), 2: [split, NS) and r^2)
-// added into acc[0 ..) of that part, before their weights (spin_weight).
+// Spin-form statistics of part PART (0: all and r^2; four haplotype populations:
+// 1 and 2, the two halves) added into acc[0 ..) of that part, before their weights.
 template <int P, bool GENO, int PART>
 LDK_DEV void spin_stats(const SpinPop* f, double* acc, unsigned& nr2) {
     if constexpr (GENO) {
@@ -1044,13 +1050,18 @@ LDK_DEV void spin_stats(const SpinPop* f, double* acc, unsigned& nr2) {
         else spin_hap_P4_2(f, acc, nr2);
     }
 }
-// Weight of statistic s of P populations (s = number of statistics: r^2, weight 1).
+// Weight and statistic (number of statistics: r^2, weight 1) of staged sum s.
 template <int P, bool GENO>
 LDK_DEV double spin_weight(int s) {
     if constexpr (GENO)
         return P == 1 ? spin_weight_geno_P1[s] : P == 2 ? spin_weight_geno_P2[s] : P == 3 ? spin_weight_geno_P3[s] : spin_weight_geno_P4[s];
     else
         return P == 1 ? spin_weight_hap_P1[s] : P == 2 ? spin_weight_hap_P2[s] : P == 3 ? spin_weight_hap_P3[s] : spin_weight_hap_P4[s];
+}
+template <int P, bool GENO>
+LDK_DEV int spin_stat(int s) {
+    if constexpr (GENO || P < 4) return s;
+    else return spin_stat_hap_P4[s];
 }
 template <typename T, int P, int S = 1>
 LDK_DEV void hap_stats(const HapFeat<T>* f, T* acc) {

@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
-    if (warp == 0) run_producer<C>(pipe, &tmA, &tmB, a, lane);
+    if (warp == 0) run_producer<C, false>(pipe, &tmA, &tmB, a, lane);
     else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
     if (warp >= 4) {
         // lanes 2r, 2r+1 share SNP r (16 per warp) and split its partners by parity; the
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
-    if (warp == 0) run_producer<C>(pipe, &tmA, &tmB, a, lane);
+    if (warp == 0) run_producer<C, false>(pipe, &tmA, &tmB, a, lane);
     else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
     if (warp >= 4) {
         // lane = SNP of the row block (32 per warp); the warp takes half `part` of every tile

@@ -18,13 +18,14 @@
 // with s8 inputs and s32 accumulation in tensor memory: TMEM lane 2r holds (R, S) and
 // lane 2r+1 holds (T, n) of SNP i0+r against every j of the tile.
 //
-// What bounds it: the FP64 estimators of the epilogue, not the counts.  The spin forms take
-// 30 / 112 / 267 FP64 operations a pair for 1 / 2 / 3 haplotype populations (the factored
-// raw-call forms they replaced: 404 measured for three) and 35 / 144 / 316 for genotypes
-// (the nine-cell polynomials: 404 for one population's numerators alone).  B200, 1965 MHz:
-// 500 diploids x 100,000 SNPs 9.63 -> 3.79 ms a pass, two genotype populations x 20,001 SNPs
-// 5.28 -> 2.77, three haplotype populations x 200 windows 48.0 -> 39.5, two x 50,000 SNPs
-// 6.93 -> 5.74, four x 8,000 SNPs 5.59 -> 4.72.
+// What bounds it: with two or more populations the FP64 estimators of the epilogue, not the
+// counts.  The spin forms take 30 / 112 / 267 FP64 operations a pair for 1 / 2 / 3 haplotype
+// populations (the factored raw-call forms they replaced: 404 measured for three) and
+// 35 / 144 / 316 for genotypes (the nine-cell polynomials: 404 for one population's numerators
+// alone).  B200, 1965 MHz, a pass with the old -> new forms: 500 diploids x 100,000 SNPs
+// 9.63 -> 3.79 ms, two genotype populations x 20,001 SNPs 5.28 -> 2.77, three haplotype
+// populations x 200 windows 48.0 -> 39.5, two x 50,000 SNPs 6.93 -> 5.74.  With one population
+// the TMA traffic (about 11 TB/s from L2) and the bin flushes weigh as much.
 //
 // Warp roles (one CTA per SM, persistent over work items: runs of one row block's partner
 // tiles, claimed dynamically):
@@ -46,7 +47,7 @@
 
 #include <cstdlib>
 #include <mutex>
-#include <type_traits>
+#include <utility>
 
 #include "ldk_estimators.cuh"
 #include "ldk_internal.h"
@@ -100,31 +101,50 @@ struct Cfg {
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     static constexpr int NS = HapNStats<P>::value;
     static constexpr int SLOTS = GENO ? 4 : 2;                         // bootstrap blocks staged per row block
+    // QROWS (one to three haplotype populations): A rows come in groups of sixteen, eight
+    // SNPs' sigma rows and the same SNPs' v rows, so that one tcgen05.ld.16x256b hands a
+    // thread all four moments (R, S, T, n) of one pair -- SNP lane / 4 of the eight, partner
+    // lane % 4 of four -- with no exchange between lanes (eighteen selects and six shuffles a
+    // pair for three populations).  Otherwise rows are interleaved
+    // (sigma, v per SNP; genotypes: one plane per region) and read with 32x32b.
+    static constexpr bool QROWS = !GENO && P <= 3;
     // Warp layout.  Warp w may read only TMEM lane quarter w % 4, and each of the four
     // schedulers of an SM holds warps w, w + 4, ... with a quarter of the register file.
-    // The epilogue warps of a lane quarter each take an equal share of every partner tile.
     //  * SPLIT (genotypes; haplotypes with three or four populations -- estimators that
     //    want ~240 registers): 12 warps.  Warpgroup 0 (TMA, MMA, two idle warps) gives its
     //    registers up with setmaxnreg (kRegCtrl each) and the eight epilogue warps 4..11
     //    take them (240 each), so that every scheduler holds two full-register epilogue
     //    warps beside one control warp (launch: 168 per thread).
-    //  * two haplotype populations (~155 registers) and one genotype population, also SPLIT:
-    //    16 warps, twelve epilogue warps 4..15 at 160 registers, three per scheduler and lane
-    //    quarter (launch: 128).
-    //  * one haplotype population (about 100 registers): 18 warps, TMA and MMA in warps 0 and
-    //    1, sixteen epilogue warps 2..17, four per lane quarter and scheduler, each taking a
-    //    quarter of every partner tile -- its per-pair work is short, so more warps hide the
-    //    latency of its dependency chains (113 registers at most).
+    //  * one genotype population, also SPLIT: 16 warps, twelve epilogue warps 4..15 at 160
+    //    registers, three per scheduler and lane quarter (launch: 128).
+    //  * one or two haplotype populations: 18 warps, TMA and MMA in warps 0 and 1, sixteen
+    //    epilogue warps 2..17, four per lane quarter and scheduler (113 registers at most).
+    static constexpr int EPI = (!GENO && P == 1) ? 16 : (GENO && P == 1) ? 12 : 8;
     static constexpr bool SPLIT = GENO || P >= 2;
-    static constexpr int EPI = (!GENO && P == 1) ? 16 : ((!GENO && P == 2) || (GENO && P == 1)) ? 12 : 8;
     static constexpr int W0 = SPLIT ? 4 : 2;  // first epilogue warp
     static constexpr int THREADS = 32 * (W0 + EPI);
-    static constexpr int REG_LAUNCH = (EPI == 12) ? 128 : 168;  // SPLIT layouts only
-    static constexpr int REG_EPI = (EPI == 12) ? 160 : 240;
+    static constexpr int REG_LAUNCH = (EPI == 16) ? 96 : (EPI == 12) ? 128 : 168;  // SPLIT layouts only
+    static constexpr int REG_EPI = (EPI == 16) ? 112 : (EPI == 12) ? 160 : 240;
+    // SSPL (four haplotype populations): the two warps of a lane quarter split the
+    // statistics, not the partners -- both take every pair, part 0 accumulates statistics
+    // [0, K) (DD, Dz) and counts pairs, part 1 the pi2 statistics [K, NS) and r^2 -- so that
+    // each holds about half of the 105 accumulators.
+    static constexpr bool SSPL = !GENO && P == 4;
+    static constexpr int PARTS = SSPL ? 2 : 1;
+    // Steps (TMEM reads) per tile and their shares: with QROWS two warps of a quarter split
+    // its SNPs, further ones the partners; otherwise the warps split the partners.
+    static constexpr int STEPS = GENO ? NJ : QROWS ? NJ / 4 : NJ / 2;
+    static constexpr int SHARES = EPI / (4 * PARTS * (QROWS ? 2 : 1));
+    static constexpr int MY_STEPS = STEPS / SHARES;
+    // Staging row of the bin flush: a lane's sums, then {pairs, finite r^2, key, -}
+    static constexpr int K = GENO ? 0 : SpinSplit<P>::value;
+    static constexpr int NA = SSPL ? (K > NS + 1 - K ? K : NS + 1 - K) : NS + 1;  // sums per lane
+    static constexpr int FROW = P == 1 ? 0 : NA + 2;  // one population reduces in registers
+    static constexpr int FROWS_MAX = 8;
     static_assert(!SPLIT || 4 * kRegCtrl + EPI * REG_EPI <= (W0 + EPI) * REG_LAUNCH,
                   "register split must fit the launch allocation");
     static_assert(!SPLIT || THREADS * REG_LAUNCH <= 65536, "register file");
-    static_assert(EPI % 4 == 0 && (GENO ? NJ : NJ / 2) % (EPI / 4) == 0, "epilogue warps share tiles equally");
+    static_assert(EPI % 4 == 0 && STEPS % SHARES == 0 && (!QROWS || NJ % 4 == 0), "epilogue warps share tiles equally");
     static_assert(NBUF * COLS <= kTmemCols, "TMEM budget");
     static_assert(N % 16 == 0 && N <= 256, "MMA N");
 };
@@ -224,6 +244,13 @@ LDK_DEV void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(taddr));
 }
+// Sixteen lanes x eight columns: thread t gets columns 2 (t % 4), + 1 of lane t / 4 in r[0],
+// r[1] and of lane t / 4 + 8 in r[2], r[3].
+LDK_DEV void tmem_ld_q(uint32_t taddr, uint32_t (&r)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+}
 template <int P>
 LDK_DEV void tmem_wait4(uint32_t (&r)[P][4]) {
 #pragma unroll
@@ -266,6 +293,51 @@ LDK_DEV void spin_ns(uint64_t ns) {
 // the fused count + estimator + bin kernel
 // ---------------------------------------------------------------------------
 
+// Flush of one population's four sums: for every (block, bin) among the flushing lanes the
+// warp adds the lanes' values with a butterfly that halves the values each lane carries (two
+// exchanges leave lane / 8 % 4 with one value, three more add it up), and the four lanes that
+// hold a total add it to the staged sums.  About ten lanes of a warp flush the same key in the
+// same step when a row block crosses a bin edge; one lane per round, ~60 cycles each, took
+// 25.0 ms for 1,000,000 SNPs x 2,000 haplotypes in 32 bins, this 21.6 (5,000 SNPs x 100:
+// 0.119 -> 0.098; 500 diploids x 100,000: 3.82 -> 3.43).
+template <bool PRIV>
+LDK_DEV void flush_one_pop(unsigned mask, int key, const double* acc, unsigned np, unsigned nr2, double* my_sacc,
+                           unsigned* my_scnt, int lane) {
+    while (mask) {
+        const int kk = __shfl_sync(0xffffffffu, key, __ffs(mask) - 1);
+        const bool in = ((mask >> lane) & 1u) && key == kk;
+        mask &= ~__ballot_sync(0xffffffffu, in);
+        const bool h1 = lane & 16, h2 = lane & 8;
+        double v[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) v[s] = in ? acc[s] : 0.0;
+        const unsigned cp = __reduce_add_sync(0xffffffffu, in ? np : 0u);
+        const unsigned cr = __reduce_add_sync(0xffffffffu, in ? nr2 : 0u);
+        double x0 = h1 ? v[2] : v[0], x1 = h1 ? v[3] : v[1];
+        x0 += __shfl_xor_sync(0xffffffffu, h1 ? v[0] : v[2], 16);
+        x1 += __shfl_xor_sync(0xffffffffu, h1 ? v[1] : v[3], 16);
+        double y = h2 ? x1 : x0;
+        y += __shfl_xor_sync(0xffffffffu, h2 ? x0 : x1, 8);
+        y += __shfl_xor_sync(0xffffffffu, y, 4);
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        if ((lane & 7) == 0) {  // lanes 0, 8, 16, 24 hold sums 0, 1, 2, 3
+            double* dst = my_sacc + kk * 4 + (lane >> 3);
+            if constexpr (PRIV) *dst += y;
+            else atomicAdd(dst, y);
+        } else if (lane == 1) {
+            if constexpr (PRIV) {
+                my_scnt[2 * kk] += cp;
+                my_scnt[2 * kk + 1] += cr;
+            } else {
+                atomicAdd(my_scnt + 2 * kk, cp);
+                atomicAdd(my_scnt + 2 * kk + 1, cr);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 struct TcArgs {
     const double* coord;
     const int32_t* jmax;
@@ -282,6 +354,7 @@ struct TcArgs {
     unsigned long long* pairs;
     unsigned long long* r2_counts;
     unsigned* status;
+    int frows;              // staging rows per epilogue warp of the bin flush
     const double4* rtab_g;  // haplotype path: reciprocal table in global memory, or null when
                             // each CTA builds it in shared memory
     const double4* gtab;    // genotype path: reciprocal table in global memory
@@ -318,13 +391,19 @@ LDK_DEV int item_tiles(const TcArgs& a, int item, int& row0, int& row1, int& jt0
 }
 
 // TMA loads of K chunk c of the tile (row block at row0, partners from j0) into stage s.
-template <class C>
+template <class C, bool QR>
 LDK_DEV void issue_loads(const Pipe& S, const CUtensorMap* tmA, const CUtensorMap* tmB, int s, int c, int row0,
                          int j0) {
     unsigned char* dst = S.stages + s * C::STAGE_BYTES;
     mbar_expect_tx(&S.full_bar[s], C::STAGE_BYTES);
+    if constexpr (QR) {  // box {128 k, 8 SNPs, 2 planes}: one group of sixteen rows
 #pragma unroll
-    for (int x = 0; x < C::REGIONS; ++x) tma_load_3d(dst + x * C::A_BOX, tmA, &S.full_bar[s], c * kKChunk, x, row0);
+        for (int g = 0; g < C::ROWS / 8; ++g)
+            tma_load_3d(dst + g * 16 * kKChunk, tmA, &S.full_bar[s], c * kKChunk, row0 + 8 * g, 0);
+    } else {
+#pragma unroll
+        for (int x = 0; x < C::REGIONS; ++x) tma_load_3d(dst + x * C::A_BOX, tmA, &S.full_bar[s], c * kKChunk, x, row0);
+    }
     tma_load_3d(dst + C::A_BYTES, tmB, &S.full_bar[s], c * kKChunk, 0, j0);
 }
 
@@ -352,7 +431,7 @@ LDK_DEV void issue_mmas(const Pipe& S, uint32_t tmem, const TcArgs& a, int s, in
 
 // Warp 0: claims work items from the global counter, publishes each with its tile count
 // through the ring and issues the TMA loads of every partner tile's K chunks.
-template <class C>
+template <class C, bool QR>
 LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorMap* tmB, const TcArgs& a,
                           int lane) {
     if (lane == 0) {
@@ -376,7 +455,7 @@ LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorM
                     const int s = it % C::STAGES;
                     const uint32_t ph = (it / C::STAGES) & 1u;
                     if (!mbar_wait(&S.empty_bar[s], ph ^ 1u, S.abort_s, a.status)) { ok = false; break; }
-                    issue_loads<C>(S, tmA, tmB, s, c, row0, j0);
+                    issue_loads<C, QR>(S, tmA, tmB, s, c, row0, j0);
                 }
             }
         }
@@ -420,7 +499,7 @@ LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a, int lane) {
 // GT: the haplotype path's reciprocal table is read from the workspace (a.rtab_g) instead of
 // being built in shared memory -- a compile-time choice, so that the shared-memory form keeps
 // its hot loop unchanged.
-template <int P, typename T, bool PRIV, bool GENO, int V, bool GT = false>
+template <int P, bool PRIV, bool GENO, int V, bool GT = false>
 __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     k_parse_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a) {
     using C = Cfg<P, GENO, V>;
@@ -435,6 +514,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     double* sacc = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // [NCOPY][SLOTS][nb][NS+1]
     unsigned* scnt = reinterpret_cast<unsigned*>(sacc + NCOPY * SLOTS * nb * (NS + 1));  // [NCOPY][SLOTS][nb][2]
     double4* rtab = reinterpret_cast<double4*>(scnt + ((NCOPY * SLOTS * nb * 2 + 7) & ~7));  // [max_n + 1]
+    double* fstage = reinterpret_cast<double*>(rtab + (GENO || GT ? 0 : a.max_n + 1));  // [EPI][frows][FROW]
 
     __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
@@ -486,35 +566,33 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     // kRegCtrl registers raised an illegal-instruction fault.
     if (warp < C::W0) {
         if constexpr (C::SPLIT) setmaxnreg_dec<kRegCtrl>();
-        if (warp == 0) run_producer<C>(pipe, &tmA, &tmB, a, lane);
+        if (warp == 0) run_producer<C, C::QROWS>(pipe, &tmA, &tmB, a, lane);
         else if (warp == 1) run_mma<C, P>(pipe, tmem, a, lane);
     } else {
         if constexpr (C::SPLIT) setmaxnreg_inc<C::REG_EPI>();
         // ------------------------------------------------------------- epilogue
-        const int e = warp - C::W0;
-        const int L = (warp & 3) * 32 + lane;
-        // haplotype rows: lanes 2r, 2r+1 share SNP r and split its partners by parity;
-        // genotype rows: lane L is SNP L and takes every partner.  With two warps per lane
-        // quarter each takes a contiguous half of every partner tile, so every lane still
-        // sees its partners in increasing order.
-        const int r = GENO ? L : L >> 1, role = GENO ? 0 : L & 1;
-        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+        const int e = warp - C::W0, quarter = warp & 3;
+        const int unit = e >> 2;  // this warp among its lane quarter's
+        constexpr bool SSPL = C::SSPL;
+        constexpr int K = C::K, NA = C::NA;
+        const int half = C::QROWS ? unit & 1 : 0;  // which eight SNPs of the quarter's sixteen
+        const int rest = C::QROWS ? unit >> 1 : unit;
+        const int part = SSPL ? rest : 0, share = SSPL ? 0 : rest;
+        // SNP r of the row block and partner jb + stride * step of a tile
+        const int r = C::QROWS ? quarter * 16 + half * 8 + (lane >> 2)
+                      : GENO   ? quarter * 32 + lane
+                               : (quarter * 32 + lane) >> 1;
+        const int role = (GENO || C::QROWS) ? 0 : lane & 1;
+        constexpr int JSTRIDE = GENO ? 1 : C::QROWS ? 4 : 2;
+        const int q0 = share * C::MY_STEPS;
+        const int jb = JSTRIDE * q0 + (GENO ? 0 : lane & (JSTRIDE - 1));
+        const uint32_t tbase = tmem + ((uint32_t)(quarter * 32 + half * 16) << 16) +
+                               (uint32_t)q0 * (C::QROWS ? 8 : 4);
         const int stage_n = SLOTS * nb * (NS + 1);
-        double* my_sacc = sacc + (PRIV ? e * stage_n : 0);
-        unsigned* my_scnt = scnt + (PRIV ? e * SLOTS * nb * 2 : 0);
-        constexpr int STEPS = GENO ? C::NJ : C::NJ / 2;   // TMEM reads per tile
-        constexpr int PARTS = EPI / 4;                    // epilogue warps per lane quarter
-        // SSPL (four haplotype populations): the two warps of a lane quarter split the
-        // statistics, not the partners -- both take every pair, warp part 0 accumulates
-        // statistics [0, K) and counts pairs, part 1 statistics [K, NS) and r^2 -- so that
-        // each holds about half of the 105 accumulators.  (The same split of the genotype
-        // path measured slower: both warps then compute all four populations' features.)
-        constexpr bool SSPL = !GENO && P == 4;
-        constexpr int K = SpinSplit<P>::value;
-        constexpr int NA = SSPL ? ((K > NS - K + 1 ? K : NS - K + 1)) : NS + 1;  // accumulators per lane
-        constexpr int MY_STEPS = SSPL ? STEPS : STEPS / PARTS;  // ... each reading a contiguous share
-        const int part = e >> 2;
-        constexpr int CREGS = (C::NJ + 31) / 32;          // partner coordinates per lane
+        const int copy = PRIV ? e : 0;
+        double* my_sacc = sacc + copy * stage_n;
+        unsigned* my_scnt = scnt + copy * SLOTS * nb * 2;
+        double* my_fst = fstage + e * a.frows * C::FROW;
         uint32_t tcount = 0;
         for (uint32_t k = 0;; ++k) {
             const int sl = k % kRing;
@@ -538,7 +616,6 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             if (te <= tb) continue;
             const int i = row0 + r;
             bool row_ok = i < row1;
-            const int my_jmax = row_ok ? a.jmax[i] : 0;
             const double ci = row_ok ? a.coord[i] : 0.0;
             const int blk0 = a.snp_block ? a.snp_block[row0] : 0;
             int slot = 0;
@@ -549,61 +626,150 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     row_ok = false;
                 }
             }
+            // partners i < j < jmax[i]: j - i - 1 < span as unsigned numbers
+            const unsigned span = row_ok ? (unsigned)(a.jmax[i] - i - 1) : 0u;
             // Sums of the current bin live in registers.  Partners come in increasing j,
             // so the distance to them never decreases and each (row, bin) run is flushed
             // to shared memory once, when the lane's next partner falls past the bin's
             // upper edge (held in `nxt`).
-            T acc[NA];
+            double acc[NA];
             // statistic s of this warp's accumulators and where it goes in the staging row
-            const int na = SSPL ? (part == 0 ? K : NS - K + 1) : NS + 1;
+            const int na = SSPL ? (part == 0 ? K : NS + 1 - K) : NS + 1;
             const int gofs = SSPL && part == 1 ? K : 0;
 #pragma unroll
-            for (int s = 0; s < NA; ++s) acc[s] = T(0);
+            for (int s = 0; s < NA; ++s) acc[s] = 0.0;
             unsigned np = 0, nr2 = 0;
             int cur = -1;
+            bool in_bin = false;  // 0 <= cur < nb
             double nxt = sedges[0];
-            // Adds the flushing lanes' sums into shared memory.  With PRIV every epilogue
-            // warp owns its staging copy and the lanes of one warp that flush the same
-            // (block, bin) take turns (one lane per key per round), so plain adds suffice;
-            // otherwise the copy is shared by the warps and the adds are atomic.  Called by
-            // all 32 lanes.
+            // Adds the flushing lanes' sums into the staged sums; called by all 32 lanes.
+            // The flushing lanes write their sums into rows of the warp's scratch (in
+            // batches of `frows`, all lanes of a batch at once), then the warp adds the
+            // rows one after the other, lane s taking value s, carrying the total while
+            // the (block, bin) stays the same.  One lane per round adding its own 46
+            // values took one pass per flushing lane of a key -- on average 6.5 for 200
+            // windows x 3 populations, 39.5 -> 35.4 ms with the rows; with shared staging
+            // (atomics) two genotype populations 2.77 -> 1.25 ms, four haplotype 4.72 -> 2.56.  With PRIV every epilogue warp owns its staged sums
+            // and plain adds suffice; otherwise the warps share them (atomics).  The pairs are
+            // counted by the first of two warps that share them.
             auto flush = [&](bool want) {
-                const int key = slot * nb + cur;
-                if constexpr (PRIV) {
+                const unsigned mask = __ballot_sync(0xffffffffu, want);
+                if constexpr (P == 1) {
+                    flush_one_pop<PRIV>(mask, slot * nb + cur, acc, np, nr2, my_sacc, my_scnt, lane);
+                    return;
+                }
+                const int rank = __popc(mask & ((1u << lane) - 1u)), total = __popc(mask);
+                if constexpr (P > 1) {
+                if (a.frows == 0) {  // no room: one lane per (block, bin) at a time
+                    const int key = slot * nb + cur;
                     const unsigned grp = __match_any_sync(0xffffffffu, want ? key : -1);
-                    const int rank = __popc(grp & ((1u << lane) - 1u));
-                    const int rounds = (int)__reduce_max_sync(0xffffffffu, want ? (unsigned)__popc(grp) : 0u);
-                    double* dst = my_sacc + key * (NS + 1);
-                    for (int rr = 0; rr < rounds; ++rr) {
-                        if (want && rank == rr) {
-                            if constexpr (SSPL) {
+                    const int turn = __popc(grp & ((1u << lane) - 1u));
+                    const int turns = PRIV ? (int)__reduce_max_sync(0xffffffffu, want ? (unsigned)__popc(grp) : 0u) : 1;
+                    double* dst = my_sacc + key * (NS + 1) + gofs;
+                    unsigned* cnt = my_scnt + 2 * key;
+                    for (int rr = 0; rr < turns; ++rr) {
+                        if (want && (!PRIV || turn == rr)) {
 #pragma unroll
-                                for (int s = 0; s < NA; ++s)
-                                    if (s < na) dst[gofs + s] += (double)acc[s];
-                                if (part == 0) my_scnt[2 * key] += np;
-                            } else {
-#pragma unroll
-                                for (int s = 0; s <= NS; ++s) dst[s] += (double)acc[s];
-                                my_scnt[2 * key] += np;
+                            for (int s = 0; s < NA; ++s)
+                                if (!SSPL || s < na) {
+                                    if constexpr (PRIV) dst[s] += acc[s];
+                                    else atomicAdd(dst + s, acc[s]);
+                                }
+                            if (part == 0) {
+                                if constexpr (PRIV) {
+                                    cnt[0] += np;
+                                    cnt[1] += nr2;
+                                } else {
+                                    atomicAdd(cnt, np);
+                                    atomicAdd(cnt + 1, nr2);
+                                }
                             }
-                            my_scnt[2 * key + 1] += nr2;
                         }
                         __syncwarp();
                     }
-                } else if (want) {
-                    double* dst = my_sacc + key * (NS + 1);
-                    if constexpr (SSPL) {
+                    return;
+                }
+                constexpr int VPL = (NA + 31) / 32;  // values per lane; lane 31 also adds the counts
+                for (int b0 = 0; b0 < total; b0 += a.frows) {
+                    const int rows = total - b0 < a.frows ? total - b0 : a.frows;
+                    if (want && rank >= b0 && rank < b0 + rows) {
+                        double* row = my_fst + (rank - b0) * C::FROW;
 #pragma unroll
                         for (int s = 0; s < NA; ++s)
-                            if (s < na) atomicAdd(dst + gofs + s, (double)acc[s]);
-                        if (part == 0) atomicAdd(my_scnt + 2 * key, np);
-                    } else {
-#pragma unroll
-                        for (int s = 0; s <= NS; ++s) atomicAdd(dst + s, (double)acc[s]);
-                        atomicAdd(my_scnt + 2 * key, np);
+                            if (!SSPL || s < na) row[s] = acc[s];
+                        *reinterpret_cast<uint2*>(row + NA) = make_uint2(np, nr2);
+                        *reinterpret_cast<int*>(row + NA + 1) = slot * nb + cur;
                     }
-                    atomicAdd(my_scnt + 2 * key + 1, nr2);
+                    __syncwarp();
+                    int pk = -1;
+                    double d[VPL];
+                    uint2 dc = make_uint2(0u, 0u);
+                    auto put = [&]() {
+#pragma unroll
+                        for (int v = 0; v < VPL; ++v) {
+                            const int s = lane + 32 * v;
+                            if (s < na) {
+                                double* dst = my_sacc + pk * (NS + 1) + gofs + s;
+                                if constexpr (PRIV) *dst = d[v];
+                                else atomicAdd(dst, d[v]);
+                            }
+                        }
+                        if (lane == 31 && part == 0) {
+                            unsigned* dst = my_scnt + 2 * pk;
+                            if constexpr (PRIV) {
+                                dst[0] = dc.x;
+                                dst[1] = dc.y;
+                            } else {
+                                atomicAdd(dst, dc.x);
+                                atomicAdd(dst + 1, dc.y);
+                            }
+                        }
+                    };
+                    for (int rr = 0; rr < rows; ++rr) {
+                        const double* row = my_fst + rr * C::FROW;
+                        const int kk = *reinterpret_cast<const int*>(row + NA + 1);
+                        if (kk != pk) {
+                            if (pk >= 0) put();
+                            pk = kk;
+#pragma unroll
+                            for (int v = 0; v < VPL; ++v) {
+                                const int s = lane + 32 * v;
+                                d[v] = PRIV && s < na ? my_sacc[kk * (NS + 1) + gofs + s] : 0.0;
+                            }
+                            if (lane == 31) dc = PRIV ? make_uint2(my_scnt[2 * kk], my_scnt[2 * kk + 1]) : make_uint2(0u, 0u);
+                        }
+#pragma unroll
+                        for (int v = 0; v < VPL; ++v) {
+                            const int s = lane + 32 * v;
+                            if (s < na) d[v] += row[s];
+                        }
+                        if (lane == 31) {
+                            const uint2 c = *reinterpret_cast<const uint2*>(row + NA);
+                            dc.x += c.x;
+                            dc.y += c.y;
+                        }
+                    }
+                    if (pk >= 0) put();
+                    __syncwarp();
                 }
+                }
+            };
+            // One TMEM read per step, indexed with constants only so the counts stay in
+            // registers.  (Issuing the next step's read before this step's estimators, so that
+            // it lands under them, measured slower: the raw counts held across the estimators
+            // cost the scheduler registers -- 200 windows x 3 populations 35.0 -> 37.4 ms, two
+            // populations spilled.)
+            constexpr int CREGS = (C::NJ + 31) / 32;  // partner coordinates per lane
+            uint32_t v[P][C::REGIONS][4];
+            auto issue = [&](uint32_t buf, int qq) {
+#pragma unroll
+                for (int p = 0; p < P; ++p)
+#pragma unroll
+                    for (int x = 0; x < C::REGIONS; ++x) {
+                        const uint32_t ta = tbase + buf * C::COLS + (p * C::REGIONS + x) * C::N + qq * (C::QROWS ? 8 : 4);
+                        if constexpr (C::QROWS) tmem_ld_q(ta, v[p][x]);
+                        else tmem_ld4(ta, v[p][x]);
+                    }
             };
             bool ok = true;
             for (int t = tb; t < te; ++t, ++tcount) {
@@ -618,20 +784,10 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 }
                 if (!mbar_wait(&tfull[buf], tph, &abort_s, a.status)) { ok = false; break; }
                 tc_fence_after();
-                // One TMEM read per step, indexed with constants only so the counts stay in
-                // registers.  Haplotypes: two partners per step, 4 columns per population.
-                // Genotypes: one partner per step, 4 columns per region and population.
 #pragma unroll 1
-                for (int qq = 0; qq < MY_STEPS; ++qq) {
-                    const int q = SSPL ? qq : part * MY_STEPS + qq;
-                    uint32_t v[P][C::REGIONS][4];
-#pragma unroll
-                    for (int p = 0; p < P; ++p)
-#pragma unroll
-                        for (int x = 0; x < C::REGIONS; ++x)
-                            tmem_ld4(tmem + lane_base + buf * C::COLS + (p * C::REGIONS + x) * C::N + q * 4,
-                                     v[p][x]);
-                    const int jj = GENO ? q : 2 * q + role;
+                for (int qq = 0; qq < C::MY_STEPS; ++qq) {
+                    issue(buf, qq);
+                    const int jj = jb + JSTRIDE * qq, j = j0 + jj;
                     double csrc = creg[0];
 #pragma unroll
                     for (int kk = 1; kk < CREGS; ++kk)
@@ -639,40 +795,11 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     const double cj = __shfl_sync(0xffffffffu, csrc, jj & 31);
 #pragma unroll
                     for (int p = 0; p < P; ++p) tmem_wait4<C::REGIONS>(v[p]);
-                    if (qq == MY_STEPS - 1) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&tempty[buf]);
-                    }
-                    const int j = j0 + jj;
-                    const bool valid = row_ok && j > i && j < my_jmax;
-                    const double dist = fabs(cj - ci);
-                    const bool change = valid && dist >= nxt;
-                    const bool want = change && cur >= 0 && np > 0;
-                    if (__ballot_sync(0xffffffffu, want)) flush(want);
-                    if (change) {
-                        cur = bin_advance(sedges, nb, cur, dist);
-                        nxt = cur < nb ? sedges[cur + 1] : CUDART_INF;
-#pragma unroll
-                        for (int s = 0; s < NA; ++s) acc[s] = T(0);
-                        np = nr2 = 0;
-                    }
                     SpinPop f[P];
                     int nval[P];
 #pragma unroll
                     for (int p = 0; p < P; ++p) {
-                        if constexpr (!GENO) {
-                            // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
-                            const uint32_t* w = v[p][0];
-                            const uint32_t sx = role ? w[0] : w[2];
-                            const uint32_t sy = role ? w[1] : w[3];
-                            const uint32_t rx = __shfl_xor_sync(0xffffffffu, sx, 1);
-                            const uint32_t ry = __shfl_xor_sync(0xffffffffu, sy, 1);
-                            f[p].R = i2d_exact((int)(role ? rx : w[0]));
-                            f[p].S = i2d_exact((int)(role ? ry : w[1]));
-                            f[p].T = i2d_exact((int)(role ? w[2] : rx));
-                            nval[p] = (int)(role ? w[3] : ry);
-                        } else {
+                        if constexpr (GENO) {
                             // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma,
                             // 1: sigma^2, 2: valid)
                             const uint32_t (&G)[3][4] = v[p];
@@ -685,9 +812,43 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                             f[p].T = i2d_exact((int)G[2][0]);
                             f[p].TT = i2d_exact((int)G[2][1]);
                             nval[p] = (int)G[2][2];
+                        } else if constexpr (C::QROWS) {
+                            f[p].R = i2d_exact((int)v[p][0][0]);
+                            f[p].S = i2d_exact((int)v[p][0][1]);
+                            f[p].T = i2d_exact((int)v[p][0][2]);
+                            nval[p] = (int)v[p][0][3];
+                        } else {
+                            // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
+                            const uint32_t* w = v[p][0];
+                            const uint32_t rx = __shfl_xor_sync(0xffffffffu, role ? w[0] : w[2], 1);
+                            const uint32_t ry = __shfl_xor_sync(0xffffffffu, role ? w[1] : w[3], 1);
+                            f[p].R = i2d_exact((int)(role ? rx : w[0]));
+                            f[p].S = i2d_exact((int)(role ? ry : w[1]));
+                            f[p].T = i2d_exact((int)(role ? w[2] : rx));
+                            nval[p] = (int)(role ? w[3] : ry);
                         }
                     }
-                    if (valid && cur >= 0 && cur < nb) {
+                    if (qq == C::MY_STEPS - 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&tempty[buf]);
+                    }
+                    const bool valid = (unsigned)(j - i - 1) < span;
+                    const double dist = fabs(cj - ci);
+                    const bool change = valid && dist >= nxt;
+                    if (__ballot_sync(0xffffffffu, change)) {
+                        const bool want = change && in_bin && np > 0;
+                        if (__ballot_sync(0xffffffffu, want)) flush(want);
+                        if (change) {
+                            cur = bin_advance(sedges, nb, cur, dist);
+                            nxt = cur < nb ? sedges[cur + 1] : CUDART_INF;
+                            in_bin = (unsigned)cur < (unsigned)nb;
+#pragma unroll
+                            for (int s = 0; s < NA; ++s) acc[s] = 0.0;
+                            np = nr2 = 0;
+                        }
+                    }
+                    if (valid && in_bin) {
 #pragma unroll
                         for (int p = 0; p < P; ++p) {
                             f[p].n = i2d_exact(nval[p]);
@@ -705,7 +866,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     }
                 }
             }
-            flush(cur >= 0 && cur < nb && np > 0);
+            flush(in_bin && np > 0);
             (void)ok;
             // staging -> global, once per work item
             epi_bar<EPI>();
@@ -713,7 +874,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             for (int idx = et; idx < stage_n; idx += 32 * EPI) {
                 double val = 0.0;
 #pragma unroll
-                for (int w = 0; w < (PRIV ? EPI : 1); ++w) {
+                for (int w = 0; w < NCOPY; ++w) {
                     val += sacc[w * stage_n + idx];
                     sacc[w * stage_n + idx] = 0.0;
                 }
@@ -722,13 +883,13 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 const int bb = rem / (NS + 1), s = rem % (NS + 1);
                 const int blk = blk0 + sl;
                 if (val != 0.0 && blk < a.n_blocks)
-                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + s) * kFxLimbs, val * spin_weight<P, GENO>(s),
+                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + spin_stat<P, GENO>(s)) * kFxLimbs, val * spin_weight<P, GENO>(s),
                            a.status);
             }
             for (int idx = et; idx < SLOTS * nb; idx += 32 * EPI) {
                 unsigned long long c0 = 0, c1 = 0;
 #pragma unroll
-                for (int w = 0; w < (PRIV ? EPI : 1); ++w) {
+                for (int w = 0; w < NCOPY; ++w) {
                     unsigned* sc = scnt + w * SLOTS * nb * 2;
                     c0 += sc[2 * idx];
                     c1 += sc[2 * idx + 1];
@@ -770,27 +931,34 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // planes[snp][plane][k]: boxes of 128 k x plane_box planes x rows_box SNPs
+// (snp_first: 128 k x rows_box SNPs x plane_box planes, coordinates in that order)
 bool make_map(CUtensorMap* m, const uint8_t* planes, int64_t n_var, int ktot, int n_planes, int plane_box,
-              int rows_box) {
+              int rows_box, bool snp_first = false) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dims[3] = {(cuuint64_t)ktot, (cuuint64_t)n_planes, (cuuint64_t)n_var};
     cuuint64_t strides[2] = {(cuuint64_t)ktot, (cuuint64_t)ktot * n_planes};
     cuuint32_t box[3] = {(cuuint32_t)kKChunk, (cuuint32_t)plane_box, (cuuint32_t)rows_box};
     cuuint32_t estr[3] = {1, 1, 1};
+    if (snp_first) {
+        std::swap(dims[1], dims[2]);
+        std::swap(strides[0], strides[1]);
+        std::swap(box[1], box[2]);
+    }
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(planes), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
 
-// Dynamic shared memory: pipeline stages, `ncopy` staging copies and `table` reciprocal
-// table entries (32 B each).
+// Dynamic shared memory: pipeline stages, `ncopy` staging copies, `table` reciprocal
+// table entries (32 B each) and `frows` flush rows per epilogue warp.
 template <int P, bool GENO, int V = 0>
-size_t smem_bytes_t(int nb, int table, int ncopy) {
+size_t smem_bytes_t(int nb, int table, int ncopy, int frows = 0) {
     using C = Cfg<P, GENO, V>;
     return 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)ncopy * C::SLOTS * nb * (C::NS + 1) * sizeof(double) +
-           (size_t)((ncopy * C::SLOTS * nb * 2 + 7) & ~7) * sizeof(unsigned) + (size_t)table * sizeof(double4) + 32;
+           (size_t)((ncopy * C::SLOTS * nb * 2 + 7) & ~7) * sizeof(unsigned) + (size_t)table * sizeof(double4) + 32 +
+           (size_t)frows * C::EPI * C::FROW * sizeof(double);
 }
 
 // Reciprocal table entries held in shared memory (none on the genotype path, none when the
@@ -827,14 +995,14 @@ bool rtab_global_t(const ParseShape& sh) {
     return smem_bytes_t<P, false, 0>(nb, t, 1) > kMaxSmem;
 }
 
-template <int P, typename T, bool PRIV, bool GENO, int V, bool GT>
+template <int P, bool PRIV, bool GENO, int V, bool GT>
 cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
                                      const ParseShape& sh, int max_items, cudaStream_t s) {
     using C = Cfg<P, GENO, V>;
-    // A: the row block (haplotypes: both planes of 64 SNPs; genotypes: one plane of 128
-    // SNPs per box); B: every plane of NJ partners
+    // A: the row block (haplotypes: both planes of 64 SNPs, with QROWS of eight per box;
+    // genotypes: one plane of 128 SNPs per box); B: every plane of NJ partners
     CUtensorMap mA, mB;
-    if (!make_map(&mA, w.hv, d->n_var, sh.ktot, C::PLANES, GENO ? 1 : C::PLANES, C::ROWS) ||
+    if (!make_map(&mA, w.hv, d->n_var, sh.ktot, C::PLANES, GENO ? 1 : C::PLANES, C::QROWS ? 8 : C::ROWS, C::QROWS) ||
         !make_map(&mB, w.hv, d->n_var, sh.ktot, C::PLANES, C::PLANES, C::NJ))
         return cudaErrorInvalidValue;
     TcArgs a;
@@ -858,17 +1026,21 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     a.gtab = static_cast<const double4*>(w.gtab);
     // at least half of an SM's shared memory, so that one CTA (holding all 512 TMEM
     // columns) runs per SM
-    size_t smem = smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), PRIV ? C::EPI : 1);
+    const int ncopy = PRIV ? C::EPI : 1;
+    a.frows = C::FROWS_MAX;  // as many flush rows as fit beside what decides the staging
+    while (a.frows > 0 && smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows) > kMaxSmem)
+        a.frows >>= 1;
+    size_t smem = smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows);
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
-        cudaFuncSetAttribute(k_parse_tc<P, T, PRIV, GENO, V, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if constexpr (C::SPLIT) {
         // the register split adds up only at C::REG_LAUNCH registers per thread; any other
         // allocation would leave setmaxnreg.inc waiting, so such a build is not launched
         cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, k_parse_tc<P, T, PRIV, GENO, V, GT>);
+        e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT>);
         if (e != cudaSuccess) return e;
         if (fa.numRegs != C::REG_LAUNCH) return cudaErrorInvalidKernelImage;
     }
@@ -877,7 +1049,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (max_items == 0) return cudaSuccess;
     const int grid = max_items < sms ? max_items : sms;
-    k_parse_tc<P, T, PRIV, GENO, V, GT><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
+    k_parse_tc<P, PRIV, GENO, V, GT><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
     return cudaGetLastError();
 }
 
@@ -886,28 +1058,28 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
 // table in shared memory or (FP64 estimators, widest tile only) in the workspace.  Other
 // variants answer cudaErrorInvalidConfiguration for a workspace table, which the tile
 // autotuner reads as "does not fit this shape".
-template <int PP, bool GENO, int V, typename T>
+template <int PP, bool GENO, int V>
 cudaError_t launch_staged(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                           int max_items, cudaStream_t s) {
     const bool priv = private_staging<PP, GENO, V>(sh.n_bins, smem_table(sh));
     if (!GENO && sh.rtab_global) {
-        if constexpr (!GENO && V == 0 && std::is_same<T, double>::value)
-            return priv ? launch_parse_tc_p<PP, T, true, GENO, V, true>(d, o, w, sh, max_items, s)
-                        : launch_parse_tc_p<PP, T, false, GENO, V, true>(d, o, w, sh, max_items, s);
+        if constexpr (!GENO && V == 0)
+            return priv ? launch_parse_tc_p<PP, true, GENO, V, true>(d, o, w, sh, max_items, s)
+                        : launch_parse_tc_p<PP, false, GENO, V, true>(d, o, w, sh, max_items, s);
         else
             return cudaErrorInvalidConfiguration;
     }
-    return priv ? launch_parse_tc_p<PP, T, true, GENO, V, false>(d, o, w, sh, max_items, s)
-                : launch_parse_tc_p<PP, T, false, GENO, V, false>(d, o, w, sh, max_items, s);
+    return priv ? launch_parse_tc_p<PP, true, GENO, V, false>(d, o, w, sh, max_items, s)
+                : launch_parse_tc_p<PP, false, GENO, V, false>(d, o, w, sh, max_items, s);
 }
 
-// One tile variant of one path, over the population count, accumulator type and staging.
-template <bool GENO, int V, typename T>
+// One tile variant of one path, over the population count and staging.
+template <bool GENO, int V>
 cudaError_t dispatch_tc(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                         int max_items, cudaStream_t s) {
 #define LDK_TC_CASE(PP)                                                                                   \
     case PP:                                                                                              \
-        return launch_staged<PP, GENO, V, T>(d, o, w, sh, max_items, s);
+        return launch_staged<PP, GENO, V>(d, o, w, sh, max_items, s);
     switch (sh.P) {
         LDK_TC_CASE(1)
         LDK_TC_CASE(2)
