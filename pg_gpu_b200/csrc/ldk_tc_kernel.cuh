@@ -66,6 +66,7 @@ constexpr uint64_t kTimeoutNs = 5000000000ull;  // 5 s per wait
 constexpr int kRegCtrl = 24;
 constexpr size_t kMinSmem = 116 * 1024;
 constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kStaticSmem = 1536;  // at most: the kernel's __shared__ variables (barriers, bin edges)
 
 // Tile geometry.  Haplotype path: a row block of 64 SNPs x {sigma, v} = 128 MMA rows against
 // NJ partners x {sigma, v} (N = 2 NJ), one MMA per K step and population.  Genotype path: a row
@@ -1028,7 +1029,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     // columns) runs per SM
     const int ncopy = PRIV ? C::EPI : 1;
     a.frows = C::FROWS_MAX;  // as many flush rows as fit beside what decides the staging
-    while (a.frows > 0 && smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows) > kMaxSmem)
+    while (a.frows > 0 && smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows) + kStaticSmem > kMaxSmem)
         a.frows >>= 1;
     size_t smem = smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows);
     if (smem < kMinSmem) smem = kMinSmem;

@@ -1,5 +1,5 @@
 """The bin flush of the tensor-core parse at the edges of its shared-memory room: three
-populations and twenty bins leave eight, two, one or no scratch rows per epilogue warp,
+populations and twenty bins leave eight, one or no scratch rows per epilogue warp,
 depending on the largest population (its reciprocal table), and many bins share one staging
 copy (atomics).  Bootstrap blocks change inside row blocks, so lanes of one warp flush
 different (block, bin) sums in the same step.  Pair tallies exact; per-bin sums within the
