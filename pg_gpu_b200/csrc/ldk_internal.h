@@ -95,7 +95,9 @@ constexpr int kMinItemTiles = 4;
 constexpr int kFlushValuesPerTile = 64;
 inline int tc_item_capacity(int n_row_blocks) { return n_row_blocks + kItemTarget; }
 int tc_min_item_tiles(const ParseShape& sh);
-cudaError_t launch_split_items(const Scratch& w, int n_row_blocks, int nj, int min_tiles, cudaStream_t s);
+// w.row_blocks null: row blocks of `rows` SNPs of one window [0, end).
+cudaError_t launch_split_items(const Scratch& w, int n_row_blocks, int nj, int min_tiles, int rows, int end,
+                               cudaStream_t s);
 
 // all-pairs LD of one SNP set (ldk_ldm.cu)
 size_t ld_matrix_workspace(int64_t n_var, int32_t n_sel);

@@ -1,16 +1,18 @@
 // All-pairs LD of one SNP set on the tensor-core count pipeline: pairwise r^2, the
-// unbiased sigma_D^2 and r^2 from jointly valid counts for every pair i < j, written as a
-// full symmetric matrix and/or reduced to the sum and count behind ZnS.
+// unbiased sigma_D^2, r^2 from jointly valid counts, dosage r^2 and Rogers-Huff r for every
+// pair i < j, written as a full symmetric matrix and/or reduced to the sum and count behind
+// ZnS.
 //
-// The Gram counts come from the same TMA + tcgen05 pipeline as the binned parse (64-SNP
+// The Gram moments come from the same TMA + tcgen05 pipeline as the binned parse (64-SNP
 // row blocks against 128-SNP partner tiles, no distance cutoff, so every partner j > i of
-// the set).  Four epilogue warps share each TMEM lane quarter (16 SNPs), one per quarter
-// of the partner tile; each evaluates its 16 rows x 32 partners into a padded
-// shared-memory tile and then writes the tile's rows (upper triangle, 256-byte runs) and
-// columns (lower triangle, 128-byte runs) with coalesced stores.
+// the set; work items of a few tiles, claimed dynamically, because the row blocks shrink
+// along the triangle: whole row blocks left 148 SMs waiting for the longest).  Sixteen
+// epilogue warps each take eight SNPs x 64 partners of a tile; a thread holds one SNP and
+// every fourth partner and stores its value to the upper and the lower triangle straight
+// from registers (32-byte and 64-byte runs).  Everything that depends on one SNP alone
+// (frequency, reciprocal variance) is tabulated first, so a pair costs no division.
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "ldk_tc_kernel.cuh"
 #include "ldk_spin.cuh"
@@ -21,40 +23,76 @@ namespace {
 
 using LdmCfg = Cfg<1, false, 0>;
 constexpr int kLdmEpi = 16;                    // epilogue warps: four per TMEM lane quarter
-constexpr int kLdmParts = kLdmEpi / 4;         // partner ranges a tile is split into
-constexpr int kLdmHalf = LdmCfg::NJ / kLdmParts;  // partners per epilogue warp and tile
-constexpr int kLdmStride = kLdmHalf + 1;       // staging row stride (doubles): rows hit distinct banks
+constexpr int kLdmPart = LdmCfg::NJ / 2;       // partners per epilogue warp and tile
+constexpr int kLdmGroup = 4;                   // steps (four partners each) in flight together
+constexpr int kLdmTable = 8192;                // most entries of the 1/n table in shared memory
 
 struct LdmArgs {
-    const double* psite;  // per SNP: derived allele frequency over the site's valid haplotypes
+    const double2* site;  // per SNP, by estimator (k_site)
     double* out;          // (n_var rows, stride ld_out) or null
     int64_t ld_out;
     double* sums;         // [sum over pairs i < j, pairs counted] or null
 };
 
-__global__ void k_fill_int(int32_t* p, int64_t n, int32_t v) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-        p[t] = v;
-}
-
-__global__ void k_fill_diag(double* out, int64_t ld, int64_t n, double v) {
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
-        out[t * ld + t] = v;
-}
-
-// p_i = (sum of derived calls) / (valid calls), 0 for a site without valid calls
-// (haplotype_matrix.py:1119-1120), over the selected rows.
-__global__ void k_site_freq(const int8_t* __restrict__ X, int64_t ld, int64_t n_var, const int32_t* __restrict__ rows,
-                            int n_rows, double* __restrict__ p) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_var; v += (int64_t)gridDim.x * blockDim.x) {
-        int dac = 0, nv = 0;
-        for (int k = 0; k < n_rows; ++k) {
-            const int8_t x = X[(int64_t)rows[k] * ld + v];
-            dac += x > 0 ? x : 0;
-            nv += x >= 0;
+// Per SNP over the selected rows, into site[v]:
+//   LDK_LDM_R2              {p, 1 / (p (1 - p))}, p = derived / valid calls (haplotype_matrix.py:1119-1120)
+//   LDK_LDM_DIPLOID_R2      {m, 1 / V}, m the mean spin (1 - dosage) of the valid calls, V their sum
+//   LDK_LDM_ROGERS_HUFF_R   {m, 1 / sqrt(V)}        of squared deviations (ld_statistics.py:1000-1011)
+// with 0 for the reciprocal of 0; and the partner range (the rest of the set) and the matrix
+// diagonal.  With `strict` a missing call sets LDK_DEVERR_BAD_INPUT (the Rogers-Huff and
+// sigma_D^2 genotype estimators take complete data, ld_statistics.py:389-399).
+// A block takes 128 SNPs, its eight warps every eighth row: 200 rows x 12,000 SNPs in one pass
+// of a few loads in flight per thread instead of 200 dependent-latency rows per thread.
+constexpr int kSiteWarps = 8;
+__global__ void __launch_bounds__(32 * kSiteWarps)
+    k_site(const int8_t* __restrict__ X, int64_t ld, int64_t n_var, const int32_t* __restrict__ rows, int n_rows,
+           int estimator, double2* __restrict__ site, int32_t* __restrict__ jmax, double* __restrict__ out,
+           int64_t ld_out, double diag, unsigned* status) {
+    __shared__ int part[kSiteWarps][128][3];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t v0 = (int64_t)blockIdx.x * 128;
+    int nv[4] = {}, n1[4] = {}, n2[4] = {};
+#pragma unroll 4
+    for (int k = warp; k < n_rows; k += kSiteWarps) {
+        const int8_t* row = X + (int64_t)rows[k] * ld + v0;
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int c = v0 + lane + 32 * m < n_var ? row[lane + 32 * m] : -1;
+            nv[m] += c >= 0;
+            n1[m] += c == 1;
+            n2[m] += c == 2;
         }
-        p[v] = nv > 0 ? (double)dac / (double)nv : 0.0;
     }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        part[warp][lane + 32 * m][0] = nv[m];
+        part[warp][lane + 32 * m][1] = n1[m];
+        part[warp][lane + 32 * m][2] = n2[m];
+    }
+    __syncthreads();
+    const int64_t v = v0 + threadIdx.x;
+    if (threadIdx.x >= 128 || v >= n_var) return;
+    int c[3] = {0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < kSiteWarps; ++w)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) c[q] += part[w][threadIdx.x][q];
+    jmax[v] = (int32_t)n_var;
+    if (out) out[v * ld_out + v] = diag;
+    double2 r = make_double2(0.0, 0.0);
+    if (estimator == LDK_LDM_R2) {
+        r.x = c[0] > 0 ? (double)c[1] / (double)c[0] : 0.0;
+        const double pq = r.x * (1.0 - r.x);
+        r.y = pq > 0.0 ? 1.0 / pq : 0.0;
+    } else if (estimator >= LDK_LDM_DIPLOID_R2) {
+        if (estimator != LDK_LDM_DIPLOID_R2 && c[0] < n_rows) atomicOr(status, LDK_DEVERR_BAD_INPUT);
+        // spins: 1 for dosage 0, 0 for 1, -1 for 2; V = (n sum s^2 - (sum s)^2) / n, exact numerator
+        const double n = c[0], S = (double)(c[0] - c[1] - 2 * c[2]), SS = (double)(c[0] - c[1]);
+        const double V = c[0] > 0 ? fma(n, SS, -(S * S)) / n : 0.0;
+        r.x = c[0] > 0 ? S / n : 0.0;
+        if (V > 0.0) r.y = estimator == LDK_LDM_DIPLOID_R2 ? 1.0 / V : 1.0 / sqrt(V);
+    }
+    site[v] = r;
 }
 
 template <int EST>
@@ -62,11 +100,12 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     k_ld_matrix(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                 const LdmArgs m) {
     using C = LdmCfg;
-    constexpr int NJ = C::NJ, SP = kLdmStride;
+    constexpr int NJ = C::NJ;
+    constexpr bool SITE = EST == LDK_LDM_R2 || EST >= LDK_LDM_DIPLOID_R2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* stages = base;
-    double* stile = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // [kLdmEpi][16][SP]
+    double* rn = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // EST R2: 1 / n
 
     __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
@@ -91,6 +130,9 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    const bool table = EST == LDK_LDM_R2 && a.max_n < kLdmTable;
+    if (table)
+        for (int n = threadIdx.x; n <= a.max_n; n += blockDim.x) rn[n] = n > 0 ? 1.0 / (double)n : 0.0;
     if (warp == 1) {
         tmem_alloc(&tmem_base_s, kTmemCols);
         tmem_relinquish();
@@ -100,16 +142,15 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
-    if (warp == 0) run_producer<C, false>(pipe, &tmA, &tmB, a, lane);
+    if (warp == 0) run_producer<C, true>(pipe, &tmA, &tmB, a, lane);
     else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
     if (warp >= 4) {
-        // lanes 2r, 2r+1 share SNP r (16 per warp) and split its partners by parity; the
-        // warp takes part `half` (of kLdmParts) of every partner tile
-        const int e = warp - 4, quarter = warp & 3, half = e >> 2;
-        const int rr = lane >> 1, role = lane & 1;
-        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        double* st = stile + e * 16 * SP;
-        double zsum = 0.0, zcnt = 0.0;
+        // thread: SNP `r` of the row block, partners jb + 4 step of the tile
+        const int e = warp - 4, quarter = warp & 3, half = (e >> 2) & 1, share = e >> 3;
+        const int r = quarter * 16 + half * 8 + (lane >> 2), jb = share * kLdmPart + (lane & 3);
+        const uint32_t tbase = tmem + ((uint32_t)(quarter * 32 + half * 16) << 16) + (uint32_t)share * (2 * kLdmPart);
+        double zsum = 0.0;
+        unsigned long long zcnt = 0;
         uint32_t tcount = 0;
         for (uint32_t k = 0;; ++k) {
             const int sl = k % kRing;
@@ -126,112 +167,108 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
             const int n_jt = item_tiles<C>(a, item, row0, row1, jt0);
             if (n_jt == 0) continue;
             const int jend = a.jmax[row1 - 1];
-            const int i = row0 + quarter * 16 + rr;
+            const int i = row0 + r;
             const bool row_ok = i < row1;
-            const double pi = (EST == 0 && row_ok) ? m.psite[i] : 0.0;
+            double2 si = make_double2(0.0, 0.0);
+            if (SITE && row_ok) si = m.site[i];
             bool ok = true;
             for (int t = 0; t < n_jt; ++t, ++tcount) {
                 const uint32_t buf = tcount % C::NBUF, tph = (tcount / C::NBUF) & 1u;
                 const int j0 = jt0 + t * NJ;
-                double preg[(kLdmHalf + 31) / 32];
-#pragma unroll
-                for (int kk = 0; kk < (kLdmHalf + 31) / 32; ++kk) {
-                    const int j = j0 + half * kLdmHalf + 32 * kk + lane;
-                    preg[kk] = (EST == 0 && j < jend) ? m.psite[j] : 0.0;
-                }
+                // a tile off the diagonal, inside the matrix and of a whole row block needs no bounds
+                const bool whole = row1 - row0 == C::ROWS && j0 >= row1 && j0 + NJ <= jend;
                 if (!mbar_wait(&tfull[buf], tph, &abort_s, a.status)) { ok = false; break; }
                 tc_fence_after();
+                int j = j0 + jb;
+                double* up = m.out ? m.out + (int64_t)i * m.ld_out + j : nullptr;
+                double* lo = m.out ? m.out + (int64_t)j * m.ld_out + i : nullptr;
+                unsigned cnt = 0;
 #pragma unroll 1
-                for (int qh = 0; qh < kLdmHalf / 2; ++qh) {
-                    const int q = half * (kLdmHalf / 2) + qh;
-                    uint32_t v[1][4];
-                    tmem_ld4(tmem + lane_base + buf * C::COLS + q * 4, v[0]);
-                    const int jl = 2 * qh + role;  // partner within this warp's half tile
-                    const int jj = half * kLdmHalf + jl;
-                    double psrc = preg[0];
+                for (int q = 0; q < kLdmPart / 4; q += kLdmGroup) {
+                    uint32_t v[kLdmGroup][4];
+                    double2 sj[kLdmGroup];
 #pragma unroll
-                    for (int kk = 1; kk < (kLdmHalf + 31) / 32; ++kk)
-                        if ((jl >> 5) == kk) psrc = preg[kk];
-                    const double pj = __shfl_sync(0xffffffffu, psrc, jl & 31);
-                    tmem_wait4<1>(v);
-                    if (qh == kLdmHalf / 2 - 1) {
+                    for (int g = 0; g < kLdmGroup; ++g) tmem_ld_q(tbase + buf * C::COLS + (q + g) * 8, v[g]);
+                    if constexpr (SITE) {
+#pragma unroll
+                        for (int g = 0; g < kLdmGroup; ++g)
+                            sj[g] = whole || j + 4 * g < jend ? __ldg(m.site + j + 4 * g) : make_double2(0.0, 0.0);
+                    }
+                    tmem_wait4<kLdmGroup>(v);
+                    if (q == kLdmPart / 4 - kLdmGroup) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&tempty[buf]);
                     }
-                    // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
-                    const uint32_t sx = role ? v[0][0] : v[0][2];
-                    const uint32_t sy = role ? v[0][1] : v[0][3];
-                    const uint32_t rx = __shfl_xor_sync(0xffffffffu, sx, 1);
-                    const uint32_t ry = __shfl_xor_sync(0xffffffffu, sy, 1);
-                    const int iR = (int)(role ? rx : v[0][0]), iS = (int)(role ? ry : v[0][1]);
-                    const int iT = (int)(role ? v[0][2] : rx), in = (int)(role ? v[0][3] : ry);
-                    const int j = j0 + jj;
-                    const bool valid = row_ok && j > i && j < jend;
-                    double val = 0.0;
-                    if (valid) {
-                        const double n = i2d_exact(in);
-                        if constexpr (EST == 0) {
+#pragma unroll
+                    for (int g = 0; g < kLdmGroup; ++g, j += 4) {
+                        const int iR = (int)v[g][0], iS = (int)v[g][1], iT = (int)v[g][2], in = (int)v[g][3];
+                        double val;
+                        bool counted = true;  // enters the sum and count
+                        if constexpr (EST == LDK_LDM_R2) {
                             // haplotype_matrix.py:1122-1128, 1171-1175; n11 = (n - S - T + R) / 4
                             const double c1 = i2d_exact((in - iS - iT + iR) >> 2);
-                            const double pab = n > 0.0 ? c1 * recip_cubic(n) : 0.0;
-                            const double D = pab - pi * pj;
-                            const double den = (pi * (1.0 - pi)) * (pj * (1.0 - pj));
-                            val = den > 0.0 ? (D * D) * recip_cubic(den) : 0.0;
-                            zsum += val;
-                            zcnt += 1.0;
+                            const double r1 = table ? rn[in] : (in > 0 ? recip_cubic(i2d_exact(in)) : 0.0);
+                            const double D = fma(c1, r1, -(si.x * sj[g].x));
+                            val = (D * D) * (si.y * sj[g].y);
+                        } else if constexpr (EST == LDK_LDM_DIPLOID_R2) {
+                            // covariance of the centred spins of the jointly called individuals
+                            // (centred dosages with the other sign, ld_statistics.py:1000-1018)
+                            const double S = i2d_exact(iS), T = i2d_exact(iT), R = i2d_exact(iR), n = i2d_exact(in);
+                            const double cov = fma(-sj[g].x, fma(-si.x, n, S), fma(-si.x, T, R));
+                            val = (cov * cov) * (si.y * sj[g].y);
+                        } else if constexpr (EST == LDK_LDM_ROGERS_HUFF_R) {
+                            // ld_statistics.py:392-437 (complete data); NaN where a site is constant
+                            const double cov = fma(-(si.x * sj[g].x), i2d_exact(in), i2d_exact(iR));
+                            const double s = si.y * sj[g].y;
+                            counted = s > 0.0;
+                            val = counted ? cov * s : CUDART_NAN;
                         } else {
-                            const double S = i2d_exact(iS), T = i2d_exact(iT), R = i2d_exact(iR);
-                            if constexpr (EST == 1) {
+                            const double n = i2d_exact(in), S = i2d_exact(iS), T = i2d_exact(iT), R = i2d_exact(iR);
+                            if constexpr (EST == LDK_LDM_SIGMA_D2) {
                                 // ld_statistics.py:326-343: the DD and pi2 numerators (exact
                                 // integers in FP64), 16 times each
                                 double dd, pi2;
                                 spin_hap_numerators(n, S, T, R, dd, pi2);
-                                const bool nok = n >= 4.0;
-                                val = (nok && pi2 != 0.0) ? dd * recip_cubic(pi2) : 0.0;
-                                zsum += val;
-                                zcnt += nok ? 1.0 : 0.0;
+                                counted = in >= 4;
+                                val = (counted && pi2 != 0.0) ? dd * recip_cubic(pi2) : 0.0;
                             } else {
                                 // haplotype_kernels.py:32-42: NaN where pA qA pB qB = 0
                                 const double E = fma(n, R, -(S * T));
                                 const double den = fma(n, n, -(S * S)) * fma(n, n, -(T * T));
-                                if (den > 0.0) {
-                                    val = (E * E) * recip_cubic(den);
-                                    zsum += val;
-                                    zcnt += 1.0;
-                                } else {
-                                    val = CUDART_NAN;
-                                }
+                                counted = den > 0.0;
+                                val = counted ? (E * E) * recip_cubic(den) : CUDART_NAN;
                             }
                         }
+                        const bool valid = whole || (row_ok && j > i && j < jend);
+                        if (m.sums && valid && counted) {
+                            zsum += EST == LDK_LDM_ROGERS_HUFF_R ? val * val : val;
+                            ++cnt;
+                        }
+                        if (m.out) {
+                            if (valid) {
+                                *up = val;
+                                *lo = val;
+                            }
+                            up += 4;
+                            lo += 4 * m.ld_out;
+                        }
                     }
-                    st[rr * SP + jl] = val;
                 }
-                __syncwarp();
-                if (m.out) {
-                    const int gi0 = row0 + quarter * 16, gj0 = j0 + half * kLdmHalf;
-                    for (int idx = lane; idx < 16 * kLdmHalf; idx += 32) {  // rows: upper triangle
-                        const int r = idx / kLdmHalf, c = idx % kLdmHalf, gi = gi0 + r, gj = gj0 + c;
-                        if (gi < row1 && gj > gi && gj < jend) m.out[(int64_t)gi * m.ld_out + gj] = st[r * SP + c];
-                    }
-                    for (int idx = lane; idx < 16 * kLdmHalf; idx += 32) {  // columns: lower triangle
-                        const int r = idx % 16, c = idx / 16, gi = gi0 + r, gj = gj0 + c;
-                        if (gi < row1 && gj > gi && gj < jend) m.out[(int64_t)gj * m.ld_out + gi] = st[r * SP + c];
-                    }
-                }
-                __syncwarp();
+                zcnt += cnt;
             }
             (void)ok;
         }
         if (m.sums) {
+            double zc = (double)zcnt;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 zsum += __shfl_xor_sync(0xffffffffu, zsum, o);
-                zcnt += __shfl_xor_sync(0xffffffffu, zcnt, o);
+                zc += __shfl_xor_sync(0xffffffffu, zc, o);
             }
             if (lane == 0) {
                 atomicAdd(&m.sums[0], zsum);
-                atomicAdd(&m.sums[1], zcnt);
+                atomicAdd(&m.sums[1], zc);
             }
         }
     }
@@ -244,7 +281,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
 }
 
 
-// ---- genotype path: dosage r^2, Rogers-Huff r, sigma_D^2 of genotype pairs ----------------
+// ---- sigma_D^2 of genotype pairs: nine moments per pair ----------------------------------
 
 using LdmGCfg = Cfg<1, true, 0>;               // 128-SNP row blocks, 16-partner tiles
 constexpr int kLdmGEpi = 8;                    // two epilogue warps per TMEM lane quarter
@@ -252,39 +289,11 @@ constexpr int kLdmGPart = LdmGCfg::NJ / 2;     // partners per epilogue warp and
 constexpr int kLdmGStride = kLdmGPart + 1;
 
 struct LdmGArgs {
-    const double* mu;   // per SNP: mean dosage over the site's valid individuals
-    const double* var;  // per SNP: sum of squared deviations from it over those individuals
     double* out;
     int64_t ld_out;
     double* sums;
-    double n_ind;       // individuals (Rogers-Huff r: all valid)
 };
 
-// mu and the sum of squared deviations per SNP over the selected rows (ld_statistics.py:
-// 1000-1011); with `strict` a missing call sets LDK_DEVERR_BAD_INPUT (the Rogers-Huff and
-// sigma_D^2 genotype estimators take complete data, ld_statistics.py:389-399).
-__global__ void k_site_moments(const int8_t* __restrict__ X, int64_t ld, int64_t n_var, const int32_t* __restrict__ rows,
-                               int n_rows, int strict, double* __restrict__ mu, double* __restrict__ var,
-                               unsigned* status) {
-    for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n_var; v += (int64_t)gridDim.x * blockDim.x) {
-        int sum = 0, nv = 0;
-        for (int k = 0; k < n_rows; ++k) {
-            const int8_t x = X[(int64_t)rows[k] * ld + v];
-            if (x >= 0) { sum += x; ++nv; }
-        }
-        if (strict && nv < n_rows) atomicOr(status, LDK_DEVERR_BAD_INPUT);
-        const double m = nv > 0 ? (double)sum / (double)nv : 0.0;
-        double ss = 0.0;
-        for (int k = 0; k < n_rows; ++k) {
-            const int8_t x = X[(int64_t)rows[k] * ld + v];
-            if (x >= 0) ss += ((double)x - m) * ((double)x - m);
-        }
-        mu[v] = m;
-        var[v] = ss;
-    }
-}
-
-template <int EST>
 __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     k_ld_matrix_geno(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                      const LdmGArgs m) {
@@ -353,7 +362,6 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
             const int jend = a.jmax[row1 - 1];
             const int i = row0 + quarter * 32 + lane;
             const bool row_ok = i < row1;
-            const double mui = row_ok ? m.mu[i] : 0.0, vari = row_ok ? m.var[i] : 0.0;
             bool ok = true;
             for (int t = 0; t < n_jt; ++t, ++tcount) {
                 const uint32_t buf = tcount % C::NBUF, tph = (tcount / C::NBUF) & 1u;
@@ -367,7 +375,6 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
 #pragma unroll
                     for (int x = 0; x < 3; ++x) tmem_ld4(tmem + lane_base + buf * C::COLS + x * C::N + 4 * c, G[x]);
                     const int j = j0 + c;
-                    const double muj = j < jend ? m.mu[j] : 0.0, varj = j < jend ? m.var[j] : 0.0;
                     tmem_wait4<3>(G);
                     if (cl == kLdmGPart - 1) {
                         tc_fence_before();
@@ -378,41 +385,16 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
                     double val = 0.0;
                     if (valid) {
                         // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma = 1 - g,
-                        // 1: sigma^2, 2: valid)
-                        const int nv = (int)G[2][2], iS = (int)G[0][2], iT = (int)G[2][0], iR = (int)G[0][0];
-                        if constexpr (EST == 3 || EST == 4) {
-                            const double sxy = (double)(nv - iS - iT + iR);  // sum of dosage products
-                            if constexpr (EST == 3) {
-                                // centred dosages zeroed where missing (ld_statistics.py:1000-1018)
-                                const double sx = (double)(nv - iS), sy = (double)(nv - iT);
-                                const double cov = sxy - muj * sx - mui * sy + mui * muj * (double)nv;
-                                const double vv = vari * varj;
-                                val = vv > 0.0 ? (cov * cov) / vv : 0.0;
-                                zsum += val;
-                                zcnt += 1.0;
-                            } else {
-                                // ld_statistics.py:392-437
-                                const double cov = sxy - m.n_ind * mui * muj;
-                                const double den = sqrt(vari * varj);
-                                if (den > 0.0) {
-                                    val = cov / den;
-                                    zsum += val * val;
-                                    zcnt += 1.0;
-                                } else {
-                                    val = CUDART_NAN;
-                                }
-                            }
+                        // 1: sigma^2, 2: valid); DD over pi2 of one population
+                        // (genotype_kernels.py:91-170)
+                        double dd, pi2;
+                        spin_geno_numerators(G, dd, pi2);
+                        if ((int)G[2][2] >= 4 && pi2 > 0.0) {
+                            val = 4.0 * dd * recip_cubic(pi2);
+                            zsum += val;
+                            zcnt += 1.0;
                         } else {
-                            // DD over pi2 of one population (genotype_kernels.py:91-170)
-                            double dd, pi2;
-                            spin_geno_numerators(G, dd, pi2);
-                            if (nv >= 4 && pi2 > 0.0) {
-                                val = 4.0 * dd / pi2;
-                                zsum += val;
-                                zcnt += 1.0;
-                            } else {
-                                val = CUDART_NAN;
-                            }
+                            val = CUDART_NAN;
                         }
                     }
                     st[lane * SP + cl] = val;
@@ -454,116 +436,91 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
 }
 
 struct LdmLayout {
-    size_t status = 0, jmax = 0, items = 0, planes = 0, psite = 0, var = 0, total = 0;
-    int n_items = 0, ktot = 0;
+    size_t jmax = 0, items = 0, planes = 0, site = 0, total = 0;
+    int n_row_blocks = 0, rows = 0, ktot = 0;
 };
 
 LdmLayout ldm_layout(int64_t n_var, int32_t n_sel, bool geno) {
     LdmLayout L;
     L.ktot = (int)(((n_sel + 31) / 32 * 32 + 127) / 128 * 128);
-    const int rows = geno ? LdmGCfg::ROWS : LdmCfg::ROWS;
-    L.n_items = (int)((n_var + rows - 1) / rows);
+    L.rows = geno ? LdmGCfg::ROWS : LdmCfg::ROWS;
+    L.n_row_blocks = (int)((n_var + L.rows - 1) / L.rows);
     auto up = [](size_t x, size_t a) { return (x + a - 1) / a * a; };
     size_t off = 256;
     L.jmax = off;
     off = up(off + (size_t)n_var * 4, 256);
-    L.items = off;  // (row0, row1, 0, INT32_MAX): whole row blocks
-    off = up(off + (size_t)L.n_items * 16, 1024);
+    L.items = off;
+    off = up(off + (size_t)tc_item_capacity(L.n_row_blocks) * 16, 1024);
     L.planes = off;
     off = up(off + (size_t)n_var * (geno ? 4 : 2) * L.ktot, 256);
-    L.psite = off;
-    off = up(off + (size_t)n_var * 8, 256);
-    L.var = off;
-    off = up(off + (size_t)n_var * 8, 256);
+    L.site = off;
+    off = up(off + (size_t)n_var * sizeof(double2), 256);
     L.total = off;
     return L;
 }
 
-template <int EST>
+int sm_count() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 cudaError_t launch_ldm_geno(const CUtensorMap& mA, const CUtensorMap& mB, const TcArgs& a, const LdmGArgs& m,
-                            int n_items, cudaStream_t s) {
+                            cudaStream_t s) {
     using C = LdmGCfg;
     size_t smem = 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)kLdmGEpi * 32 * kLdmGStride * sizeof(double);
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix_geno<EST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix_geno, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = n_items < sms ? n_items : sms;
-    k_ld_matrix_geno<EST><<<grid, 128 + 32 * kLdmGEpi, smem, s>>>(mA, mB, a, m);
+    k_ld_matrix_geno<<<sm_count(), 128 + 32 * kLdmGEpi, smem, s>>>(mA, mB, a, m);
     return cudaGetLastError();
 }
 
 template <int EST>
-cudaError_t launch_ldm(const CUtensorMap& mA, const CUtensorMap& mB, const TcArgs& a, const LdmArgs& m, int n_items,
-                       cudaStream_t s) {
+cudaError_t launch_ldm(const CUtensorMap& mA, const CUtensorMap& mB, const TcArgs& a, const LdmArgs& m, cudaStream_t s) {
     using C = LdmCfg;
-    size_t smem = 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)kLdmEpi * 16 * kLdmStride * sizeof(double);
+    size_t smem = 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (a.max_n < kLdmTable ? a.max_n + 1 : 0) * sizeof(double);
     if (smem < kMinSmem) smem = kMinSmem;
     cudaError_t e = cudaFuncSetAttribute(k_ld_matrix<EST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = n_items < sms ? n_items : sms;
-    k_ld_matrix<EST><<<grid, 128 + 32 * kLdmEpi, smem, s>>>(mA, mB, a, m);
+    k_ld_matrix<EST><<<sm_count(), 128 + 32 * kLdmEpi, smem, s>>>(mA, mB, a, m);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t ld_matrix_workspace(int64_t n_var, int32_t n_sel) { return ldm_layout(n_var, n_sel, true).total; }
+size_t ld_matrix_workspace(int64_t n_var, int32_t n_sel) {
+    return std::max(ldm_layout(n_var, n_sel, true).total, ldm_layout(n_var, n_sel, false).total);
+}
 
 // Enqueues the all-pairs LD of the n_sel selected rows of X (see ldk_ld_matrix).
 cudaError_t launch_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const int32_t* rows, int32_t n_sel,
                              int estimator, double* out, int64_t ld_out, double* sums, unsigned char* ws,
                              unsigned* status, cudaStream_t s) {
-    const bool geno = estimator >= 3;
-    const LdmLayout L = ldm_layout(n_var, n_sel, geno);
+    const bool dosage = estimator >= LDK_LDM_DIPLOID_R2;       // codes {-1, 0, 1, 2}
+    const bool nine = estimator == LDK_LDM_SIGMA_D2_GENO;      // the nine-moment kernel
+    const LdmLayout L = ldm_layout(n_var, n_sel, nine);
     cudaError_t e;
-    int32_t* jmax = reinterpret_cast<int32_t*>(ws + L.jmax);
-    int32_t* items = reinterpret_cast<int32_t*>(ws + L.items);
-    uint8_t* planes = ws + L.planes;
-    double* psite = reinterpret_cast<double*>(ws + L.psite);
-    double* svar = reinterpret_cast<double*>(ws + L.var);
     if (sums && (e = cudaMemsetAsync(sums, 0, 2 * sizeof(double), s)) != cudaSuccess) return e;
-    if (out && n_var > 0) {
-        const bool nan_diag = estimator == LDK_LDM_R2_COUNTS || estimator >= LDK_LDM_ROGERS_HUFF_R;
-        k_fill_diag<<<(unsigned)((n_var + 255) / 256), 256, 0, s>>>(out, ld_out, n_var, nan_diag ? std::nan("") : 0.0);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if (n_var < 2) return cudaSuccess;
-    // every SNP's partner range is the rest of the set
-    k_fill_int<<<(unsigned)((n_var + 255) / 256), 256, 0, s>>>(jmax, n_var, (int32_t)n_var);
+    if (n_var < 1) return cudaSuccess;
+    Scratch w{};
+    w.status = status;
+    w.jmax = reinterpret_cast<int32_t*>(ws + L.jmax);
+    w.items = reinterpret_cast<int32_t*>(ws + L.items);
+    w.n_items = reinterpret_cast<int*>(ws + 192);
+    w.item_counter = reinterpret_cast<int*>(ws + 128);
+    w.hv = ws + L.planes;
+    double2* site = reinterpret_cast<double2*>(ws + L.site);
+    const bool nan_diag = estimator == LDK_LDM_R2_COUNTS || estimator >= LDK_LDM_ROGERS_HUFF_R;
+    k_site<<<(unsigned)((n_var + 127) / 128), 32 * kSiteWarps, 0, s>>>(X, ld_x, n_var, rows, n_sel, estimator, site, w.jmax,
+                                                                    out, ld_out, nan_diag ? std::nan("") : 0.0, status);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int rows_per_block = geno ? LdmGCfg::ROWS : LdmCfg::ROWS;
-    std::vector<int32_t> it;
-    it.reserve((size_t)L.n_items * 4);
-    for (int64_t r0 = 0; r0 < n_var; r0 += rows_per_block) {  // most partners first
-        it.push_back((int32_t)r0);
-        it.push_back((int32_t)std::min<int64_t>(r0 + rows_per_block, n_var));
-        it.push_back(0);
-        it.push_back(INT32_MAX);
-    }
-    int* n_items = reinterpret_cast<int*>(ws + 192);
-    const int n_items_h = L.n_items;
-    if ((e = cudaMemcpyAsync(items, it.data(), it.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(n_items, &n_items_h, sizeof(int), cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return e;
-    if (estimator == LDK_LDM_R2) {
-        k_site_freq<<<(unsigned)((n_var + 255) / 256), 256, 0, s>>>(X, ld_x, n_var, rows, n_sel, psite);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    if (geno) {
-        k_site_moments<<<(unsigned)((n_var + 255) / 256), 256, 0, s>>>(
-            X, ld_x, n_var, rows, n_sel, estimator != LDK_LDM_DIPLOID_R2, psite, svar, status);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
+    if (n_var < 2) return cudaSuccess;
     // the spin planes of the selected rows, as for a one-population parse
     ldk_parse_t d{};
-    d.genotypes = geno ? 1 : 0;
+    d.genotypes = dosage ? 1 : 0;
     d.X = X;
     d.ld_x = ld_x;
     d.n_var = n_var;
@@ -573,42 +530,39 @@ cudaError_t launch_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const
     for (int p = 1; p <= LDK_MAX_POPS; ++p) d.pop_offsets[p] = n_sel;
     ParseShape sh{};
     sh.P = 1;
-    sh.genotypes = geno ? 1 : 0;
-    sh.planes = geno ? 4 : 2;
+    sh.genotypes = dosage ? 1 : 0;
+    sh.planes = nine ? 4 : 2;
     sh.ktot = L.ktot;
     for (int p = 0; p <= LDK_MAX_POPS; ++p) sh.kofs[p] = p == 0 ? 0 : (n_sel + 31) / 32 * 32;
     sh.max_n = n_sel;
-    Scratch w{};
-    w.status = status;
-    w.hv = planes;
     if ((e = launch_prep_planes(&d, w, sh, s)) != cudaSuccess) return e;
+    // items of one tile at least: unlike the parse's, they end without a flush
+    if ((e = launch_split_items(w, L.n_row_blocks, nine ? LdmGCfg::NJ : LdmCfg::NJ, 1, L.rows, (int)n_var, s)) !=
+        cudaSuccess)
+        return e;
     CUtensorMap mA, mB;
-    if (geno ? (!make_map(&mA, planes, n_var, L.ktot, 4, 1, LdmGCfg::ROWS) ||
-                !make_map(&mB, planes, n_var, L.ktot, 4, 4, LdmGCfg::NJ))
-             : (!make_map(&mA, planes, n_var, L.ktot, 2, 2, LdmCfg::ROWS) ||
-                !make_map(&mB, planes, n_var, L.ktot, 2, 2, LdmCfg::NJ)))
+    if (nine ? (!make_map(&mA, w.hv, n_var, L.ktot, 4, 1, LdmGCfg::ROWS) ||
+                !make_map(&mB, w.hv, n_var, L.ktot, 4, 4, LdmGCfg::NJ))
+             : (!make_map(&mA, w.hv, n_var, L.ktot, 2, 2, 8, true) ||
+                !make_map(&mB, w.hv, n_var, L.ktot, 2, 2, LdmCfg::NJ)))
         return cudaErrorInvalidValue;
     TcArgs a{};
-    a.jmax = jmax;
-    a.items = items;
-    a.n_items = n_items;
-    a.item_counter = reinterpret_cast<int*>(ws + 128);
+    a.jmax = w.jmax;
+    a.items = w.items;
+    a.n_items = w.n_items;
+    a.item_counter = w.item_counter;
     a.nkc = L.ktot / kKChunk;
     for (int p = 0; p <= LDK_MAX_POPS; ++p) a.kofs[p] = sh.kofs[p];
+    a.max_n = n_sel;
     a.status = status;
-    if (geno) {
-        LdmGArgs g{psite, svar, out, ld_out, sums, (double)n_sel};
-        switch (estimator) {
-            case LDK_LDM_DIPLOID_R2: return launch_ldm_geno<3>(mA, mB, a, g, L.n_items, s);
-            case LDK_LDM_ROGERS_HUFF_R: return launch_ldm_geno<4>(mA, mB, a, g, L.n_items, s);
-            default: return launch_ldm_geno<5>(mA, mB, a, g, L.n_items, s);
-        }
-    }
-    LdmArgs m{psite, out, ld_out, sums};
+    if (nine) return launch_ldm_geno(mA, mB, a, LdmGArgs{out, ld_out, sums}, s);
+    const LdmArgs m{site, out, ld_out, sums};
     switch (estimator) {
-        case LDK_LDM_R2: return launch_ldm<0>(mA, mB, a, m, L.n_items, s);
-        case LDK_LDM_SIGMA_D2: return launch_ldm<1>(mA, mB, a, m, L.n_items, s);
-        default: return launch_ldm<2>(mA, mB, a, m, L.n_items, s);
+        case LDK_LDM_R2: return launch_ldm<LDK_LDM_R2>(mA, mB, a, m, s);
+        case LDK_LDM_SIGMA_D2: return launch_ldm<LDK_LDM_SIGMA_D2>(mA, mB, a, m, s);
+        case LDK_LDM_R2_COUNTS: return launch_ldm<LDK_LDM_R2_COUNTS>(mA, mB, a, m, s);
+        case LDK_LDM_DIPLOID_R2: return launch_ldm<LDK_LDM_DIPLOID_R2>(mA, mB, a, m, s);
+        default: return launch_ldm<LDK_LDM_ROGERS_HUFF_R>(mA, mB, a, m, s);
     }
 }
 

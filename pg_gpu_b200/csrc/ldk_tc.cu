@@ -33,7 +33,7 @@ constexpr int kPrepV = 128, kPrepK = 128;
 // quad of a SNP into its plane bytes with byte-wise compares and writes every plane as
 // 128-byte runs along K.  Plane bytes (GENO: 4 planes, haplotypes: 2):
 //   haplotypes  sigma = 1 - 2x, v = [x in {0, 1}]
-//   genotypes   sigma = 1 - x, sigma^2, v = [x in {0, 1, 2}], 0
+//   genotypes   sigma = 1 - x, sigma^2, v = [x in {0, 1, 2}], 0 (PL = 2: sigma, v)
 // Padding (127) and invalid codes give 0 in every plane; invalid codes also raise
 // LDK_DEVERR_BAD_INPUT.
 //
@@ -48,9 +48,8 @@ constexpr int kPrepV = 128, kPrepK = 128;
 // The second word is read only where it holds SNPs of the quad, and an aligned word holding
 // one byte of the matrix lies in that byte's memory page, so no read can fault; its other
 // bytes are shifted or masked out.
-template <bool GENO, bool PACKED>
+template <bool GENO, bool PACKED, int PL = GENO ? 4 : 2>
 __global__ void __launch_bounds__(256) k_prep_planes(PrepArgs a) {
-    constexpr int PL = GENO ? 4 : 2;
     constexpr int RS = kPrepK + 4;  // bytes per SNP row: 33 words, so the scatter's word loads
                                     // (one K quad per lane) hit distinct banks
     __shared__ __align__(16) int8_t tile[kPrepV * RS];
@@ -137,7 +136,11 @@ __global__ void __launch_bounds__(256) k_prep_planes(PrepArgs a) {
         const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + vv * RS + 4 * kq);
         const uint32_t eq0 = __vcmpeq4(w, 0u), eq1 = __vcmpeq4(w, kOne);
         uint8_t* dst = a.planes_out + v * PL * (int64_t)a.ktot + k0 + 4 * kq;
-        if constexpr (GENO) {
+        if constexpr (GENO && PL == 2) {  // sigma and the mask only
+            const uint32_t eq2 = __vcmpeq4(w, 2u * kOne);
+            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq2;
+            *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq1 | eq2) & kOne;
+        } else if constexpr (GENO) {
             const uint32_t eq2 = __vcmpeq4(w, 2u * kOne);
             *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq2;  // 0xFF = -1
             *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq2) & kOne;
@@ -297,7 +300,9 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
     a.status = w.status;
     dim3 grid((unsigned)((d->n_var + kPrepV - 1) / kPrepV), (unsigned)(sh.ktot / kPrepK));
     const bool packed = d->x_format == LDK_X_PACKED2;
-    if (sh.genotypes) {
+    if (sh.genotypes && sh.planes == 2) {
+        k_prep_planes<true, false, 2><<<grid, 256, 0, s>>>(a);
+    } else if (sh.genotypes) {
         if (packed) k_prep_planes<true, true><<<grid, 256, 0, s>>>(a);
         else k_prep_planes<true, false><<<grid, 256, 0, s>>>(a);
     } else {
@@ -319,14 +324,25 @@ namespace {
 // scan of the pieces per row block, 1024 row blocks per round.
 constexpr int kSplitThreads = 1024;
 
-__device__ __forceinline__ int rb_tiles(const int32_t* __restrict__ rb, const int32_t* __restrict__ jmax, int k,
-                                        int nj) {
-    const int r0 = rb[2 * k], r1 = rb[2 * k + 1];
+// Row block k: from the list, or (no list: one window) [k * rows, (k + 1) * rows) up to `end`.
+struct RowBlocks {
+    const int32_t* list;
+    int rows, end;
+    __device__ __forceinline__ int2 at(int k) const {
+        if (list) return make_int2(list[2 * k], list[2 * k + 1]);
+        const int r0 = k * rows;
+        return make_int2(r0, end - r0 < rows ? end : r0 + rows);
+    }
+};
+
+__device__ __forceinline__ int rb_tiles(const RowBlocks& rb, const int32_t* __restrict__ jmax, int k, int nj) {
+    const int2 b = rb.at(k);
+    const int r0 = b.x, r1 = b.y;
     const int jend = jmax[r1 - 1];
     return jend > r0 + 1 ? (jend - r0 + nj - 1) / nj : 0;
 }
 
-__global__ void __launch_bounds__(kSplitThreads) k_split_items(const int32_t* __restrict__ rb, int n_rb,
+__global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks rb, int n_rb,
                                                                const int32_t* __restrict__ jmax, int nj,
                                                                int min_tiles, int4* __restrict__ items,
                                                                int* __restrict__ n_items) {
@@ -371,7 +387,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const int32_t* __
         __syncthreads();
         const int first = s_base + (wid ? s_scan[wid - 1] : 0) + x - parts;
         if (parts) {
-            const int r0 = rb[2 * k], r1 = rb[2 * k + 1];
+            const int r0 = rb.at(k).x, r1 = rb.at(k).y;
             for (int q = 0; q < parts; ++q)
                 items[first + q] = make_int4(r0, r1, q * c, q == parts - 1 ? INT32_MAX : (q + 1) * c);
         }
@@ -390,8 +406,9 @@ int tc_min_item_tiles(const ParseShape& sh) {
     return t > kMinItemTiles ? t : kMinItemTiles;
 }
 
-cudaError_t launch_split_items(const Scratch& w, int n_row_blocks, int nj, int min_tiles, cudaStream_t s) {
-    k_split_items<<<1, kSplitThreads, 0, s>>>(w.row_blocks, n_row_blocks, w.jmax, nj, min_tiles,
+cudaError_t launch_split_items(const Scratch& w, int n_row_blocks, int nj, int min_tiles, int rows, int end,
+                               cudaStream_t s) {
+    k_split_items<<<1, kSplitThreads, 0, s>>>(RowBlocks{w.row_blocks, rows, end}, n_row_blocks, w.jmax, nj, min_tiles,
                                               reinterpret_cast<int4*>(w.items), w.n_items);
     return cudaGetLastError();
 }
