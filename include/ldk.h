@@ -68,6 +68,28 @@ LDK_API int ldk_counts_geno(const int8_t* X, int64_t ld_x, int64_t n_var, const 
 LDK_API int ldk_stats(int genotypes, int P, const int32_t* counts, const int32_t* n_valid,
               int64_t n_pairs, double* out, void* stream);
 
+/* ldk_stats from one array per population: counts[p] (n_pairs, 4 or 9) -- haplotype counts on a
+ * 16-byte boundary -- and n_valid[p] (n_pairs) or NULL (the counts' sum); the pointer arrays
+ * are host memory, n_valid itself may be NULL. */
+LDK_API int ldk_stats_pops(int genotypes, int P, const int32_t* const* counts, const int32_t* const* n_valid,
+                   int64_t n_pairs, double* out, void* stream);
+
+/* ldk_counts_hap through bit planes packed into `workspace` (ldk_counts_workspace_size bytes,
+ * 256-byte aligned; counts 16-byte aligned): the same counts.  X has n_total_rows rows.  The
+ * workspace's first int is left with bit 0 set if any entry of the selected rows is -1 (the
+ * reference's "has missing data", ld_pipeline.py:155) and bit 1 if a row index lies outside the
+ * matrix (that row then counts as missing). */
+LDK_API size_t ldk_counts_workspace_size(int64_t n_var, int32_t n_rows);
+LDK_API int ldk_counts_hap_packed(const int8_t* X, int64_t ld_x, int64_t n_var, int64_t n_total_rows, const int32_t* rows,
+                   int32_t n_rows, const int32_t* idx_i, const int32_t* idx_j, int64_t n_pairs, int32_t* counts,
+                   int32_t* n_valid, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Per SNP over the rows `rows[0..n_rows)` of X (NULL: the first n_rows rows): the sum of its
+ * positive codes and the number of codes that are not negative -- what the segregating-site
+ * filter asks (ld_statistics.py:249-278). */
+LDK_API int ldk_site_counts(const int8_t* X, int64_t ld_x, int64_t n_var, const int32_t* rows, int32_t n_rows,
+                   int32_t* positive_sum, int32_t* n_valid, void* stream);
+
 /* One raw haplotype estimator call on float64 counts (n_pairs, 4*P_total) with
  * n_valid (n_pairs, P_total) or NULL.  case_id and args are the canonical case of
  * the call (see pg_gpu_b200/csrc/gen_estimators.py: RAW_CASES); out is n_pairs.

@@ -66,6 +66,12 @@ EXPORTS = {
     "ldk_counts_geno": (ctypes.c_int, [c_vp, ctypes.c_int64, ctypes.c_int64, c_vp, ctypes.c_int32, c_vp, c_vp,
                                        ctypes.c_int64, c_vp, c_vp, c_vp]),
     "ldk_stats": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, c_vp, c_vp, ctypes.c_int64, c_vp, c_vp]),
+    "ldk_stats_pops": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(c_vp), ctypes.POINTER(c_vp),
+                                      ctypes.c_int64, c_vp, c_vp]),
+    "ldk_counts_workspace_size": (ctypes.c_size_t, [ctypes.c_int64, ctypes.c_int32]),
+    "ldk_counts_hap_packed": (ctypes.c_int, [c_vp, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64, c_vp, ctypes.c_int32,
+                                             c_vp, c_vp, ctypes.c_int64, c_vp, c_vp, c_vp, ctypes.c_size_t, c_vp]),
+    "ldk_site_counts": (ctypes.c_int, [c_vp, ctypes.c_int64, ctypes.c_int64, c_vp, ctypes.c_int32, c_vp, c_vp, c_vp]),
     "ldk_raw_hap": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_int32), ctypes.c_int, c_vp, c_vp,
                                    ctypes.c_int64, c_vp, c_vp]),
     "ldk_r_family": (ctypes.c_int, [ctypes.c_int, c_vp, c_vp, ctypes.c_int64, c_vp, c_vp]),

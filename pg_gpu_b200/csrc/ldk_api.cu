@@ -503,10 +503,56 @@ int ldk_counts_geno(const int8_t* X, int64_t ld_x, int64_t n_var, const int32_t*
                                     (cudaStream_t)stream), "ldk_counts_geno");
 }
 
+size_t ldk_counts_workspace_size(int64_t n_var, int32_t n_rows) {
+    if (n_var < 0 || n_rows < 0) return 0;
+    return counts_workspace(n_var, n_rows);
+}
+
+int ldk_counts_hap_packed(const int8_t* X, int64_t ld_x, int64_t n_var, int64_t n_total_rows, const int32_t* rows,
+                          int32_t n_rows, const int32_t* idx_i, const int32_t* idx_j, int64_t n_pairs, int32_t* counts,
+                          int32_t* n_valid, void* workspace, size_t workspace_bytes, void* stream) {
+    if (n_pairs < 0 || n_rows < 0 || n_var < 0 || n_total_rows < 0 || ld_x < n_var) { set_error("bad sizes"); return LDK_ERR_ARG; }
+    if (n_rows > 32 * 65535) { set_error("more than 2,097,120 rows"); return LDK_ERR_UNSUPPORTED; }
+    if (n_rows > 0 && n_var > 0 && (!X || !rows)) { set_error("null pointer"); return LDK_ERR_ARG; }
+    if (n_pairs > 0 && (!idx_i || !idx_j || !counts)) { set_error("null pointer"); return LDK_ERR_ARG; }
+    if (!workspace || workspace_bytes < counts_workspace(n_var, n_rows)) {
+        set_error("workspace of %zu bytes is smaller than the %zu required", workspace_bytes, counts_workspace(n_var, n_rows));
+        return LDK_ERR_WORKSPACE;
+    }
+    if (reinterpret_cast<uintptr_t>(workspace) % 256) { set_error("workspace must be 256-byte aligned"); return LDK_ERR_ARG; }
+    if (reinterpret_cast<uintptr_t>(counts) % 16) { set_error("counts must be 16-byte aligned"); return LDK_ERR_ARG; }
+    if (int rc = check_arch()) return rc;
+    return check_cuda(launch_counts_bits(X, ld_x, n_var, n_total_rows, rows, n_rows, idx_i, idx_j, n_pairs, counts, n_valid,
+                                         static_cast<unsigned char*>(workspace), (cudaStream_t)stream),
+                      "ldk_counts_hap_packed");
+}
+
+int ldk_site_counts(const int8_t* X, int64_t ld_x, int64_t n_var, const int32_t* rows, int32_t n_rows,
+                    int32_t* positive_sum, int32_t* n_valid, void* stream) {
+    if (n_rows < 0 || n_var < 0 || ld_x < n_var) { set_error("bad sizes"); return LDK_ERR_ARG; }
+    if (n_var > 0 && ((!X && n_rows > 0) || !positive_sum || !n_valid)) { set_error("null pointer"); return LDK_ERR_ARG; }
+    if (int rc = check_arch()) return rc;
+    return check_cuda(launch_site_counts(X, ld_x, n_var, rows, n_rows, positive_sum, n_valid, (cudaStream_t)stream),
+                      "ldk_site_counts");
+}
+
 int ldk_stats(int genotypes, int P, const int32_t* counts, const int32_t* n_valid, int64_t n_pairs, double* out,
               void* stream) {
     if (P < 1 || P > LDK_MAX_POPS || n_pairs < 0) { set_error("bad P or n_pairs"); return LDK_ERR_ARG; }
-    if (n_pairs > 0 && (!counts || !out)) { set_error("null pointer"); return LDK_ERR_ARG; }
+    const int32_t* c[LDK_MAX_POPS] = {};
+    const int32_t* nv[LDK_MAX_POPS] = {};
+    for (int p = 0; p < P; ++p) {
+        c[p] = counts ? counts + (int64_t)p * n_pairs * (genotypes ? 9 : 4) : nullptr;
+        nv[p] = n_valid ? n_valid + (int64_t)p * n_pairs : nullptr;
+    }
+    return ldk_stats_pops(genotypes, P, c, nv, n_pairs, out, stream);
+}
+
+int ldk_stats_pops(int genotypes, int P, const int32_t* const* counts, const int32_t* const* n_valid, int64_t n_pairs,
+                   double* out, void* stream) {
+    if (P < 1 || P > LDK_MAX_POPS || n_pairs < 0) { set_error("bad P or n_pairs"); return LDK_ERR_ARG; }
+    for (int p = 0; p < P; ++p)
+        if (n_pairs > 0 && (!counts || !counts[p] || !out)) { set_error("null pointer"); return LDK_ERR_ARG; }
     if (int rc = check_arch()) return rc;
     return check_cuda(launch_stats(genotypes, P, counts, n_valid, n_pairs, out, (cudaStream_t)stream), "ldk_stats");
 }

@@ -57,6 +57,18 @@ LDK_DEV uint64_t global_ns() {
     return t;
 }
 
+// Codes of SNPs v .. v + 3 of one row (bytes; -1 beyond the matrix): one aligned word, or two
+// joined with a funnel shift.  The second word is read only where it holds SNPs of the quad, so
+// no read leaves the 4-byte words that hold the row's codes.
+LDK_DEV uint32_t load_quad(const int8_t* p, int left) {
+    const uintptr_t ad = reinterpret_cast<uintptr_t>(p);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(ad & ~uintptr_t(3));
+    const int s = (int)(ad & 3u);
+    uint32_t x = __ldg(q);
+    if (s) x = __funnelshift_r(x, s + left > 4 ? __ldg(q + 1) : 0u, 8 * s);
+    return left >= 4 ? x : x | (0xFFFFFFFFu << (8 * left));
+}
+
 // FP64 add into shared memory.
 LDK_DEV void smem_add_f64(double* p, double v) { atomicAdd(p, v); }
 

@@ -44,7 +44,7 @@ struct ParseShape {
 cudaError_t launch_counts(int genotypes, const int8_t* X, int64_t ld, const int32_t* rows, int n_rows,
                           const int32_t* ii, const int32_t* jj, int64_t n, int32_t* counts,
                           int32_t* n_valid, cudaStream_t s);
-cudaError_t launch_stats(int genotypes, int P, const int32_t* counts, const int32_t* n_valid, int64_t n,
+cudaError_t launch_stats(int genotypes, int P, const int32_t* const* counts, const int32_t* const* n_valid, int64_t n,
                          double* out, cudaStream_t s);
 cudaError_t launch_raw_hap(int case_id, const int32_t* args, int P_total, const double* counts,
                            const double* n_valid, int64_t n, double* out, cudaStream_t s);
@@ -58,6 +58,15 @@ cudaError_t launch_fx_finish(const ldk_parse_t* d, const ldk_parse_out_t* o, con
                              cudaStream_t s);
 cudaError_t launch_block_combine(const double* block_sums, int64_t n_blocks, int64_t k,
                                  const int32_t* weights, int64_t n_rep, double* out, cudaStream_t s);
+
+// launchers (ldk_bits.cu): pair counts from bit planes in `ws` (its first int: 1 = a missing
+// entry in the rows, 2 = a row outside the matrix) and per-SNP call counts
+size_t counts_workspace(int64_t n_var, int32_t n_rows);
+cudaError_t launch_counts_bits(const int8_t* X, int64_t ld, int64_t n_var, int64_t n_total, const int32_t* rows,
+                               int n_rows, const int32_t* ii, const int32_t* jj, int64_t n, int32_t* counts,
+                               int32_t* n_valid, unsigned char* ws, cudaStream_t s);
+cudaError_t launch_site_counts(const int8_t* X, int64_t ld, int64_t n_var, const int32_t* rows, int n_rows, int32_t* pos,
+                               int32_t* valid, cudaStream_t s);
 
 // launchers (ldk_tc.cu)
 cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh,

@@ -56,13 +56,21 @@ def segregating(hap, missing_data="include"):
     sites with 0 < derived count < valid count."""
     torch = _lib.require_cuda()
     X = _hap_tensor(hap, torch)
-    keep = torch.arange(X.shape[1], device="cuda")
+    n_rows, m = X.shape
+    dac = torch.empty(m, dtype=torch.int32, device="cuda")
+    nv = torch.empty(m, dtype=torch.int32, device="cuda")
+    _lib.check(_lib.load().ldk_site_counts(_lib.ptr(X), m, m, None, n_rows, _lib.ptr(dac), _lib.ptr(nv),
+                                           _lib.stream_handle()))
+    keep = (dac > 0) & (dac < nv)
     if missing_data == "exclude":
-        keep = keep[(X < 0).sum(0) == 0]
-    sub = X.index_select(1, keep)
-    dac = sub.clamp(min=0).to(torch.int64).sum(0)
-    nv = (sub >= 0).sum(0)
-    return keep[(dac > 0) & (dac < nv)]
+        keep &= nv == n_rows
+    return keep.nonzero().flatten()
+
+
+def _segregating_sites(X, missing_data):
+    """The columns of X that ``segregating`` keeps: X itself where it keeps all."""
+    seg = segregating(X, missing_data)
+    return X if seg.numel() == X.shape[1] else X.index_select(1, seg)
 
 
 def _resolve(estimator):
@@ -82,11 +90,11 @@ def zns(hap, missing_data="include", estimator="auto"):
     torch = _lib.require_cuda()
     est = _resolve(estimator)
     X = _hap_tensor(hap, torch)
-    seg = segregating(X, missing_data if est == "r2" else "include")
-    m = int(seg.numel())
+    X = _segregating_sites(X, missing_data if est == "r2" else "include")
+    m = X.shape[1]
     if m < 2:
         return 0.0
-    _, S = ld_matrix(X.index_select(1, seg), estimator=est, matrix=False, reduce=True)
+    _, S = ld_matrix(X, estimator=est, matrix=False, reduce=True)
     total, count = S.tolist()
     if est == "r2":
         return total / (m * (m - 1) / 2)
@@ -100,11 +108,10 @@ def omega(hap, missing_data="include", estimator="auto"):
     torch = _lib.require_cuda()
     est = _resolve(estimator)
     X = _hap_tensor(hap, torch)
-    seg = segregating(X, missing_data)
-    m = int(seg.numel())
-    if m < 5:
+    X = _segregating_sites(X, missing_data)
+    if X.shape[1] < 5:
         return 0.0
-    M, _ = ld_matrix(X.index_select(1, seg), estimator=est)
+    M, _ = ld_matrix(X, estimator=est)
     return omega_from_matrix(M)
 
 

@@ -7,6 +7,8 @@ estimators run in libldk, pair enumeration uses device tensor ops.
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 
 from . import _lib
@@ -74,15 +76,17 @@ def iter_pairs_within_distance(positions, max_dist, chunk_size):
 # ---------------------------------------------------------------------------
 
 
-def _rows_and_missing(mat, pop_indices, missing_pred):
+def _rows(mat, pop_indices):
     torch = _lib.require_cuda()
     if pop_indices is None:
-        rows = torch.arange(mat.shape[0], dtype=torch.int32, device="cuda")
-        sub = mat
-    else:
-        rows = _device_tensor(np.asarray(pop_indices) if not isinstance(pop_indices, torch.Tensor)
-                              else pop_indices, torch.int32)
-        sub = mat.index_select(0, rows.long())
+        return torch.arange(mat.shape[0], dtype=torch.int32, device="cuda")
+    return _device_tensor(np.asarray(pop_indices) if not isinstance(pop_indices, torch.Tensor) else pop_indices,
+                          torch.int32)
+
+
+def _rows_and_missing(mat, pop_indices, missing_pred):
+    rows = _rows(mat, pop_indices)
+    sub = mat if pop_indices is None else mat.index_select(0, rows.long())
     return rows, bool(missing_pred(sub).any().item())
 
 
@@ -94,13 +98,18 @@ def compute_counts_for_pairs(haplotypes, idx_i, idx_j, pop_indices=None):
     X = _device_tensor(haplotypes, torch.int8)
     I = _device_tensor(idx_i, torch.int32)
     J = _device_tensor(idx_j, torch.int32)
-    rows, has_missing = _rows_and_missing(X, pop_indices, lambda s: s == -1)
+    rows = _rows(X, pop_indices)
     n = I.numel()
     counts = torch.empty((n, 4), dtype=torch.int32, device="cuda")
     nv = torch.empty(n, dtype=torch.int32, device="cuda")
-    _lib.check(lib.ldk_counts_hap(_lib.ptr(X), X.shape[1], X.shape[1], _lib.ptr(rows), rows.numel(), _lib.ptr(I),
-                                  _lib.ptr(J), n, _lib.ptr(counts), _lib.ptr(nv), _lib.stream_handle()))
-    return counts, (nv if has_missing else None)
+    ws = torch.empty(int(lib.ldk_counts_workspace_size(X.shape[1], rows.numel())), dtype=torch.uint8, device="cuda")
+    _lib.check(lib.ldk_counts_hap_packed(_lib.ptr(X), X.shape[1], X.shape[1], X.shape[0], _lib.ptr(rows), rows.numel(),
+                                         _lib.ptr(I), _lib.ptr(J), n, _lib.ptr(counts), _lib.ptr(nv), _lib.ptr(ws),
+                                         ws.numel(), _lib.stream_handle()))
+    flag = int(ws[:4].view(torch.int32).item())
+    if flag & 2:
+        raise IndexError("population row index out of range")
+    return counts, (nv if flag & 1 else None)
 
 
 def compute_genotype_counts_for_pairs(genotypes, idx_i, idx_j, pop_indices=None):
@@ -133,15 +142,20 @@ def compute_multi_pop_statistics_batch(counts_per_pop, n_valid_per_pop=None, gen
     lib = _lib.load()
     P = len(counts_per_pop)
     width = 9 if genotypes else 4
-    C = torch.stack([_device_tensor(c, torch.int32).reshape(-1, width) for c in counts_per_pop]).contiguous()
-    n = C.shape[1]
-    NV = None
-    if n_valid_per_pop is not None and any(v is not None for v in n_valid_per_pop):
-        NV = torch.stack([_device_tensor(v, torch.int32) if v is not None else C[p].sum(dim=1, dtype=torch.int32)
-                          for p, v in enumerate(n_valid_per_pop)]).contiguous()
+    C = [_device_tensor(c, torch.int32).reshape(-1, width) for c in counts_per_pop]
+    # the library reads haplotype counts as 16-byte rows
+    C = [c if c.data_ptr() % 16 == 0 else c.clone() for c in C]
+    n = C[0].shape[0]
+    NV = [None] * P
+    if n_valid_per_pop is not None:
+        NV = [None if v is None else _device_tensor(v, torch.int32).reshape(-1) for v in n_valid_per_pop]
+    if any(c.shape[0] != n for c in C) or any(v is not None and v.numel() != n for v in NV):
+        raise RuntimeError("counts and n_valid of the populations differ in length")
     out = torch.empty((n, len(ld_names(P))), dtype=torch.float64, device="cuda")
-    _lib.check(lib.ldk_stats(int(bool(genotypes)), P, _lib.ptr(C), _lib.ptr(NV), n, _lib.ptr(out),
-                             _lib.stream_handle()))
+    ptrs = ctypes.c_void_p * P
+    _lib.check(lib.ldk_stats_pops(int(bool(genotypes)), P, ptrs(*[c.data_ptr() for c in C]),
+                                  ptrs(*[None if v is None else v.data_ptr() for v in NV]), n, _lib.ptr(out),
+                                  _lib.stream_handle()))
     return out
 
 
