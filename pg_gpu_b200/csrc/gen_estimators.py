@@ -932,9 +932,9 @@ def emit_spin(P, geno):
         if NS in mine:
             at = mine.index(NS)
             use("E0 vx0 vy0")
-            lines += ["    const double den = vx0 * vy0;", "    if (den > 0.0) {",
-                      f"        acc[{at}] = fma(E0 * E0, recip_cubic(den), acc[{at}]);", "        ++nr2;", "    }"]
-        L.append(f"LDK_DEV void spin_{path}_P{P}_{part}(const SpinPop* f, double* acc, unsigned& nr2) {{")
+            lines += ["    const double den = vx0 * vy0;", "    const bool has = ok && den > 0.0;",
+                      f"    acc[{at}] = fma(E0 * E0, has ? recip_cubic(den) : 0.0, acc[{at}]);", "    nr2 += has;"]
+        L.append(f"LDK_DEV void spin_{path}_P{P}_{part}(const SpinPop* f, bool ok, double* acc, unsigned& nr2) {{")
         L += lines
         L.append("}")
     w = [x[1] for x in stats] + [1.0]
@@ -1034,20 +1034,21 @@ LDK_DEV void geno_stats(const GenoFeat<T>* f, T* acc) {
     else geno_stats_P4<T, S>(f, acc);
 }
 // Spin-form statistics of part PART (0: all and r^2; four haplotype populations:
-// 1 and 2, the two halves) added into acc[0 ..) of that part, before their weights.
+// 1 and 2, the two halves) added into acc[0 ..) of that part, before their weights.  A pair that
+// does not count (!ok) has its reciprocals set to 0 by the caller; r^2 looks at ok itself.
 template <int P, bool GENO, int PART>
-LDK_DEV void spin_stats(const SpinPop* f, double* acc, unsigned& nr2) {
+LDK_DEV void spin_stats(const SpinPop* f, bool ok, double* acc, unsigned& nr2) {
     if constexpr (GENO) {
-        if constexpr (P == 1) spin_geno_P1_0(f, acc, nr2);
-        else if constexpr (P == 2) spin_geno_P2_0(f, acc, nr2);
-        else if constexpr (P == 3) spin_geno_P3_0(f, acc, nr2);
-        else spin_geno_P4_0(f, acc, nr2);
+        if constexpr (P == 1) spin_geno_P1_0(f, ok, acc, nr2);
+        else if constexpr (P == 2) spin_geno_P2_0(f, ok, acc, nr2);
+        else if constexpr (P == 3) spin_geno_P3_0(f, ok, acc, nr2);
+        else spin_geno_P4_0(f, ok, acc, nr2);
     } else {
-        if constexpr (P == 1) spin_hap_P1_0(f, acc, nr2);
-        else if constexpr (P == 2) spin_hap_P2_0(f, acc, nr2);
-        else if constexpr (P == 3) spin_hap_P3_0(f, acc, nr2);
-        else if constexpr (PART == 1) spin_hap_P4_1(f, acc, nr2);
-        else spin_hap_P4_2(f, acc, nr2);
+        if constexpr (P == 1) spin_hap_P1_0(f, ok, acc, nr2);
+        else if constexpr (P == 2) spin_hap_P2_0(f, ok, acc, nr2);
+        else if constexpr (P == 3) spin_hap_P3_0(f, ok, acc, nr2);
+        else if constexpr (PART == 1) spin_hap_P4_1(f, ok, acc, nr2);
+        else spin_hap_P4_2(f, ok, acc, nr2);
     }
 }
 // Weight and statistic (number of statistics: r^2, weight 1) of staged sum s.

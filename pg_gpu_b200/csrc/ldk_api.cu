@@ -71,6 +71,7 @@ bool shape_of(const ldk_parse_t* d, ParseShape& sh) {
     sh.n_stats = stats_of(d->n_pops);
     sh.n_bins = d->n_bins;
     sh.planes = tc_planes(sh);
+    sh.slots = d->snp_block ? tc_block_slots(sh) : 1;
     int k = 0;
     sh.max_n = 0;
     for (int p = 0; p < LDK_MAX_POPS + 1; ++p) sh.kofs[p] = 0;

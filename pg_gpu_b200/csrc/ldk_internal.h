@@ -36,6 +36,7 @@ struct ParseShape {
     int ktot;                    // TC path: total K bytes (multiple of 128)
     int planes;                  // TC path: spin planes per SNP (2 haplotype, 4 genotype)
     int max_n;                   // largest population size
+    int slots;                   // TC path: bootstrap blocks staged per row block (1 without blocks)
     int rtab_global;             // TC haplotype path: the reciprocal table (32 B per n_valid)
                                  // does not fit beside the pipeline in shared memory
 };

@@ -112,9 +112,9 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* stages = base;
-    double* rn = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // EST R2: 1 / n
+    double* rn = reinterpret_cast<double*>(stages + a.stages * C::STAGE_BYTES);  // EST R2: 1 / n
 
-    __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], tfull[C::NBUF], tempty[C::NBUF];
+    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
     __shared__ volatile int ring[2 * kRing];
     __shared__ uint32_t tmem_base_s;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; ++s) {
+        for (int s = 0; s < a.stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
+    const Pipe pipe{su32(stages), full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
     if (warp == 0) run_producer<C, true>(pipe, &tmA, &tmB, a, lane);
     else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
     if (warp >= 4) {
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* stages = base;
-    double* stile = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // [kLdmGEpi][32][SP]
+    double* stile = reinterpret_cast<double*>(stages + a.stages * C::STAGE_BYTES);  // [kLdmGEpi][32][SP]
 
-    __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], tfull[C::NBUF], tempty[C::NBUF];
+    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
     __shared__ volatile int ring[2 * kRing];
     __shared__ uint32_t tmem_base_s;
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; ++s) {
+        for (int s = 0; s < a.stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
+    const Pipe pipe{su32(stages), full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
     if (warp == 0) run_producer<C, false>(pipe, &tmA, &tmB, a, lane);
     else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
     if (warp >= 4) {
@@ -473,10 +473,17 @@ int sm_count() {
     return sms;
 }
 
-cudaError_t launch_ldm_geno(const CUtensorMap& mA, const CUtensorMap& mB, const TcArgs& a, const LdmGArgs& m,
+// Shared memory of a launch: `other` bytes beside the pipeline of C::STAGES stages.  (A longer
+// ring takes the L1 that serves the per-SNP factors: r^2 matrix 369 -> 392 us.)
+template <class C>
+size_t ldm_smem(TcArgs& a, size_t other) {
+    a.stages = C::STAGES;
+    return other + (size_t)a.stages * C::STAGE_BYTES;
+}
+
+cudaError_t launch_ldm_geno(const CUtensorMap& mA, const CUtensorMap& mB, TcArgs& a, const LdmGArgs& m,
                             cudaStream_t s) {
-    using C = LdmGCfg;
-    size_t smem = 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)kLdmGEpi * 32 * kLdmGStride * sizeof(double);
+    size_t smem = ldm_smem<LdmGCfg>(a, 1024 + (size_t)kLdmGEpi * 32 * kLdmGStride * sizeof(double));
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaFuncSetAttribute(k_ld_matrix_geno, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -486,9 +493,8 @@ cudaError_t launch_ldm_geno(const CUtensorMap& mA, const CUtensorMap& mB, const 
 }
 
 template <int EST>
-cudaError_t launch_ldm(const CUtensorMap& mA, const CUtensorMap& mB, const TcArgs& a, const LdmArgs& m, cudaStream_t s) {
-    using C = LdmCfg;
-    size_t smem = 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (a.max_n < kLdmTable ? a.max_n + 1 : 0) * sizeof(double);
+cudaError_t launch_ldm(const CUtensorMap& mA, const CUtensorMap& mB, TcArgs& a, const LdmArgs& m, cudaStream_t s) {
+    size_t smem = ldm_smem<LdmCfg>(a, 1024 + (a.max_n < kLdmTable ? a.max_n + 1 : 0) * sizeof(double));
     if (smem < kMinSmem) smem = kMinSmem;
     cudaError_t e = cudaFuncSetAttribute(k_ld_matrix<EST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
 }  // namespace
 
 int tc_min_item_tiles(const ParseShape& sh) {
-    const int staged = tc_block_slots(sh) * sh.n_bins * (sh.n_stats + 1);
+    const int staged = sh.slots * sh.n_bins * (sh.n_stats + 1);
     const int t = (staged + kFlushValuesPerTile - 1) / kFlushValuesPerTile;
     return t > kMinItemTiles ? t : kMinItemTiles;
 }

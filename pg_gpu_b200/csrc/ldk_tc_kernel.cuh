@@ -45,8 +45,10 @@
 #include <cudaTypedefs.h>
 #include <math_constants.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 
 #include "ldk_estimators.cuh"
@@ -60,10 +62,9 @@ constexpr int kRing = 2;                // claimed work items in flight between 
 constexpr int kTmemCols = 512;
 constexpr uint64_t kTimeoutNs = 5000000000ull;  // 5 s per wait
 // Register split of the SPLIT layouts: the launch gives every thread Cfg::REG_LAUNCH
-// registers; warpgroup 0 drops to kRegCtrl and the epilogue warpgroups rise to Cfg::REG_EPI,
+// registers; warpgroup 0 drops to Cfg::REG_CTRL and the epilogue warpgroups rise to Cfg::REG_EPI,
 // which the freed registers cover (Cfg asserts the sum).  The host launches only a kernel
 // compiled to Cfg::REG_LAUNCH registers.
-constexpr int kRegCtrl = 24;
 constexpr size_t kMinSmem = 116 * 1024;
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kStaticSmem = 1536;  // at most: the kernel's __shared__ variables (barriers, bin edges)
@@ -113,8 +114,8 @@ struct Cfg {
     // schedulers of an SM holds warps w, w + 4, ... with a quarter of the register file.
     //  * SPLIT (genotypes; haplotypes with three or four populations -- estimators that
     //    want ~240 registers): 12 warps.  Warpgroup 0 (TMA, MMA, two idle warps) gives its
-    //    registers up with setmaxnreg (kRegCtrl each) and the eight epilogue warps 4..11
-    //    take them (240 each), so that every scheduler holds two full-register epilogue
+    //    registers up with setmaxnreg (24 or 40 each) and the eight epilogue warps 4..11
+    //    take them (240 or 232 each), so that every scheduler holds two full-register epilogue
     //    warps beside one control warp (launch: 168 per thread).
     //  * one genotype population, also SPLIT: 16 warps, twelve epilogue warps 4..15 at 160
     //    registers, three per scheduler and lane quarter (launch: 128).
@@ -125,7 +126,10 @@ struct Cfg {
     static constexpr int W0 = SPLIT ? 4 : 2;  // first epilogue warp
     static constexpr int THREADS = 32 * (W0 + EPI);
     static constexpr int REG_LAUNCH = (EPI == 16) ? 96 : (EPI == 12) ? 128 : 168;  // SPLIT layouts only
-    static constexpr int REG_EPI = (EPI == 16) ? 112 : (EPI == 12) ? 160 : 240;
+    // control and epilogue registers; three and four haplotype populations need every register
+    // in the epilogue, the others give the control warps enough not to spill
+    static constexpr int REG_CTRL = (EPI == 12) ? 32 : (!GENO && P >= 3) ? 24 : 40;
+    static constexpr int REG_EPI = (EPI == 16) ? 112 : (EPI == 12) ? 160 : (!GENO && P >= 3) ? 240 : 232;
     // SSPL (four haplotype populations): the two warps of a lane quarter split the
     // statistics, not the partners -- both take every pair, part 0 accumulates statistics
     // [0, K) (DD, Dz) and counts pairs, part 1 the pi2 statistics [K, NS) and r^2 -- so that
@@ -137,12 +141,22 @@ struct Cfg {
     static constexpr int STEPS = GENO ? NJ : QROWS ? NJ / 4 : NJ / 2;
     static constexpr int SHARES = EPI / (4 * PARTS * (QROWS ? 2 : 1));
     static constexpr int MY_STEPS = STEPS / SHARES;
+    // Pairs a lane evaluates together: one population's chain of ~45 FP64 operations waits for
+    // itself, two interleaved chains less (1,000,000 SNPs x 2,000 haplotypes 21.7 -> 20.7 ms,
+    // 5,000 x 100 0.099 -> 0.090); with two populations a pair at a time is faster (5.18 against
+    // 5.44 ms), and two pairs of three do not fit the registers.
+    static constexpr int U = P == 1 ? 2 : 1;
+    static_assert(MY_STEPS % U == 0, "pairs per step");
+    using Recip = typename std::conditional<P == 1, double, double4>::type;
+    // The ring: as many stages as shared memory has left (STAGES at least), or STAGES where the
+    // control warps have 24 registers, which do not hold a run-time length.
+    static constexpr bool MORE_STAGES = !SPLIT || REG_CTRL >= 32;
     // Staging row of the bin flush: a lane's sums, then {pairs, finite r^2, key, -}
     static constexpr int K = GENO ? 0 : SpinSplit<P>::value;
     static constexpr int NA = SSPL ? (K > NS + 1 - K ? K : NS + 1 - K) : NS + 1;  // sums per lane
-    static constexpr int FROW = P == 1 ? 0 : NA + 2;  // one population reduces in registers
+    static constexpr int FROW = P == 1 ? 0 : (NA + 2) | 1;  // odd: rows in other banks; one population reduces in registers
     static constexpr int FROWS_MAX = 8;
-    static_assert(!SPLIT || 4 * kRegCtrl + EPI * REG_EPI <= (W0 + EPI) * REG_LAUNCH,
+    static_assert(!SPLIT || 4 * REG_CTRL + EPI * REG_EPI <= (W0 + EPI) * REG_LAUNCH,
                   "register split must fit the launch allocation");
     static_assert(!SPLIT || THREADS * REG_LAUNCH <= 65536, "register file");
     static_assert(EPI % 4 == 0 && STEPS % SHARES == 0 && (!QROWS || NJ % 4 == 0), "epilogue warps share tiles equally");
@@ -191,10 +205,10 @@ LDK_DEV bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag, u
     }
 }
 
-LDK_DEV void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+LDK_DEV void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(su32(dst)),
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(su32(bar)), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
@@ -355,6 +369,8 @@ struct TcArgs {
     unsigned long long* pairs;
     unsigned long long* r2_counts;
     unsigned* status;
+    int slots;              // bootstrap blocks staged per row block (1 without snp_block)
+    int stages;             // ring stages
     int frows;              // staging rows per epilogue warp of the bin flush
     const double4* rtab_g;  // haplotype path: reciprocal table in global memory, or null when
                             // each CTA builds it in shared memory
@@ -362,8 +378,9 @@ struct TcArgs {
 };
 
 // Shared-memory state of the persistent pipeline (one CTA).
+constexpr int kMaxStages = 8;
 struct Pipe {
-    unsigned char* stages;
+    uint32_t stages;  // shared address of the ring
     uint64_t* full_bar;
     uint64_t* empty_bar;
     uint64_t* tfull;
@@ -391,28 +408,22 @@ LDK_DEV int item_tiles(const TcArgs& a, int item, int& row0, int& row1, int& jt0
     return te > it.z ? te - it.z : 0;
 }
 
-// TMA loads of K chunk c of the tile (row block at row0, partners from j0) into stage s.
+// TMA loads of K chunk c of a row block into `dst`, signalled on `bar`.
 template <class C, bool QR>
-LDK_DEV void issue_loads(const Pipe& S, const CUtensorMap* tmA, const CUtensorMap* tmB, int s, int c, int row0,
-                         int j0) {
-    unsigned char* dst = S.stages + s * C::STAGE_BYTES;
-    mbar_expect_tx(&S.full_bar[s], C::STAGE_BYTES);
+LDK_DEV void load_rows(uint32_t dst, const CUtensorMap* tmA, uint64_t* bar, int c, int row0) {
     if constexpr (QR) {  // box {128 k, 8 SNPs, 2 planes}: one group of sixteen rows
 #pragma unroll
-        for (int g = 0; g < C::ROWS / 8; ++g)
-            tma_load_3d(dst + g * 16 * kKChunk, tmA, &S.full_bar[s], c * kKChunk, row0 + 8 * g, 0);
+        for (int g = 0; g < C::ROWS / 8; ++g) tma_load_3d(dst + g * 16 * kKChunk, tmA, bar, c * kKChunk, row0 + 8 * g, 0);
     } else {
 #pragma unroll
-        for (int x = 0; x < C::REGIONS; ++x) tma_load_3d(dst + x * C::A_BOX, tmA, &S.full_bar[s], c * kKChunk, x, row0);
+        for (int x = 0; x < C::REGIONS; ++x) tma_load_3d(dst + x * C::A_BOX, tmA, bar, c * kKChunk, x, row0);
     }
-    tma_load_3d(dst + C::A_BYTES, tmB, &S.full_bar[s], c * kKChunk, 0, j0);
 }
 
-// MMAs of K chunk c (in stage s) into accumulator buffer buf; frees the stage on completion.
+// MMAs of K chunk c (staged at a_addr) into accumulator buffer buf.
 template <class C, int P>
-LDK_DEV void issue_mmas(const Pipe& S, uint32_t tmem, const TcArgs& a, int s, int c, uint32_t buf) {
+LDK_DEV void issue_mmas(uint32_t tmem, const TcArgs& a, uint32_t a_addr, int c, uint32_t buf) {
     constexpr uint32_t idesc = idesc_s8<C::N>();
-    const uint32_t a_addr = su32(S.stages + s * C::STAGE_BYTES);
     const uint32_t b_addr = a_addr + C::A_BYTES;
 #pragma unroll
     for (int ks = 0; ks < kKChunk / 32; ++ks) {
@@ -427,7 +438,6 @@ LDK_DEV void issue_mmas(const Pipe& S, uint32_t tmem, const TcArgs& a, int s, in
             mma_i8(d, sw128_desc(a_addr + x * C::A_BOX + ks * 32), sw128_desc(b_addr + ks * 32), idesc, first ^ 1u);
         }
     }
-    mma_commit(&S.empty_bar[s]);
 }
 
 // Warp 0: claims work items from the global counter, publishes each with its tile count
@@ -436,7 +446,9 @@ template <class C, bool QR>
 LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorMap* tmB, const TcArgs& a,
                           int lane) {
     if (lane == 0) {
-        uint32_t it = 0;
+        const int nst = C::MORE_STAGES ? a.stages : C::STAGES;
+        int s = 0;        // ring stage and its phase
+        uint32_t ph = 0;
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             // claim the next item and publish it to the MMA issuer and the epilogue
@@ -450,13 +462,14 @@ LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorM
             S.ring[kRing + sl] = n_jt;
             mbar_arrive(&S.ifull[sl]);
             if (item < 0) break;
-            const int jstop = jt0 + n_jt * C::NJ;
-            for (int j0 = jt0; j0 < jstop && ok; j0 += C::NJ) {
-                for (int c = 0; c < a.nkc; ++c, ++it) {
-                    const int s = it % C::STAGES;
-                    const uint32_t ph = (it / C::STAGES) & 1u;
+            for (int t = 0; t < n_jt && ok; ++t) {
+                for (int c = 0; c < a.nkc; ++c) {
                     if (!mbar_wait(&S.empty_bar[s], ph ^ 1u, S.abort_s, a.status)) { ok = false; break; }
-                    issue_loads<C, QR>(S, tmA, tmB, s, c, row0, j0);
+                    const uint32_t dst = S.stages + s * C::STAGE_BYTES;
+                    mbar_expect_tx(&S.full_bar[s], C::STAGE_BYTES);
+                    load_rows<C, QR>(dst, tmA, &S.full_bar[s], c, row0);
+                    tma_load_3d(dst + C::A_BYTES, tmB, &S.full_bar[s], c * kKChunk, 0, jt0 + t * C::NJ);
+                    if (++s == nst) { s = 0; ph ^= 1u; }
                 }
             }
         }
@@ -469,7 +482,9 @@ LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorM
 template <class C, int P>
 LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a, int lane) {
     if (lane == 0) {
-        uint32_t it = 0, tcount = 0;
+        const int nst = C::MORE_STAGES ? a.stages : C::STAGES;
+        int s = 0;
+        uint32_t ph = 0, tcount = 0;
         bool ok = true;
         for (uint32_t k = 0; ok; ++k) {
             const int sl = k % kRing;
@@ -481,12 +496,12 @@ LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a, int lane) {
                 const uint32_t buf = tcount % C::NBUF, tph = (tcount / C::NBUF) & 1u;
                 if (!mbar_wait(&S.tempty[buf], tph ^ 1u, S.abort_s, a.status)) { ok = false; break; }
                 tc_fence_after();
-                for (int c = 0; c < a.nkc; ++c, ++it) {
-                    const int s = it % C::STAGES;
-                    const uint32_t ph = (it / C::STAGES) & 1u;
+                for (int c = 0; c < a.nkc; ++c) {
                     if (!mbar_wait(&S.full_bar[s], ph, S.abort_s, a.status)) { ok = false; break; }
                     tc_fence_after();
-                    issue_mmas<C, P>(S, tmem, a, s, c, buf);
+                    issue_mmas<C, P>(tmem, a, S.stages + s * C::STAGE_BYTES, c, buf);
+                    mma_commit(&S.empty_bar[s]);
+                    if (++s == nst) { s = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
                 mma_commit(&S.tfull[buf]);
@@ -506,18 +521,20 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     using C = Cfg<P, GENO, V>;
     constexpr int NS = C::NS;
     constexpr int EPI = C::EPI;
-    constexpr int SLOTS = C::SLOTS;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int nb = a.edges.n_bins;
+    const int slots = a.slots;
     unsigned char* stages = base;
     constexpr int NCOPY = PRIV ? EPI : 1;  // staging copies: one per epilogue warp, or shared
-    double* sacc = reinterpret_cast<double*>(base + C::STAGES * C::STAGE_BYTES);  // [NCOPY][SLOTS][nb][NS+1]
-    unsigned* scnt = reinterpret_cast<unsigned*>(sacc + NCOPY * SLOTS * nb * (NS + 1));  // [NCOPY][SLOTS][nb][2]
-    double4* rtab = reinterpret_cast<double4*>(scnt + ((NCOPY * SLOTS * nb * 2 + 7) & ~7));  // [max_n + 1]
-    double* fstage = reinterpret_cast<double*>(rtab + (GENO || GT ? 0 : a.max_n + 1));  // [EPI][frows][FROW]
+    double* sacc = reinterpret_cast<double*>(stages + a.stages * C::STAGE_BYTES);  // [NCOPY][slots][nb][NS+1]
+    unsigned* scnt = reinterpret_cast<unsigned*>(sacc + NCOPY * slots * nb * (NS + 1));  // [NCOPY][slots][nb][2]
+    // reciprocals of the valid counts [max_n + 1] (one population reads the last one only)
+    using Recip = typename C::Recip;
+    Recip* rtab = reinterpret_cast<Recip*>(scnt + ((NCOPY * slots * nb * 2 + 7) & ~7));
+    double* fstage = reinterpret_cast<double*>(rtab + (GENO || GT ? 0 : (a.max_n + 2) & ~1));  // [EPI][frows][FROW]
 
-    __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES], tfull[C::NBUF], tempty[C::NBUF];
+    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
     __shared__ volatile int ring[2 * kRing];
     __shared__ uint32_t tmem_base_s;
@@ -526,7 +543,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; ++s) {
+        for (int s = 0; s < a.stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -542,10 +559,13 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int b = threadIdx.x; b <= nb; b += blockDim.x) sedges[b] = a.edges.e[b];
-    for (int idx = threadIdx.x; idx < NCOPY * SLOTS * nb * (NS + 1); idx += blockDim.x) sacc[idx] = 0.0;
-    for (int idx = threadIdx.x; idx < NCOPY * SLOTS * nb * 2; idx += blockDim.x) scnt[idx] = 0u;
+    for (int idx = threadIdx.x; idx < NCOPY * slots * nb * (NS + 1); idx += blockDim.x) sacc[idx] = 0.0;
+    for (int idx = threadIdx.x; idx < NCOPY * slots * nb * 2; idx += blockDim.x) scnt[idx] = 0u;
     if constexpr (!GENO && !GT)
-        for (int idx = threadIdx.x; idx <= a.max_n; idx += blockDim.x) rtab[idx] = recip_entry(idx);
+        for (int idx = threadIdx.x; idx <= a.max_n; idx += blockDim.x) {
+            if constexpr (P == 1) rtab[idx] = recip_entry(idx).w;
+            else rtab[idx] = recip_entry(idx);
+        }
     if (warp == 1) {
         tmem_alloc(&tmem_base_s, kTmemCols);
         tmem_relinquish();
@@ -554,7 +574,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    const Pipe pipe{stages, full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
+    const Pipe pipe{su32(stages), full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
     // Each side changes its register budget once, at its start, and never back: warpgroup
     // 0 releases registers (setmaxnreg.dec never waits) and the epilogue warps take them
     // (setmaxnreg.inc waits only for that release, which comes unconditionally first).
@@ -564,9 +584,9 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     // code both sides share, the teardown below, fits the smaller budget.  Neither the
     // roles nor the teardown may call a function (printf, a non-inlined helper): a
     // callee's registers are not bounded by the budget, and a call from a warp holding
-    // kRegCtrl registers raised an illegal-instruction fault.
+    // 24 registers raised an illegal-instruction fault.
     if (warp < C::W0) {
-        if constexpr (C::SPLIT) setmaxnreg_dec<kRegCtrl>();
+        if constexpr (C::SPLIT) setmaxnreg_dec<C::REG_CTRL>();
         if (warp == 0) run_producer<C, C::QROWS>(pipe, &tmA, &tmB, a, lane);
         else if (warp == 1) run_mma<C, P>(pipe, tmem, a, lane);
     } else {
@@ -589,10 +609,10 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
         const int jb = JSTRIDE * q0 + (GENO ? 0 : lane & (JSTRIDE - 1));
         const uint32_t tbase = tmem + ((uint32_t)(quarter * 32 + half * 16) << 16) +
                                (uint32_t)q0 * (C::QROWS ? 8 : 4);
-        const int stage_n = SLOTS * nb * (NS + 1);
+        const int stage_n = slots * nb * (NS + 1);
         const int copy = PRIV ? e : 0;
         double* my_sacc = sacc + copy * stage_n;
-        unsigned* my_scnt = scnt + copy * SLOTS * nb * 2;
+        unsigned* my_scnt = scnt + copy * slots * nb * 2;
         double* my_fst = fstage + e * a.frows * C::FROW;
         uint32_t tcount = 0;
         for (uint32_t k = 0;; ++k) {
@@ -622,7 +642,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             int slot = 0;
             if (row_ok && a.snp_block) {
                 slot = a.snp_block[i] - blk0;
-                if (slot < 0 || slot >= SLOTS) {
+                if (slot < 0 || slot >= slots) {
                     atomicOr(a.status, LDK_DEVERR_BLOCK_SPAN);
                     row_ok = false;
                 }
@@ -645,12 +665,12 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             double nxt = sedges[0];
             // Adds the flushing lanes' sums into the staged sums; called by all 32 lanes.
             // The flushing lanes write their sums into rows of the warp's scratch (in
-            // batches of `frows`, all lanes of a batch at once), then the warp adds the
-            // rows one after the other, lane s taking value s, carrying the total while
-            // the (block, bin) stays the same.  One lane per round adding its own 46
+            // batches of `frows`, all lanes of a batch at once), then for every (block, bin)
+            // among them the warp adds the rows that hold it, lane s taking value s.  One lane per round adding its own 46
             // values took one pass per flushing lane of a key -- on average 6.5 for 200
-            // windows x 3 populations, 39.5 -> 35.4 ms with the rows; with shared staging
-            // (atomics) two genotype populations 2.77 -> 1.25 ms, four haplotype 4.72 -> 2.56.  With PRIV every epilogue warp owns its staged sums
+            // windows x 3 populations, 39.5 -> 32.4 ms with eight rows of odd stride (four
+            // rows: 33.5; rows added one after the other: 33.4); with shared staging
+            // (atomics) two genotype populations 2.77 -> 1.07 ms, four haplotype 4.72 -> 2.32.  With PRIV every epilogue warp owns its staged sums
             // and plain adds suffice; otherwise the warps share them (atomics).  The pairs are
             // counted by the first of two warps that share them.
             auto flush = [&](bool want) {
@@ -691,6 +711,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     return;
                 }
                 constexpr int VPL = (NA + 31) / 32;  // values per lane; lane 31 also adds the counts
+                constexpr int RB = C::FROWS_MAX;
                 for (int b0 = 0; b0 < total; b0 += a.frows) {
                     const int rows = total - b0 < a.frows ? total - b0 : a.frows;
                     if (want && rank >= b0 && rank < b0 + rows) {
@@ -702,21 +723,36 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                         *reinterpret_cast<int*>(row + NA + 1) = slot * nb + cur;
                     }
                     __syncwarp();
-                    int pk = -1;
-                    double d[VPL];
-                    uint2 dc = make_uint2(0u, 0u);
-                    auto put = [&]() {
+                    // lane r knows row r's key; one pass per key adds the rows that hold it
+                    const int my_key = lane < rows ? *reinterpret_cast<const int*>(my_fst + lane * C::FROW + NA + 1) : -1;
+                    unsigned left = (1u << rows) - 1u;
+                    do {
+                        const int kk = __shfl_sync(0xffffffffu, my_key, __ffs(left) - 1);
+                        const unsigned grp = __ballot_sync(0xffffffffu, my_key == kk);
+                        left &= ~grp;
 #pragma unroll
                         for (int v = 0; v < VPL; ++v) {
                             const int s = lane + 32 * v;
                             if (s < na) {
-                                double* dst = my_sacc + pk * (NS + 1) + gofs + s;
-                                if constexpr (PRIV) *dst = d[v];
-                                else atomicAdd(dst, d[v]);
+                                double* dst = my_sacc + kk * (NS + 1) + gofs + s;
+                                double d = PRIV ? *dst : 0.0;
+#pragma unroll
+                                for (int rr = 0; rr < RB; ++rr)
+                                    if ((grp >> rr) & 1u) d += my_fst[rr * C::FROW + s];
+                                if constexpr (PRIV) *dst = d;
+                                else atomicAdd(dst, d);
                             }
                         }
-                        if (lane == 31 && part == 0) {
-                            unsigned* dst = my_scnt + 2 * pk;
+                        if (part == 0 && lane == 31) {
+                            unsigned* dst = my_scnt + 2 * kk;
+                            uint2 dc = PRIV ? make_uint2(dst[0], dst[1]) : make_uint2(0u, 0u);
+#pragma unroll
+                            for (int rr = 0; rr < RB; ++rr)
+                                if ((grp >> rr) & 1u) {
+                                    const uint2 c = *reinterpret_cast<const uint2*>(my_fst + rr * C::FROW + NA);
+                                    dc.x += c.x;
+                                    dc.y += c.y;
+                                }
                             if constexpr (PRIV) {
                                 dst[0] = dc.x;
                                 dst[1] = dc.y;
@@ -725,32 +761,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                                 atomicAdd(dst + 1, dc.y);
                             }
                         }
-                    };
-                    for (int rr = 0; rr < rows; ++rr) {
-                        const double* row = my_fst + rr * C::FROW;
-                        const int kk = *reinterpret_cast<const int*>(row + NA + 1);
-                        if (kk != pk) {
-                            if (pk >= 0) put();
-                            pk = kk;
-#pragma unroll
-                            for (int v = 0; v < VPL; ++v) {
-                                const int s = lane + 32 * v;
-                                d[v] = PRIV && s < na ? my_sacc[kk * (NS + 1) + gofs + s] : 0.0;
-                            }
-                            if (lane == 31) dc = PRIV ? make_uint2(my_scnt[2 * kk], my_scnt[2 * kk + 1]) : make_uint2(0u, 0u);
-                        }
-#pragma unroll
-                        for (int v = 0; v < VPL; ++v) {
-                            const int s = lane + 32 * v;
-                            if (s < na) d[v] += row[s];
-                        }
-                        if (lane == 31) {
-                            const uint2 c = *reinterpret_cast<const uint2*>(row + NA);
-                            dc.x += c.x;
-                            dc.y += c.y;
-                        }
-                    }
-                    if (pk >= 0) put();
+                    } while (left);
                     __syncwarp();
                 }
                 }
@@ -761,23 +772,12 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             // cost the scheduler registers -- 200 windows x 3 populations 35.0 -> 37.4 ms, two
             // populations spilled.)
             constexpr int CREGS = (C::NJ + 31) / 32;  // partner coordinates per lane
-            uint32_t v[P][C::REGIONS][4];
-            auto issue = [&](uint32_t buf, int qq) {
-#pragma unroll
-                for (int p = 0; p < P; ++p)
-#pragma unroll
-                    for (int x = 0; x < C::REGIONS; ++x) {
-                        const uint32_t ta = tbase + buf * C::COLS + (p * C::REGIONS + x) * C::N + qq * (C::QROWS ? 8 : 4);
-                        if constexpr (C::QROWS) tmem_ld_q(ta, v[p][x]);
-                        else tmem_ld4(ta, v[p][x]);
-                    }
-            };
+            constexpr int U = C::U;
             bool ok = true;
             for (int t = tb; t < te; ++t, ++tcount) {
                 const uint32_t buf = tcount % C::NBUF, tph = (tcount / C::NBUF) & 1u;
                 const int j0 = row0 + t * C::NJ;
-                // partner coordinates of this tile, one per lane and register
-                double creg[CREGS];
+                double creg[CREGS];  // partner coordinates of this tile, one per lane and register
 #pragma unroll
                 for (int kk = 0; kk < CREGS; ++kk) {
                     const int j = j0 + 32 * kk + lane;
@@ -786,84 +786,120 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 if (!mbar_wait(&tfull[buf], tph, &abort_s, a.status)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll 1
-                for (int qq = 0; qq < C::MY_STEPS; ++qq) {
-                    issue(buf, qq);
-                    const int jj = jb + JSTRIDE * qq, j = j0 + jj;
-                    double csrc = creg[0];
+                for (int qq = 0; qq < C::MY_STEPS; qq += U) {
+                    uint32_t v[U][P][C::REGIONS][4];
+                    double dist[U];
+                    bool valid[U];
 #pragma unroll
-                    for (int kk = 1; kk < CREGS; ++kk)
-                        if ((jj >> 5) == kk) csrc = creg[kk];
-                    const double cj = __shfl_sync(0xffffffffu, csrc, jj & 31);
+                    for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int p = 0; p < P; ++p) tmem_wait4<C::REGIONS>(v[p]);
-                    SpinPop f[P];
-                    int nval[P];
+                        for (int p = 0; p < P; ++p)
 #pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        if constexpr (GENO) {
-                            // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma,
-                            // 1: sigma^2, 2: valid)
-                            const uint32_t (&G)[3][4] = v[p];
-                            f[p].R = i2d_exact((int)G[0][0]);
-                            f[p].STT = i2d_exact((int)G[0][1]);
-                            f[p].S = i2d_exact((int)G[0][2]);
-                            f[p].SST = i2d_exact((int)G[1][0]);
-                            f[p].SSTT = i2d_exact((int)G[1][1]);
-                            f[p].SS = i2d_exact((int)G[1][2]);
-                            f[p].T = i2d_exact((int)G[2][0]);
-                            f[p].TT = i2d_exact((int)G[2][1]);
-                            nval[p] = (int)G[2][2];
-                        } else if constexpr (C::QROWS) {
-                            f[p].R = i2d_exact((int)v[p][0][0]);
-                            f[p].S = i2d_exact((int)v[p][0][1]);
-                            f[p].T = i2d_exact((int)v[p][0][2]);
-                            nval[p] = (int)v[p][0][3];
-                        } else {
-                            // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
-                            const uint32_t* w = v[p][0];
-                            const uint32_t rx = __shfl_xor_sync(0xffffffffu, role ? w[0] : w[2], 1);
-                            const uint32_t ry = __shfl_xor_sync(0xffffffffu, role ? w[1] : w[3], 1);
-                            f[p].R = i2d_exact((int)(role ? rx : w[0]));
-                            f[p].S = i2d_exact((int)(role ? ry : w[1]));
-                            f[p].T = i2d_exact((int)(role ? w[2] : rx));
-                            nval[p] = (int)(role ? w[3] : ry);
-                        }
+                            for (int x = 0; x < C::REGIONS; ++x) {
+                                const uint32_t ta = tbase + buf * C::COLS + (p * C::REGIONS + x) * C::N +
+                                                    (qq + u) * (C::QROWS ? 8 : 4);
+                                if constexpr (C::QROWS) tmem_ld_q(ta, v[u][p][x]);
+                                else tmem_ld4(ta, v[u][p][x]);
+                            }
+                    bool any = false;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int jj = jb + JSTRIDE * (qq + u);
+                        double csrc = creg[0];
+#pragma unroll
+                        for (int kk = 1; kk < CREGS; ++kk)
+                            if ((jj >> 5) == kk) csrc = creg[kk];
+                        dist[u] = fabs(__shfl_sync(0xffffffffu, csrc, jj & 31) - ci);
+                        valid[u] = (unsigned)(j0 + jj - i - 1) < span;
+                        any |= valid[u] && dist[u] >= nxt;
                     }
-                    if (qq == C::MY_STEPS - 1) {
+                    const bool change = __ballot_sync(0xffffffffu, any) != 0u;
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int p = 0; p < P; ++p) tmem_wait4<C::REGIONS>(v[u][p]);
+                    SpinPop f[U][P];
+                    int nval[U][P];
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int p = 0; p < P; ++p) {
+                            SpinPop& m = f[u][p];
+                            if constexpr (GENO) {
+                                // G[x][y]: plane x of SNP i . plane y of SNP j (0: sigma,
+                                // 1: sigma^2, 2: valid)
+                                const uint32_t (&G)[3][4] = v[u][p];
+                                m.R = i2d_exact((int)G[0][0]);
+                                m.STT = i2d_exact((int)G[0][1]);
+                                m.S = i2d_exact((int)G[0][2]);
+                                m.SST = i2d_exact((int)G[1][0]);
+                                m.SSTT = i2d_exact((int)G[1][1]);
+                                m.SS = i2d_exact((int)G[1][2]);
+                                m.T = i2d_exact((int)G[2][0]);
+                                m.TT = i2d_exact((int)G[2][1]);
+                                nval[u][p] = (int)G[2][2];
+                            } else if constexpr (C::QROWS) {
+                                m.R = i2d_exact((int)v[u][p][0][0]);
+                                m.S = i2d_exact((int)v[u][p][0][1]);
+                                m.T = i2d_exact((int)v[u][p][0][2]);
+                                nval[u][p] = (int)v[u][p][0][3];
+                            } else {
+                                // lane 2r: (R, S) of partners 2q, 2q+1; lane 2r+1: (T, n)
+                                const uint32_t* w = v[u][p][0];
+                                const uint32_t rx = __shfl_xor_sync(0xffffffffu, role ? w[0] : w[2], 1);
+                                const uint32_t ry = __shfl_xor_sync(0xffffffffu, role ? w[1] : w[3], 1);
+                                m.R = i2d_exact((int)(role ? rx : w[0]));
+                                m.S = i2d_exact((int)(role ? ry : w[1]));
+                                m.T = i2d_exact((int)(role ? w[2] : rx));
+                                nval[u][p] = (int)(role ? w[3] : ry);
+                            }
+                        }
+                    if (qq == C::MY_STEPS - U) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&tempty[buf]);
                     }
-                    const bool valid = (unsigned)(j - i - 1) < span;
-                    const double dist = fabs(cj - ci);
-                    const bool change = valid && dist >= nxt;
-                    if (__ballot_sync(0xffffffffu, change)) {
-                        const bool want = change && in_bin && np > 0;
-                        if (__ballot_sync(0xffffffffu, want)) flush(want);
-                        if (change) {
-                            cur = bin_advance(sedges, nb, cur, dist);
-                            nxt = cur < nb ? sedges[cur + 1] : CUDART_INF;
-                            in_bin = (unsigned)cur < (unsigned)nb;
-#pragma unroll
-                            for (int s = 0; s < NA; ++s) acc[s] = 0.0;
-                            np = nr2 = 0;
-                        }
-                    }
-                    if (valid && in_bin) {
+                    auto evaluate = [&](int u, bool counts) {  // pair u into the current bin's sums
 #pragma unroll
                         for (int p = 0; p < P; ++p) {
-                            f[p].n = i2d_exact(nval[p]);
-                            if constexpr (GENO) spin_reciprocals(f[p], a.gtab[nval[p]]);
-                            else if constexpr (GT) spin_reciprocals(f[p], a.rtab_g[nval[p]]);
-                            else spin_reciprocals(f[p], rtab[nval[p]]);
+                            SpinPop& m = f[u][p];
+                            m.n = i2d_exact(nval[u][p]);
+                            if constexpr (GENO) spin_reciprocals(m, a.gtab[nval[u][p]]);
+                            else if constexpr (GT) spin_reciprocals(m, a.rtab_g[nval[u][p]]);
+                            else if constexpr (P == 1) m.r4 = rtab[nval[u][p]];
+                            else spin_reciprocals(m, rtab[nval[u][p]]);
+                            if (U > 1 && !counts) m.r1 = m.r2 = m.r3 = m.r4 = 0.0;
                         }
                         if constexpr (SSPL) {
-                            if (part == 0) spin_stats<P, GENO, 1>(f, acc, nr2);
-                            else spin_stats<P, GENO, 2>(f, acc, nr2);
+                            if (part == 0) spin_stats<P, GENO, 1>(f[u], counts, acc, nr2);
+                            else spin_stats<P, GENO, 2>(f[u], counts, acc, nr2);
                         } else {
-                            spin_stats<P, GENO, 0>(f, acc, nr2);
+                            spin_stats<P, GENO, 0>(f[u], counts, acc, nr2);
                         }
-                        ++np;
+                        np += counts;
+                    };
+                    if (U > 1 && !change) {
+                        // every pair stays in its lane's bin: evaluated together, without branches
+#pragma unroll
+                        for (int u = 0; u < U; ++u) evaluate(u, valid[u] && in_bin);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const bool step = valid[u] && dist[u] >= nxt;
+                            if (U == 1 ? change : __ballot_sync(0xffffffffu, step) != 0u) {
+                                const bool want = step && in_bin && np > 0;
+                                if (__ballot_sync(0xffffffffu, want)) flush(want);
+                                if (step) {
+                                    cur = bin_advance(sedges, nb, cur, dist[u]);
+                                    nxt = cur < nb ? sedges[cur + 1] : CUDART_INF;
+                                    in_bin = (unsigned)cur < (unsigned)nb;
+#pragma unroll
+                                    for (int s = 0; s < NA; ++s) acc[s] = 0.0;
+                                    np = nr2 = 0;
+                                }
+                            }
+                            if (valid[u] && in_bin) evaluate(u, true);
+                        }
                     }
                 }
             }
@@ -887,11 +923,11 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + spin_stat<P, GENO>(s)) * kFxLimbs, val * spin_weight<P, GENO>(s),
                            a.status);
             }
-            for (int idx = et; idx < SLOTS * nb; idx += 32 * EPI) {
+            for (int idx = et; idx < slots * nb; idx += 32 * EPI) {
                 unsigned long long c0 = 0, c1 = 0;
 #pragma unroll
                 for (int w = 0; w < NCOPY; ++w) {
-                    unsigned* sc = scnt + w * SLOTS * nb * 2;
+                    unsigned* sc = scnt + w * slots * nb * 2;
                     c0 += sc[2 * idx];
                     c1 += sc[2 * idx + 1];
                     sc[2 * idx] = 0u;
@@ -962,6 +998,14 @@ size_t smem_bytes_t(int nb, int table, int ncopy, int frows = 0) {
            (size_t)frows * C::EPI * C::FROW * sizeof(double);
 }
 
+// Ring stages in `room` bytes: C::STAGES, or as many as fit (two stages of 48 KB left the MMAs of
+// 2,000 haplotypes waiting 1,000 cycles a chunk for their loads; three: 20.7 -> 20.3 ms).
+template <class C>
+int ring_stages(size_t room) {
+    const size_t n = room / C::STAGE_BYTES;
+    return C::MORE_STAGES && n > (size_t)C::STAGES ? (int)std::min<size_t>(n, kMaxStages) : C::STAGES;
+}
+
 // Reciprocal table entries held in shared memory (none on the genotype path, none when the
 // table lives in the workspace).
 inline int smem_table(const ParseShape& sh) { return (sh.genotypes || sh.rtab_global) ? 0 : sh.max_n + 1; }
@@ -1025,13 +1069,22 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     a.status = w.status;
     a.rtab_g = static_cast<const double4*>(w.rtab);
     a.gtab = static_cast<const double4*>(w.gtab);
+    const int ncopy = PRIV ? C::EPI : 1;
+    // What decides the staging (per-warp copies, the reciprocal table's place) is sized with
+    // every slot and C::STAGES streamed stages; what this call leaves of shared memory goes to
+    // flush rows, then to the ring.
+    a.slots = sh.slots;
+    size_t other = 1024 + (size_t)ncopy * a.slots * d->n_bins * (C::NS + 1) * sizeof(double) +
+                   (size_t)((ncopy * a.slots * d->n_bins * 2 + 7) & ~7) * sizeof(unsigned) +
+                   (size_t)(smem_table(sh) ? (sh.max_n + 2) & ~1 : 0) * sizeof(typename C::Recip) + 32;
+    const size_t row = (size_t)C::EPI * C::FROW * sizeof(double), full = kMaxSmem - kStaticSmem;
+    a.frows = C::FROWS_MAX;
+    while (a.frows > 0 && other + (size_t)C::STAGES * C::STAGE_BYTES + a.frows * row > full) a.frows >>= 1;
+    other += a.frows * row;
+    a.stages = ring_stages<C>(full > other ? full - other : 0);
+    size_t smem = other + (size_t)a.stages * C::STAGE_BYTES;
     // at least half of an SM's shared memory, so that one CTA (holding all 512 TMEM
     // columns) runs per SM
-    const int ncopy = PRIV ? C::EPI : 1;
-    a.frows = C::FROWS_MAX;  // as many flush rows as fit beside what decides the staging
-    while (a.frows > 0 && smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows) + kStaticSmem > kMaxSmem)
-        a.frows >>= 1;
-    size_t smem = smem_bytes_t<P, GENO, V>(d->n_bins, smem_table(sh), ncopy, a.frows);
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
