@@ -89,6 +89,9 @@ bool shape_of(const ldk_parse_t* d, ParseShape& sh) {
 }
 
 int window_count(const ldk_parse_t* d) { return d->window_offsets ? d->n_windows : 1; }
+// One window needs no plan in the workspace: its bounds go with the launches and its row blocks
+// follow from them.
+bool planless(const ldk_parse_t* d) { return window_count(d) == 1; }
 
 int64_t window_bound(const ldk_parse_t* d, int w) {
     if (d->window_offsets) return d->window_offsets[w];
@@ -239,7 +242,7 @@ int prepare(const ldk_parse_t* d, void* workspace, size_t workspace_bytes, Prepa
     P.w.win_off = reinterpret_cast<int64_t*>(ws + P.L.win_off);
     P.w.anc_end = P.w.win_off + window_count(d) + 1;
     P.w.fx = reinterpret_cast<unsigned long long*>(ws + P.L.fx_off);
-    P.w.row_blocks = reinterpret_cast<int32_t*>(ws + P.L.rb_off);
+    P.w.row_blocks = planless(d) ? nullptr : reinterpret_cast<int32_t*>(ws + P.L.rb_off);
     P.w.items = reinterpret_cast<int32_t*>(ws + P.L.items_off);
     P.w.hv = ws + P.L.hv_off;
     P.w.rtab = P.sh.rtab_global ? static_cast<void*>(ws + P.L.rtab_off) : nullptr;
@@ -262,6 +265,7 @@ int check_outputs(const ldk_parse_out_t* out) {
 // order.  Each launch splits it into work items (launch_split_items), which the kernel's
 // CTAs claim in list order.
 int upload_items(const ldk_parse_t* d, const Prepared& P, cudaStream_t s, int claim_order) {
+    if (planless(d)) return LDK_OK;
     int rc;
     const int rows = tc_rows_per_block(P.sh);
     std::vector<int> order(window_count(d));
@@ -290,6 +294,7 @@ int upload_items(const ldk_parse_t* d, const Prepared& P, cudaStream_t s, int cl
 // row-block list in the tuned claim order (largest windows first if the shape is untuned)
 // -- or, with device_items, the list is built on the device in window order.
 int upload_plan(const ldk_parse_t* d, const Prepared& P, cudaStream_t s, bool device_items) {
+    if (planless(d)) return LDK_OK;
     int rc;
     const int nw = window_count(d);
     std::vector<int64_t> woff(2 * nw + 1);  // window offsets, then anchor ends (the workspace layout)
@@ -319,6 +324,14 @@ int clear(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepared& P, c
     return LDK_OK;
 }
 
+// What a parse clears before its kernels: everything, or for the tensor-core method (whose
+// preparation kernel clears its accumulators and whose bin sums are written, not added) the
+// status block.
+int clear_for(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepared& P, cudaStream_t s) {
+    if (d->n_var < 2 || d->method == LDK_METHOD_PLAIN_FP64) return clear(d, out, P, s);
+    return check_cuda(cudaMemsetAsync(P.ws + P.L.status_off, 0, 256, s), "memset");
+}
+
 // Device work of one parse (after the plan is in the workspace): pair ranges, spin
 // planes and the parse kernel.  Host work: tensor-map encoding and launch configuration.
 // ---- autotuning: the fastest (tile variant, row-block order) per shape class (ldk_tune.cu)
@@ -337,6 +350,22 @@ bool autotune_on() {
 int tuned_variant(const ldk_parse_t* d, const ParseShape& sh) {
     TuneChoice c;
     return tune_lookup(tune_key_of(d, sh), &c) ? c.variant : -1;
+}
+
+// The variant a call runs: the tuned one, else the default -- for one haplotype population the
+// narrower tile where the wide one leaves most SMs without a tile (an upper bound: every pair of
+// every window within the cutoff).
+int variant_of(const ldk_parse_t* d, const ParseShape& sh) {
+    const int v = tuned_variant(d, sh);
+    if (v >= 0) return v;
+    if (sh.genotypes || sh.P != 1 || sh.rtab_global) return 0;
+    const int64_t rows = tc_rows_per_block(sh), nj = tc_tile_width(sh, 0);
+    int64_t tiles = 0;
+    for (int w = 0; w < window_count(d) && tiles <= kSpreadCtas; ++w) {
+        const int64_t m = window_bound(d, w + 1) - window_bound(d, w);
+        tiles += (m + rows - 1) / rows * ((m + 2 * nj - 1) / (2 * nj));
+    }
+    return tiles <= kSpreadCtas ? 1 : 0;
 }
 
 // Candidates worth timing: the alternative tile only where its width differs, the window
@@ -376,23 +405,20 @@ int enqueue_device(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepa
     int rc;
     ldk_parse_t dd = *d;
     dd.n_windows = window_count(d);
-    if ((rc = check_cuda(launch_jmax(&dd, P.w, s), "pair ranges"))) return rc;
     if (d->method == LDK_METHOD_PLAIN_FP64) {
+        if ((rc = check_cuda(launch_jmax(&dd, P.w, s), "pair ranges"))) return rc;
         if (prof) cudaEventRecord(g_ev[0], s);
         if ((rc = check_cuda(launch_parse_plain(&dd, out, P.w, P.sh, s), "plain parse"))) return rc;
         if (prof) cudaEventRecord(g_ev[1], s);
         if ((rc = check_cuda(launch_fx_finish(&dd, out, P.w, P.sh.n_stats, s), "bin sums"))) return rc;
     } else {
-        if ((rc = check_cuda(launch_prep_planes(&dd, P.w, P.sh, s), "spin planes"))) return rc;
-        if (P.w.rtab && (rc = check_cuda(launch_fill_rtab(P.w.rtab, P.sh.max_n, s), "reciprocal table"))) return rc;
-        if (P.w.gtab && (rc = check_cuda(launch_fill_gtab(P.w.gtab, P.sh.max_n, s), "reciprocal table"))) return rc;
+        if ((rc = check_cuda(launch_prep_planes(&dd, P.w, P.sh, out, s), "pair ranges and spin planes"))) return rc;
         if (tune && n_variants(d, P.sh) * n_orders(d) > 1 && tuned_variant(d, P.sh) < 0) {
             if ((rc = autotune_tc(&dd, out, P, s))) return rc;
             // the candidate runs left their sums and a spent row-block counter behind
             if ((rc = clear(&dd, out, P, s))) return rc;
         }
-        const int v = tuned_variant(d, P.sh);
-        if ((rc = check_cuda(launch_tc(&dd, out, P, v < 0 ? 0 : v, s, prof), "tensor-core parse"))) return rc;
+        if ((rc = check_cuda(launch_tc(&dd, out, P, variant_of(d, P.sh), s, prof), "tensor-core parse"))) return rc;
         if ((rc = check_cuda(launch_fx_finish(&dd, out, P.w, P.sh.n_stats, s), "bin sums"))) return rc;
     }
     return LDK_OK;
@@ -465,7 +491,7 @@ int ldk::parse_impl(const ldk_parse_t* d, const ldk_parse_out_t* out, void* work
     Prepared P;
     if (int rc = prepare(d, workspace, workspace_bytes, P)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = clear(d, out, P, s)) return rc;
+    if (int rc = clear_for(d, out, P, s)) return rc;
     if (d->n_var < 2) return LDK_OK;
     if (int rc = upload_plan(d, P, s, device_items)) return rc;
     const bool prof = !device_items && g_prof && prof_events();
@@ -609,7 +635,7 @@ int ldk_parse_enqueue(const ldk_parse_t* d, const ldk_parse_out_t* out, void* wo
     Prepared P;
     if (int rc = prepare(d, workspace, workspace_bytes, P)) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (int rc = clear(d, out, P, s)) return rc;
+    if (int rc = clear_for(d, out, P, s)) return rc;
     if (d->n_var < 2) return LDK_OK;
     return enqueue_device(d, out, P, s, false);
 }
@@ -655,8 +681,7 @@ int ldk_tile_width(const ldk_parse_t* d) {
     if (d->method == LDK_METHOD_PLAIN_FP64) return 0;
     ParseShape sh;
     shape_of(d, sh);
-    const int v = tuned_variant(d, sh);
-    return tc_tile_width(sh, v < 0 ? 0 : v);
+    return tc_tile_width(sh, variant_of(d, sh));
 }
 
 int ldk_parse_reproducible(const ldk_parse_t* d) {
@@ -664,8 +689,7 @@ int ldk_parse_reproducible(const ldk_parse_t* d) {
     if (d->method == LDK_METHOD_PLAIN_FP64) return 1;
     ParseShape sh;
     shape_of(d, sh);
-    const int v = tuned_variant(d, sh);
-    return tc_private_staging(sh, v < 0 ? 0 : v) ? 1 : 0;
+    return tc_private_staging(sh, variant_of(d, sh)) ? 1 : 0;
 }
 
 int ldk_tc_row_blocks(int genotypes, int32_t* rows, int32_t* max_blocks) {

@@ -70,7 +70,8 @@ cudaError_t launch_site_counts(const int8_t* X, int64_t ld, int64_t n_var, const
                                int32_t* valid, cudaStream_t s);
 
 // launchers (ldk_tc.cu)
-cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh,
+// o null: the planes only (all-pairs LD)
+cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh, const ldk_parse_out_t* o,
                                cudaStream_t s);
 // max_items bounds the work items in w (their count is on the device): at most that many CTAs
 cudaError_t launch_parse_tc(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
@@ -90,17 +91,16 @@ cudaError_t probe_peaks(double* int8_ops_per_s, double* fp64_fma_per_s, unsigned
 size_t tc_smem_bytes(const ParseShape& sh);
 bool tc_rtab_global(const ParseShape& sh);  // where the reciprocal table must live
 bool tc_private_staging(const ParseShape& sh, int variant);  // one staging copy per epilogue warp
-cudaError_t launch_fill_rtab(void* rtab, int max_n, cudaStream_t s);
-cudaError_t launch_fill_gtab(void* gtab, int max_n, cudaStream_t s);
 
 cudaError_t launch_build_items(const Scratch& w, int n_windows, int rows, cudaStream_t s);
 // Work items of the tensor-core parse: each row block of w.row_blocks split into pieces of
-// at most c partner tiles of width nj, c = max(min_tiles, ceil(total tiles / kItemTarget)),
+// at most c partner tiles of width nj, c = max(min(min_tiles, ceil(total tiles / kSpreadCtas)), ceil(total tiles / kItemTarget)),
 // from the pair ranges in w.jmax; the count goes to *w.n_items.  At most
 // n_row_blocks + kItemTarget items.  min_tiles = tc_min_item_tiles(shape): every item ends
 // with a flush of the epilogue's staged sums (block slots x bins x (statistics + 1) values),
 // so an item is kept at least one tile per kFlushValuesPerTile staged values long.
 constexpr int kItemTarget = 2048;
+constexpr int kSpreadCtas = 148;  // SMs: fewer tiles than these are spread one by one
 constexpr int kMinItemTiles = 4;
 constexpr int kFlushValuesPerTile = 64;
 inline int tc_item_capacity(int n_row_blocks) { return n_row_blocks + kItemTarget; }

@@ -548,7 +548,7 @@ cudaError_t launch_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const
     sh.ktot = L.ktot;
     for (int p = 0; p <= LDK_MAX_POPS; ++p) sh.kofs[p] = p == 0 ? 0 : (n_sel + 31) / 32 * 32;
     sh.max_n = n_sel;
-    if ((e = launch_prep_planes(&d, w, sh, s)) != cudaSuccess) return e;
+    if ((e = launch_prep_planes(&d, w, sh, nullptr, s)) != cudaSuccess) return e;
     // items of one tile at least: unlike the parse's, they end without a flush
     if ((e = launch_split_items(w, L.n_row_blocks, nine ? LdmGCfg::NJ : LdmCfg::NJ, 1, L.rows, (int)n_var, s)) !=
         cudaSuccess)

@@ -5,6 +5,7 @@
 
 #include "ldk_estimators.cuh"
 #include "ldk_internal.h"
+#include "ldk_jmax.cuh"
 
 namespace ldk {
 
@@ -183,36 +184,9 @@ __global__ void k_r_family(int which, const double* __restrict__ counts, const d
     }
 }
 
-// ---------------------------------------------------------------------------
-// pair ranges: jmax[i] = end of SNP i's partners (cutoff on pos, window end); i + 1 for
-// SNPs after their window's anchor end (a split parse's right halo)
-// ---------------------------------------------------------------------------
-
-__global__ void k_jmax(const double* __restrict__ pos, const double* __restrict__ coord, int64_t n_var, const int64_t* __restrict__ win_off,
-                       const int64_t* __restrict__ anc_end, int n_win, double max_dist, const int32_t* __restrict__ snp_block, int n_blocks,
-                       int32_t* __restrict__ jmax, unsigned* __restrict__ status) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n_var;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        int lo = 0, hi = n_win;  // window w with win_off[w] <= i < win_off[w+1]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (win_off[mid] <= i) lo = mid; else hi = mid;
-        }
-        const int64_t we = win_off[lo + 1];
-        const double lim = pos[i] + max_dist;
-        int64_t a = i + 1, b = we;  // first j in [i+1, we) with pos[j] > lim
-        while (a < b) {
-            const int64_t m = (a + b) >> 1;
-            if (pos[m] <= lim) a = m + 1; else b = m;
-        }
-        jmax[i] = (int32_t)(i < anc_end[lo] ? a : i + 1);  // SNPs past the anchors have no pairs of their own
-        if (i + 1 < we && pos[i + 1] < pos[i]) atomicOr(status, LDK_DEVERR_BAD_INPUT);
-        if (coord && i + 1 < we && coord[i + 1] < coord[i]) atomicOr(status, LDK_DEVERR_BAD_INPUT);
-        if (snp_block) {
-            const int blk = snp_block[i];
-            if (blk < 0 || blk >= n_blocks) atomicOr(status, LDK_DEVERR_BLOCK_RANGE);
-        }
-    }
+__global__ void k_jmax(const JmaxArgs a) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n_var; i += (int64_t)gridDim.x * blockDim.x)
+        pair_range(a, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -513,9 +487,7 @@ cudaError_t launch_r_family(int which, const double* counts, const double* n_val
 
 cudaError_t launch_jmax(const ldk_parse_t* d, const Scratch& w, cudaStream_t s) {
     if (d->n_var == 0) return cudaSuccess;
-    k_jmax<<<blocks_for(d->n_var), kThreads, 0, s>>>(d->pos, d->coord, d->n_var, w.win_off, w.anc_end, d->n_windows,
-                                                      d->max_dist,
-                                                      d->snp_block, d->n_blocks, w.jmax, w.status);
+    k_jmax<<<blocks_for(d->n_var), kThreads, 0, s>>>(jmax_args(d, w));
     return cudaGetLastError();
 }
 

@@ -1,6 +1,7 @@
 // Tensor-core path of the binned parse: spin-plane preparation, tile-variant
 // dispatch and the peak probes (the kernel itself is in ldk_tc_kernel.cuh).
 #include "ldk_tc_kernel.cuh"
+#include "ldk_jmax.cuh"
 
 namespace ldk {
 
@@ -23,6 +24,13 @@ struct PrepArgs {
     int planes;
     uint8_t* planes_out;
     unsigned* status;
+    // a parse's other preparations, in the blocks of one more y slice (slice < 0: none)
+    int slice;
+    JmaxArgs ranges;
+    unsigned long long* zero[3];  // accumulators to clear and their 64-bit words
+    int64_t zero_n[3];
+    double4* table;  // reciprocal table in the workspace, or null
+    int table_n;
 };  // X: int8 codes, or (PACKED) 2-bit codes + 1, four SNPs per byte (LDK_X_PACKED2)
 
 constexpr int kPrepV = 128, kPrepK = 128;
@@ -48,12 +56,32 @@ constexpr int kPrepV = 128, kPrepK = 128;
 // The second word is read only where it holds SNPs of the quad, and an aligned word holding
 // one byte of the matrix lies in that byte's memory page, so no read can fault; its other
 // bytes are shifted or masked out.
+// Pair ranges of the block's 128 SNPs (first half of the threads); zeroed accumulators and the
+// reciprocal table (second half).
+template <bool GENO>
+LDK_DEV void prepare_rest(const PrepArgs& a) {
+    if (threadIdx.x < 128) {
+        const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+        if (i < a.n_var) pair_range(a.ranges, i);
+        return;
+    }
+    const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x - 128, step = (int64_t)gridDim.x * 128;
+#pragma unroll
+    for (int z = 0; z < 3; ++z)
+        for (int64_t k = t; k < a.zero_n[z]; k += step) a.zero[z][k] = 0ull;
+    for (int64_t k = t; k < a.table_n; k += step) a.table[k] = GENO ? recip_entry_geno((int)k) : recip_entry((int)k);
+}
+
 template <bool GENO, bool PACKED, int PL = GENO ? 4 : 2>
 __global__ void __launch_bounds__(256) k_prep_planes(PrepArgs a) {
     constexpr int RS = kPrepK + 4;  // bytes per SNP row: 33 words, so the scatter's word loads
                                     // (one K quad per lane) hit distinct banks
     __shared__ __align__(16) int8_t tile[kPrepV * RS];
     __shared__ int srow[kPrepK];
+    if ((int)blockIdx.y == a.slice) {
+        prepare_rest<GENO>(a);
+        return;
+    }
     const int64_t v0 = (int64_t)blockIdx.x * kPrepV;
     const int k0 = blockIdx.y * kPrepK;
     constexpr int xmax = GENO ? 2 : 1;
@@ -257,33 +285,16 @@ bool tc_rtab_global(const ParseShape& sh) {
     }
 }
 
-namespace {
-__global__ void k_fill_rtab(double4* t, int max_n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= max_n) t[i] = recip_entry(i);
-}
-}  // namespace
-
-namespace {
-__global__ void k_fill_gtab(double4* t, int max_n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= max_n) t[i] = recip_entry_geno(i);
-}
-}  // namespace
-
-cudaError_t launch_fill_gtab(void* gtab, int max_n, cudaStream_t s) {
-    k_fill_gtab<<<(max_n + 256) / 256, 256, 0, s>>>(static_cast<double4*>(gtab), max_n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fill_rtab(void* rtab, int max_n, cudaStream_t s) {
-    k_fill_rtab<<<(max_n + 256) / 256, 256, 0, s>>>(static_cast<double4*>(rtab), max_n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh, cudaStream_t s) {
+// The spin planes, and with `o` the rest of a parse's preparation in the same launch: pair
+// ranges, the cleared accumulators and pair tallies, the reciprocal table.  (Separate kernels and
+// memsets each waited for the one before: with the outputs' own memsets, which the bin sums
+// overwrite anyway, thirteen operations for a window of 400 SNPs, 92 us a call; five, 56, of which the narrower tile and
+// one-tile pieces on more SMs give 18.)
+cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh, const ldk_parse_out_t* o,
+                               cudaStream_t s) {
     if (d->n_var == 0) return cudaSuccess;
-    PrepArgs a;
+    PrepArgs a{};
+    a.slice = -1;
     a.X = d->X;
     a.ld = d->ld_x;
     a.n_var = d->n_var;
@@ -299,6 +310,24 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
     a.planes_out = w.hv;
     a.status = w.status;
     dim3 grid((unsigned)((d->n_var + kPrepV - 1) / kPrepV), (unsigned)(sh.ktot / kPrepK));
+    if (o) {
+        a.slice = (int)grid.y++;
+        a.ranges = jmax_args(d, w);
+        const int64_t cells = (int64_t)d->n_blocks * d->n_bins;
+        a.zero[0] = w.fx;
+        a.zero_n[0] = cells * (sh.n_stats + 1) * kFxLimbs;
+        a.zero[1] = reinterpret_cast<unsigned long long*>(o->pairs);
+        a.zero[2] = reinterpret_cast<unsigned long long*>(o->r2_counts);
+        a.zero_n[1] = a.zero_n[2] = cells;
+        // more than a few words a thread (many blocks of few SNPs): by memset
+        if (a.zero_n[0] > 64ll * 128 * grid.x) {
+            cudaError_t e = cudaMemsetAsync(w.fx, 0, a.zero_n[0] * sizeof(unsigned long long), s);
+            if (e != cudaSuccess) return e;
+            a.zero_n[0] = 0;
+        }
+        a.table = static_cast<double4*>(w.rtab ? w.rtab : w.gtab);
+        a.table_n = a.table ? sh.max_n + 1 : 0;
+    }
     const bool packed = d->x_format == LDK_X_PACKED2;
     if (sh.genotypes && sh.planes == 2) {
         k_prep_planes<true, false, 2><<<grid, 256, 0, s>>>(a);
@@ -316,7 +345,8 @@ namespace {
 // Work items of the persistent parse kernel.  A row block alone is too coarse a unit where
 // there are few row blocks per SM (a 5,000-SNP window has 79) or where their count leaves a
 // partial last wave; pieces of at most c partner tiles bound the spread of the CTAs' finishing
-// times by one piece.  c = max(min_tiles, ceil(total tiles / kItemTarget)), so shapes with
+// times by one piece.  c = max(min_tiles, ceil(total tiles / kItemTarget)) -- min_tiles at
+// most the tiles there are per SM -- so shapes with
 // many small row blocks keep one item per row block, and no piece is so short that the flush
 // of its staged sums (which ends every item) outweighs its tiles.  Pieces of one row block are consecutive
 // (the claim order of the row blocks stays), its last piece runs to INT32_MAX, and a row block
@@ -361,8 +391,9 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
     long long total = 0;
 #pragma unroll 4
     for (int x = 0; x < NW; ++x) total += s_sum[x];
-    const long long cl = (total + kItemTarget - 1) / kItemTarget;
-    const int c = cl > min_tiles ? (int)cl : min_tiles;
+    const long long cl = (total + kItemTarget - 1) / kItemTarget, spread = (total + kSpreadCtas - 1) / kSpreadCtas;
+    const int least = spread < min_tiles ? (spread > 0 ? (int)spread : 1) : min_tiles;
+    const int c = cl > least ? (int)cl : least;
     for (int b0 = 0; b0 < n_rb; b0 += kSplitThreads) {
         const int k = b0 + tid;
         const int nt = k < n_rb ? rb_tiles(rb, jmax, k, nj) : 0;

@@ -46,6 +46,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -1093,10 +1094,14 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     if constexpr (C::SPLIT) {
         // the register split adds up only at C::REG_LAUNCH registers per thread; any other
         // allocation would leave setmaxnreg.inc waiting, so such a build is not launched
-        cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT>);
-        if (e != cudaSuccess) return e;
-        if (fa.numRegs != C::REG_LAUNCH) return cudaErrorInvalidKernelImage;
+        static std::atomic<int> regs{-1};  // of this build's kernel: asked for once
+        if (regs.load() < 0) {
+            cudaFuncAttributes fa;
+            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT>);
+            if (e != cudaSuccess) return e;
+            regs.store(fa.numRegs);
+        }
+        if (regs.load() != C::REG_LAUNCH) return cudaErrorInvalidKernelImage;
     }
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
