@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     const uint32_t tmem = tmem_base_s;
     const Pipe pipe{su32(stages), full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
     if (warp == 0) run_producer<C, true>(pipe, &tmA, &tmB, a, lane);
-    else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
+    else if (warp == 1) run_mma<C, 1>(pipe, tmem, a);
     if (warp >= 4) {
         // thread: SNP `r` of the row block, partners jb + 4 step of the tile
         const int e = warp - 4, quarter = warp & 3, half = (e >> 2) & 1, share = e >> 3;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     const uint32_t tmem = tmem_base_s;
     const Pipe pipe{su32(stages), full_bar, empty_bar, tfull, tempty, ifull, iempty, ring, &abort_s};
     if (warp == 0) run_producer<C, false>(pipe, &tmA, &tmB, a, lane);
-    else if (warp == 1) run_mma<C, 1>(pipe, tmem, a, lane);
+    else if (warp == 1) run_mma<C, 1>(pipe, tmem, a);
     if (warp >= 4) {
         // lane = SNP of the row block (32 per warp); the warp takes half `part` of every tile
         const int e = warp - 4, quarter = warp & 3, part = e >> 2;

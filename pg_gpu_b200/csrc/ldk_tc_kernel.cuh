@@ -255,6 +255,30 @@ LDK_DEV void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
+// The same from a whole warp, issued by the lane whose `one` is set: predicated, not branched,
+// so that the descriptors stay in uniform registers.
+LDK_DEV void mma_i8_one(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc, uint32_t one) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(one));
+}
+LDK_DEV void mma_commit_one(uint64_t* bar, uint32_t one) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(su32(bar)),
+        "r"(one)
+        : "memory");
+}
+LDK_DEV uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
+
 LDK_DEV void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -423,7 +447,7 @@ LDK_DEV void load_rows(uint32_t dst, const CUtensorMap* tmA, uint64_t* bar, int 
 
 // MMAs of K chunk c (staged at a_addr) into accumulator buffer buf.
 template <class C, int P>
-LDK_DEV void issue_mmas(uint32_t tmem, const TcArgs& a, uint32_t a_addr, int c, uint32_t buf) {
+LDK_DEV void issue_mmas(uint32_t tmem, const TcArgs& a, uint32_t a_addr, int c, uint32_t buf, uint32_t one) {
     constexpr uint32_t idesc = idesc_s8<C::N>();
     const uint32_t b_addr = a_addr + C::A_BYTES;
 #pragma unroll
@@ -436,7 +460,7 @@ LDK_DEV void issue_mmas(uint32_t tmem, const TcArgs& a, uint32_t a_addr, int c, 
 #pragma unroll
         for (int x = 0; x < C::REGIONS; ++x) {
             const uint32_t d = tmem + buf * C::COLS + (p * C::REGIONS + x) * C::N;
-            mma_i8(d, sw128_desc(a_addr + x * C::A_BOX + ks * 32), sw128_desc(b_addr + ks * 32), idesc, first ^ 1u);
+            mma_i8_one(d, sw128_desc(a_addr + x * C::A_BOX + ks * 32), sw128_desc(b_addr + ks * 32), idesc, first ^ 1u, one);
         }
     }
 }
@@ -479,37 +503,39 @@ LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorM
     __syncwarp();
 }
 
-// Warp 1: one thread issues the MMAs of every tile into the double-buffered accumulators.
+// Warp 1: the MMAs of every tile into the double-buffered accumulators.  The whole warp runs the
+// loop, one elected lane issues: in code that only one lane runs, every MMA's descriptors went
+// through vector registers, and issuing took longer than the small MMAs themselves.
 template <class C, int P>
-LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a, int lane) {
-    if (lane == 0) {
-        const int nst = C::MORE_STAGES ? a.stages : C::STAGES;
-        int s = 0;
-        uint32_t ph = 0, tcount = 0;
-        bool ok = true;
-        for (uint32_t k = 0; ok; ++k) {
-            const int sl = k % kRing;
-            if (!mbar_wait(&S.ifull[sl], (k / kRing) & 1u, S.abort_s, a.status)) { ok = false; break; }
-            const int item = S.ring[sl], n_jt = S.ring[kRing + sl];
-            mbar_arrive(&S.iempty[sl]);
-            if (item < 0) break;
-            for (int t = 0; t < n_jt && ok; ++t, ++tcount) {
-                const uint32_t buf = tcount % C::NBUF, tph = (tcount / C::NBUF) & 1u;
-                if (!mbar_wait(&S.tempty[buf], tph ^ 1u, S.abort_s, a.status)) { ok = false; break; }
+LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a) {
+    const int nst = C::MORE_STAGES ? a.stages : C::STAGES;
+    const uint32_t one = elect_one();
+    int s = 0;
+    uint32_t ph = 0, buf = 0, tph = 0;
+    bool ok = true;
+    for (uint32_t k = 0; ok; ++k) {
+        const int sl = k % kRing;
+        if (!__all_sync(0xffffffffu, mbar_wait(&S.ifull[sl], (k / kRing) & 1u, S.abort_s, a.status))) { ok = false; break; }
+        const int item = __shfl_sync(0xffffffffu, S.ring[sl], 0), n_jt = __shfl_sync(0xffffffffu, S.ring[kRing + sl], 0);
+        if (one) mbar_arrive(&S.iempty[sl]);
+        __syncwarp();
+        if (item < 0) break;
+        for (int t = 0; t < n_jt && ok; ++t) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&S.tempty[buf], tph ^ 1u, S.abort_s, a.status))) { ok = false; break; }
+            tc_fence_after();
+            for (int c = 0; c < a.nkc; ++c) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&S.full_bar[s], ph, S.abort_s, a.status))) { ok = false; break; }
                 tc_fence_after();
-                for (int c = 0; c < a.nkc; ++c) {
-                    if (!mbar_wait(&S.full_bar[s], ph, S.abort_s, a.status)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_mmas<C, P>(tmem, a, S.stages + s * C::STAGE_BYTES, c, buf);
-                    mma_commit(&S.empty_bar[s]);
-                    if (++s == nst) { s = 0; ph ^= 1u; }
-                }
-                if (!ok) break;
-                mma_commit(&S.tfull[buf]);
+                issue_mmas<C, P>(tmem, a, S.stages + s * C::STAGE_BYTES, c, buf, one);
+                mma_commit_one(&S.empty_bar[s], one);
+                if (++s == nst) { s = 0; ph ^= 1u; }
             }
+            if (!ok) break;
+            mma_commit_one(&S.tfull[buf], one);
+            if (++buf == C::NBUF) { buf = 0; tph ^= 1u; }
         }
-        if (!ok) spin_ns(2000000);
     }
+    if (!ok) spin_ns(2000000);
     __syncwarp();
 }
 
@@ -589,7 +615,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     if (warp < C::W0) {
         if constexpr (C::SPLIT) setmaxnreg_dec<C::REG_CTRL>();
         if (warp == 0) run_producer<C, C::QROWS>(pipe, &tmA, &tmB, a, lane);
-        else if (warp == 1) run_mma<C, P>(pipe, tmem, a, lane);
+        else if (warp == 1) run_mma<C, P>(pipe, tmem, a);
     } else {
         if constexpr (C::SPLIT) setmaxnreg_inc<C::REG_EPI>();
         // ------------------------------------------------------------- epilogue
