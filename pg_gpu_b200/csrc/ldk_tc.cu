@@ -24,7 +24,8 @@ struct PrepArgs {
     int planes;
     uint8_t* planes_out;
     unsigned* status;
-    // a parse's other preparations, in the blocks of one more y slice (slice < 0: none)
+    int64_t nx;  // SNP tiles
+    int ny;      // K tiles, and one more slice for a parse's other preparations (slice < 0: none)
     int slice;
     JmaxArgs ranges;
     unsigned long long* zero[3];  // accumulators to clear and their 64-bit words
@@ -34,149 +35,181 @@ struct PrepArgs {
 };  // X: int8 codes, or (PACKED) 2-bit codes + 1, four SNPs per byte (LDK_X_PACKED2)
 
 constexpr int kPrepV = 128, kPrepK = 128;
+// Blocks run in groups of eight SNP tiles x all K tiles: what is in flight together then reads
+// rows of X in runs of a kilobyte and completes whole rows of planes.  2,000 haplotypes x 10^6
+// SNPs (2 GB read, 4 GB written, DRAM the bound): K tile by K tile 2.2 ms, in groups 1.85, and
+// with the sixteen-row gather below 1.2 (5 TB/s).
+constexpr int kPrepGroup = 8;
 
-// One block: 128 K positions (haplotypes / individuals) x 128 SNPs.  The rows of the 128 K
-// positions are resolved once; the gather reads 128-byte row segments of X (consecutive
-// threads, consecutive SNPs) into a SNP-major shared tile, the scatter turns each 4-byte K
-// quad of a SNP into its plane bytes with byte-wise compares and writes every plane as
-// 128-byte runs along K.  Plane bytes (GENO: 4 planes, haplotypes: 2):
-//   haplotypes  sigma = 1 - 2x, v = [x in {0, 1}]
-//   genotypes   sigma = 1 - x, sigma^2, v = [x in {0, 1, 2}], 0 (PL = 2: sigma, v)
-// Padding (127) and invalid codes give 0 in every plane; invalid codes also raise
-// LDK_DEVERR_BAD_INPUT.
-//
-// Gather: a lane takes four consecutive SNPs and a warp four consecutive K rows; each row's
-// four codes come as one 32-bit word (int8 input) or one byte (packed input: four 2-bit
-// fields holding code + 1, SNP v in bits 2 (v % 4) of byte v / 4), the 4 x 4 byte block is
-// transposed in registers with byte permutes, and each SNP's four K bytes go to the tile in
-// one 32-bit store (the SNP order rotated by lane / 8 so that the 32 lanes' stores fall in 32
-// banks).  An int8 row segment that does not start on a 4-byte boundary (odd row stride, or
-// an unaligned base) is read as the two aligned words around it and joined with a funnel
-// shift; the offset is the same for the 32 lanes of a row, so the branch is warp-uniform.
-// The second word is read only where it holds SNPs of the quad, and an aligned word holding
-// one byte of the matrix lies in that byte's memory page, so no read can fault; its other
-// bytes are shifted or masked out.
 // Pair ranges of the block's 128 SNPs (first half of the threads); zeroed accumulators and the
 // reciprocal table (second half).
 template <bool GENO>
-LDK_DEV void prepare_rest(const PrepArgs& a) {
+LDK_DEV void prepare_rest(const PrepArgs& a, int64_t bx) {
     if (threadIdx.x < 128) {
-        const int64_t i = (int64_t)blockIdx.x * 128 + threadIdx.x;
+        const int64_t i = bx * 128 + threadIdx.x;
         if (i < a.n_var) pair_range(a.ranges, i);
         return;
     }
-    const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x - 128, step = (int64_t)gridDim.x * 128;
+    const int64_t t = bx * 128 + threadIdx.x - 128, step = a.nx * 128;
 #pragma unroll
     for (int z = 0; z < 3; ++z)
         for (int64_t k = t; k < a.zero_n[z]; k += step) a.zero[z][k] = 0ull;
     for (int64_t k = t; k < a.table_n; k += step) a.table[k] = GENO ? recip_entry_geno((int)k) : recip_entry((int)k);
 }
 
+// One block: 128 K positions (haplotypes / individuals) x 128 SNPs.  The rows of the 128 K
+// positions are resolved once; the gather reads 128-byte row segments of X (a lane four
+// consecutive SNPs) into a SNP-major shared tile, the scatter turns sixteen K positions of a SNP
+// into their plane bytes and writes every plane as 128-byte runs along K.  Plane bytes (GENO: 4
+// planes, haplotypes: 2):
+//   haplotypes  sigma = 1 - 2x, v = [x in {0, 1}]
+//   genotypes   sigma = 1 - x, sigma^2, v = [x in {0, 1, 2}], 0 (PL = 2: sigma, v)
+// Padding (127) and invalid codes give 0 in every plane; invalid codes also raise
+// LDK_DEVERR_BAD_INPUT.
+//
+// Gather: a warp takes sixteen K rows, all of them in flight before the first is used (what
+// bounds this kernel is how many bytes are under way); each row's four codes come as one 32-bit
+// word (int8 input) or one byte (packed input: four 2-bit fields holding code + 1, SNP v in bits
+// 2 (v % 4) of byte v / 4), 4 x 4 byte blocks are transposed in registers with byte permutes,
+// and each SNP's sixteen K bytes go to the tile in one 128-bit store, at a place rotated by the
+// lane so that eight lanes fall in the 32 banks.  An int8 row segment that does not start on a
+// 4-byte boundary (odd row stride, or an unaligned base) is read as the two aligned words around
+// it and joined with a funnel shift; the offset is the same for the 32 lanes of a row, so the
+// branch is warp-uniform.  The second word is read only where it holds SNPs of the quad, and an
+// aligned word holding one byte of the matrix lies in that byte's memory page, so no read can
+// fault; its other bytes are shifted or masked out.  The range check and the plane bytes are
+// computed on four bytes at a time in plain 32-bit arithmetic.
 template <bool GENO, bool PACKED, int PL = GENO ? 4 : 2>
 __global__ void __launch_bounds__(256) k_prep_planes(PrepArgs a) {
-    constexpr int RS = kPrepK + 4;  // bytes per SNP row: 33 words, so the scatter's word loads
-                                    // (one K quad per lane) hit distinct banks
-    __shared__ __align__(16) int8_t tile[kPrepV * RS];
+    static_assert(kPrepV == 128 && kPrepK == 128, "a warp gathers 16 K rows, a lane four SNPs");
+    constexpr uint32_t kOne = 0x01010101u, kPad = 0x7F7F7F7Fu;
+    __shared__ uint4 tile[kPrepV][kPrepK / 16];  // 16 K positions at [v][their index ^ (v / 4) % 8]
     __shared__ int srow[kPrepK];
-    if ((int)blockIdx.y == a.slice) {
-        prepare_rest<GENO>(a);
+    const int64_t g = blockIdx.x / ((int64_t)kPrepGroup * a.ny), q = blockIdx.x % ((int64_t)kPrepGroup * a.ny);
+    const int64_t bx = g * kPrepGroup + q % kPrepGroup;
+    const int by = (int)(q / kPrepGroup);
+    if (bx >= a.nx) return;
+    if (by == a.slice) {
+        prepare_rest<GENO>(a, bx);
         return;
     }
-    const int64_t v0 = (int64_t)blockIdx.x * kPrepV;
-    const int k0 = blockIdx.y * kPrepK;
-    constexpr int xmax = GENO ? 2 : 1;
-    for (int kk = threadIdx.x; kk < kPrepK; kk += blockDim.x) {
-        const int k = k0 + kk;
+    const int64_t v0 = bx * kPrepV;
+    const int k0 = by * kPrepK;
+    if (threadIdx.x < kPrepK) {
+        const int k = k0 + threadIdx.x;
         int p = 0;
         while (p + 1 < a.P && k >= a.kofs[p + 1]) ++p;
         const int local = k - a.kofs[p];
         const int np = a.pop_off[p + 1] - a.pop_off[p];
-        srow[kk] = (local >= 0 && local < np && k < a.kofs[a.P]) ? a.pop_rows[a.pop_off[p] + local] : -1;
+        srow[threadIdx.x] = (local >= 0 && local < np && k < a.kofs[a.P]) ? a.pop_rows[a.pop_off[p] + local] : -1;
     }
     __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // gather: tile[v][k] = X[row(k), v0 + v]; 127 marks padding
-    constexpr int kThreads = 256;
-    bool bad = false;
     {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        static_assert(kPrepV == 4 * 32 && kPrepK % (4 * (kThreads / 32)) == 0, "wide gather geometry");
         const int64_t v = v0 + 4 * lane;
         const int64_t left = a.n_var - v;
         const int nv = left >= 4 ? 4 : (left > 0 ? (int)left : 0);  // SNPs of this quad in the matrix
-        // bytes of the quad outside the matrix read as padding (127)
         const uint32_t keep = nv >= 4 ? 0xFFFFFFFFu : ((1u << (8 * nv)) - 1u);
         const int8_t* base = a.X + (PACKED ? (v >> 2) : v);
-        const int rot = lane >> 3;
-        for (int kk = 4 * warp; kk < kPrepK; kk += 4 * (kThreads / 32)) {
-            uint32_t w[4];
+        uint32_t w[16];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int row = srow[kk + m];
-                uint32_t x = 0x7F7F7F7Fu;
-                if (row >= 0 && nv > 0) {
-                    if constexpr (PACKED) {
-                        const uint32_t b = (uint8_t)__ldg(base + (int64_t)row * a.ld);
-                        // field j = code + 1 -> byte j = code (two's complement), or 0xFF for missing
-                        x = 0u;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) x |= (((b >> (2 * j)) & 3u) - 1u & 0xFFu) << (8 * j);
-                    } else {
-                        const uintptr_t ad = reinterpret_cast<uintptr_t>(base + (int64_t)row * a.ld);
-                        const uint32_t* q = reinterpret_cast<const uint32_t*>(ad & ~uintptr_t(3));
-                        const int s = (int)(ad & 3u);
-                        x = __ldg(q);
-                        if (s != 0) {
-                            const uint32_t hi = s + nv > 4 ? __ldg(q + 1) : 0u;
-                            x = __funnelshift_r(x, hi, 8 * s);
-                        }
-                    }
-                    x = (x & keep) | (0x7F7F7F7Fu & ~keep);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (j < nv) {
-                            const int8_t c = (int8_t)(x >> (8 * j));
-                            bad |= (c < -1 || c > xmax);
-                        }
+        for (int m = 0; m < 16; ++m) {
+            const int row = srow[16 * warp + m];
+            w[m] = kPad;
+            if (row >= 0 && nv > 0) {
+                if constexpr (PACKED) {
+                    w[m] = (uint8_t)__ldg(base + (int64_t)row * a.ld);
+                } else {
+                    const uintptr_t ad = reinterpret_cast<uintptr_t>(base + (int64_t)row * a.ld);
+                    const uint32_t* q = reinterpret_cast<const uint32_t*>(ad & ~uintptr_t(3));
+                    const int s = (int)(ad & 3u);
+                    w[m] = __ldg(q);
+                    if (s != 0) {
+                        const uint32_t hi = s + nv > 4 ? __ldg(q + 1) : 0u;
+                        w[m] = __funnelshift_r(w[m], hi, 8 * s);
                     }
                 }
-                w[m] = x;
-            }
-            // 4 x 4 byte transpose: t[j] holds SNP j's codes of rows kk .. kk + 3
-            const uint32_t x0 = __byte_perm(w[0], w[1], 0x5140), x1 = __byte_perm(w[0], w[1], 0x7362);
-            const uint32_t x2 = __byte_perm(w[2], w[3], 0x5140), x3 = __byte_perm(w[2], w[3], 0x7362);
-            const uint32_t t[4] = {__byte_perm(x0, x2, 0x5410), __byte_perm(x0, x2, 0x7632),
-                                   __byte_perm(x1, x3, 0x5410), __byte_perm(x1, x3, 0x7632)};
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int j = (jj + rot) & 3;
-                *reinterpret_cast<uint32_t*>(tile + (4 * lane + j) * RS + kk) = t[j];
             }
         }
+        uint32_t bad = 0u;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            if constexpr (PACKED) {
+                // field j = code + 1 -> byte j = code (two's complement), or 0xFF for missing
+                if (srow[16 * warp + m] >= 0 && nv > 0) {
+                    const uint32_t b = w[m];
+                    w[m] = 0u;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) w[m] |= (((b >> (2 * j)) & 3u) - 1u & 0xFFu) << (8 * j);
+                }
+            }
+            // code + 1 of each byte (no carry between bytes); valid: 0 .. 2 (haplotypes), 0 .. 3
+            if (srow[16 * warp + m] >= 0) {
+                const uint32_t y = (((w[m] & 0x7F7F7F7Fu) + kOne) ^ (w[m] & 0x80808080u)) & keep;
+                uint32_t odd = y & 0xFCFCFCFCu;
+                if constexpr (!GENO) odd |= y & (y >> 1) & kOne;
+                if (odd) {  // invalid codes become padding
+                    bad |= odd;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if ((odd >> (8 * j)) & 0xFFu) w[m] |= 0x7Fu << (8 * j);
+                }
+                w[m] = (w[m] & keep) | (kPad & ~keep);
+            }
+        }
+        if (bad) atomicOr(a.status, LDK_DEVERR_BAD_INPUT);
+        // 4 x 4 byte transposes: t[q][j] holds SNP j's codes of rows 4 q .. 4 q + 3
+        uint32_t t[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t x0 = __byte_perm(w[4 * q], w[4 * q + 1], 0x5140), x1 = __byte_perm(w[4 * q], w[4 * q + 1], 0x7362);
+            const uint32_t x2 = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x5140);
+            const uint32_t x3 = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x7362);
+            t[q][0] = __byte_perm(x0, x2, 0x5410);
+            t[q][1] = __byte_perm(x0, x2, 0x7632);
+            t[q][2] = __byte_perm(x1, x3, 0x5410);
+            t[q][3] = __byte_perm(x1, x3, 0x7632);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            tile[4 * lane + j][warp ^ (lane & 7)] = make_uint4(t[0][j], t[1][j], t[2][j], t[3][j]);
     }
-    if (bad) atomicOr(a.status, LDK_DEVERR_BAD_INPUT);
     __syncthreads();
-    // scatter: lane = K quad, warps stride over the SNPs
-    const int kq = threadIdx.x % 32;
-    constexpr uint32_t kOne = 0x01010101u;
-    for (int vv = threadIdx.x / 32; vv < kPrepV; vv += kThreads / 32) {
+    // scatter: a warp takes four SNPs at a time, a lane 16 K positions of one
+    const int kg = lane & 7;
+    uint8_t* out = a.planes_out + k0 + 16 * kg;
+#pragma unroll
+    for (int it = 0; it < kPrepV / 32; ++it) {
+        const int vv = 32 * it + 4 * warp + (lane >> 3);
         const int64_t v = v0 + vv;
         if (v >= a.n_var) break;
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + vv * RS + 4 * kq);
-        const uint32_t eq0 = __vcmpeq4(w, 0u), eq1 = __vcmpeq4(w, kOne);
-        uint8_t* dst = a.planes_out + v * PL * (int64_t)a.ktot + k0 + 4 * kq;
-        if constexpr (GENO && PL == 2) {  // sigma and the mask only
-            const uint32_t eq2 = __vcmpeq4(w, 2u * kOne);
-            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq2;
-            *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq1 | eq2) & kOne;
-        } else if constexpr (GENO) {
-            const uint32_t eq2 = __vcmpeq4(w, 2u * kOne);
-            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq2;  // 0xFF = -1
-            *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq2) & kOne;
-            *reinterpret_cast<uint32_t*>(dst + 2 * (int64_t)a.ktot) = (eq0 | eq1 | eq2) & kOne;
-            *reinterpret_cast<uint32_t*>(dst + 3 * (int64_t)a.ktot) = 0u;
+        const uint4 q = tile[vv][kg ^ ((vv >> 2) & 7)];
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        uint32_t sg[4], sq[4], va[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            // the codes are 0, 1 (, 2), 0x7F or 0xFF: bit 1 (2) is clear in the valid ones only,
+            // and adding 254 to a byte of 1 makes it -1
+            va[k] = (~w[k] >> (GENO ? 2 : 1)) & kOne;
+            if constexpr (GENO) {
+                sq[k] = va[k] & ~w[k];
+                sg[k] = sq[k] + ((w[k] >> 1) & va[k]) * 254u;
+            } else {
+                sg[k] = va[k] + (w[k] & va[k]) * 254u;
+            }
+        }
+        uint8_t* dst = out + v * PL * (int64_t)a.ktot;
+        auto put = [&](int plane, const uint32_t (&x)[4]) {
+            *reinterpret_cast<uint4*>(dst + plane * (int64_t)a.ktot) = make_uint4(x[0], x[1], x[2], x[3]);
+        };
+        put(0, sg);
+        if constexpr (PL == 4) {
+            put(1, sq);
+            put(2, va);
+            *reinterpret_cast<uint4*>(dst + 3 * (int64_t)a.ktot) = make_uint4(0u, 0u, 0u, 0u);
         } else {
-            *reinterpret_cast<uint32_t*>(dst) = (eq0 & kOne) | eq1;
-            *reinterpret_cast<uint32_t*>(dst + a.ktot) = (eq0 | eq1) & kOne;
+            put(1, va);
         }
     }
 }
@@ -309,9 +342,10 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
     a.planes = sh.planes;
     a.planes_out = w.hv;
     a.status = w.status;
-    dim3 grid((unsigned)((d->n_var + kPrepV - 1) / kPrepV), (unsigned)(sh.ktot / kPrepK));
+    a.nx = (d->n_var + kPrepV - 1) / kPrepV;
+    a.ny = sh.ktot / kPrepK;
     if (o) {
-        a.slice = (int)grid.y++;
+        a.slice = a.ny++;
         a.ranges = jmax_args(d, w);
         const int64_t cells = (int64_t)d->n_blocks * d->n_bins;
         a.zero[0] = w.fx;
@@ -320,7 +354,7 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
         a.zero[2] = reinterpret_cast<unsigned long long*>(o->r2_counts);
         a.zero_n[1] = a.zero_n[2] = cells;
         // more than a few words a thread (many blocks of few SNPs): by memset
-        if (a.zero_n[0] > 64ll * 128 * grid.x) {
+        if (a.zero_n[0] > 64ll * 128 * a.nx) {
             cudaError_t e = cudaMemsetAsync(w.fx, 0, a.zero_n[0] * sizeof(unsigned long long), s);
             if (e != cudaSuccess) return e;
             a.zero_n[0] = 0;
@@ -328,6 +362,9 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
         a.table = static_cast<double4*>(w.rtab ? w.rtab : w.gtab);
         a.table_n = a.table ? sh.max_n + 1 : 0;
     }
+    const int64_t blocks = (a.nx + kPrepGroup - 1) / kPrepGroup * kPrepGroup * a.ny;
+    if (blocks > INT32_MAX) return cudaErrorInvalidValue;
+    const unsigned grid = (unsigned)blocks;
     const bool packed = d->x_format == LDK_X_PACKED2;
     if (sh.genotypes && sh.planes == 2) {
         k_prep_planes<true, false, 2><<<grid, 256, 0, s>>>(a);
