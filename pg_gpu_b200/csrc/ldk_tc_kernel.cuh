@@ -157,6 +157,16 @@ struct Cfg {
     static constexpr int NA = SSPL ? (K > NS + 1 - K ? K : NS + 1 - K) : NS + 1;  // sums per lane
     static constexpr int FROW = P == 1 ? 0 : (NA + 2) | 1;  // odd: rows in other banks; one population reduces in registers
     static constexpr int FROWS_MAX = 8;
+    // The rows of a warp's 32 SNPs (8 with QROWS) cross a bin edge a few partners apart.
+    // LATE: a lane's finished sums wait in registers until some lane of the warp leaves the
+    // next bin, so one flush serves a whole edge: 500 diploids x 100,000 SNPs 3.10 -> 2.79 ms,
+    // 1,000,000 SNPs x 2,000 haplotypes 20.7 -> 20.1 (two haplotype populations 4.80 -> 5.22:
+    // their registers cost more than the few flushes).
+    // PEND: rows wait in the scratch until it is full, where the staged sums are shared by
+    // atomics: two genotype populations 1.03 -> 0.94 ms, four haplotype 2.25 -> 2.23 (two
+    // haplotype populations 4.80 -> 5.0, three 31.8 -> 31.9).
+    static constexpr bool LATE = P == 1;
+    static constexpr bool PEND = P > 1 && (GENO || P == 4);
     static_assert(!SPLIT || 4 * REG_CTRL + EPI * REG_EPI <= (W0 + EPI) * REG_LAUNCH,
                   "register split must fit the launch allocation");
     static_assert(!SPLIT || THREADS * REG_LAUNCH <= 65536, "register file");
@@ -687,29 +697,75 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
 #pragma unroll
             for (int s = 0; s < NA; ++s) acc[s] = 0.0;
             unsigned np = 0, nr2 = 0;
+            double pacc[C::LATE ? NA : 1];  // LATE: sums of the bin this lane left last
+            unsigned pnp = 0, pnr2 = 0;
+            int pkey = 0;
             int cur = -1;
             bool in_bin = false;  // 0 <= cur < nb
             double nxt = sedges[0];
-            // Adds the flushing lanes' sums into the staged sums; called by all 32 lanes.
-            // The flushing lanes write their sums into rows of the warp's scratch (in
-            // batches of `frows`, all lanes of a batch at once), then for every (block, bin)
-            // among them the warp adds the rows that hold it, lane s taking value s.  One lane per round adding its own 46
-            // values took one pass per flushing lane of a key -- on average 6.5 for 200
-            // windows x 3 populations, 39.5 -> 32.4 ms with eight rows of odd stride (four
-            // rows: 33.5; rows added one after the other: 33.4); with shared staging
-            // (atomics) two genotype populations 2.77 -> 1.07 ms, four haplotype 4.72 -> 2.32.  With PRIV every epilogue warp owns its staged sums
-            // and plain adds suffice; otherwise the warps share them (atomics).  The pairs are
-            // counted by the first of two warps that share them.
-            auto flush = [&](bool want) {
-                const unsigned mask = __ballot_sync(0xffffffffu, want);
-                if constexpr (P == 1) {
-                    flush_one_pop<PRIV>(mask, slot * nb + cur, acc, np, nr2, my_sacc, my_scnt, lane);
-                    return;
+            // Adds lanes' sums into the staged sums; called by all 32 lanes.  With more than one
+            // population they go into rows of the warp's scratch (all lanes of a batch at
+            // once), and for every (block, bin) among the rows the warp adds the rows that hold
+            // it, lane s taking value s.  One lane per round adding its own 46 values took one
+            // pass per lane of a key -- on average 6.5 for 200 windows x 3 populations, 39.5 ->
+            // 32.4 ms with eight rows of odd stride (four rows: 33.5; rows added one after the
+            // other: 33.4); with shared staging (atomics) two genotype populations 2.77 -> 1.07
+            // ms, four haplotype 4.72 -> 2.32.  With PRIV every epilogue warp owns its staged
+            // sums and plain adds suffice; otherwise the warps share them (atomics).  The pairs
+            // are counted by the first of two warps that share them.
+            int used = 0;  // rows of the scratch that wait
+            auto drain = [&]() {
+                constexpr int VPL = (NA + 31) / 32;  // values per lane; lane 31 also adds the counts
+                constexpr int RB = C::FROWS_MAX;
+                __syncwarp();
+                // lane r knows row r's key; one pass per key adds the rows that hold it
+                const int my_key = lane < used ? *reinterpret_cast<const int*>(my_fst + lane * C::FROW + NA + 1) : -1;
+                unsigned left = (1u << used) - 1u;
+                while (left) {
+                    const int kk = __shfl_sync(0xffffffffu, my_key, __ffs(left) - 1);
+                    const unsigned grp = __ballot_sync(0xffffffffu, my_key == kk);
+                    left &= ~grp;
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) {
+                        const int s = lane + 32 * v;
+                        if (s < na) {
+                            double* dst = my_sacc + kk * (NS + 1) + gofs + s;
+                            double d = PRIV ? *dst : 0.0;
+#pragma unroll
+                            for (int rr = 0; rr < RB; ++rr)
+                                if ((grp >> rr) & 1u) d += my_fst[rr * C::FROW + s];
+                            if constexpr (PRIV) *dst = d;
+                            else atomicAdd(dst, d);
+                        }
+                    }
+                    if (part == 0 && lane == 31) {
+                        unsigned* dst = my_scnt + 2 * kk;
+                        uint2 dc = PRIV ? make_uint2(dst[0], dst[1]) : make_uint2(0u, 0u);
+#pragma unroll
+                        for (int rr = 0; rr < RB; ++rr)
+                            if ((grp >> rr) & 1u) {
+                                const uint2 c = *reinterpret_cast<const uint2*>(my_fst + rr * C::FROW + NA);
+                                dc.x += c.x;
+                                dc.y += c.y;
+                            }
+                        if constexpr (PRIV) {
+                            dst[0] = dc.x;
+                            dst[1] = dc.y;
+                        } else {
+                            atomicAdd(dst, dc.x);
+                            atomicAdd(dst + 1, dc.y);
+                        }
+                    }
                 }
+                __syncwarp();
+                used = 0;
+            };
+            auto add = [&](bool want, bool last, const double* acc, unsigned np, unsigned nr2, int key) {
+                const unsigned mask = __ballot_sync(0xffffffffu, want);
+                if constexpr (P == 1) flush_one_pop<PRIV>(mask, key, acc, np, nr2, my_sacc, my_scnt, lane);
                 const int rank = __popc(mask & ((1u << lane) - 1u)), total = __popc(mask);
                 if constexpr (P > 1) {
                 if (a.frows == 0) {  // no room: one lane per (block, bin) at a time
-                    const int key = slot * nb + cur;
                     const unsigned grp = __match_any_sync(0xffffffffu, want ? key : -1);
                     const int turn = __popc(grp & ((1u << lane) - 1u));
                     const int turns = PRIV ? (int)__reduce_max_sync(0xffffffffu, want ? (unsigned)__popc(grp) : 0u) : 1;
@@ -737,60 +793,39 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     }
                     return;
                 }
-                constexpr int VPL = (NA + 31) / 32;  // values per lane; lane 31 also adds the counts
-                constexpr int RB = C::FROWS_MAX;
-                for (int b0 = 0; b0 < total; b0 += a.frows) {
-                    const int rows = total - b0 < a.frows ? total - b0 : a.frows;
+                int b0 = 0;
+                do {
+                    const int rows = total - b0 < a.frows - used ? total - b0 : a.frows - used;
                     if (want && rank >= b0 && rank < b0 + rows) {
-                        double* row = my_fst + (rank - b0) * C::FROW;
+                        double* row = my_fst + (used + rank - b0) * C::FROW;
 #pragma unroll
                         for (int s = 0; s < NA; ++s)
                             if (!SSPL || s < na) row[s] = acc[s];
                         *reinterpret_cast<uint2*>(row + NA) = make_uint2(np, nr2);
-                        *reinterpret_cast<int*>(row + NA + 1) = slot * nb + cur;
+                        *reinterpret_cast<int*>(row + NA + 1) = key;
                     }
-                    __syncwarp();
-                    // lane r knows row r's key; one pass per key adds the rows that hold it
-                    const int my_key = lane < rows ? *reinterpret_cast<const int*>(my_fst + lane * C::FROW + NA + 1) : -1;
-                    unsigned left = (1u << rows) - 1u;
-                    do {
-                        const int kk = __shfl_sync(0xffffffffu, my_key, __ffs(left) - 1);
-                        const unsigned grp = __ballot_sync(0xffffffffu, my_key == kk);
-                        left &= ~grp;
-#pragma unroll
-                        for (int v = 0; v < VPL; ++v) {
-                            const int s = lane + 32 * v;
-                            if (s < na) {
-                                double* dst = my_sacc + kk * (NS + 1) + gofs + s;
-                                double d = PRIV ? *dst : 0.0;
-#pragma unroll
-                                for (int rr = 0; rr < RB; ++rr)
-                                    if ((grp >> rr) & 1u) d += my_fst[rr * C::FROW + s];
-                                if constexpr (PRIV) *dst = d;
-                                else atomicAdd(dst, d);
-                            }
-                        }
-                        if (part == 0 && lane == 31) {
-                            unsigned* dst = my_scnt + 2 * kk;
-                            uint2 dc = PRIV ? make_uint2(dst[0], dst[1]) : make_uint2(0u, 0u);
-#pragma unroll
-                            for (int rr = 0; rr < RB; ++rr)
-                                if ((grp >> rr) & 1u) {
-                                    const uint2 c = *reinterpret_cast<const uint2*>(my_fst + rr * C::FROW + NA);
-                                    dc.x += c.x;
-                                    dc.y += c.y;
-                                }
-                            if constexpr (PRIV) {
-                                dst[0] = dc.x;
-                                dst[1] = dc.y;
-                            } else {
-                                atomicAdd(dst, dc.x);
-                                atomicAdd(dst + 1, dc.y);
-                            }
-                        }
-                    } while (left);
-                    __syncwarp();
+                    used += rows;
+                    b0 += rows;
+                    if (!C::PEND || used == a.frows || (last && b0 == total)) drain();
+                } while (b0 < total);
                 }
+            };
+            auto flush = [&](bool want, bool last) {
+                if constexpr (C::LATE) {
+                    if (__ballot_sync(0xffffffffu, want && pnp > 0)) {
+                        add(pnp > 0, false, pacc, pnp, pnr2, pkey);
+                        pnp = 0;
+                    }
+                    if (want) {
+#pragma unroll
+                        for (int s = 0; s < NA; ++s) pacc[s] = acc[s];
+                        pnp = np;
+                        pnr2 = nr2;
+                        pkey = slot * nb + cur;
+                    }
+                    if (last) add(pnp > 0, true, pacc, pnp, pnr2, pkey);
+                } else {
+                    add(want, last, acc, np, nr2, slot * nb + cur);
                 }
             };
             // One TMEM read per step, indexed with constants only so the counts stay in
@@ -915,7 +950,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                             const bool step = valid[u] && dist[u] >= nxt;
                             if (U == 1 ? change : __ballot_sync(0xffffffffu, step) != 0u) {
                                 const bool want = step && in_bin && np > 0;
-                                if (__ballot_sync(0xffffffffu, want)) flush(want);
+                                if (__ballot_sync(0xffffffffu, want)) flush(want, false);
                                 if (step) {
                                     cur = bin_advance(sedges, nb, cur, dist[u]);
                                     nxt = cur < nb ? sedges[cur + 1] : CUDART_INF;
@@ -930,7 +965,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     }
                 }
             }
-            flush(in_bin && np > 0);
+            flush(in_bin && np > 0, true);
             (void)ok;
             // staging -> global, once per work item
             epi_bar<EPI>();
