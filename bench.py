@@ -7,7 +7,7 @@ missing, 16 log-spaced distance bins (10 bp .. 1 Mb), per-window per-bin FP64
 DD/Dz/pi2 (45 statistics), 50-kb bootstrap blocks and 100 block-bootstrap replicates.
 Seeded synthetic data (founder mosaics, see pg_gpu_b200/synth.py).
 
-One step = the whole batched parse of that workload: pair ranges, indicator planes,
+One step = the whole batched parse of that workload: pair ranges, spin planes,
 the fused INT8 tcgen05 count + estimator + bin kernel, per-window totals and bootstrap
 replicates.  ``value`` has inputs resident in HBM; ``e2e`` copies the inputs from
 pinned host memory and the results back every step.  ``--impl reference`` times pg_gpu's
@@ -565,7 +565,7 @@ def main():
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
             "warmup": max(3, args.warmup), "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "strong" if args.split else "weak", "vs_baseline": None,
-            "dtype": {"tc": "u8 counts / s32 accumulate / f64 estimators",
+            "dtype": {"tc": "s8 counts / s32 accumulate / f64 estimators",
                       "plain": "i8 byte counts / f64 estimators"}[args.method],
             "data": "synthetic (seeded founder mosaics; no public dataset offline)",
             "config": {"workload": w.name, "config_index": args.config, "scale": args.scale,
@@ -584,20 +584,17 @@ def main():
                        "tile_partners": int(parser.tile_width()),
                        "tile_source": "autotuned (ldk_autotune)" if not args.no_autotune else "default",
                        "tuned": tuned_entry,
-                       "l2": "inputs larger than L2 (haplotypes %d MB, indicator planes %d MB)" % (
+                       "l2": "inputs larger than L2 (haplotypes %d MB, spin planes %d MB)" % (
                            w.data.nbytes >> 20, (w.n_var * 2 * parser_ktot(w)) >> 20)},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
             "roofline": roofline,
-            # per step: k_jmax, k_prep_planes, k_split_items, k_parse_tc, k_fx_finish,
-            # 2 x k_block_combine, and on
-            # the genotype path (1-3 populations) k_fill_gtab; plain: k_jmax, k_parse_plain,
-            # k_fx_finish, 2 x combine (a workspace reciprocal table, k_fill_rtab, serves only
-            # populations whose table does not fit in shared memory: none of configurations 1-5)
-            "gpu_launches": int(args.steps * (5 if parser.method == "plain" else
-                                              7 + int(bool(w.genotypes) and len(w.pop_rows) <= 3))),
-            "launch": "CUDA graph replay (memsets, k_jmax, planes, work items + parse kernel, k_fx_finish, "
-                      "2 x k_block_combine"
-                      + (", genotype reciprocal table" if w.genotypes and parser.method != "plain" else "") + ")"
+            # per step: k_prep_planes (also the pair ranges, cleared accumulators and reciprocal
+            # table), k_split_items, k_parse_tc, k_fx_finish, 2 x k_block_combine; plain: k_jmax,
+            # k_parse_plain, k_fx_finish, 2 x combine
+            "gpu_launches": int(args.steps * (5 if parser.method == "plain" else 6)),
+            "launch": ("CUDA graph replay (status memset, preparation, work items, parse kernel, k_fx_finish, "
+                       "2 x k_block_combine)" if parser.method != "plain" else
+                       "CUDA graph replay (memsets, k_jmax, parse kernel, k_fx_finish, 2 x k_block_combine)")
                       if not args.no_graph else "ldk_parse per step",
             "clocks": clocks,
         }
@@ -675,12 +672,12 @@ def run_all_pairs(args):
     print(json.dumps({
         "metric": "all-pairs LD SNP-pairs/s", "value": pairs / (ms / 1e3), "unit": "SNP-pairs/s", "n_gpus": 1,
         "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "u8 counts / s32 accumulate / f64 values",
+        "scaling": "weak", "vs_baseline": None, "dtype": "s8 counts / s32 accumulate / f64 values",
         "data": "synthetic (seeded founder mosaics, 1% missing)",
         "config": {"workload": f"all-pairs {args.estimator}, {m} SNPs x {n} {'individuals' if geno else 'haplotypes'}",
                    "matrix": M is not None, "pairs": pairs, "l2": "matrix larger than L2" if M is not None else
                    "reduction only"},
-        "roofline": roof, "gpu_launches": int(args.steps * ((M is not None) + (est == 0) + geno + 3)),
+        "roofline": roof, "gpu_launches": int(args.steps * 4),  # k_site, k_prep_planes, k_split_items, the matrix kernel
         "clocks": clk.summary()}),
         flush=True)
 

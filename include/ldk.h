@@ -40,7 +40,7 @@ extern "C" {
 
 /* counting / estimator method of ldk_parse */
 #define LDK_METHOD_PLAIN_FP64 0 /* per-pair byte counting + FP64 estimators (the drop-in) */
-#define LDK_METHOD_TC 1         /* INT8 tcgen05 Gram counts; exact-integer features, FP64 combination and bins */
+#define LDK_METHOD_TC 1         /* INT8 tcgen05 Gram moments; FP64 estimators on them (exact integers) and bins */
 
 LDK_API int ldk_version(void);
 LDK_API const char* ldk_last_error(void);
@@ -182,9 +182,10 @@ LDK_API int ldk_parse_noalloc(const ldk_parse_t* d, const ldk_parse_out_t* out, 
  * counterpart in pg_gpu (its parse is a Python loop of CuPy calls).
  *
  * ldk_parse_setup writes the call's plan into the workspace -- window offsets and the
- * tensor-core method's row-block list, from host memory -- and synchronises `stream`.
- * ldk_parse_enqueue then enqueues only device work on `stream` (zeroing the outputs and
- * the status word, pair ranges, indicator planes, the parse kernel): no host <-> device
+ * tensor-core method's row-block list, from host memory (a tensor-core parse of one window
+ * needs neither and has no plan) -- and synchronises `stream`.
+ * ldk_parse_enqueue then enqueues only device work on `stream` (clearing the status word and
+ * the accumulators, pair ranges, spin planes, the parse kernel, the outputs): no host <-> device
  * copies, no synchronisation, no allocation, so it can be captured into a CUDA graph and
  * the graph replayed while the input arrays change contents in place.  It requires a
  * preceding ldk_parse_setup with the same descriptor shape (n_var, populations, windows,
@@ -248,7 +249,8 @@ LDK_API int ldk_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const in
  * bytes, bin count, decade of max_dist, log2 of the mean window size).  Later ldk_parse,
  * ldk_parse_setup (the order) and ldk_parse_enqueue (the width) calls of the class use the
  * kept choice, tuning enabled or not; classes never tuned use the defaults (the widest
- * haplotype tile, 12 / 8 partners for one / two genotype populations; largest windows first).  ldk_tile_width returns the width (SNPs per partner tile) a call
+ * haplotype tile, the narrower one for one population in windows with no more tiles than SMs,
+ * 12 / 8 partners for one / two genotype populations; largest windows first).  ldk_tile_width returns the width (SNPs per partner tile) a call
  * with this descriptor would use now, 0 for the plain method, or a negative status.  No
  * counterpart in pg_gpu. */
 LDK_API int ldk_autotune(int enable);

@@ -321,8 +321,8 @@ bool tc_rtab_global(const ParseShape& sh) {
 // The spin planes, and with `o` the rest of a parse's preparation in the same launch: pair
 // ranges, the cleared accumulators and pair tallies, the reciprocal table.  (Separate kernels and
 // memsets each waited for the one before: with the outputs' own memsets, which the bin sums
-// overwrite anyway, thirteen operations for a window of 400 SNPs, 92 us a call; five, 56, of which the narrower tile and
-// one-tile pieces on more SMs give 18.)
+// overwrite anyway, thirteen operations for a window of 400 SNPs, 92 us a call; five, 56, of
+// which the narrower tile and one-tile pieces on more SMs give 18.)
 cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const ParseShape& sh, const ldk_parse_out_t* o,
                                cudaStream_t s) {
     if (d->n_var == 0) return cudaSuccess;
@@ -383,9 +383,11 @@ namespace {
 // there are few row blocks per SM (a 5,000-SNP window has 79) or where their count leaves a
 // partial last wave; pieces of at most c partner tiles bound the spread of the CTAs' finishing
 // times by one piece.  c = max(min_tiles, ceil(total tiles / kItemTarget)) -- min_tiles at
-// most the tiles there are per SM -- so shapes with
-// many small row blocks keep one item per row block, and no piece is so short that the flush
-// of its staged sums (which ends every item) outweighs its tiles.  Pieces of one row block are consecutive
+// most the tiles there are per SM -- so shapes with many small row blocks keep one item per row
+// block, and no piece is so short that the flush of its staged sums (which ends every item)
+// outweighs its tiles.  Where there are fewer tiles than SMs a tile is a piece: 400 SNPs
+// (28 tiles of 64 partners) x 60 haplotypes 0.028 ms with pieces of four, 0.020 with one; x 2,000
+// haplotypes 0.050 and 0.028; from 2,000 SNPs on the same.  Pieces of one row block are consecutive
 // (the claim order of the row blocks stays), its last piece runs to INT32_MAX, and a row block
 // without partners gets no item.  One block of 1024 threads: the total, then a block-wide
 // scan of the pieces per row block, 1024 row blocks per round.

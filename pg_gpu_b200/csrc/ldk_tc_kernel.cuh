@@ -22,23 +22,26 @@
 // counts.  The spin forms take 30 / 112 / 267 FP64 operations a pair for 1 / 2 / 3 haplotype
 // populations (the factored raw-call forms they replaced: 404 measured for three) and
 // 35 / 144 / 316 for genotypes (the nine-cell polynomials: 404 for one population's numerators
-// alone).  B200, 1965 MHz, a pass with the old -> new forms: 500 diploids x 100,000 SNPs
-// 9.63 -> 3.79 ms, two genotype populations x 20,001 SNPs 5.28 -> 2.77, three haplotype
-// populations x 200 windows 48.0 -> 39.5, two x 50,000 SNPs 6.93 -> 5.74.  With one population
-// the TMA traffic (about 11 TB/s from L2) and the bin flushes weigh as much.
+// alone).  B200, 1965 MHz, a pass with the old forms -> with the spin forms -> with what the
+// comments below describe: 500 diploids x 100,000 SNPs 9.63 -> 3.79 -> 2.88 ms, two genotype
+// populations x 20,001 SNPs 5.28 -> 2.77 -> 0.98, three haplotype populations x 200 windows
+// 48.0 -> 39.5 -> 32.2 (FP64 pipe about 55%: estimators 12 of a warp's 17 thousand cycles a
+// tile), two x 50,000 SNPs 6.93 -> 5.74 -> 4.84.  With one population the loads weigh as much as
+// the estimators: 2,000 haplotypes x 10^6 SNPs 28.3 -> 21.3 ms, where a tile's 21.7 thousand
+// cycles hold 10 of waiting for TMA traffic (about 10 TB/s from L2) and the epilogue takes 20.
 //
 // Warp roles (one CTA per SM, persistent over work items: runs of one row block's partner
 // tiles, claimed dynamically):
-//   warp 0     TMA producer (A: row block, B: 12..128 partner SNPs, per 128-byte K chunk)
-//   warp 1     TMEM allocator and single-thread MMA issuer, double-buffered accumulators
+//   warp 0     TMA producer (A: row block, B: 8..128 partner SNPs, per 128-byte K chunk)
+//   warp 1     TMEM allocator and MMA issuer, double-buffered accumulators
 //   epilogue   8, 12 or 16 warps (see Cfg), two to four per TMEM lane quarter, each
-//              taking its share of every partner tile: tcgen05.ld the counts, swap halves
-//              between lane pairs, evaluate the estimators in FP64, sum per
-//              distance bin in registers (bins are monotone
-//              in j for a fixed i), flush each finished bin run into a per-warp FP64
-//              staging copy in shared memory, and add the staged sums to the
-//              per-bootstrap-block fixed-point accumulators once per work item (integer
-//              atomics, so the result does not depend on the order of the items).
+//              taking its share of every partner tile: tcgen05.ld the moments (QROWS: all
+//              four of a pair in one thread), evaluate the estimators in FP64, sum per
+//              distance bin in registers (bins are monotone in j for a fixed i), flush each
+//              finished bin run into an FP64 staging copy in shared memory, and add the
+//              staged sums to the per-bootstrap-block fixed-point accumulators once per work
+//              item (integer atomics, so the result does not depend on the order of the
+//              items).
 // Every wait is bounded (LDK_DEVERR_TIMEOUT) so a fault cannot hang the GPU.
 #pragma once
 #include <cuda.h>
@@ -79,8 +82,8 @@ constexpr size_t kStaticSmem = 1536;  // at most: the kernel's __shared__ variab
 // Partners per tile: tile variant 0 is the default, variant 1 the alternative the
 // autotuner also times (half the width on the haplotype path; on the genotype path 8 for
 // one population, 16 for two -- one TMEM buffer -- and the default for more).
-// Two haplotype populations and one genotype population: 48 (or 24) and 12 (or 24), so that
-// each of the three epilogue warps of a lane quarter takes an equal share of the tile.
+// One genotype population: 12 (or 24), so that each of the three epilogue warps of a lane
+// quarter takes an equal share of the tile.
 constexpr int tile_nj(int P, bool GENO, int V) {
     return GENO ? (V == 0 ? (P == 1 ? 12 : 8) : (P == 1 ? 24 : P == 2 ? 16 : 8))
                 : ((P == 1 ? 128 : P == 2 ? 48 : 32) >> V);
@@ -113,15 +116,17 @@ struct Cfg {
     static constexpr bool QROWS = !GENO && P <= 3;
     // Warp layout.  Warp w may read only TMEM lane quarter w % 4, and each of the four
     // schedulers of an SM holds warps w, w + 4, ... with a quarter of the register file.
-    //  * SPLIT (genotypes; haplotypes with three or four populations -- estimators that
-    //    want ~240 registers): 12 warps.  Warpgroup 0 (TMA, MMA, two idle warps) gives its
+    //  * SPLIT (genotypes; haplotypes with two or more populations -- estimators that want
+    //    150 to 240 registers): 12 warps.  Warpgroup 0 (TMA, MMA, two idle warps) gives its
     //    registers up with setmaxnreg (24 or 40 each) and the eight epilogue warps 4..11
     //    take them (240 or 232 each), so that every scheduler holds two full-register epilogue
-    //    warps beside one control warp (launch: 168 per thread).
+    //    warps beside one control warp (launch: 168 per thread).  Two haplotype populations
+    //    with twelve epilogue warps at 160 registers: 5.65 ms, with eight 5.14.
     //  * one genotype population, also SPLIT: 16 warps, twelve epilogue warps 4..15 at 160
     //    registers, three per scheduler and lane quarter (launch: 128).
-    //  * one or two haplotype populations: 18 warps, TMA and MMA in warps 0 and 1, sixteen
-    //    epilogue warps 2..17, four per lane quarter and scheduler (113 registers at most).
+    //  * one haplotype population: 18 warps, TMA and MMA in warps 0 and 1, sixteen epilogue
+    //    warps 2..17, four per lane quarter and scheduler (96 registers: five warps share a
+    //    scheduler's quarter of the register file).
     static constexpr int EPI = (!GENO && P == 1) ? 16 : (GENO && P == 1) ? 12 : 8;
     static constexpr bool SPLIT = GENO || P >= 2;
     static constexpr int W0 = SPLIT ? 4 : 2;  // first epilogue warp
@@ -346,10 +351,10 @@ LDK_DEV void spin_ns(uint64_t ns) {
 // Flush of one population's four sums: for every (block, bin) among the flushing lanes the
 // warp adds the lanes' values with a butterfly that halves the values each lane carries (two
 // exchanges leave lane / 8 % 4 with one value, three more add it up), and the four lanes that
-// hold a total add it to the staged sums.  About ten lanes of a warp flush the same key in the
-// same step when a row block crosses a bin edge; one lane per round, ~60 cycles each, took
-// 25.0 ms for 1,000,000 SNPs x 2,000 haplotypes in 32 bins, this 21.6 (5,000 SNPs x 100:
-// 0.119 -> 0.098; 500 diploids x 100,000: 3.82 -> 3.43).
+// hold a total add it to the staged sums.  About ten lanes of a warp hold the same key when a row
+// block crosses a bin edge (all of them since they wait for one another); one lane per round,
+// ~60 cycles each, took 25.0 ms for 1,000,000 SNPs x 2,000 haplotypes in 32 bins, this 21.6 (5,000 SNPs x 100:
+// 0.119 -> 0.098; 500 diploids x 100,000: 3.82 -> 3.43), all kernel times before the later steps.
 template <bool PRIV>
 LDK_DEV void flush_one_pop(unsigned mask, int key, const double* acc, unsigned np, unsigned nr2, double* my_sacc,
                            unsigned* my_scnt, int lane) {
@@ -515,7 +520,9 @@ LDK_DEV void run_producer(const Pipe& S, const CUtensorMap* tmA, const CUtensorM
 
 // Warp 1: the MMAs of every tile into the double-buffered accumulators.  The whole warp runs the
 // loop, one elected lane issues: in code that only one lane runs, every MMA's descriptors went
-// through vector registers, and issuing took longer than the small MMAs themselves.
+// through vector registers, and issuing took longer than the small MMAs themselves (a tile of
+// 48 MMAs with N = 48 3,680 -> 2,170 cycles, near the 48 each that the tensor core takes for
+// N <= 64; 500 diploids x 100,000 SNPs 3.33 -> 3.11 ms, two haplotype populations 4.95 -> 4.82).
 template <class C, int P>
 LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a) {
     const int nst = C::MORE_STAGES ? a.stages : C::STAGES;
