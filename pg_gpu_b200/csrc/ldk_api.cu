@@ -352,22 +352,31 @@ int tuned_variant(const ldk_parse_t* d, const ParseShape& sh) {
     return tune_lookup(tune_key_of(d, sh), &c) ? c.variant : -1;
 }
 
-// The variant a call runs: the tuned one, else the default -- for one haplotype population the
-// narrower tile where the wide one leaves most SMs without a tile (an upper bound: every pair of
-// every window within the cutoff).  60 haplotypes, one window, kernel ms wide / narrow: 400 SNPs
-// 0.0236 / 0.0195, 1,500 (144 wide tiles by this bound) 0.0276 / 0.0256, 2,000 0.0276 / 0.0276,
-// 2,500 0.040 / 0.046, 5,000 0.087 / 0.097.
+// The variant a call runs: the tuned one, else the default.  Variant 0, but with one population the
+// wider tile where there are more tiles than SMs and the narrower one where there are not (an upper
+// bound: every pair of every window within the cutoff).  Kernel ms, one window, wide / narrow:
+//   haplotypes (128 / 64 partners), 60 of them: 400 SNPs 0.0236 / 0.0195, 1,500 (144 wide tiles by
+//   this bound) 0.0276 / 0.0256, 2,000 0.0276 / 0.0276, 2,500 0.040 / 0.046, 5,000 0.087 / 0.097;
+//   genotypes (24 / 12 partners, one accumulator buffer / two), 200 kb cutoff, 20 bins: 500
+//   individuals 300 SNPs 0.0192 / 0.0172, 2,000 0.057 / 0.054, 5,000 0.130 / 0.152, 100,000 2.65 /
+//   2.85; 1,200 individuals 1,000 SNPs 0.0295 / 0.0307, 100,000 3.97 / 5.36.  An MMA takes about as
+//   long for 12 partners as for 24, so the wide tile pays from kWideGenoK bytes of K on: 200
+//   individuals 100,000 SNPs 2.19 / 2.16, 60 1.96 / 1.82.  It is taken only with a staging copy per
+//   warp, which makes the sums reproducible (up to 24 bins; the narrow tile 34).
+constexpr int kWideGenoK = 384;
 int variant_of(const ldk_parse_t* d, const ParseShape& sh) {
     const int v = tuned_variant(d, sh);
     if (v >= 0) return v;
-    if (sh.genotypes || sh.P != 1 || sh.rtab_global) return 0;
-    const int64_t rows = tc_rows_per_block(sh), nj = tc_tile_width(sh, 0);
+    if (sh.P != 1 || sh.rtab_global) return 0;
+    if (sh.genotypes && (sh.ktot < kWideGenoK || !tc_private_staging(sh, 1))) return 0;
+    const int wide = sh.genotypes ? 1 : 0;  // the variant of the wider tile
+    const int64_t rows = tc_rows_per_block(sh), nj = tc_tile_width(sh, wide);
     int64_t tiles = 0;
     for (int w = 0; w < window_count(d) && tiles <= kSpreadCtas; ++w) {
         const int64_t m = window_bound(d, w + 1) - window_bound(d, w);
         tiles += (m + rows - 1) / rows * ((m + 2 * nj - 1) / (2 * nj));
     }
-    return tiles <= kSpreadCtas ? 1 : 0;
+    return tiles <= kSpreadCtas ? 1 - wide : wide;
 }
 
 // Candidates worth timing: the alternative tile only where its width differs, the window

@@ -94,3 +94,21 @@ def test_clearing_of_many_blocks(n_blocks):
     want = O.bin_sums(data, pos, rows, edges, **kw)
     for _ in range(2):  # the second run clears what the first one left
         _check(p.run().numpy(), want)
+
+
+# untuned genotypes of one population: 12 partners a tile up to 256 individuals or with no more
+# tiles than SMs (1,100 SNPs are nine row blocks x 23 tiles of 48 by the rule's bound, 300 three x
+# seven), else 24 where that leaves every warp its staging copy (32 bins do not)
+@pytest.mark.parametrize("n,m,bins,width", [(256, 1100, 9, 12), (257, 1100, 9, 24), (257, 300, 9, 12),
+                                            (400, 1100, 20, 24), (400, 1100, 32, 12)])
+def test_genotype_tile_rule(n, m, bins, width):
+    rng = np.random.default_rng(n + m)
+    data, rows = _hap(rng, (n,), m)
+    data = np.where(data < 0, -1, data + (rng.random(data.shape) < 0.3)).astype(np.int8)
+    pos = np.cumsum(rng.integers(1, 40, size=m)).astype(np.float64)
+    edges = np.linspace(0.0, 2000.0, bins + 1)
+    kw = dict(genotypes=True, max_dist=2000.0)
+    p = parse.Parser(data, pos, rows, edges, method="tc", **kw)
+    assert p.tile_width() == width
+    _check(p.run().numpy(), O.bin_sums(data, pos, rows, edges, **kw))
+    assert p.reproducible()
