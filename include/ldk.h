@@ -40,7 +40,8 @@ extern "C" {
 
 /* counting / estimator method of ldk_parse */
 #define LDK_METHOD_PLAIN_FP64 0 /* per-pair byte counting + FP64 estimators (the drop-in) */
-#define LDK_METHOD_TC 1         /* INT8 tcgen05 Gram moments; FP64 estimators on them (exact integers) and bins */
+#define LDK_METHOD_TC 1         /* INT8 tcgen05 Gram moments; FP64 estimators on them (integers, exact in
+                                 * populations of up to 5,792; above, on the counts they give) and bins */
 
 LDK_API int ldk_version(void);
 LDK_API const char* ldk_last_error(void);

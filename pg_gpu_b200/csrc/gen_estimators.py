@@ -16,8 +16,7 @@ The feature algebra was derived with sympy from the reference's formulas
 (``haplotype_kernels.py:69-304``); ``check()`` re-verifies every identity
 symbolically and the unit tests evaluate the same expression strings with NumPy
 against the float64 oracle.  The genotype path (``genotype_kernels.py``) keeps the
-reference's polynomial forms, which are written once in
-``ldk_geno_poly.cuh`` and shared by every kernel.
+reference's polynomials in Horner form.
 
 Run ``python -m pg_gpu_b200.csrc.gen_estimators`` to regenerate; ``build()`` does it.
 """
@@ -645,8 +644,8 @@ def emit_geno(P):
     feats = geno_features_needed(P)
     calls, stats = plan(P, geno=True)
     L = [f"// genotype path, P = {P}: {len(stats)} statistics from {len(calls)} distinct raw calls",
-         "template <typename T>", f"LDK_DEV void geno_features_P{P}(GenoFeat<T>& x) {{",
-         "    geno_prepare(x);"]
+         "template <typename T, bool PREP = true>", f"LDK_DEV void geno_features_P{P}(GenoFeat<T>& x) {{",
+         "    if constexpr (PREP) geno_prepare(x);"]
     for n, e in geno_features():
         if n in feats:
             L.append(f"    x.{n} = {_cexpr(e)};")
@@ -727,21 +726,33 @@ def emit_hap(P):
         if n in feats:
             L.append(f"    x.{n} = {_cexpr(e)};")
     L.append("}")
-    L.append("template <typename T, int S = 1>")
-    L.append(f"LDK_DEV void hap_stats_P{P}(const HapFeat<T>* f, T* acc) {{")
-    for ci, (case, args) in enumerate(calls):
-        L.append(f"    const T v{ci} = {_cexpr(hap_call_expr(case, args))};  // {case}{args}")
-    for si, (name, terms) in enumerate(stats):
-        groups = {}
-        for idx, w in terms:
-            groups.setdefault(w, []).append(f"v{idx}")
-        parts = []
-        for w, vs in sorted(groups.items(), reverse=True):
-            sw = _fmt_weight(w)
-            body = " + ".join(vs)
-            parts.append(body if sw is None else f"T({sw}) * ({body})")
-        L.append(f"    acc[{si} * S] += {' + '.join(parts)};  // {name}")
-    L.append("}")
+    # every statistic, and (four populations) the halves that two warps share as in spin_order
+    order, K = spin_order(P, False)
+    halves = [("template <typename T, int S = 1>", f"hap_stats_P{P}", range(len(stats)), " * S")]
+    if K:
+        halves += [("template <typename T>", f"hap_half_P{P}_{h}", mine, "") for h, mine in ((1, order[:K]), (2, order[K:]))]
+    for head, fn, mine, stride in halves:
+        mine = list(mine)
+        used = {idx for si in mine if si < len(stats) for idx, _ in stats[si][1]}
+        L.append(head)
+        L.append(f"LDK_DEV void {fn}(const HapFeat<T>* f, T* acc) {{")
+        for ci, (case, args) in enumerate(calls):
+            if ci in used:
+                L.append(f"    const T v{ci} = {_cexpr(hap_call_expr(case, args))};  // {case}{args}")
+        for at, si in enumerate(mine):
+            if si == len(stats):
+                continue  # r^2: the caller's
+            name, terms = stats[si]
+            groups = {}
+            for idx, w in terms:
+                groups.setdefault(w, []).append(f"v{idx}")
+            parts = []
+            for w, vs in sorted(groups.items(), reverse=True):
+                sw = _fmt_weight(w)
+                body = " + ".join(vs)
+                parts.append(body if sw is None else f"T({sw}) * ({body})")
+            L.append(f"    acc[{at}{stride}] += {' + '.join(parts)};  // {name}")
+        L.append("}")
     return "\n".join(L)
 
 
@@ -765,15 +776,29 @@ def emit_hap(P):
 #   Q4 = u v - 4 Q3 - 2 Q2    = sum over distinct k, m, l, o of sigma_k sigma_m tau_l tau_o
 # (the pairs {k, m} and {l, o} of u v overlap in one index in four ways, in both in two).
 # A haplotype has sigma^2 = 1, so SS = TT = SSTT = n, SST = T, STT = S and Q3 = R W - u - v.
-# All numerators are integers, exact in FP64 below 2^53 (populations of up to ~8,000), so a
-# statistic that is exactly zero stays zero; each is scaled by the tabulated reciprocals and
-# added with one FMA.  The constant factors (powers of two) are applied once per staged sum
-# (SPIN weights), not per pair.  ``check()`` proves the forms equal to the raw calls.
+# All numerators are integers and no intermediate of theirs exceeds 8 N^4 in populations of at
+# most N, so up to N = SPIN_MAX_N = 5,792 (8 N^4 <= 2^53) FP64 holds them exactly and a statistic
+# that is exactly zero stays zero; each is scaled by the tabulated reciprocals and added with one
+# FMA.  The constant factors (powers of two) are applied once per staged sum (SPIN weights), not
+# per pair.  ``check()`` proves the forms equal to the raw calls.
+#
+# Above SPIN_MAX_N the n^4 terms would cancel to rounding remainders where the alleles are rare
+# (DD of singletons 1e-7 off at n = 100,000, sigma_D^2 = 1 where both numerators are 0), so the
+# kernels recover the two-locus counts from the moments (HAP_CELLS, GENO_CELLS: exact) and
+# evaluate the raw calls on them, whose terms are as small as the rare counts.
 #
 # Expressions are C and Python syntax over the names below, suffixed with the population.
 
+SPIN_MAX_N = 5792
 SPIN_INPUTS = ["n", "S", "T", "R", "r1", "r2", "r3", "r4"]
 SPIN_INPUTS_GENO = SPIN_INPUTS + ["SS", "TT", "SST", "STT", "SSTT"]
+# counts n11, n10, n01, n00 and n00, n01, ..., n22 (genotypes; column g_i * 3 + g_j) of the moments:
+# [x = 1] = (1 - sigma) / 2; [g = 0] = (sigma^2 + sigma) / 2, [g = 1] = 1 - sigma^2, [g = 2] = (sigma^2 - sigma) / 2
+HAP_CELLS = ["0.25 * ((n - S) - (T - R))", "0.25 * ((n - S) + (T - R))", "0.25 * ((n + S) - (T + R))",
+             "0.25 * ((n + S) + (T + R))"]
+GENO_CELLS = ["0.25 * ((SSTT + R) + (SST + STT))", "0.5 * ((SS + S) - (SSTT + STT))", "0.25 * ((SSTT - R) - (SST - STT))",
+              "0.5 * ((TT + T) - (SSTT + SST))", "(n - SS) - (TT - SSTT)", "0.5 * ((TT - T) - (SSTT - SST))",
+              "0.25 * ((SSTT - R) + (SST - STT))", "0.5 * ((SS - S) - (SSTT - STT))", "0.25 * ((SSTT + R) - (SST + STT))"]
 
 
 def _spin_pop(p, geno):
@@ -968,6 +993,18 @@ def emit_spin_numerators(geno):
     return "\n".join(head + lines + ["    dd = DD0;", "    pi2 = PI0;", "}"])
 
 
+def emit_cells():
+    """The two-locus counts of a population's moments."""
+    import re
+    members = lambda e: re.sub(r"[A-Z]+\b|\bn\b", lambda m: "m." + m.group(0), e)  # noqa: E731
+    L = [f"constexpr int kSpinMaxN = {SPIN_MAX_N};  // largest population of the spin forms",
+         "LDK_DEV void spin_hap_cells(const SpinPop& m, double (&c)[4]) {"]
+    L += [f"    c[{k}] = {members(e)};" for k, e in enumerate(HAP_CELLS)]
+    L += ["}", "LDK_DEV void spin_geno_cells(const SpinPop& m, double (&c)[9]) {"]
+    L += [f"    c[{k}] = {members(e)};" for k, e in enumerate(GENO_CELLS)]
+    return "\n".join(L + ["}"])
+
+
 def _cexpr(e):
     """Numeric literals as T(...) so float and double instantiations stay exact."""
     import re
@@ -979,8 +1016,9 @@ HEADER = """// GENERATED by gen_estimators.py -- do not edit by hand.
 // Straight-line two-locus LD estimators for P = 1..4 populations (haplotype path).
 // Statistic order and averaging weights follow moments.LD (pg_gpu ld_pipeline.py:357-457);
 // raw-call algebra restates pg_gpu haplotype_kernels.py:69-304 in factored form.
-// hap_stats_P* evaluate every distinct raw call (plain kernel, raw-call entry points);
-// spin_hap_P* / spin_geno_P* are the statistic-level forms of the tensor-core parse.
+// hap_stats_P* / geno_stats_P* evaluate every distinct raw call (plain kernel, raw-call entry
+// points, tensor-core parse of populations above kSpinMaxN); spin_hap_P* / spin_geno_P* are the
+// statistic-level forms of the tensor-core parse.
 #pragma once
 """
 
@@ -1002,6 +1040,8 @@ def generate(path=None):
     for geno in (False, True):
         parts.append(emit_spin_numerators(geno))
         parts.append("")
+    parts.append(emit_cells())
+    parts.append("")
     parts.append(emit_raw_dispatch())
     parts.append("")
     parts.append("template <int P> struct HapNStats;")
@@ -1019,12 +1059,19 @@ LDK_DEV void hap_features(HapFeat<T>& x) {
     else if constexpr (P == 3) hap_features_P3<T>(x);
     else hap_features_P4<T>(x);
 }
-template <typename T, int P>
+template <typename T, int P, int S = 1>
+LDK_DEV void hap_stats(const HapFeat<T>* f, T* acc) {
+    if constexpr (P == 1) hap_stats_P1<T, S>(f, acc);
+    else if constexpr (P == 2) hap_stats_P2<T, S>(f, acc);
+    else if constexpr (P == 3) hap_stats_P3<T, S>(f, acc);
+    else hap_stats_P4<T, S>(f, acc);
+}
+template <typename T, int P, bool PREP = true>
 LDK_DEV void geno_features(GenoFeat<T>& x) {
-    if constexpr (P == 1) geno_features_P1<T>(x);
-    else if constexpr (P == 2) geno_features_P2<T>(x);
-    else if constexpr (P == 3) geno_features_P3<T>(x);
-    else geno_features_P4<T>(x);
+    if constexpr (P == 1) geno_features_P1<T, PREP>(x);
+    else if constexpr (P == 2) geno_features_P2<T, PREP>(x);
+    else if constexpr (P == 3) geno_features_P3<T, PREP>(x);
+    else geno_features_P4<T, PREP>(x);
 }
 template <typename T, int P, int S = 1>
 LDK_DEV void geno_stats(const GenoFeat<T>* f, T* acc) {
@@ -1051,6 +1098,57 @@ LDK_DEV void spin_stats(const SpinPop* f, bool ok, double* acc, unsigned& nr2) {
         else spin_hap_P4_2(f, ok, acc, nr2);
     }
 }
+// The same statistics, weights applied, from the counts behind the moments: populations of more
+// than kSpinMaxN.  The caller sets the pair's n and reciprocals.
+template <int P, bool GENO, int PART>
+LDK_DEV void count_stats(const SpinPop* m, double* acc, unsigned& nr2) {
+    constexpr int NS = HapNStats<P>::value;
+    if constexpr (GENO) {
+        GenoFeat<double> f[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            double c[9];
+            spin_geno_cells(m[p], c);
+            geno_set_counts(f[p], c);
+            f[p].n = m[p].n;
+            if constexpr (P < 4) {
+                geno_prepare_from(f[p], m[p].r1, m[p].r2, m[p].r3, m[p].r4);
+                geno_features<double, P, false>(f[p]);
+            } else {  // four populations divide: the table's registers double their spill
+                geno_features<double, P>(f[p]);
+            }
+        }
+        geno_stats<double, P>(f, acc);
+        const double E = fma(m[0].n, m[0].R, -(m[0].S * m[0].T));
+        const double den = fma(m[0].n, m[0].SS, -(m[0].S * m[0].S)) * fma(m[0].n, m[0].TT, -(m[0].T * m[0].T));
+        if (den > 0.0) {
+            acc[NS] = fma(E * E, recip_cubic(den), acc[NS]);
+            ++nr2;
+        }
+    } else {
+        HapFeat<double> f[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            double c[4];
+            spin_hap_cells(m[p], c);
+            hap_set_counts(f[p], c[0], c[1], c[2], c[3]);
+            f[p].r1 = m[p].r1;
+            f[p].r2 = m[p].r2;
+            f[p].r3 = m[p].r3;
+            f[p].r4 = m[p].r4;
+            hap_features<double, P>(f[p]);
+        }
+        constexpr int R2 = PART == 1 ? SpinSplit<P>::value - 1 : NS;  // where r^2 is staged
+        if constexpr (PART == 0) hap_stats<double, P>(f, acc);
+        else if constexpr (PART == 1) hap_half_P4_1<double>(f, acc);
+        else hap_half_P4_2<double>(f, acc);
+        double r2;
+        if (PART != 2 && hap_r2(f[0], r2)) {
+            acc[R2] += r2;
+            ++nr2;
+        }
+    }
+}
 // Weight and statistic (number of statistics: r^2, weight 1) of staged sum s.
 template <int P, bool GENO>
 LDK_DEV double spin_weight(int s) {
@@ -1063,13 +1161,6 @@ template <int P, bool GENO>
 LDK_DEV int spin_stat(int s) {
     if constexpr (GENO || P < 4) return s;
     else return spin_stat_hap_P4[s];
-}
-template <typename T, int P, int S = 1>
-LDK_DEV void hap_stats(const HapFeat<T>* f, T* acc) {
-    if constexpr (P == 1) hap_stats_P1<T, S>(f, acc);
-    else if constexpr (P == 2) hap_stats_P2<T, S>(f, acc);
-    else if constexpr (P == 3) hap_stats_P3<T, S>(f, acc);
-    else hap_stats_P4<T, S>(f, acc);
 }
 """)
     text = "\n".join(parts)
@@ -1172,6 +1263,9 @@ def check_spin(seed=0, trials=12, small_haplotypes=False):
                                          "STT": (1, 2), "SSTT": (2, 2)}.items():
                         env[f"{name}{p}"] = Fr(sum(k * s ** a * t ** b for k, (s, t) in zip(c, st)))
                     env[f"n{p}"] = n
+                    loc = {"n": n, **{k[:-len(str(p))]: v for k, v in env.items() if k.endswith(str(p)) and k[0] in "STR"}}
+                    cells = [eval(code(e), {"Fr": Fr}, loc) for e in (GENO_CELLS if geno else HAP_CELLS)]
+                    assert cells == (c[::-1] if geno else c), (geno, cells, c)
                     for k in range(4):
                         env[f"r{k + 1}{p}"] = inv(d[k])
                 for k, e in defs.items():

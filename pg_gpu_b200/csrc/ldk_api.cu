@@ -85,6 +85,7 @@ bool shape_of(const ldk_parse_t* d, ParseShape& sh) {
     sh.ktot = (k + 127) / 128 * 128;
     sh.rtab_global = 0;
     sh.rtab_global = (d->method != LDK_METHOD_PLAIN_FP64 && !sh.genotypes && tc_rtab_global(sh)) ? 1 : 0;
+    sh.from_counts = (d->method != LDK_METHOD_PLAIN_FP64 && tc_from_counts(sh)) ? 1 : 0;
     return true;
 }
 

@@ -39,6 +39,21 @@ LDK_DEV void geno_prepare(GenoFeat<T>& x) {
     x.w4 = (ns >= T(4)) ? T(1) / (ns * (ns - T(1)) * (ns - T(2)) * (ns - T(3))) : T(0);
 }
 
+// geno_prepare for n = ns >= 0 without a division: from 1/n, 1/(n(n-1)), 1/(n(n-1)(n-2)), not
+// finite where n is too small, and the guarded four-fold reciprocal (recip_entry_geno).
+LDK_DEV void geno_prepare_from(GenoFeat<double>& x, double u1, double u2, double u3, double w4) {
+    const double n = x.n;
+    x.inn1 = n >= 2.0 ? 0.25 * u2 : 1.0;
+    x.invn = u1;
+    x.r1 = n >= 1.0 ? u1 : 0.0;
+    x.r2 = n >= 2.0 ? u2 : 0.0;
+    x.r3 = n >= 3.0 ? u3 : 0.0;
+    x.u1 = u1;
+    x.u2 = u2;
+    x.u3 = u3;
+    x.w4 = w4;
+}
+
 // Pairwise-complete dosage (Rogers-Huff) r^2 from the nine cells; false where either
 // locus is constant (pg_gpu ld_statistics.py:410-443 returns NaN there).
 template <typename T>

@@ -39,6 +39,7 @@ struct ParseShape {
     int slots;                   // TC path: bootstrap blocks staged per row block (1 without blocks)
     int rtab_global;             // TC haplotype path: the reciprocal table (32 B per n_valid)
                                  // does not fit beside the pipeline in shared memory
+    int from_counts;             // TC path: a population is too large for the spin forms
 };
 
 // launchers (ldk_plain.cu)
@@ -83,6 +84,11 @@ cudaError_t launch_tc_hap_v1(const ldk_parse_t* d, const ldk_parse_out_t* o, con
                              int max_items, cudaStream_t s);
 cudaError_t launch_tc_geno(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                            int max_items, int variant, cudaStream_t s);
+// the same for sh.from_counts (ldk_tc_counts_hap.cu, the wider tile only; ldk_tc_counts_geno.cu)
+cudaError_t launch_tc_counts_hap(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
+                                 int max_items, int variant, cudaStream_t s);
+cudaError_t launch_tc_counts_geno(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
+                                  int max_items, int variant, cudaStream_t s);
 int tc_tile_width(const ParseShape& sh, int variant);  // partners per tile of a tile variant
 int tc_rows_per_block(const ParseShape& sh);
 int tc_block_slots(const ParseShape& sh);  // bootstrap blocks one row block may cover
@@ -90,6 +96,7 @@ int tc_planes(const ParseShape& sh);
 cudaError_t probe_peaks(double* int8_ops_per_s, double* fp64_fma_per_s, unsigned* status, cudaStream_t s);
 size_t tc_smem_bytes(const ParseShape& sh);
 bool tc_rtab_global(const ParseShape& sh);  // where the reciprocal table must live
+bool tc_from_counts(const ParseShape& sh);  // the spin forms are not exact for its largest population
 bool tc_private_staging(const ParseShape& sh, int variant);  // one staging copy per epilogue warp
 
 cudaError_t launch_build_items(const Scratch& w, int n_windows, int rows, cudaStream_t s);

@@ -318,6 +318,8 @@ bool tc_rtab_global(const ParseShape& sh) {
     }
 }
 
+bool tc_from_counts(const ParseShape& sh) { return sh.max_n > kSpinMaxN; }
+
 // The spin planes, and with `o` the rest of a parse's preparation in the same launch: pair
 // ranges, the cleared accumulators and pair tallies, the reciprocal table.  (Separate kernels and
 // memsets each waited for the one before: with the outputs' own memsets, which the bin sums
@@ -485,6 +487,9 @@ cudaError_t launch_split_items(const Scratch& w, int n_row_blocks, int nj, int m
 
 cudaError_t launch_parse_tc(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
                             const ParseShape& sh, int max_items, int variant, cudaStream_t s) {
+    if (sh.from_counts)
+        return sh.genotypes ? launch_tc_counts_geno(d, o, w, sh, max_items, variant, s)
+                            : launch_tc_counts_hap(d, o, w, sh, max_items, variant, s);
     if (sh.genotypes) return launch_tc_geno(d, o, w, sh, max_items, variant, s);
     return variant == 1 ? launch_tc_hap_v1(d, o, w, sh, max_items, s) : launch_tc_hap_v0(d, o, w, sh, max_items, s);
 }

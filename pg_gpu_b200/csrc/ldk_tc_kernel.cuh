@@ -559,7 +559,12 @@ LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a) {
 // GT: the haplotype path's reciprocal table is read from the workspace (a.rtab_g) instead of
 // being built in shared memory -- a compile-time choice, so that the shared-memory form keeps
 // its hot loop unchanged.
-template <int P, bool PRIV, bool GENO, int V, bool GT = false>
+// CNT: populations of more than kSpinMaxN, where the spin forms are no longer exact; the
+// statistics come from the counts behind the moments.  Loads and MMAs of so many haplotypes hide
+// most of the raw calls' extra FP64 operations: 6,000 haplotypes x 20,000 SNPs 3.33 ms with the spin
+// forms, 3.36 with this; 100,000 x 1,000 0.523, 0.527; 6,000 + 6,000 x 4,000 0.84, 0.86; genotypes,
+// whose raw calls are long polynomials, 20,000 x 2,000 0.43, 0.47, 6,000 + 60 + 60 x 2,000 0.45, 0.80.
+template <int P, bool PRIV, bool GENO, int V, bool GT = false, bool CNT = false>
 __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     k_parse_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a) {
     using C = Cfg<P, GENO, V>;
@@ -939,7 +944,11 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                             else spin_reciprocals(m, rtab[nval[u][p]]);
                             if (U > 1 && !counts) m.r1 = m.r2 = m.r3 = m.r4 = 0.0;
                         }
-                        if constexpr (SSPL) {
+                        if constexpr (CNT) {  // called for counted pairs only
+                            if constexpr (!SSPL) count_stats<P, GENO, 0>(f[u], acc, nr2);
+                            else if (part == 0) count_stats<P, GENO, 1>(f[u], acc, nr2);
+                            else count_stats<P, GENO, 2>(f[u], acc, nr2);
+                        } else if constexpr (SSPL) {
                             if (part == 0) spin_stats<P, GENO, 1>(f[u], counts, acc, nr2);
                             else spin_stats<P, GENO, 2>(f[u], counts, acc, nr2);
                         } else {
@@ -947,7 +956,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                         }
                         np += counts;
                     };
-                    if (U > 1 && !change) {
+                    if (U > 1 && !CNT && !change) {
                         // every pair stays in its lane's bin: evaluated together, without branches
 #pragma unroll
                         for (int u = 0; u < U; ++u) evaluate(u, valid[u] && in_bin);
@@ -989,8 +998,8 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 const int bb = rem / (NS + 1), s = rem % (NS + 1);
                 const int blk = blk0 + sl;
                 if (val != 0.0 && blk < a.n_blocks)
-                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + spin_stat<P, GENO>(s)) * kFxLimbs, val * spin_weight<P, GENO>(s),
-                           a.status);
+                    fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + spin_stat<P, GENO>(s)) * kFxLimbs,
+                           CNT ? val : val * spin_weight<P, GENO>(s), a.status);
             }
             for (int idx = et; idx < slots * nb; idx += 32 * EPI) {
                 unsigned long long c0 = 0, c1 = 0;
@@ -1109,7 +1118,7 @@ bool rtab_global_t(const ParseShape& sh) {
     return smem_bytes_t<P, false, 0>(nb, t, 1) > kMaxSmem;
 }
 
-template <int P, bool PRIV, bool GENO, int V, bool GT>
+template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT>
 cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
                                      const ParseShape& sh, int max_items, cudaStream_t s) {
     using C = Cfg<P, GENO, V>;
@@ -1157,7 +1166,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
-        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if constexpr (C::SPLIT) {
         // the register split adds up only at C::REG_LAUNCH registers per thread; any other
@@ -1165,7 +1174,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
         static std::atomic<int> regs{-1};  // of this build's kernel: asked for once
         if (regs.load() < 0) {
             cudaFuncAttributes fa;
-            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT>);
+            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT>);
             if (e != cudaSuccess) return e;
             regs.store(fa.numRegs);
         }
@@ -1176,7 +1185,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (max_items == 0) return cudaSuccess;
     const int grid = max_items < sms ? max_items : sms;
-    k_parse_tc<P, PRIV, GENO, V, GT><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
+    k_parse_tc<P, PRIV, GENO, V, GT, CNT><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
     return cudaGetLastError();
 }
 
@@ -1185,28 +1194,34 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
 // table in shared memory or (FP64 estimators, widest tile only) in the workspace.  Other
 // variants answer cudaErrorInvalidConfiguration for a workspace table, which the tile
 // autotuner reads as "does not fit this shape".
-template <int PP, bool GENO, int V>
+template <int PP, bool GENO, int V, bool CNT>
 cudaError_t launch_staged(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                           int max_items, cudaStream_t s) {
     const bool priv = private_staging<PP, GENO, V>(sh.n_bins, smem_table(sh));
     if (!GENO && sh.rtab_global) {
         if constexpr (!GENO && V == 0)
-            return priv ? launch_parse_tc_p<PP, true, GENO, V, true>(d, o, w, sh, max_items, s)
-                        : launch_parse_tc_p<PP, false, GENO, V, true>(d, o, w, sh, max_items, s);
+            return priv ? launch_parse_tc_p<PP, true, GENO, V, true, CNT>(d, o, w, sh, max_items, s)
+                        : launch_parse_tc_p<PP, false, GENO, V, true, CNT>(d, o, w, sh, max_items, s);
         else
             return cudaErrorInvalidConfiguration;
     }
-    return priv ? launch_parse_tc_p<PP, true, GENO, V, false>(d, o, w, sh, max_items, s)
-                : launch_parse_tc_p<PP, false, GENO, V, false>(d, o, w, sh, max_items, s);
+    if constexpr (!GENO && CNT) {  // a table of kSpinMaxN entries never fits in shared memory
+        static_assert((size_t)kSpinMaxN * sizeof(double4) + Cfg<PP, GENO, V>::STAGES * Cfg<PP, GENO, V>::STAGE_BYTES > kMaxSmem,
+                      "counted haplotypes keep their table in the workspace");
+        return cudaErrorInvalidConfiguration;
+    } else {
+        return priv ? launch_parse_tc_p<PP, true, GENO, V, false, CNT>(d, o, w, sh, max_items, s)
+                    : launch_parse_tc_p<PP, false, GENO, V, false, CNT>(d, o, w, sh, max_items, s);
+    }
 }
 
 // One tile variant of one path, over the population count and staging.
-template <bool GENO, int V>
+template <bool GENO, int V, bool CNT = false>
 cudaError_t dispatch_tc(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                         int max_items, cudaStream_t s) {
 #define LDK_TC_CASE(PP)                                                                                   \
     case PP:                                                                                              \
-        return launch_staged<PP, GENO, V>(d, o, w, sh, max_items, s);
+        return launch_staged<PP, GENO, V, CNT>(d, o, w, sh, max_items, s);
     switch (sh.P) {
         LDK_TC_CASE(1)
         LDK_TC_CASE(2)
