@@ -53,6 +53,13 @@ LDK_DEV double recip_newton(double x) {
 }
 LDK_DEV float recip_newton(float x) { return 1.0f / x; }
 
+// The DD and pi2 numerators of one population from its counts (ld_statistics.py:326-343).
+LDK_DEV void hap_numerators(double c1, double c2, double c3, double c4, double& dd, double& pi2) {
+    dd = c1 * (c1 - 1.0) * c4 * (c4 - 1.0) + c2 * (c2 - 1.0) * c3 * (c3 - 1.0) - 2.0 * c1 * c2 * c3 * c4;
+    pi2 = (c1 + c2) * (c1 + c3) * (c2 + c4) * (c3 + c4) - c1 * c4 * (-1.0 + c1 + 3.0 * c2 + 3.0 * c3 + c4) -
+          c2 * c3 * (-1.0 + 3.0 * c1 + c2 + c3 + 3.0 * c4);
+}
+
 template <typename T>
 LDK_DEV bool hap_r2(const HapFeat<T>& x, T& r2) {
     const T den = (x.c1 + x.c2) * (x.c3 + x.c4) * ((x.c1 + x.c3) * (x.c2 + x.c4));

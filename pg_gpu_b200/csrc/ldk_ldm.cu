@@ -15,7 +15,6 @@
 #include <cmath>
 
 #include "ldk_tc_kernel.cuh"
-#include "ldk_spin.cuh"
 
 namespace ldk {
 
@@ -102,7 +101,11 @@ __global__ void __launch_bounds__(32 * kSiteWarps)
     site[v] = r;
 }
 
-template <int EST>
+// CNT (sigma_D^2 of more than kSpinMaxN rows): the numerators from the counts, because the moment
+// form's n^4 terms no longer cancel exactly there (two singletons on one haplotype of 20,000: 0 / 0
+// became -16 / -16).  6,000 haplotypes x 4,000 SNPs 0.371 ms with the moment form, 0.375 with this;
+// genotypes 1.157, 1.208.
+template <int EST, bool CNT = false>
 __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
     k_ld_matrix(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                 const LdmArgs m) {
@@ -233,10 +236,16 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
                         } else {
                             const double n = i2d_exact(in), S = i2d_exact(iS), T = i2d_exact(iT), R = i2d_exact(iR);
                             if constexpr (EST == LDK_LDM_SIGMA_D2) {
-                                // ld_statistics.py:326-343: the DD and pi2 numerators (exact
-                                // integers in FP64), 16 times each
+                                // ld_statistics.py:326-343: the DD and pi2 numerators, exact
+                                // integers in FP64 (up to kSpinMaxN; 16 times each) or, from the
+                                // counts, where these are small
                                 double dd, pi2;
-                                spin_hap_numerators(n, S, T, R, dd, pi2);
+                                if constexpr (CNT)
+                                    hap_numerators(i2d_exact((in - iS - iT + iR) >> 2), i2d_exact((in - iS + iT - iR) >> 2),
+                                                   i2d_exact((in + iS - iT - iR) >> 2), i2d_exact((in + iS + iT + iR) >> 2),
+                                                   dd, pi2);
+                                else
+                                    spin_hap_numerators(n, S, T, R, dd, pi2);
                                 counted = in >= 4;
                                 val = (counted && pi2 != 0.0) ? dd * recip_cubic(pi2) : 0.0;
                             } else {
@@ -301,6 +310,7 @@ struct LdmGArgs {
     double* sums;
 };
 
+template <bool CNT>  // as for k_ld_matrix
 __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
     k_ld_matrix_geno(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a,
                      const LdmGArgs m) {
@@ -395,7 +405,21 @@ __global__ void __launch_bounds__(128 + 32 * kLdmGEpi, 1)
                         // 1: sigma^2, 2: valid); DD over pi2 of one population
                         // (genotype_kernels.py:91-170)
                         double dd, pi2;
-                        spin_geno_numerators(G, dd, pi2);
+                        if constexpr (CNT) {
+                            const SpinPop s{i2d_exact((int)G[2][2]), i2d_exact((int)G[0][2]), i2d_exact((int)G[2][0]),
+                                            i2d_exact((int)G[0][0]), i2d_exact((int)G[1][2]), i2d_exact((int)G[2][1]),
+                                            i2d_exact((int)G[1][0]), i2d_exact((int)G[0][1]), i2d_exact((int)G[1][1])};
+                            double c[9];
+                            spin_geno_cells(s, c);
+                            GenoFeat<double> f{};
+                            f.w4 = 1.0;  // n(n-1)(n-2)(n-3) cancels
+                            geno_set_counts(f, c);
+                            geno_features<double, 1, false>(f);
+                            dd = 0.25 * f.DD1;  // the genotype DD is four times the moment form's
+                            pi2 = f.PI1;
+                        } else {
+                            spin_geno_numerators(G, dd, pi2);
+                        }
                         if ((int)G[2][2] >= 4 && pi2 > 0.0) {
                             val = 4.0 * dd * recip_cubic(pi2);
                             zsum += val;
@@ -481,24 +505,25 @@ size_t ldm_smem(TcArgs& a, size_t other) {
     return other + (size_t)a.stages * C::STAGE_BYTES;
 }
 
+template <bool CNT>
 cudaError_t launch_ldm_geno(const CUtensorMap& mA, const CUtensorMap& mB, TcArgs& a, const LdmGArgs& m,
                             cudaStream_t s) {
     size_t smem = ldm_smem<LdmGCfg>(a, 1024 + (size_t)kLdmGEpi * 32 * kLdmGStride * sizeof(double));
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix_geno, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix_geno<CNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ld_matrix_geno<<<sm_count(), 128 + 32 * kLdmGEpi, smem, s>>>(mA, mB, a, m);
+    k_ld_matrix_geno<CNT><<<sm_count(), 128 + 32 * kLdmGEpi, smem, s>>>(mA, mB, a, m);
     return cudaGetLastError();
 }
 
-template <int EST>
+template <int EST, bool CNT = false>
 cudaError_t launch_ldm(const CUtensorMap& mA, const CUtensorMap& mB, TcArgs& a, const LdmArgs& m, cudaStream_t s) {
     size_t smem = ldm_smem<LdmCfg>(a, 1024 + (a.max_n < kLdmTable ? a.max_n + 1 : 0) * sizeof(double));
     if (smem < kMinSmem) smem = kMinSmem;
-    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix<EST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_ld_matrix<EST, CNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_ld_matrix<EST><<<sm_count(), 128 + 32 * kLdmEpi, smem, s>>>(mA, mB, a, m);
+    k_ld_matrix<EST, CNT><<<sm_count(), 128 + 32 * kLdmEpi, smem, s>>>(mA, mB, a, m);
     return cudaGetLastError();
 }
 
@@ -568,11 +593,16 @@ cudaError_t launch_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const
     for (int p = 0; p <= LDK_MAX_POPS; ++p) a.kofs[p] = sh.kofs[p];
     a.max_n = n_sel;
     a.status = status;
-    if (nine) return launch_ldm_geno(mA, mB, a, LdmGArgs{out, ld_out, sums}, s);
+    const bool counts = n_sel > kSpinMaxN;
+    if (nine) {
+        const LdmGArgs g{out, ld_out, sums};
+        return counts ? launch_ldm_geno<true>(mA, mB, a, g, s) : launch_ldm_geno<false>(mA, mB, a, g, s);
+    }
     const LdmArgs m{site, out, ld_out, sums};
     switch (estimator) {
         case LDK_LDM_R2: return launch_ldm<LDK_LDM_R2>(mA, mB, a, m, s);
-        case LDK_LDM_SIGMA_D2: return launch_ldm<LDK_LDM_SIGMA_D2>(mA, mB, a, m, s);
+        case LDK_LDM_SIGMA_D2:
+            return counts ? launch_ldm<LDK_LDM_SIGMA_D2, true>(mA, mB, a, m, s) : launch_ldm<LDK_LDM_SIGMA_D2>(mA, mB, a, m, s);
         case LDK_LDM_R2_COUNTS: return launch_ldm<LDK_LDM_R2_COUNTS>(mA, mB, a, m, s);
         case LDK_LDM_DIPLOID_R2: return launch_ldm<LDK_LDM_DIPLOID_R2>(mA, mB, a, m, s);
         default: return launch_ldm<LDK_LDM_ROGERS_HUFF_R>(mA, mB, a, m, s);
