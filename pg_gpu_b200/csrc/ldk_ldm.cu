@@ -36,7 +36,8 @@ struct LdmArgs {
 // Per SNP over the selected rows, into site[v]:
 //   LDK_LDM_R2              {p, 1 / (p (1 - p))}, p = derived / valid calls (haplotype_matrix.py:1119-1120)
 //   LDK_LDM_DIPLOID_R2      {m, 1 / V}, m the mean spin (1 - dosage) of the valid calls, V their sum
-//   LDK_LDM_ROGERS_HUFF_R   {m, 1 / sqrt(V)}        of squared deviations (ld_statistics.py:1000-1011)
+//                           of squared deviations (ld_statistics.py:1000-1011)
+//   LDK_LDM_ROGERS_HUFF_R   {d, 1 / sqrt(V)}, d the mean dosage
 // with 0 for the reciprocal of 0; and the partner range (the rest of the set) and the matrix
 // diagonal.  With `strict` a missing call sets LDK_DEVERR_BAD_INPUT (the Rogers-Huff and
 // sigma_D^2 genotype estimators take complete data, ld_statistics.py:389-399).
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(32 * kSiteWarps)
         // spins: 1 for dosage 0, 0 for 1, -1 for 2; V = (n sum s^2 - (sum s)^2) / n, exact numerator
         const double n = c[0], S = (double)(c[0] - c[1] - 2 * c[2]), SS = (double)(c[0] - c[1]);
         const double V = c[0] > 0 ? fma(n, SS, -(S * S)) / n : 0.0;
-        r.x = c[0] > 0 ? S / n : 0.0;
+        if (c[0] > 0) r.x = (estimator == LDK_LDM_DIPLOID_R2 ? S : (double)(c[1] + 2 * c[2])) / n;
         if (V > 0.0) r.y = estimator == LDK_LDM_DIPLOID_R2 ? 1.0 / V : 1.0 / sqrt(V);
     }
     site[v] = r;
@@ -228,8 +229,10 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
                             const double cov = fma(-sj[g].x, fma(-si.x, n, S), fma(-si.x, T, R));
                             val = (cov * cov) * (si.y * sj[g].y);
                         } else if constexpr (EST == LDK_LDM_ROGERS_HUFF_R) {
-                            // ld_statistics.py:392-437 (complete data); NaN where a site is constant
-                            const double cov = fma(-(si.x * sj[g].x), i2d_exact(in), i2d_exact(iR));
+                            // ld_statistics.py:392-437 (complete data); NaN where a site is constant.
+                            // Of dosages 1 - sigma, not spins: of rare alleles their sums are small,
+                            // where R - mean mean n cancels n - n
+                            const double cov = fma(-(si.x * sj[g].x), i2d_exact(in), i2d_exact(in - iS - iT + iR));
                             const double s = si.y * sj[g].y;
                             counted = s > 0.0;
                             val = counted ? cov * s : CUDART_NAN;
