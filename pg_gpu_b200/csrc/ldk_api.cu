@@ -229,7 +229,7 @@ int prepare(const ldk_parse_t* d, void* workspace, size_t workspace_bytes, Prepa
     }
     if (reinterpret_cast<uintptr_t>(workspace) % 256) { set_error("workspace must be 256-byte aligned"); return LDK_ERR_ARG; }
     if (int rc = check_arch()) return rc;
-    if (d->method != LDK_METHOD_PLAIN_FP64 && tc_smem_bytes(P.sh) > 227 * 1024) {
+    if (d->method != LDK_METHOD_PLAIN_FP64 && !tc_fits(P.sh)) {
         set_error("bins x statistics exceed the tensor-core kernel's shared-memory staging");
         return LDK_ERR_UNSUPPORTED;
     }
@@ -363,7 +363,7 @@ int tuned_variant(const ldk_parse_t* d, const ParseShape& sh) {
 //   2.85; 1,200 individuals 1,000 SNPs 0.0295 / 0.0307, 100,000 3.97 / 5.36.  An MMA takes about as
 //   long for 12 partners as for 24, so the wide tile pays from kWideGenoK bytes of K on: 200
 //   individuals 100,000 SNPs 2.19 / 2.16, 60 1.96 / 1.82.  It is taken only with a staging copy per
-//   warp, which makes the sums reproducible (up to 24 bins; the narrow tile 34).
+//   warp, which makes the sums reproducible (up to 24 bins; the narrow tile 33, without blocks 34).
 constexpr int kWideGenoK = 384;
 int variant_of(const ldk_parse_t* d, const ParseShape& sh) {
     const int v = tuned_variant(d, sh);

@@ -94,7 +94,7 @@ int tc_rows_per_block(const ParseShape& sh);
 int tc_block_slots(const ParseShape& sh);  // bootstrap blocks one row block may cover
 int tc_planes(const ParseShape& sh);
 cudaError_t probe_peaks(double* int8_ops_per_s, double* fp64_fma_per_s, unsigned* status, cudaStream_t s);
-size_t tc_smem_bytes(const ParseShape& sh);
+bool tc_fits(const ParseShape& sh);  // the default tile's kernel, with one staging copy, into shared memory
 bool tc_rtab_global(const ParseShape& sh);  // where the reciprocal table must live
 bool tc_from_counts(const ParseShape& sh);  // the spin forms are not exact for its largest population
 bool tc_private_staging(const ParseShape& sh, int variant);  // one staging copy per epilogue warp

@@ -289,20 +289,30 @@ int tc_block_slots(const ParseShape& sh) { return sh.genotypes ? Cfg<1, true>::S
 int tc_tile_width(const ParseShape& sh, int variant) { return tile_nj(sh.P, sh.genotypes != 0, variant); }
 int tc_planes(const ParseShape& sh) { return sh.genotypes ? Cfg<1, true>::PLANES : Cfg<1, false>::PLANES; }
 
-size_t tc_smem_bytes(const ParseShape& sh) {
-    return sh.genotypes ? tc_smem_bytes_g<true>(sh) : tc_smem_bytes_g<false>(sh);
+namespace {
+template <bool GENO>
+bool tc_fits_g(const ParseShape& sh) {
+    const int t = smem_table(sh);
+    switch (sh.P) {
+        case 1: return smem_fits<Cfg<1, GENO>>(sh, 1, t);
+        case 2: return smem_fits<Cfg<2, GENO>>(sh, 1, t);
+        case 3: return smem_fits<Cfg<3, GENO>>(sh, 1, t);
+        default: return smem_fits<Cfg<4, GENO>>(sh, 1, t);
+    }
 }
 
 template <bool GENO, int V>
 bool private_staging_of(const ParseShape& sh) {
-    const int t = smem_table(sh);
     switch (sh.P) {
-        case 1: return private_staging<1, GENO, V>(sh.n_bins, t);
-        case 2: return private_staging<2, GENO, V>(sh.n_bins, t);
-        case 3: return private_staging<3, GENO, V>(sh.n_bins, t);
-        default: return private_staging<4, GENO, V>(sh.n_bins, t);
+        case 1: return private_staging<1, GENO, V>(sh);
+        case 2: return private_staging<2, GENO, V>(sh);
+        case 3: return private_staging<3, GENO, V>(sh);
+        default: return private_staging<4, GENO, V>(sh);
     }
 }
+}  // namespace
+
+bool tc_fits(const ParseShape& sh) { return sh.genotypes ? tc_fits_g<true>(sh) : tc_fits_g<false>(sh); }
 
 bool tc_private_staging(const ParseShape& sh, int variant) {
     if (sh.genotypes) return (variant == 1 && sh.P <= 2) ? private_staging_of<true, 1>(sh) : private_staging_of<true, 0>(sh);

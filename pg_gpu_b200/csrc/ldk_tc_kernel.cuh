@@ -70,8 +70,9 @@ constexpr uint64_t kTimeoutNs = 5000000000ull;  // 5 s per wait
 // which the freed registers cover (Cfg asserts the sum).  The host launches only a kernel
 // compiled to Cfg::REG_LAUNCH registers.
 constexpr size_t kMinSmem = 116 * 1024;
-constexpr size_t kMaxSmem = 227 * 1024;
-constexpr size_t kStaticSmem = 1536;  // at most: the kernel's __shared__ variables (barriers, bin edges)
+constexpr size_t kMaxSmem = 227 * 1024;  // of a CTA, its __shared__ variables (Cfg::SHARED) included
+constexpr size_t kSpareSmem = 1536;      // kept free of flush rows and further ring stages
+constexpr int kMaxStages = 8;
 
 // Tile geometry.  Haplotype path: a row block of 64 SNPs x {sigma, v} = 128 MMA rows against
 // NJ partners x {sigma, v} (N = 2 NJ), one MMA per K step and population.  Genotype path: a row
@@ -157,6 +158,11 @@ struct Cfg {
     // The ring: as many stages as shared memory has left (STAGES at least), or STAGES where the
     // control warps have 24 registers, which do not hold a run-time length.
     static constexpr bool MORE_STAGES = !SPLIT || REG_CTRL >= 32;
+    static constexpr int MAX_STAGES = !MORE_STAGES ? STAGES
+                                      : kMaxSmem / STAGE_BYTES < kMaxStages ? (int)(kMaxSmem / STAGE_BYTES) : kMaxStages;
+    // bytes of the kernel's __shared__ variables: barriers of the ring, of the accumulators and of the
+    // claimed items, the item ring, two words, bin edges (the launch checks it against the build)
+    static constexpr size_t SHARED = 16 * MAX_STAGES + 16 * NBUF + 16 * kRing + 8 * kRing + 8 + 8 * (LDK_MAX_BINS + 1);
     // Staging row of the bin flush: a lane's sums, then {pairs, finite r^2, key, -}
     static constexpr int K = GENO ? 0 : SpinSplit<P>::value;
     static constexpr int NA = SSPL ? (K > NS + 1 - K ? K : NS + 1 - K) : NS + 1;  // sums per lane
@@ -418,7 +424,6 @@ struct TcArgs {
 };
 
 // Shared-memory state of the persistent pipeline (one CTA).
-constexpr int kMaxStages = 8;
 struct Pipe {
     uint32_t stages;  // shared address of the ring
     uint64_t* full_bar;
@@ -583,7 +588,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     Recip* rtab = reinterpret_cast<Recip*>(scnt + ((NCOPY * slots * nb * 2 + 7) & ~7));
     double* fstage = reinterpret_cast<double*>(rtab + (GENO || GT ? 0 : (a.max_n + 2) & ~1));  // [EPI][frows][FROW]
 
-    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tfull[C::NBUF], tempty[C::NBUF];
+    __shared__ __align__(8) uint64_t full_bar[C::MAX_STAGES], empty_bar[C::MAX_STAGES], tfull[C::NBUF], tempty[C::NBUF];
     __shared__ __align__(8) uint64_t ifull[kRing], iempty[kRing];
     __shared__ volatile int ring[2 * kRing];
     __shared__ uint32_t tmem_base_s;
@@ -1066,14 +1071,21 @@ bool make_map(CUtensorMap* m, const uint8_t* planes, int64_t n_var, int ktot, in
     return r == CUDA_SUCCESS;
 }
 
-// Dynamic shared memory: pipeline stages, `ncopy` staging copies, `table` reciprocal
-// table entries (32 B each) and `frows` flush rows per epilogue warp.
-template <int P, bool GENO, int V = 0>
-size_t smem_bytes_t(int nb, int table, int ncopy, int frows = 0) {
-    using C = Cfg<P, GENO, V>;
-    return 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)ncopy * C::SLOTS * nb * (C::NS + 1) * sizeof(double) +
-           (size_t)((ncopy * C::SLOTS * nb * 2 + 7) & ~7) * sizeof(unsigned) + (size_t)table * sizeof(double4) + 32 +
-           (size_t)frows * C::EPI * C::FROW * sizeof(double);
+// Shared memory of a CTA but for flush rows and further ring stages: `ncopy` staging copies of
+// `slots` bootstrap blocks, `table` reciprocal table entries of `entry` bytes.
+template <class C>
+size_t smem_bytes(int nb, int ncopy, int slots, int table, size_t entry) {
+    return 1024 + (size_t)C::STAGES * C::STAGE_BYTES + (size_t)ncopy * slots * nb * (C::NS + 1) * sizeof(double) +
+           (size_t)((ncopy * slots * nb * 2 + 7) & ~7) * sizeof(unsigned) + (size_t)table * entry + 32;
+}
+
+// Whether a shape fits with `ncopy` staging copies and `table` table entries in shared memory.
+// Decided for every bootstrap slot and entries of 32 bytes, whatever the call stages, and it has to
+// fit as it is launched: the slots in use, the kernel's entries, its __shared__ variables.
+template <class C>
+bool smem_fits(const ParseShape& sh, int ncopy, int table) {
+    return smem_bytes<C>(sh.n_bins, ncopy, C::SLOTS, table, sizeof(double4)) <= kMaxSmem &&
+           smem_bytes<C>(sh.n_bins, ncopy, sh.slots, table, sizeof(typename C::Recip)) + C::SHARED <= kMaxSmem;
 }
 
 // Ring stages in `room` bytes: C::STAGES, or as many as fit (two stages of 48 KB left the MMAs of
@@ -1081,7 +1093,7 @@ size_t smem_bytes_t(int nb, int table, int ncopy, int frows = 0) {
 template <class C>
 int ring_stages(size_t room) {
     const size_t n = room / C::STAGE_BYTES;
-    return C::MORE_STAGES && n > (size_t)C::STAGES ? (int)std::min<size_t>(n, kMaxStages) : C::STAGES;
+    return C::MORE_STAGES && n > (size_t)C::STAGES ? (int)std::min<size_t>(n, C::MAX_STAGES) : C::STAGES;
 }
 
 // Reciprocal table entries held in shared memory (none on the genotype path, none when the
@@ -1090,19 +1102,8 @@ inline int smem_table(const ParseShape& sh) { return (sh.genotypes || sh.rtab_gl
 
 // Per-warp staging copies when they fit next to the pipeline stages.
 template <int P, bool GENO, int V>
-bool private_staging(int nb, int table) {
-    return smem_bytes_t<P, GENO, V>(nb, table, Cfg<P, GENO, V>::EPI) <= kMaxSmem;
-}
-
-template <bool GENO>
-size_t tc_smem_bytes_g(const ParseShape& sh) {
-    const int t = smem_table(sh);
-    switch (sh.P) {
-        case 1: return smem_bytes_t<1, GENO>(sh.n_bins, t, 1);
-        case 2: return smem_bytes_t<2, GENO>(sh.n_bins, t, 1);
-        case 3: return smem_bytes_t<3, GENO>(sh.n_bins, t, 1);
-        default: return smem_bytes_t<4, GENO>(sh.n_bins, t, 1);
-    }
+bool private_staging(const ParseShape& sh) {
+    return smem_fits<Cfg<P, GENO, V>>(sh, Cfg<P, GENO, V>::EPI, smem_table(sh));
 }
 
 // Haplotype path: the reciprocal table goes to the workspace when it does not fit in shared
@@ -1112,10 +1113,10 @@ size_t tc_smem_bytes_g(const ParseShape& sh) {
 template <int P>
 bool rtab_global_t(const ParseShape& sh) {
     using C = Cfg<P, false, 0>;
-    const int nb = sh.n_bins, t = sh.max_n + 1;
-    if (smem_bytes_t<P, false, 0>(nb, t, C::EPI) <= kMaxSmem) return false;
-    if (smem_bytes_t<P, false, 0>(nb, 0, C::EPI) <= kMaxSmem) return true;
-    return smem_bytes_t<P, false, 0>(nb, t, 1) > kMaxSmem;
+    const int t = sh.max_n + 1;
+    if (smem_fits<C>(sh, C::EPI, t)) return false;
+    if (smem_fits<C>(sh, C::EPI, 0)) return true;
+    return !smem_fits<C>(sh, 1, t);
 }
 
 template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT>
@@ -1148,37 +1149,35 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     a.rtab_g = static_cast<const double4*>(w.rtab);
     a.gtab = static_cast<const double4*>(w.gtab);
     const int ncopy = PRIV ? C::EPI : 1;
-    // What decides the staging (per-warp copies, the reciprocal table's place) is sized with
-    // every slot and C::STAGES streamed stages; what this call leaves of shared memory goes to
-    // flush rows, then to the ring.
+    // What the staging (smem_fits) leaves of shared memory goes to flush rows, then to the ring.
     a.slots = sh.slots;
-    size_t other = 1024 + (size_t)ncopy * a.slots * d->n_bins * (C::NS + 1) * sizeof(double) +
-                   (size_t)((ncopy * a.slots * d->n_bins * 2 + 7) & ~7) * sizeof(unsigned) +
-                   (size_t)(smem_table(sh) ? (sh.max_n + 2) & ~1 : 0) * sizeof(typename C::Recip) + 32;
-    const size_t row = (size_t)C::EPI * C::FROW * sizeof(double), full = kMaxSmem - kStaticSmem;
+    size_t other = smem_bytes<C>(d->n_bins, ncopy, a.slots, smem_table(sh), sizeof(typename C::Recip)) -
+                   (size_t)C::STAGES * C::STAGE_BYTES;
+    const size_t row = (size_t)C::EPI * C::FROW * sizeof(double), full = kMaxSmem - kSpareSmem;
     a.frows = C::FROWS_MAX;
     while (a.frows > 0 && other + (size_t)C::STAGES * C::STAGE_BYTES + a.frows * row > full) a.frows >>= 1;
-    other += a.frows * row;
+    if (a.frows > 0) other += a.frows * row + sizeof(typename C::Recip);  // they start at an even table entry
     a.stages = ring_stages<C>(full > other ? full - other : 0);
     size_t smem = other + (size_t)a.stages * C::STAGE_BYTES;
     // at least half of an SM's shared memory, so that one CTA (holding all 512 TMEM
     // columns) runs per SM
     if (smem < kMinSmem) smem = kMinSmem;
-    if (smem > kMaxSmem) return cudaErrorInvalidConfiguration;
+    if (smem + C::SHARED > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
         cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    if constexpr (C::SPLIT) {
-        // the register split adds up only at C::REG_LAUNCH registers per thread; any other
-        // allocation would leave setmaxnreg.inc waiting, so such a build is not launched
-        static std::atomic<int> regs{-1};  // of this build's kernel: asked for once
-        if (regs.load() < 0) {
+    {
+        // the register split adds up only at C::REG_LAUNCH registers per thread (any other
+        // allocation would leave setmaxnreg.inc waiting) and what fits is decided with C::SHARED,
+        // so a build with others is not launched
+        static std::atomic<int> built{-1};  // of this build's kernel: asked for once
+        if (built.load() < 0) {
             cudaFuncAttributes fa;
             e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT>);
             if (e != cudaSuccess) return e;
-            regs.store(fa.numRegs);
+            built.store((!C::SPLIT || fa.numRegs == C::REG_LAUNCH) && fa.sharedSizeBytes <= C::SHARED);
         }
-        if (regs.load() != C::REG_LAUNCH) return cudaErrorInvalidKernelImage;
+        if (!built.load()) return cudaErrorInvalidKernelImage;
     }
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1197,7 +1196,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
 template <int PP, bool GENO, int V, bool CNT>
 cudaError_t launch_staged(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                           int max_items, cudaStream_t s) {
-    const bool priv = private_staging<PP, GENO, V>(sh.n_bins, smem_table(sh));
+    const bool priv = private_staging<PP, GENO, V>(sh);
     if (!GENO && sh.rtab_global) {
         if constexpr (!GENO && V == 0)
             return priv ? launch_parse_tc_p<PP, true, GENO, V, true, CNT>(d, o, w, sh, max_items, s)
