@@ -39,8 +39,8 @@ struct LdmArgs {
 //                           of squared deviations (ld_statistics.py:1000-1011)
 //   LDK_LDM_ROGERS_HUFF_R   {d, 1 / sqrt(V)}, d the mean dosage
 // with 0 for the reciprocal of 0; and the partner range (the rest of the set) and the matrix
-// diagonal.  With `strict` a missing call sets LDK_DEVERR_BAD_INPUT (the Rogers-Huff and
-// sigma_D^2 genotype estimators take complete data, ld_statistics.py:389-399).
+// diagonal.  For the Rogers-Huff and sigma_D^2 genotype estimators, which take complete data
+// (ld_statistics.py:389-399), a missing call sets LDK_DEVERR_BAD_INPUT, unless the set has no pair.
 // A block takes 128 SNPs (four a lane, one word per row), its sixteen warps every sixteenth
 // group of eight rows: 12,000 SNPs x 200 rows 24 us with a thread per SNP walking the rows, 13.
 constexpr int kSiteWarps = 16;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(32 * kSiteWarps)
         const double pq = r.x * (1.0 - r.x);
         r.y = pq > 0.0 ? 1.0 / pq : 0.0;
     } else if (estimator >= LDK_LDM_DIPLOID_R2) {
-        if (estimator != LDK_LDM_DIPLOID_R2 && c[0] < n_rows) atomicOr(status, LDK_DEVERR_BAD_INPUT);
+        if (estimator != LDK_LDM_DIPLOID_R2 && n_var > 1 && c[0] < n_rows) atomicOr(status, LDK_DEVERR_BAD_INPUT);
         // spins: 1 for dosage 0, 0 for 1, -1 for 2; V = (n sum s^2 - (sum s)^2) / n, exact numerator
         const double n = c[0], S = (double)(c[0] - c[1] - 2 * c[2]), SS = (double)(c[0] - c[1]);
         const double V = c[0] > 0 ? fma(n, SS, -(S * S)) / n : 0.0;
