@@ -1002,7 +1002,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                 const int rem = idx % (nb * (NS + 1));
                 const int bb = rem / (NS + 1), s = rem % (NS + 1);
                 const int blk = blk0 + sl;
-                if (val != 0.0 && blk < a.n_blocks)
+                if (val != 0.0 && (unsigned)blk < (unsigned)a.n_blocks)  // others: reported by pair_range
                     fx_add(a.fx + (((int64_t)blk * nb + bb) * (NS + 1) + spin_stat<P, GENO>(s)) * kFxLimbs,
                            CNT ? val : val * spin_weight<P, GENO>(s), a.status);
             }
@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     sc[2 * idx + 1] = 0u;
                 }
                 const int blk = blk0 + idx / nb, bb = idx % nb;
-                if (blk < a.n_blocks) {
+                if ((unsigned)blk < (unsigned)a.n_blocks) {
                     if (c0) atomicAdd(&a.pairs[(int64_t)blk * nb + bb], c0);
                     if (c1) atomicAdd(&a.r2_counts[(int64_t)blk * nb + bb], c1);
                 }
