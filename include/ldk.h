@@ -249,7 +249,8 @@ LDK_API int ldk_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const in
  * candidate.  A shape class is (population count, haplotype or genotype path, padded sample
  * bytes, bin count, decade of max_dist, log2 of the mean window size).  Later ldk_parse,
  * ldk_parse_setup (the order) and ldk_parse_enqueue (the width) calls of the class use the
- * kept choice, tuning enabled or not; classes never tuned use the defaults (the widest
+ * kept choice, tuning enabled or not; classes never tuned, and shapes of a class that the kept
+ * width does not fit (large populations' tables), use the defaults (the widest
  * haplotype tile, the narrower one for one population in windows with no more tiles than SMs;
  * 12 partners for one genotype population, 24 from 257 individuals and more tiles than SMs on,
  * 8 for two; largest windows first).  ldk_tile_width returns the width (SNPs per partner tile) a call

@@ -367,7 +367,7 @@ int tuned_variant(const ldk_parse_t* d, const ParseShape& sh) {
 constexpr int kWideGenoK = 384;
 int variant_of(const ldk_parse_t* d, const ParseShape& sh) {
     const int v = tuned_variant(d, sh);
-    if (v >= 0) return v;
+    if (v >= 0 && tc_variant_runs(sh, v)) return v;  // a shape class may hold shapes that its choice does not fit
     if (sh.P != 1 || sh.rtab_global) return 0;
     if (sh.genotypes && (sh.ktot < kWideGenoK || !tc_private_staging(sh, 1))) return 0;
     const int wide = sh.genotypes ? 1 : 0;  // the variant of the wider tile

@@ -97,6 +97,7 @@ cudaError_t probe_peaks(double* int8_ops_per_s, double* fp64_fma_per_s, unsigned
 bool tc_fits(const ParseShape& sh);  // the default tile's kernel, with one staging copy, into shared memory
 bool tc_rtab_global(const ParseShape& sh);  // where the reciprocal table must live
 bool tc_from_counts(const ParseShape& sh);  // the spin forms are not exact for its largest population
+bool tc_variant_runs(const ParseShape& sh, int variant);  // whether that tile variant launches for this shape
 bool tc_private_staging(const ParseShape& sh, int variant);  // one staging copy per epilogue warp
 
 cudaError_t launch_build_items(const Scratch& w, int n_windows, int rows, cudaStream_t s);

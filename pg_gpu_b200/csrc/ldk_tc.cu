@@ -314,6 +314,10 @@ bool private_staging_of(const ParseShape& sh) {
 
 bool tc_fits(const ParseShape& sh) { return sh.genotypes ? tc_fits_g<true>(sh) : tc_fits_g<false>(sh); }
 
+// The narrow haplotype tile reads no table in the workspace; the wide genotype tiles fit with any
+// number of bins (one staging copy of 64: 196 and 208 KB).
+bool tc_variant_runs(const ParseShape& sh, int variant) { return variant == 0 || sh.genotypes || !sh.rtab_global; }
+
 bool tc_private_staging(const ParseShape& sh, int variant) {
     if (sh.genotypes) return (variant == 1 && sh.P <= 2) ? private_staging_of<true, 1>(sh) : private_staging_of<true, 0>(sh);
     return variant == 1 ? private_staging_of<false, 1>(sh) : private_staging_of<false, 0>(sh);
