@@ -426,6 +426,8 @@ int enqueue_device(const ldk_parse_t* d, const ldk_parse_out_t* out, const Prepa
     } else {
         if ((rc = check_cuda(launch_prep_planes(&dd, P.w, P.sh, out, s), "pair ranges and spin planes"))) return rc;
         if (tune && n_variants(d, P.sh) * n_orders(d) > 1 && tuned_variant(d, P.sh) < 0) {
+            // what the preparation reports would be cleared with the candidates' counters
+            if ((rc = read_status(P.w.status, s))) return rc;
             if ((rc = autotune_tc(&dd, out, P, s))) return rc;
             // the candidate runs left their sums and a spent row-block counter behind
             if ((rc = clear(&dd, out, P, s))) return rc;
