@@ -145,16 +145,20 @@ def compute_multi_pop_statistics_batch(counts_per_pop, n_valid_per_pop=None, gen
     C = [_device_tensor(c, torch.int32).reshape(-1, width) for c in counts_per_pop]
     # the library reads haplotype counts as 16-byte rows
     C = [c if c.data_ptr() % 16 == 0 else c.clone() for c in C]
+    if not C:
+        raise RuntimeError("no populations")
     n = C[0].shape[0]
-    NV = [None] * P
+    NV = []
     if n_valid_per_pop is not None:
         NV = [None if v is None else _device_tensor(v, torch.int32).reshape(-1) for v in n_valid_per_pop]
+    if any(v is not None for v in NV) and any(v is None for v in NV[P:]):
+        raise IndexError("more n_valid entries than populations")
     if any(c.shape[0] != n for c in C) or any(v is not None and v.numel() != n for v in NV):
         raise RuntimeError("counts and n_valid of the populations differ in length")
     out = torch.empty((n, len(ld_names(P))), dtype=torch.float64, device="cuda")
     ptrs = ctypes.c_void_p * P
     _lib.check(lib.ldk_stats_pops(int(bool(genotypes)), P, ptrs(*[c.data_ptr() for c in C]),
-                                  ptrs(*[None if v is None else v.data_ptr() for v in NV]), n, _lib.ptr(out),
+                                  ptrs(*[None if v is None else v.data_ptr() for v in NV[:P]]), n, _lib.ptr(out),
                                   _lib.stream_handle()))
     return out
 
