@@ -553,7 +553,6 @@ int ldk_counts_hap_packed(const int8_t* X, int64_t ld_x, int64_t n_var, int64_t 
                           int32_t n_rows, const int32_t* idx_i, const int32_t* idx_j, int64_t n_pairs, int32_t* counts,
                           int32_t* n_valid, void* workspace, size_t workspace_bytes, void* stream) {
     if (n_pairs < 0 || n_rows < 0 || n_var < 0 || n_total_rows < 0 || ld_x < n_var) { set_error("bad sizes"); return LDK_ERR_ARG; }
-    if (n_rows > 32 * 65535) { set_error("more than 2,097,120 rows"); return LDK_ERR_UNSUPPORTED; }
     if (n_rows > 0 && n_var > 0 && (!X || !rows)) { set_error("null pointer"); return LDK_ERR_ARG; }
     if (n_pairs > 0 && (!idx_i || !idx_j || !counts)) { set_error("null pointer"); return LDK_ERR_ARG; }
     if (!workspace || workspace_bytes < counts_workspace(n_var, n_rows)) {

@@ -27,46 +27,48 @@ __global__ void __launch_bounds__(kPackThreads)
                 int* __restrict__ flag) {
     const int64_t v = 4 * ((int64_t)blockIdx.x * kPackThreads + threadIdx.x);
     if (v >= n_var) return;
-    const int w = blockIdx.y, left = n_var - v < 4 ? (int)(n_var - v) : 4;
-    uint32_t out[3][4] = {};
-    uint32_t missing = 0u;
-    bool outside = false;
+    const int left = n_var - v < 4 ? (int)(n_var - v) : 4;
+    for (int w = blockIdx.y; w < words; w += gridDim.y) {
+        uint32_t out[3][4] = {};
+        uint32_t missing = 0u;
+        bool outside = false;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        uint32_t x[8];
+        for (int g = 0; g < 4; ++g) {
+            uint32_t x[8];
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            const int k = 32 * w + 8 * g + b;
-            x[b] = 0xFEFEFEFEu;  // past the selection: in no plane, and not missing
-            if (k < n_rows) {
-                const int row = rows[k];
-                if (row >= 0 && row < n_total) x[b] = load_quad(X + row * ld + v, left);
-                else outside = true;
+            for (int b = 0; b < 8; ++b) {
+                const unsigned k = 32u * w + 8 * g + b;
+                x[b] = 0xFEFEFEFEu;  // past the selection: in no plane, and not missing
+                if (k < (unsigned)n_rows) {
+                    const int row = rows[k];
+                    if (row >= 0 && row < n_total) x[b] = load_quad(X + row * ld + v, left);
+                    else outside = true;
+                }
+            }
+            uint32_t one = 0u, zero = 0u, valid = 0u;  // byte j: eight rows of SNP v + j
+#pragma unroll
+            for (int b = 7; b >= 0; --b) {
+                one = (one << 1) | (__vcmpeq4(x[b], kOnes) & kOnes);
+                zero = (zero << 1) | (__vcmpeq4(x[b], 0u) & kOnes);
+                valid = (valid << 1) | (~(x[b] >> 7) & kOnes);
+                missing |= __vcmpeq4(x[b], 0xFFFFFFFFu);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                out[0][j] |= ((one >> (8 * j)) & 0xFFu) << (8 * g);
+                out[1][j] |= ((zero >> (8 * j)) & 0xFFu) << (8 * g);
+                out[2][j] |= ((valid >> (8 * j)) & 0xFFu) << (8 * g);
             }
         }
-        uint32_t one = 0u, zero = 0u, valid = 0u;  // byte j: eight rows of SNP v + j
 #pragma unroll
-        for (int b = 7; b >= 0; --b) {
-            one = (one << 1) | (__vcmpeq4(x[b], kOnes) & kOnes);
-            zero = (zero << 1) | (__vcmpeq4(x[b], 0u) & kOnes);
-            valid = (valid << 1) | (~(x[b] >> 7) & kOnes);
-            missing |= __vcmpeq4(x[b], 0xFFFFFFFFu);
-        }
+        for (int pl = 0; pl < 3; ++pl)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            out[0][j] |= ((one >> (8 * j)) & 0xFFu) << (8 * g);
-            out[1][j] |= ((zero >> (8 * j)) & 0xFFu) << (8 * g);
-            out[2][j] |= ((valid >> (8 * j)) & 0xFFu) << (8 * g);
-        }
+            for (int j = 0; j < 4; ++j)
+                if (j < left) planes[((int64_t)pl * words + w) * n_var + v + j] = out[pl][j];
+        if (left < 4) missing &= (1u << (8 * left)) - 1u;  // the bytes beyond the matrix
+        const int f = (missing ? 1 : 0) | (outside ? 2 : 0);
+        if (f) atomicOr(flag, f);
     }
-#pragma unroll
-    for (int pl = 0; pl < 3; ++pl)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j < left) planes[((int64_t)pl * words + w) * n_var + v + j] = out[pl][j];
-    if (left < 4) missing &= (1u << (8 * left)) - 1u;  // the bytes beyond the matrix
-    const int f = (missing ? 1 : 0) | (outside ? 2 : 0);
-    if (f) atomicOr(flag, f);
 }
 
 __global__ void __launch_bounds__(256)
@@ -91,7 +93,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-int pack_words(int n_rows) { return (n_rows + 31) / 32; }
+int pack_words(int n_rows) { return (int)(((int64_t)n_rows + 31) / 32); }
 
 }  // namespace
 
@@ -108,7 +110,7 @@ cudaError_t launch_counts_bits(const int8_t* X, int64_t ld, int64_t n_var, int64
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), s);
     if (e != cudaSuccess) return e;
     if (n_var > 0 && words > 0) {
-        const dim3 grid((unsigned)((n_var + 4 * kPackThreads - 1) / (4 * kPackThreads)), (unsigned)words);
+        const dim3 grid((unsigned)((n_var + 4 * kPackThreads - 1) / (4 * kPackThreads)), (unsigned)(words < 65535 ? words : 65535));
         k_pack_bits<<<grid, kPackThreads, 0, s>>>(X, ld, n_var, n_total, rows, n_rows, planes, words, flag);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
