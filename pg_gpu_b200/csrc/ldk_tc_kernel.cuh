@@ -418,6 +418,7 @@ struct TcArgs {
     int slots;              // bootstrap blocks staged per row block (1 without snp_block)
     int stages;             // ring stages
     int frows;              // staging rows per epilogue warp of the bin flush
+    int dense;              // DN: an item of fewer partners per bin flushes lane by lane
     const double4* rtab_g;  // haplotype path: reciprocal table in global memory, or null when
                             // each CTA builds it in shared memory
     const double4* gtab;    // genotype path: reciprocal table in global memory
@@ -569,7 +570,9 @@ LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a) {
 // most of the raw calls' extra FP64 operations: 6,000 haplotypes x 20,000 SNPs 3.33 ms with the spin
 // forms, 3.36 with this; 100,000 x 1,000 0.523, 0.527; 6,000 + 6,000 x 4,000 0.84, 0.86; genotypes,
 // whose raw calls are long polynomials, 20,000 x 2,000 0.43, 0.47, 6,000 + 60 + 60 x 2,000 0.45, 0.80.
-template <int P, bool PRIV, bool GENO, int V, bool GT = false, bool CNT = false>
+// DN: items whose bins hold few partners (dense_partners) have a tile loop of their own, whose flush
+// adds lane by lane.
+template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN>
 __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     k_parse_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a) {
     using C = Cfg<P, GENO, V>;
@@ -707,6 +710,8 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             // so the distance to them never decreases and each (row, bin) run is flushed
             // to shared memory once, when the lane's next partner falls past the bin's
             // upper edge (held in `nxt`).
+            auto run_tiles = [&](auto dense_c) {
+            constexpr bool DENSE = decltype(dense_c)::value;
             double acc[NA];
             // statistic s of this warp's accumulators and where it goes in the staging row
             const int na = SSPL ? (part == 0 ? K : NS + 1 - K) : NS + 1;
@@ -779,10 +784,10 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             };
             auto add = [&](bool want, bool last, const double* acc, unsigned np, unsigned nr2, int key) {
                 const unsigned mask = __ballot_sync(0xffffffffu, want);
-                if constexpr (P == 1) flush_one_pop<PRIV>(mask, key, acc, np, nr2, my_sacc, my_scnt, lane);
+                if constexpr (P == 1 && !DENSE) flush_one_pop<PRIV>(mask, key, acc, np, nr2, my_sacc, my_scnt, lane);
                 const int rank = __popc(mask & ((1u << lane) - 1u)), total = __popc(mask);
-                if constexpr (P > 1) {
-                if (a.frows == 0) {  // no room: one lane per (block, bin) at a time
+                if constexpr (P > 1 || DENSE) {
+                if (DENSE || (!DN && a.frows == 0)) {  // one lane per (block, bin) at a time
                     const unsigned grp = __match_any_sync(0xffffffffu, want ? key : -1);
                     const int turn = __popc(grp & ((1u << lane) - 1u));
                     const int turns = PRIV ? (int)__reduce_max_sync(0xffffffffu, want ? (unsigned)__popc(grp) : 0u) : 1;
@@ -810,6 +815,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     }
                     return;
                 }
+                if constexpr (!DENSE) {
                 int b0 = 0;
                 do {
                     const int rows = total - b0 < a.frows - used ? total - b0 : a.frows - used;
@@ -825,6 +831,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                     b0 += rows;
                     if (!C::PEND || used == a.frows || (last && b0 == total)) drain();
                 } while (b0 < total);
+                }
                 }
             };
             auto flush = [&](bool want, bool last) {
@@ -961,7 +968,7 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
                         }
                         np += counts;
                     };
-                    if (U > 1 && !CNT && !change) {
+                    if (U > 1 && !CNT && !DENSE && !change) {
                         // every pair stays in its lane's bin: evaluated together, without branches
 #pragma unroll
                         for (int u = 0; u < U; ++u) evaluate(u, valid[u] && in_bin);
@@ -988,6 +995,16 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             }
             flush(in_bin && np > 0, true);
             (void)ok;
+            };
+            bool dense = false;
+            if constexpr (DN) {  // bins between the row block and its last partner
+                const double far = fabs(a.coord[jend - 1] - a.coord[row1 - 1]);
+                int bins = __popc(__ballot_sync(0xffffffffu, lane < nb && far >= sedges[lane]));
+                if (nb > 32) bins += __popc(__ballot_sync(0xffffffffu, lane + 32 < nb && far >= sedges[lane + 32]));
+                dense = jend - row1 < (int64_t)a.dense * bins || a.frows == 0;
+                if (dense) run_tiles(std::true_type{});
+            }
+            if (!dense) run_tiles(std::false_type{});
             // staging -> global, once per work item
             epi_bar<EPI>();
             const int et = threadIdx.x - 32 * C::W0;
@@ -1119,7 +1136,23 @@ bool rtab_global_t(const ParseShape& sh) {
     return !smem_fits<C>(sh, 1, t);
 }
 
-template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT>
+// DN: partners per bin below which an item's flush adds lane by lane.  Adding key by key or through
+// scratch rows pays where many lanes leave a bin together; in bins of a few partners every lane of
+// every step leaves one, with another key.  Kernel ms of 12,000 SNPs, lane by lane / the other way:
+//   three populations (40 + 30 + 20 haplotypes, bootstrap blocks), 8 scratch rows, 16 bins: 1
+//   partner per bin 0.095 / 0.183, 2.5 0.249 / 0.247, 5 0.54 / 0.31; 4 rows, 18 bins: 1 0.105 /
+//   0.290, 2.5 0.27 / 0.43, 5 0.60 / 0.51; 2 rows, 20 bins: 1 0.11 / 0.39, 5 0.65 / 0.92, 10 0.93 /
+//   0.84; 1 row, 21 bins: 75 1.24 / 1.74;
+//   60 haplotypes, 64 bins: 1.6 0.073 / 0.124; 16 bins: 2.5 0.056 / 0.062, 6 0.097 / 0.064;
+//   600 genotypes (10,000 SNPs), 16 bins: 2.5 0.074 / 0.143, 25 0.134 / 0.109.
+template <int P, bool GENO, bool PRIV>
+int dense_partners(int frows) {
+    if (P == 1) return GENO ? 8 : 3;
+    if (!PRIV) return 0;  // shared sums: lanes of one key would wait for one another's atomics
+    return frows >= 8 ? 2 : frows == 4 ? 4 : frows == 2 ? 7 : 1 << 20;
+}
+
+template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN>
 cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
                                      const ParseShape& sh, int max_items, cudaStream_t s) {
     using C = Cfg<P, GENO, V>;
@@ -1156,6 +1189,11 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     const size_t row = (size_t)C::EPI * C::FROW * sizeof(double), full = kMaxSmem - kSpareSmem;
     a.frows = C::FROWS_MAX;
     while (a.frows > 0 && other + (size_t)C::STAGES * C::STAGE_BYTES + a.frows * row > full) a.frows >>= 1;
+    // two populations with one or two rows flush lane by lane (82 + 15 haplotypes x 12,000 SNPs, 64 bins of
+    // 3 partners 1.75 -> 0.38 ms, of 23 2.61 -> 1.25; with four rows of 62 bins 0.28 / 0.37 in bins of
+    // one partner, 1.00 / 0.85 of ten)
+    if (P == 2 && PRIV && a.frows <= 2) a.frows = 0;
+    a.dense = dense_partners<P, GENO, PRIV>(a.frows);
     if (a.frows > 0) other += a.frows * row + sizeof(typename C::Recip);  // they start at an even table entry
     a.stages = ring_stages<C>(full > other ? full - other : 0);
     size_t smem = other + (size_t)a.stages * C::STAGE_BYTES;
@@ -1164,7 +1202,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem + C::SHARED > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
-        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     {
         // the register split adds up only at C::REG_LAUNCH registers per thread (any other
@@ -1173,7 +1211,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
         static std::atomic<int> built{-1};  // of this build's kernel: asked for once
         if (built.load() < 0) {
             cudaFuncAttributes fa;
-            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT>);
+            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN>);
             if (e != cudaSuccess) return e;
             built.store((!C::SPLIT || fa.numRegs == C::REG_LAUNCH) && fa.sharedSizeBytes <= C::SHARED);
         }
@@ -1184,7 +1222,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (max_items == 0) return cudaSuccess;
     const int grid = max_items < sms ? max_items : sms;
-    k_parse_tc<P, PRIV, GENO, V, GT, CNT><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
+    k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
     return cudaGetLastError();
 }
 
@@ -1193,14 +1231,28 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
 // table in shared memory or (FP64 estimators, widest tile only) in the workspace.  Other
 // variants answer cudaErrorInvalidConfiguration for a workspace table, which the tile
 // autotuner reads as "does not fit this shape".
+// The kernel with or without DN.  The choice inside one tile loop makes that loop 1.4 to 2.7% slower;
+// two loops leave three haplotype populations (200 windows 31.8 -> 31.0 ms) and the wide genotype
+// tile (500 x 100,000 2.56 -> 2.51) faster, other kernels' main loop 2 to 3% slower: those of one
+// population have it from so many bins on that narrow ones are likely, two populations do not.
+// (Two in 16 bins of 2.5 partners take 0.115 ms, lane by lane 0.093.)
+template <int PP, bool PRIV, bool GENO, int V, bool GT, bool CNT>
+cudaError_t launch_parse_tc_d(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
+                              int max_items, cudaStream_t s) {
+    constexpr bool always = !CNT && ((!GENO && PP == 3) || (GENO && PP == 1 && V == 1));
+    if constexpr (!CNT && PP == 1 && !always)
+        if (sh.n_bins > (GENO ? 24 : 32)) return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, true>(d, o, w, sh, max_items, s);
+    return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, always>(d, o, w, sh, max_items, s);
+}
+
 template <int PP, bool GENO, int V, bool CNT>
 cudaError_t launch_staged(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                           int max_items, cudaStream_t s) {
     const bool priv = private_staging<PP, GENO, V>(sh);
     if (!GENO && sh.rtab_global) {
         if constexpr (!GENO && V == 0)
-            return priv ? launch_parse_tc_p<PP, true, GENO, V, true, CNT>(d, o, w, sh, max_items, s)
-                        : launch_parse_tc_p<PP, false, GENO, V, true, CNT>(d, o, w, sh, max_items, s);
+            return priv ? launch_parse_tc_d<PP, true, GENO, V, true, CNT>(d, o, w, sh, max_items, s)
+                        : launch_parse_tc_d<PP, false, GENO, V, true, CNT>(d, o, w, sh, max_items, s);
         else
             return cudaErrorInvalidConfiguration;
     }
@@ -1209,8 +1261,8 @@ cudaError_t launch_staged(const ldk_parse_t* d, const ldk_parse_out_t* o, const 
                       "counted haplotypes keep their table in the workspace");
         return cudaErrorInvalidConfiguration;
     } else {
-        return priv ? launch_parse_tc_p<PP, true, GENO, V, false, CNT>(d, o, w, sh, max_items, s)
-                    : launch_parse_tc_p<PP, false, GENO, V, false, CNT>(d, o, w, sh, max_items, s);
+        return priv ? launch_parse_tc_d<PP, true, GENO, V, false, CNT>(d, o, w, sh, max_items, s)
+                    : launch_parse_tc_d<PP, false, GENO, V, false, CNT>(d, o, w, sh, max_items, s);
     }
 }
 
