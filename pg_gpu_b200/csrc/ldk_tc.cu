@@ -405,10 +405,12 @@ namespace {
 // block, and no piece is so short that the flush of its staged sums (which ends every item)
 // outweighs its tiles.  Where there are fewer tiles than SMs a tile is a piece: 400 SNPs
 // (28 tiles of 64 partners) x 60 haplotypes 0.028 ms with pieces of four, 0.020 with one; x 2,000
-// haplotypes 0.050 and 0.028; from 2,000 SNPs on the same.  Pieces of one row block are consecutive
-// (the claim order of the row blocks stays), its last piece runs to INT32_MAX, and a row block
-// without partners gets no item.  One block of 1024 threads: the total, then a block-wide
-// scan of the pieces per row block, 1024 row blocks per round.
+// haplotypes 0.050 and 0.028; from 2,000 SNPs on the same.  Not, though, where at least half as
+// many row blocks as SMs would become more pieces than SMs: 5,500 SNPs of 75 partners (86 row
+// blocks of three tiles), two populations, 172 pieces 0.110 ms, 86 0.081 (8 bins 0.064, 0.048).
+// Pieces of one row block are consecutive (the claim order of the row blocks stays), its last
+// piece runs to INT32_MAX, and a row block without partners gets no item.  One block of 1024
+// threads: the total, then a block-wide scan of the pieces per row block, 1024 row blocks per round.
 constexpr int kSplitThreads = 1024;
 
 // Row block k: from the list, or (no list: one window) [k * rows, (k + 1) * rows) up to `end`.
@@ -429,6 +431,19 @@ __device__ __forceinline__ int rb_tiles(const RowBlocks& rb, const int32_t* __re
     return jend > r0 + 1 ? (jend - r0 + nj - 1) / nj : 0;
 }
 
+// Sum over the block's threads, in every thread.
+__device__ __forceinline__ long long block_sum(long long t, long long (&s_sum)[kSplitThreads / 32]) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = t;
+    __syncthreads();
+    long long total = 0;
+#pragma unroll 4
+    for (int x = 0; x < kSplitThreads / 32; ++x) total += s_sum[x];
+    return total;
+}
+
 __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks rb, int n_rb,
                                                                const int32_t* __restrict__ jmax, int nj,
                                                                int min_tiles, int4* __restrict__ items,
@@ -440,16 +455,15 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
     constexpr int NW = kSplitThreads / 32;
     long long t = 0;
     for (int k = tid; k < n_rb; k += kSplitThreads) t += rb_tiles(rb, jmax, k, nj);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) s_sum[wid] = t;
     if (tid == 0) s_base = 0;
-    __syncthreads();
-    long long total = 0;
-#pragma unroll 4
-    for (int x = 0; x < NW; ++x) total += s_sum[x];
+    const long long total = block_sum(t, s_sum);
     const long long cl = (total + kItemTarget - 1) / kItemTarget, spread = (total + kSpreadCtas - 1) / kSpreadCtas;
-    const int least = spread < min_tiles ? (spread > 0 ? (int)spread : 1) : min_tiles;
+    int least = spread < min_tiles ? (spread > 0 ? (int)spread : 1) : min_tiles;
+    if (least < min_tiles && n_rb >= kSpreadCtas / 2) {  // a second round of pieces costs more than whole row blocks
+        t = 0;
+        for (int k = tid; k < n_rb; k += kSplitThreads) t += (rb_tiles(rb, jmax, k, nj) + least - 1) / least;
+        if (block_sum(t, s_sum) > kSpreadCtas) least = min_tiles;
+    }
     const int c = cl > least ? (int)cl : least;
     for (int b0 = 0; b0 < n_rb; b0 += kSplitThreads) {
         const int k = b0 + tid;
