@@ -90,7 +90,7 @@ constexpr int tile_nj(int P, bool GENO, int V) {
                 : ((P == 1 ? 128 : P == 2 ? 48 : 32) >> V);
 }
 
-template <int P, bool GENO = false, int V = 0>
+template <int P, bool GENO = false, int V = 0, bool IL = false>
 struct Cfg {
     static constexpr int ROWS = GENO ? 128 : 64;                      // SNPs per row block
     static constexpr int PLANES = GENO ? 4 : 2;                        // stored planes per SNP
@@ -114,7 +114,9 @@ struct Cfg {
     // lane % 4 of four -- with no exchange between lanes (eighteen selects and six shuffles a
     // pair for three populations).  Otherwise rows are interleaved
     // (sigma, v per SNP; genotypes: one plane per region) and read with 32x32b.
-    static constexpr bool QROWS = !GENO && P <= 3;
+    // IL (two and three populations of many haplotypes, interleave_k): interleaved all the same,
+    // because QROWS loads a row block in eight boxes of 2 KB instead of one of 16.
+    static constexpr bool QROWS = !GENO && P <= 3 && !IL;
     // Warp layout.  Warp w may read only TMEM lane quarter w % 4, and each of the four
     // schedulers of an SM holds warps w, w + 4, ... with a quarter of the register file.
     //  * SPLIT (genotypes; haplotypes with two or more populations -- estimators that want
@@ -572,10 +574,10 @@ LDK_DEV void run_mma(const Pipe& S, uint32_t tmem, const TcArgs& a) {
 // whose raw calls are long polynomials, 20,000 x 2,000 0.43, 0.47, 6,000 + 60 + 60 x 2,000 0.45, 0.80.
 // DN: items whose bins hold few partners (dense_partners) have a tile loop of their own, whose flush
 // adds lane by lane.
-template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN>
+template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN, bool IL>
 __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
     k_parse_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TcArgs a) {
-    using C = Cfg<P, GENO, V>;
+    using C = Cfg<P, GENO, V, IL>;
     constexpr int NS = C::NS;
     constexpr int EPI = C::EPI;
     extern __shared__ unsigned char smem_raw[];
@@ -719,9 +721,9 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
 #pragma unroll
             for (int s = 0; s < NA; ++s) acc[s] = 0.0;
             unsigned np = 0, nr2 = 0;
-            double pacc[C::LATE ? NA : 1];  // LATE: sums of the bin this lane left last
-            unsigned pnp = 0, pnr2 = 0;
-            int pkey = 0;
+            [[maybe_unused]] double pacc[C::LATE ? NA : 1];  // LATE: sums of the bin this lane left last
+            [[maybe_unused]] unsigned pnp = 0, pnr2 = 0;
+            [[maybe_unused]] int pkey = 0;
             int cur = -1;
             bool in_bin = false;  // 0 <= cur < nb
             double nxt = sedges[0];
@@ -1105,6 +1107,15 @@ bool smem_fits(const ParseShape& sh, int ncopy, int table) {
            smem_bytes<C>(sh.n_bins, ncopy, sh.slots, table, sizeof(typename C::Recip)) + C::SHARED <= kMaxSmem;
 }
 
+// Two and three haplotype populations: bytes of K from which the row block's rows are interleaved
+// (Cfg::IL), and with them the table kept in the workspace.  The loads bound such parses, and the
+// small boxes take about twice as long: ms with QROWS / interleaved, 16 bins, two populations x
+// 6,000 SNPs: 1,000 + 1,000 haplotypes 0.375 / 0.375 (60 bins 0.47 / 0.52), 1,500 + 1,500 0.495 /
+// 0.421, 3,000 + 3,000 0.866 / 0.551, 5,000 + 5,000 1.376 / 0.765; three: 400 each 0.531 / 0.546, 600
+// each 0.616 / 0.593, 2,000 each x 5,000 SNPs 1.164 / 0.683.  Fewer haplotypes: QROWS, whose reads
+// need no exchange between lanes (100 + 100 x 8,000 SNPs 0.444 / 0.483).
+inline int interleave_k(int P) { return P == 2 ? 3072 : P == 3 ? 1920 : INT32_MAX; }
+
 // Ring stages in `room` bytes: C::STAGES, or as many as fit (two stages of 48 KB left the MMAs of
 // 2,000 haplotypes waiting 1,000 cycles a chunk for their loads; three: 20.7 -> 20.3 ms).
 template <class C>
@@ -1126,11 +1137,12 @@ bool private_staging(const ParseShape& sh) {
 // Haplotype path: the reciprocal table goes to the workspace when it does not fit in shared
 // memory beside the widest tile's pipeline -- with per-warp staging if that fits without
 // the table (per-warp staging matters more than a shared-memory table), else beside one
-// shared staging copy.
+// shared staging copy -- and with interleaved rows.
 template <int P>
 bool rtab_global_t(const ParseShape& sh) {
     using C = Cfg<P, false, 0>;
     const int t = sh.max_n + 1;
+    if (sh.ktot >= interleave_k(P)) return true;
     if (smem_fits<C>(sh, C::EPI, t)) return false;
     if (smem_fits<C>(sh, C::EPI, 0)) return true;
     return !smem_fits<C>(sh, 1, t);
@@ -1152,10 +1164,10 @@ int dense_partners(int frows) {
     return frows >= 8 ? 2 : frows == 4 ? 4 : frows == 2 ? 7 : 1 << 20;
 }
 
-template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN>
+template <int P, bool PRIV, bool GENO, int V, bool GT, bool CNT, bool DN, bool IL>
 cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w,
                                      const ParseShape& sh, int max_items, cudaStream_t s) {
-    using C = Cfg<P, GENO, V>;
+    using C = Cfg<P, GENO, V, IL>;
     // A: the row block (haplotypes: both planes of 64 SNPs, with QROWS of eight per box;
     // genotypes: one plane of 128 SNPs per box); B: every plane of NJ partners
     CUtensorMap mA, mB;
@@ -1202,7 +1214,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     if (smem < kMinSmem) smem = kMinSmem;
     if (smem + C::SHARED > kMaxSmem) return cudaErrorInvalidConfiguration;
     cudaError_t e =
-        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN, IL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     {
         // the register split adds up only at C::REG_LAUNCH registers per thread (any other
@@ -1211,7 +1223,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
         static std::atomic<int> built{-1};  // of this build's kernel: asked for once
         if (built.load() < 0) {
             cudaFuncAttributes fa;
-            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN>);
+            e = cudaFuncGetAttributes(&fa, k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN, IL>);
             if (e != cudaSuccess) return e;
             built.store((!C::SPLIT || fa.numRegs == C::REG_LAUNCH) && fa.sharedSizeBytes <= C::SHARED);
         }
@@ -1222,7 +1234,7 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (max_items == 0) return cudaSuccess;
     const int grid = max_items < sms ? max_items : sms;
-    k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
+    k_parse_tc<P, PRIV, GENO, V, GT, CNT, DN, IL><<<grid, C::THREADS, smem, s>>>(mA, mB, a);
     return cudaGetLastError();
 }
 
@@ -1241,8 +1253,14 @@ cudaError_t launch_parse_tc_d(const ldk_parse_t* d, const ldk_parse_out_t* o, co
                               int max_items, cudaStream_t s) {
     constexpr bool always = !CNT && ((!GENO && PP == 3) || (GENO && PP == 1 && V == 1));
     if constexpr (!CNT && PP == 1 && !always)
-        if (sh.n_bins > (GENO ? 24 : 32)) return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, true>(d, o, w, sh, max_items, s);
-    return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, always>(d, o, w, sh, max_items, s);
+        if (sh.n_bins > (GENO ? 24 : 32))
+            return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, true, false>(d, o, w, sh, max_items, s);
+    constexpr bool il = !GENO && GT && (PP == 2 || PP == 3);
+    if constexpr (il && CNT) return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, always, true>(d, o, w, sh, max_items, s);
+    if constexpr (il && !CNT)
+        if (sh.ktot >= interleave_k(PP))
+            return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, always, true>(d, o, w, sh, max_items, s);
+    if constexpr (!(il && CNT)) return launch_parse_tc_p<PP, PRIV, GENO, V, GT, CNT, always, false>(d, o, w, sh, max_items, s);
 }
 
 template <int PP, bool GENO, int V, bool CNT>
