@@ -405,9 +405,9 @@ namespace {
 // block, and no piece is so short that the flush of its staged sums (which ends every item)
 // outweighs its tiles.  Where there are fewer tiles than SMs a tile is a piece: 400 SNPs
 // (28 tiles of 64 partners) x 60 haplotypes 0.028 ms with pieces of four, 0.020 with one; x 2,000
-// haplotypes 0.050 and 0.028; from 2,000 SNPs on the same.  Not, though, where at least half as
-// many row blocks as SMs would become more pieces than SMs: 5,500 SNPs of 75 partners (86 row
-// blocks of three tiles), two populations, 172 pieces 0.110 ms, 86 0.081 (8 bins 0.064, 0.048).
+// haplotypes 0.050 and 0.028; from 2,000 SNPs on the same.  Not, though, where these pieces are
+// more than the SMs and pieces of four tiles are not: 5,500 SNPs of 75 partners (86 row blocks of
+// three tiles), two populations, 172 pieces 0.110 ms, 86 0.081 (8 bins 0.064, 0.048).
 // Pieces of one row block are consecutive (the claim order of the row blocks stays), its last
 // piece runs to INT32_MAX, and a row block without partners gets no item.  One block of 1024
 // threads: the total, then a block-wide scan of the pieces per row block, 1024 row blocks per round.
@@ -459,10 +459,15 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
     const long long total = block_sum(t, s_sum);
     const long long cl = (total + kItemTarget - 1) / kItemTarget, spread = (total + kSpreadCtas - 1) / kSpreadCtas;
     int least = spread < min_tiles ? (spread > 0 ? (int)spread : 1) : min_tiles;
-    if (least < min_tiles && n_rb >= kSpreadCtas / 2) {  // a second round of pieces costs more than whole row blocks
-        t = 0;
-        for (int k = tid; k < n_rb; k += kSplitThreads) t += (rb_tiles(rb, jmax, k, nj) + least - 1) / least;
-        if (block_sum(t, s_sum) > kSpreadCtas) least = min_tiles;
+    if (least < kMinItemTiles && min_tiles >= kMinItemTiles && n_rb >= kSpreadCtas / 2) {
+        // a second round of shorter pieces (more than a few) costs more than one round of kMinItemTiles
+        long long now = 0, whole = 0;
+        for (int k = tid; k < n_rb; k += kSplitThreads) {
+            const int nt = rb_tiles(rb, jmax, k, nj);
+            now += (nt + least - 1) / least;
+            whole += (nt + kMinItemTiles - 1) / kMinItemTiles;
+        }
+        if (block_sum(now, s_sum) > kSpreadCtas + kSpreadCtas / 16 && block_sum(whole, s_sum) <= kSpreadCtas) least = kMinItemTiles;
     }
     const int c = cl > least ? (int)cl : least;
     for (int b0 = 0; b0 < n_rb; b0 += kSplitThreads) {

@@ -999,11 +999,12 @@ __global__ void __launch_bounds__(Cfg<P, GENO, V>::THREADS, 1)
             (void)ok;
             };
             bool dense = false;
-            if constexpr (DN) {  // bins between the row block and its last partner
-                const double far = fabs(a.coord[jend - 1] - a.coord[row1 - 1]);
+            if constexpr (DN) {  // the first row's partners and the bins up to its last one
+                const int last = a.jmax[row0] - 1;
+                const double far = fabs(a.coord[last] - a.coord[row0]);
                 int bins = __popc(__ballot_sync(0xffffffffu, lane < nb && far >= sedges[lane]));
                 if (nb > 32) bins += __popc(__ballot_sync(0xffffffffu, lane + 32 < nb && far >= sedges[lane + 32]));
-                dense = jend - row1 < (int64_t)a.dense * bins || a.frows == 0;
+                dense = last - row0 < (int64_t)a.dense * bins || a.frows == 0;
                 if (dense) run_tiles(std::true_type{});
             }
             if (!dense) run_tiles(std::false_type{});
