@@ -183,8 +183,9 @@ LDK_API int ldk_parse_noalloc(const ldk_parse_t* d, const ldk_parse_out_t* out, 
  * counterpart in pg_gpu (its parse is a Python loop of CuPy calls).
  *
  * ldk_parse_setup writes the call's plan into the workspace -- window offsets and the
- * tensor-core method's row-block list, from host memory (a tensor-core parse of one window
- * needs neither and has no plan) -- and synchronises `stream`.
+ * tensor-core method's row-block list, from host memory (a parse of one window needs neither
+ * and has no plan: its bounds and anchor end go with the enqueued launches) -- and synchronises
+ * `stream`.
  * ldk_parse_enqueue then enqueues only device work on `stream` (clearing the status word and
  * the accumulators, pair ranges, spin planes, the parse kernel, the outputs): no host <-> device
  * copies, no synchronisation, no allocation, so it can be captured into a CUDA graph and
@@ -252,8 +253,8 @@ LDK_API int ldk_ld_matrix(const int8_t* X, int64_t ld_x, int64_t n_var, const in
  * kept choice, tuning enabled or not; classes never tuned, and shapes of a class that the kept
  * width does not fit (large populations' tables), use the defaults (the widest
  * haplotype tile, the narrower one for one population in windows with no more tiles than SMs;
- * 12 partners for one genotype population, 24 from 257 individuals and more tiles than SMs on,
- * 8 for two; largest windows first).  ldk_tile_width returns the width (SNPs per partner tile) a call
+ * 12 partners for one genotype population, 24 from 257 individuals and more tiles than SMs on
+ * where up to 24 bins leave every warp its staging copy, 8 for two; largest windows first).  ldk_tile_width returns the width (SNPs per partner tile) a call
  * with this descriptor would use now, 0 for the plain method, or a negative status.  No
  * counterpart in pg_gpu. */
 LDK_API int ldk_autotune(int enable);

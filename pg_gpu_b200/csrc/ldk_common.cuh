@@ -69,9 +69,6 @@ LDK_DEV uint32_t load_quad(const int8_t* p, int left) {
     return left >= 4 ? x : x | (0xFFFFFFFFu << (8 * left));
 }
 
-// FP64 add into shared memory.
-LDK_DEV void smem_add_f64(double* p, double v) { atomicAdd(p, v); }
-
 // ---------------------------------------------------------------------------
 // Order-independent bin sums.  Each FP64 partial sum is converted exactly (truncated below
 // 2^-96) into a fixed-point integer X = |v| * 2^96 < 2^160, split into kFxLimbs limbs of 32

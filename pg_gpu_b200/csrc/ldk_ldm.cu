@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(128 + 32 * kLdmEpi, 1)
 
 // ---- sigma_D^2 of genotype pairs: nine moments per pair ----------------------------------
 
-using LdmGCfg = Cfg<1, true, 0>;               // 128-SNP row blocks, 16-partner tiles
+using LdmGCfg = Cfg<1, true, 0>;               // 128-SNP row blocks, 12-partner tiles
 constexpr int kLdmGEpi = 8;                    // two epilogue warps per TMEM lane quarter
 constexpr int kLdmGPart = LdmGCfg::NJ / 2;     // partners per epilogue warp and tile
 constexpr int kLdmGStride = kLdmGPart + 1;

@@ -20,8 +20,6 @@ struct PrepArgs {
     int kofs[LDK_MAX_POPS + 1];
     int P;
     int ktot;
-    int genotypes;
-    int planes;
     uint8_t* planes_out;
     unsigned* status;
     int64_t nx;  // SNP tiles
@@ -354,8 +352,6 @@ cudaError_t launch_prep_planes(const ldk_parse_t* d, const Scratch& w, const Par
     }
     a.P = sh.P;
     a.ktot = sh.ktot;
-    a.genotypes = sh.genotypes;
-    a.planes = sh.planes;
     a.planes_out = w.hv;
     a.status = w.status;
     a.nx = (d->n_var + kPrepV - 1) / kPrepV;

@@ -1247,8 +1247,9 @@ cudaError_t launch_parse_tc_p(const ldk_parse_t* d, const ldk_parse_out_t* o, co
 // The kernel with or without DN.  The choice inside one tile loop makes that loop 1.4 to 2.7% slower;
 // two loops leave three haplotype populations (200 windows 31.8 -> 31.0 ms) and the wide genotype
 // tile (500 x 100,000 2.56 -> 2.51) faster, other kernels' main loop 2 to 3% slower: those of one
-// population have it from so many bins on that narrow ones are likely, two populations do not.
-// (Two in 16 bins of 2.5 partners take 0.115 ms, lane by lane 0.093.)
+// population have it from so many bins on that narrow ones are likely (38 haplotypes x 24,864 SNPs
+// in 64 bins of 26 partners 0.45 -> 0.48 ms), two populations do not (16 bins of 2.5 partners take
+// 0.115 ms, lane by lane 0.093).
 template <int PP, bool PRIV, bool GENO, int V, bool GT, bool CNT>
 cudaError_t launch_parse_tc_d(const ldk_parse_t* d, const ldk_parse_out_t* o, const Scratch& w, const ParseShape& sh,
                               int max_items, cudaStream_t s) {
