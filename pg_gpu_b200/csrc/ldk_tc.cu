@@ -427,11 +427,10 @@ __device__ __forceinline__ int rb_tiles(const RowBlocks& rb, const int32_t* __re
     return jend > r0 + 1 ? (jend - r0 + nj - 1) / nj : 0;
 }
 
-// Sum over the block's threads, in every thread.
+// Sum over the block's threads, in every thread; `s_sum` must not be in use.
 __device__ __forceinline__ long long block_sum(long long t, long long (&s_sum)[kSplitThreads / 32]) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    __syncthreads();
     if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = t;
     __syncthreads();
     long long total = 0;
@@ -444,7 +443,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
                                                                const int32_t* __restrict__ jmax, int nj,
                                                                int min_tiles, int4* __restrict__ items,
                                                                int* __restrict__ n_items) {
-    __shared__ long long s_sum[kSplitThreads / 32];
+    __shared__ long long s_sum[3][kSplitThreads / 32];
     __shared__ int s_scan[kSplitThreads / 32];
     __shared__ int s_base;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -452,7 +451,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
     long long t = 0;
     for (int k = tid; k < n_rb; k += kSplitThreads) t += rb_tiles(rb, jmax, k, nj);
     if (tid == 0) s_base = 0;
-    const long long total = block_sum(t, s_sum);
+    const long long total = block_sum(t, s_sum[0]);
     const long long cl = (total + kItemTarget - 1) / kItemTarget, spread = (total + kSpreadCtas - 1) / kSpreadCtas;
     int least = spread < min_tiles ? (spread > 0 ? (int)spread : 1) : min_tiles;
     if (least < kMinItemTiles && min_tiles >= kMinItemTiles && n_rb >= kSpreadCtas / 2) {
@@ -463,7 +462,7 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_items(const RowBlocks r
             now += (nt + least - 1) / least;
             whole += (nt + kMinItemTiles - 1) / kMinItemTiles;
         }
-        if (block_sum(now, s_sum) > kSpreadCtas + kSpreadCtas / 16 && block_sum(whole, s_sum) <= kSpreadCtas) least = kMinItemTiles;
+        if (block_sum(now, s_sum[1]) > kSpreadCtas + kSpreadCtas / 16 && block_sum(whole, s_sum[2]) <= kSpreadCtas) least = kMinItemTiles;
     }
     const int c = cl > least ? (int)cl : least;
     for (int b0 = 0; b0 < n_rb; b0 += kSplitThreads) {
