@@ -23,11 +23,11 @@
 // populations (the factored raw-call forms they replaced: 404 measured for three) and
 // 35 / 144 / 316 for genotypes (the nine-cell polynomials: 404 for one population's numerators
 // alone).  B200, 1965 MHz, a pass with the old forms -> with the spin forms -> with what the
-// comments below describe: 500 diploids x 100,000 SNPs 9.63 -> 3.79 -> 2.88 ms, two genotype
-// populations x 20,001 SNPs 5.28 -> 2.77 -> 0.98, three haplotype populations x 200 windows
-// 48.0 -> 39.5 -> 32.2 (FP64 pipe about 55%: estimators 12 of a warp's 17 thousand cycles a
-// tile), two x 50,000 SNPs 6.93 -> 5.74 -> 4.84.  With one population the loads weigh as much as
-// the estimators: 2,000 haplotypes x 10^6 SNPs 28.3 -> 21.3 ms, where a tile's 21.7 thousand
+// comments below describe: 500 diploids x 100,000 SNPs 9.63 -> 3.79 -> 2.57 ms, two genotype
+// populations x 20,001 SNPs 5.28 -> 2.77 -> 0.99, three haplotype populations x 200 windows
+// 48.0 -> 39.5 -> 31.4 (FP64 pipe about 56%: estimators 12 of a warp's 17 thousand cycles a
+// tile), two x 50,000 SNPs 6.93 -> 5.74 -> 4.86.  With one population the loads weigh as much as
+// the estimators: 2,000 haplotypes x 10^6 SNPs 28.3 -> 21.2 ms, where a tile's 21.7 thousand
 // cycles hold 10 of waiting for TMA traffic (about 10 TB/s from L2) and the epilogue takes 20.
 //
 // Warp roles (one CTA per SM, persistent over work items: runs of one row block's partner
